@@ -64,7 +64,7 @@ __device__ __forceinline__ bool metro_decide(float theta, float ci, float si, fl
     float sn, cn;
     __sincosf(tn, &sn, &cn);
     const float de = __fmaf_rn(__fsub_rn(ci, cn), hx, __fmul_rn(__fsub_rn(si, sn), hy));
-    const bool acc = (de <= 0.0f) || (u_acc < __expf(__fmul_rn(-beta, de)));
+    const bool acc = (de <= 0.0f) | (u_acc < __expf(__fmul_rn(-beta, de)));
     *theta_new = tn;
     *s_new = sn;
     *c_new = cn;
@@ -78,14 +78,29 @@ __device__ __forceinline__ float wolff_projection(float c, float s, float cphi, 
     return __fmaf_rn(s, sphi, __fmul_rn(c, cphi));
 }
 
+/* e^x = 2^(x log2 e) with the hardware's 2^y, results below 2^-126 flushed to
+ * zero (the instruction alone, without the range test and the two scalings
+ * that keep subnormal results). */
+__device__ __forceinline__ float exp_flush(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(x, 1.44269504088896341f)));
+    return r;
+}
+
 /* Bond activation of try_add_wolff_neighbor (src/updates.rs:537-548) with a
- * per-bond random: active iff J r_i r_j > 0 and u < 1 - exp(-2 beta J r_i r_j). */
+ * per-bond random: active iff J r_i r_j > 0 and u < p = 1 - exp(-2 beta J r_i r_j).
+ * Without branches (three of them per site cost 17 of 186 instructions), and
+ * with the comparison moved to integers times 2^-32 where it needs fewer
+ * steps: exp is at most 1 here, so p is a multiple of 2^-24 (1 - e rounds to
+ * the spacing of [1/2, 1)), 2^32 p = 2^32 - 2^32 e in one fused step is that
+ * same rounding scaled exactly, and word >> 8 < 2^24 p holds iff the word
+ * itself, rounded towards zero to 24 bits, is below 2^32 p.  A flushed exp
+ * gives p = 1, as a subnormal one does. */
 __device__ __forceinline__ bool wolff_bond_active(float coupling, float ri, float rj,
                                                   float minus_two_beta, uint32_t word) {
     const float prod = __fmul_rn(__fmul_rn(coupling, ri), rj);
-    if (!(prod > 0.0f)) return false;
-    const float p = __fsub_rn(1.0f, __expf(__fmul_rn(minus_two_beta, prod)));
-    return slsf_u24f(word) < p;
+    const float e = exp_flush(__fmul_rn(minus_two_beta, prod));
+    return (prod > 0.0f) & (__uint2float_rz(word) < __fmaf_rn(e, -4294967296.0f, 4294967296.0f));
 }
 
 /* Terms of one bond a -> b = a + mu of the observables

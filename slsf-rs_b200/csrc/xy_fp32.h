@@ -69,6 +69,13 @@ SLSF_HD float slsf_mul_rn(float a, float b) {
 
 /* One-step wrap into [0, 2 pi) with the FP32 round-up clamp. */
 SLSF_HD float slsf_wrap_once(float t) {
+#if defined(__CUDA_ARCH__)
+    /* the same without branches: t - 2 pi, t + 2 pi or t (adding -0 leaves
+     * every t as it is) */
+    const bool below = t < 0.0f;
+    const float r = __fadd_rn(t, below ? SLSF_TWO_PI_F : (t >= SLSF_TWO_PI_F ? -SLSF_TWO_PI_F : -0.0f));
+    return (below & (r >= SLSF_TWO_PI_F)) ? 0.0f : r;
+#else
     if (t >= SLSF_TWO_PI_F) {
         t = slsf_sub_rn(t, SLSF_TWO_PI_F);
     } else if (t < 0.0f) {
@@ -76,6 +83,7 @@ SLSF_HD float slsf_wrap_once(float t) {
         if (t >= SLSF_TWO_PI_F) t = 0.0f;
     }
     return t;
+#endif
 }
 
 /* Metropolis proposal theta + w (2u - 1); 2u - 1 is exact for a 24-bit u. */
@@ -87,6 +95,10 @@ SLSF_HD float slsf_propose(float theta, float width, float u) {
 /* Reflection about the axis phi: 2 phi + pi - theta, wrapped into [0, 2 pi). */
 SLSF_HD float slsf_reflect(float theta, float phi) {
     float t = slsf_sub_rn(slsf_fma_rn(2.0f, phi, SLSF_PI_F), theta);
+#if defined(__CUDA_ARCH__)
+    t = slsf_wrap_once(t);
+    return t >= SLSF_TWO_PI_F ? __fsub_rn(t, SLSF_TWO_PI_F) : t;
+#else
     if (t >= SLSF_TWO_PI_F) {
         t = slsf_sub_rn(t, SLSF_TWO_PI_F);
         if (t >= SLSF_TWO_PI_F) t = slsf_sub_rn(t, SLSF_TWO_PI_F);
@@ -95,6 +107,7 @@ SLSF_HD float slsf_reflect(float theta, float phi) {
         if (t >= SLSF_TWO_PI_F) t = 0.0f;
     }
     return t;
+#endif
 }
 
 /* 2 pi u for a 24-bit uniform; used for the Wolff axis and the initial angles. */
