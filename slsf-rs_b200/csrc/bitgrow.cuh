@@ -93,8 +93,9 @@ __device__ __forceinline__ uint32_t close_line(uint32_t c, uint32_t p, bool peri
 /* Closes the block C[z][y] (cluster words, pitch kGrowEdge + 1) through its
  * bonds BX (along x inside the word), BY[z][y] (row y to y + 1) and BZ[z][y]
  * (plane z to z + 1), with px / py / pz telling whether the block spans the
- * whole period along x (one-word rows), y and z.  Needs 1024 threads (32
- * warps); C must already be closed along x.  Passes alternate a full warp
+ * whole period along x (one-word rows), y and z.  Needs whole warps that
+ * divide 32 (a warp takes every nwarps-th plane, or row); C must already be
+ * closed along x.  Passes alternate a full warp
  * scan along y (lane = y, warp = z) or along z (lane = z, warp = y, the arrays
  * read transposed) with one step along the other axis and the closure along
  * x of the words that changed; a pass that changes nothing ends it.  Returns
@@ -104,12 +105,13 @@ __device__ __forceinline__ uint32_t close_block(uint32_t (*C)[kGrowEdge + 1], co
                                                 const uint32_t (*BZ)[kGrowEdge + 1], const uint32_t (*BX)[kGrowEdge + 1],
                                                 bool px, bool py, bool pz,
                                                 uint32_t max_pass = kGrowEdge * kGrowEdge * kGrowEdge + 1) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     constexpr uint32_t E = kGrowEdge;
     for (uint32_t pass = 0; pass < max_pass; ++pass) {
         int changed = 0;
         if ((pass & 1u) == 0) {
-            const uint32_t z = warp, y = lane;
+            for (uint32_t z = warp; z < E; z += nwarps) {
+            const uint32_t y = lane;
             const uint32_t old = C[z][y];
             const uint32_t by_ = BY[z][y];
             /* a warp scans only if some bit of it sits on a bond along the line */
@@ -124,8 +126,10 @@ __device__ __forceinline__ uint32_t close_block(uint32_t (*C)[kGrowEdge + 1], co
                 C[z][y] = v;
                 changed = 1;
             }
+            }
         } else {
-            const uint32_t z = lane, y = warp;
+            for (uint32_t y = warp; y < E; y += nwarps) {
+            const uint32_t z = lane;
             const uint32_t old = C[z][y];
             const uint32_t bz_ = BZ[z][y];
             const uint32_t bz_in = __shfl_sync(0xffffffffu, bz_, (lane + 31u) & 31u);
@@ -138,6 +142,7 @@ __device__ __forceinline__ uint32_t close_block(uint32_t (*C)[kGrowEdge + 1], co
             if (v != old) {
                 C[z][y] = v;
                 changed = 1;
+            }
             }
         }
         if (!__syncthreads_or(changed)) return pass + 1;

@@ -1154,17 +1154,17 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
     }
 }
 
-/* Without a tuned entry: the one-CTA kernel when the replica fits, with a CTA
- * of about one thread per 32 sites (128 .. 1024; measured on B200: L = 8 and
- * 16 run 1.4-2x faster on 128 threads than on 1024, L = 24 best on 512, L = 32
- * on 1024); else the smallest cluster that holds it, 1024 threads; else the
- * grid-wide kernels. */
+/* Without a tuned entry: the one-CTA kernel when the replica fits, with 64
+ * threads up to 1024 sites, 128 up to 8192, 256 up to 16384, else 512
+ * (measured on B200, 1e10 site-updates/s: L = 8 2.07 / 1.56 / 1.07 on 64 / 128
+ * / 256 threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 512, L = 20 5.13 / 4.72
+ * on 128 / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93 on 512, L = 32
+ * 6.67 on 512 and 5.8 on 1024); else the smallest cluster that holds it, 1024
+ * threads; else the grid-wide kernels. */
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
     if (slsf::resident_supports(lx, ly, lz, device)) {
         const uint64_t v = (uint64_t)lx * ly * lz;
-        uint32_t t = 128;
-        while (t < 1024 && 32ull * t < v) t <<= 1;
-        return {slsf::kKernelResident, 1, t};
+        return {slsf::kKernelResident, 1, v <= 1024 ? 64u : (v <= 8192 ? 128u : (v <= 16384 ? 256u : 512u))};
     }
     if (const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device)) return {slsf::kKernelCluster, c, 1024};
     return {slsf::kKernelGrid, 1, 256};
@@ -1640,7 +1640,7 @@ int slsf_autotune(slsf_ctx* ctx, uint32_t lx, uint32_t ly, uint32_t lz, uint32_t
     if (int rc = bind_device(ctx)) return rc;
     /* candidates */
     std::vector<slsf::KernelChoice> cand;
-    for (uint32_t t : {128u, 256u, 512u, 1024u}) {
+    for (uint32_t t : {64u, 128u, 256u, 512u, 1024u}) {
         const slsf::KernelChoice c = {slsf::kKernelResident, 1, t};
         if (choice_feasible(c, lx, ly, lz, ctx->device)) cand.push_back(c);
     }

@@ -31,6 +31,7 @@
  * Growth is monotone, so the pass count is bounded by V.
  */
 #include <algorithm>
+#include <type_traits>
 
 #include "bins.cuh"
 #include "bitgrow.cuh"
@@ -80,7 +81,7 @@ struct Geo {
     uint32_t stride1; /* offset of the colour-1 array */
     uint32_t xmask;
     bool lx_tiles_warp;
-    slsf_fastdiv div_hx, div_ly, div_lx;
+    slsf_fastdiv div_hx, div_ly, div_lx, div_nq;
 };
 
 __device__ __forceinline__ Geo make_geo(const TaskView& t) {
@@ -98,6 +99,7 @@ __device__ __forceinline__ Geo make_geo(const TaskView& t) {
     g.div_hx = slsf_fastdiv_make(t.lx >> 1);
     g.div_ly = slsf_fastdiv_make(t.ly);
     g.div_lx = slsf_fastdiv_make(t.lx);
+    g.div_nq = slsf_fastdiv_make(max(1u, t.lx >> 2));
     return g;
 }
 
@@ -168,7 +170,10 @@ struct Smem {
     float* jz;
     uint32_t* blk; /* 32^3 replicas: cluster and bond words as [z][y] blocks of pitch 33 (cube32), else NULL */
     double* corr;  /* fused correlation scratch (resident_corr_doubles) */
+    float jmax;    /* largest coupling of the replica (NaN and infinity become infinity) */
 };
+
+constexpr float kJMax = 1e30f;
 
 /* Words of the padded blocks of a 32^3 replica's Wolff growth (C, BY, BZ, BX). */
 constexpr uint32_t kBlockWords = 4 * kGrowEdge * (kGrowEdge + 1);
@@ -218,6 +223,19 @@ __device__ __forceinline__ void load_state(const TaskView& t, const Geo& g, Smem
         s.jxy[z] = t.jxy[z];
         s.jz[z] = t.jz[z];
     }
+}
+
+/* The same in every thread. */
+__device__ __forceinline__ float largest_coupling(const Geo& g, const Smem& s) {
+    float m = 0.0f;
+    bool fine = true;
+    for (uint32_t z = threadIdx.x & 31u; z < g.lz; z += 32) {
+        fine &= s.jxy[z] < kJMax && s.jz[z] < kJMax;
+        m = fmaxf(m, fmaxf(s.jxy[z], s.jz[z]));
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    return __all_sync(0xffffffffu, fine) ? m : __int_as_float(0x7f800000);
 }
 
 __device__ __forceinline__ void store_state(const TaskView& t, const Geo& g, const Smem& s) {
@@ -325,122 +343,214 @@ __device__ __forceinline__ uint32_t half_sweep(const TaskView& t, const Geo& g, 
     return accepted;
 }
 
-/* The same colour half-sweep for L_x = 32, walking along z.  A warp owns a
- * pair of rows (y0, y0 + 1) for a run of planes: lanes 0-15 hold row y0 and
- * lanes 16-31 row y0 + 1, lane k of a group updating the colour-c site of
- * compact index k (x = 2k + parity).  At every plane the lane keeps the trig
- * of the other colour's site of the same compact index on the planes below,
- * at and above (the z neighbours; a window that takes one sincos per plane);
- * the x neighbours are that value of lanes k and k -/+ 1, the y neighbour
- * inside the pair the other group's, and only the y neighbour outside the
- * pair is loaded: four sincos per update instead of eight, and no per-site
- * index division.  Operands, rounding order and randoms are those of
- * half_sweep, so decisions and new angles are bit-identical.  The lane pair
- * (2m, 2m + 1) shares one Philox block per plane: the even lane computes the
- * block of plane z and the odd lane that of plane z + 1, and each passes the
- * other the two words it needs. */
+/* The same colour half-sweep for L_x a multiple of 4, walking along z.  A
+ * thread owns a patch of two rows (y0, y0 + 1; y0 even) by two compact sites
+ * of each colour (k = 2 q, 2 q + 1, i.e. x = 4 q .. 4 q + 3) for a run of
+ * planes and updates its four colour-c sites of a plane together:
+ *   - it keeps the trig of the other colour's patch on the planes below, at
+ *     and above (the z neighbours), which is also one x neighbour, the inner
+ *     x neighbour of each pair and the inner y neighbours, so a plane takes 14
+ *     neighbour sincos for four updates instead of 24, and no shuffles;
+ *   - the two sites of a pair (h even, h + 1) share a Philox block, so a
+ *     thread uses its two blocks per plane whole, with one key schedule;
+ *   - the pair's arithmetic is packed (two FP32 operations per instruction);
+ *   - y0 is even, so the rows' parities depend on the plane alone and the
+ *     planes are unrolled by two instead of selecting by parity.
+ * The kernel is bound by instruction issue; the earlier form (one site per
+ * lane, x neighbours by shuffle, L_x = 32 only) took 186 instructions per
+ * update.  Operands, rounding order and randoms are those of half_sweep, so
+ * decisions and new angles are bit-identical. */
+struct Trig2 {
+    float2 c, s; /* cos and sin of two sites */
+};
+
+__device__ __forceinline__ Trig2 trig2(float2 th) {
+    Trig2 t;
+    __sincosf(th.x, &t.s.x, &t.c.x);
+    __sincosf(th.y, &t.s.y, &t.c.y);
+    return t;
+}
+
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+
+/* Two running sums of FP32 terms carried as a value and a remainder.  The
+ * value starts at a bias of at least twice what its terms can add up to, so
+ * it never falls below a term's magnitude and each addition's rounding error
+ * is exactly x - (t - v) (Dekker's fast two-sum); the errors add up in the
+ * remainder.  total() recovers the sum to about 2^-40 of its terms'
+ * magnitudes -- it agrees with FP64 sums of the same terms to 1e-12.  Four
+ * packed FP32 instructions per two terms; converting each term to FP64 takes
+ * eight cycles of the special-function pipe, which bound the measuring
+ * half-sweep (41k of 136k cycles per sweep at L = 32 against 18k for the
+ * other colour; 32k with these sums). */
+struct Sum2 {
+    float2 v, r;
+    __device__ __forceinline__ void start(float bias) {
+        v = make_float2(bias, bias);
+        r = make_float2(0.0f, 0.0f);
+    }
+    __device__ __forceinline__ void add(float2 x) {
+        const float2 minus = make_float2(-1.0f, -1.0f);
+        const float2 t = __fadd2_rn(v, x);
+        r = __fadd2_rn(r, __ffma2_rn(__ffma2_rn(v, minus, t), minus, x));
+        v = t;
+    }
+    __device__ __forceinline__ double total(float bias) const {
+        return ((double)__fsub_rn(v.x, bias) + (double)r.x) + ((double)__fsub_rn(v.y, bias) + (double)r.y);
+    }
+};
+
+/* Adds J cos and J sin of the forward bonds i -> p and the backward bonds
+ * m -> i of two sites i (bond_cos, bond_sin). */
+__device__ __forceinline__ void add_bonds2(Sum2& ac, Sum2& as, float jp, float jm, const Trig2& i, const Trig2& n,
+                                           const Trig2& p, const Trig2& m) {
+    ac.add(__fmul2_rn(dup2(jp), __ffma2_rn(i.c, p.c, __fmul2_rn(i.s, p.s))));
+    as.add(__fmul2_rn(dup2(jp), __ffma2_rn(i.s, p.c, __fmul2_rn(n.c, p.s))));
+    ac.add(__fmul2_rn(dup2(jm), __ffma2_rn(m.c, i.c, __fmul2_rn(m.s, i.s))));
+    as.add(__fmul2_rn(dup2(jm), __ffma2_rn(m.s, i.c, __fmul2_rn(m.c, n.s))));
+}
+
+/* field_from_pairs of two sites. */
+__device__ __forceinline__ float2 field2(float jxy, float jzp, float jzm, float2 a01, float2 a23, float2 a4, float2 a5) {
+    return __ffma2_rn(dup2(jzm), a5, __ffma2_rn(dup2(jzp), a4, __fmul2_rn(dup2(jxy), __fadd2_rn(a01, a23))));
+}
+
+/* metro_decide for the two sites of a Philox block; returns the number accepted. */
+__device__ __forceinline__ uint32_t metro_pair(float2& th, const Trig2& own, float2 hx, float2 hy, float beta,
+                                               float width, const slsf_u32x4& b) {
+    const float2 up = make_float2((float)(b.x >> 8), (float)(b.z >> 8));
+    /* 2 u - 1 with u = word >> 8 over 2^24 */
+    const float2 d = __ffma2_rn(up, dup2(1.0f / 8388608.0f), dup2(-1.0f));
+    const float2 t = __ffma2_rn(dup2(width), d, th);
+    const float2 tn = make_float2(slsf_wrap_once(t.x), slsf_wrap_once(t.y));
+    const Trig2 n = trig2(tn);
+    const float2 dc = __fadd2_rn(own.c, neg2(n.c)), ds = __fadd2_rn(own.s, neg2(n.s));
+    const float2 de = __ffma2_rn(dc, hx, __fmul2_rn(ds, hy));
+    const float2 arg = __fmul2_rn(dup2(-beta), de);
+    const bool a0 = (de.x <= 0.0f) | (slsf_u24f(b.y) < __expf(arg.x));
+    const bool a1 = (de.y <= 0.0f) | (slsf_u24f(b.w) < __expf(arg.y));
+    th.x = a0 ? tn.x : th.x;
+    th.y = a1 ? tn.y : th.y;
+    return (a0 ? 1u : 0u) + (a1 ? 1u : 0u);
+}
+
 template <bool kMeasure>
-__device__ __forceinline__ uint32_t half_sweep_walk32(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
-                                                      uint32_t colour, double (&acc)[8]) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const uint32_t grp = lane >> 4, k = lane & 15u, odd = k & 1u;
-    const uint32_t own = colour * g.stride1, other = (colour ^ 1u) * g.stride1;
-    const uint32_t pairs = g.ly >> 1;
-    /* planes per unit: every warp gets work when there are fewer pairs than warps */
-    const uint32_t nseg = max(1u, min(g.lz / 2, nwarps / max(1u, pairs)));
+__device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
+                                                     uint32_t colour, double (&acc)[8]) {
+    const uint32_t hx = g.lx >> 1, nq = g.lx >> 2, ncol = nq * (g.ly >> 1), plane = hx * g.ly;
+    /* planes per unit: every thread gets work when there are fewer patches than threads */
+    const uint32_t nseg = max(1u, min(g.lz >> 1, blockDim.x / ncol));
     const uint32_t seglen = (g.lz + nseg - 1) / nseg;
-    const uint32_t lk = grp * 16u + ((k + 15u) & 15u), rk = grp * 16u + ((k + 1u) & 15u);
+    float* own = s.th + colour * g.stride1;
+    const float* oth = s.th + (colour ^ 1u) * g.stride1;
     uint32_t accepted = 0;
-    for (uint32_t u = warp; u < pairs * nseg; u += nwarps) {
-        const uint32_t m = u / nseg, sgi = u - m * nseg;
-        const uint32_t z_lo = sgi * seglen, z_hi = min(g.lz, z_lo + seglen);
+    /* each of a thread's sums takes four terms per plane, at most 1 or J in magnitude */
+    const float bias = 8.0f * (float)(seglen * ((ncol * nseg + blockDim.x - 1) / blockDim.x));
+    Sum2 sum[kMeasure ? 8 : 1];
+    if (kMeasure)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum[k].start(k < 2 ? bias : s.jmax * bias);
+    for (uint32_t u = threadIdx.x; u < ncol * nseg; u += blockDim.x) {
+        const uint32_t sg = u / ncol, col = u - sg * ncol, m = col / nq, q = col - m * nq;
+        const uint32_t z_lo = sg * seglen, z_hi = min(g.lz, z_lo + seglen);
         if (z_lo >= z_hi) continue;
-        const uint32_t yr = 2u * m + grp;
-        const uint32_t yext = grp ? (yr + 1 == g.ly ? 0u : yr + 1) : (yr == 0 ? g.ly - 1 : yr - 1);
-        auto trig_other = [&](uint32_t y, uint32_t z) {
+        const uint32_t y0 = 2u * m;
+        /* compact offsets in a plane: the patch's rows, the rows below and above, the x neighbours left and right */
+        const uint32_t h0 = y0 * hx + 2u * q, h1 = h0 + hx;
+        const uint32_t hm = (y0 == 0 ? g.ly - 1 : y0 - 1) * hx + 2u * q;
+        const uint32_t hp = (y0 + 2 == g.ly ? 0u : y0 + 2) * hx + 2u * q;
+        const uint32_t xl = q == 0 ? h0 + hx - 1 : h0 - 1, xr = q + 1 == nq ? h0 + 2 - hx : h0 + 2;
+        auto two = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
+        auto trig1 = [&](uint32_t at) {
             float sn, cn;
-            __sincosf(s.th[other + (y + g.ly * z) * 16u + k], &sn, &cn);
+            __sincosf(oth[at], &sn, &cn);
             return make_float2(cn, sn);
         };
-        float2 om = trig_other(yr, z_lo == 0 ? g.lz - 1 : z_lo - 1);
-        float2 o0 = trig_other(yr, z_lo);
-        slsf_u32x4 blk = {0, 0, 0, 0};
-        uint32_t w0 = 0, w1 = 0;
-        for (uint32_t z = z_lo; z < z_hi; ++z) {
-            const uint32_t zi = z - z_lo;
-            if ((zi & 1u) == 0) {
-                /* the pair's blocks for planes z and z + 1 */
-                const uint32_t unit = ((yr + g.ly * (z + odd)) * 16u + k) >> 1;
-                blk = slsf_stream(t.seed, sweep, SLSF_PURPOSE_METRO, colour, unit);
-                w0 = __shfl_xor_sync(0xffffffffu, odd ? blk.x : blk.z, 1);
-                w1 = __shfl_xor_sync(0xffffffffu, odd ? blk.y : blk.w, 1);
-            }
-            /* plane z: the even lane's own block (x, y), the odd lane the even
-             * lane's (z, w); plane z + 1: the even lane the odd lane's (x, y),
-             * the odd lane its own (z, w) */
-            const bool first = (zi & 1u) == 0;
-            const uint32_t wp = first ? (odd ? w0 : blk.x) : (odd ? blk.z : w0);
-            const uint32_t wa = first ? (odd ? w1 : blk.y) : (odd ? blk.w : w1);
-            const float u_prop = slsf_u24f(wp), u_acc = slsf_u24f(wa);
-            const float2 op = trig_other(yr, z + 1 == g.lz ? 0u : z + 1);
-            const float2 oy = trig_other(yext, z);
-            /* neighbours: x from this group's window, y inside the pair from the other group */
-            const float lc = __shfl_sync(0xffffffffu, o0.x, lk), ls = __shfl_sync(0xffffffffu, o0.y, lk);
-            const float rc = __shfl_sync(0xffffffffu, o0.x, rk), rs = __shfl_sync(0xffffffffu, o0.y, rk);
-            const float pc = __shfl_xor_sync(0xffffffffu, o0.x, 16), ps = __shfl_xor_sync(0xffffffffu, o0.y, 16);
-            const uint32_t parity = (colour + yr + z) & 1u;
-            /* parity 0: +x is this lane's other-colour site, -x lane k - 1's; parity 1: -x own, +x lane k + 1's */
-            const float cxp = parity ? rc : o0.x, sxp = parity ? rs : o0.y;
-            const float cxm = parity ? o0.x : lc, sxm = parity ? o0.y : ls;
-            const float cyp = grp ? oy.x : pc, syp = grp ? oy.y : ps;
-            const float cym = grp ? pc : oy.x, sym = grp ? ps : oy.y;
-            const uint32_t q = (yr + g.ly * z) * 16u + k;
-            const float jx = s.jxy[z], jzp = s.jz[z], jzm = s.jz[z == 0 ? g.lz - 1 : z - 1];
-            const float th = s.th[own + q];
-            float si, ci;
-            __sincosf(th, &si, &ci);
-            if (kMeasure) {
-                acc[0] += (double)ci + (double)cxp;
-                acc[1] += (double)si + (double)sxp;
-                acc[2] += (double)bond_cos(jx, ci, si, cxp, sxp) + (double)bond_cos(jx, cxm, sxm, ci, si);
-                acc[5] += (double)bond_sin(jx, ci, si, cxp, sxp) + (double)bond_sin(jx, cxm, sxm, ci, si);
-                acc[3] += (double)bond_cos(jx, ci, si, cyp, syp) + (double)bond_cos(jx, cym, sym, ci, si);
-                acc[6] += (double)bond_sin(jx, ci, si, cyp, syp) + (double)bond_sin(jx, cym, sym, ci, si);
-                acc[4] += (double)bond_cos(jzp, ci, si, op.x, op.y) + (double)bond_cos(jzm, om.x, om.y, ci, si);
-                acc[7] += (double)bond_sin(jzp, ci, si, op.x, op.y) + (double)bond_sin(jzm, om.x, om.y, ci, si);
-            }
-            const float hx01 = __fadd_rn(cxp, cxm), hy01 = __fadd_rn(sxp, sxm);
-            const float hx23 = __fadd_rn(cyp, cym), hy23 = __fadd_rn(syp, sym);
-            const float hx = field_from_pairs(jx, jzp, jzm, hx01, hx23, op.x, om.x);
-            const float hy = field_from_pairs(jx, jzp, jzm, hy01, hy23, op.y, om.y);
-            float tn, sn, cn;
-            if (metro_decide(th, ci, si, hx, hy, t.beta, t.width, u_prop, u_acc, &tn, &sn, &cn)) {
-                s.th[own + q] = tn;
-                ++accepted;
-            }
-            om = o0;
-            o0 = op;
+        uint32_t base = z_lo * plane;
+        const uint32_t below = (z_lo == 0 ? g.lz - 1 : z_lo - 1) * plane;
+        Trig2 m0 = trig2(two(oth + below + h0)), m1 = trig2(two(oth + below + h1)); /* plane below */
+        Trig2 c0 = trig2(two(oth + base + h0)), c1 = trig2(two(oth + base + h1));   /* this plane */
+        float jzm = s.jz[z_lo == 0 ? g.lz - 1 : z_lo - 1];
+        /* one plane; kOdd: the parity (colour + y0 + z) & 1 of row y0, whose colour-c sites sit at x = 2 k + parity */
+        auto step = [&](uint32_t z, auto odd) {
+            constexpr bool kOdd = decltype(odd)::value;
+            const uint32_t above = z + 1 == g.lz ? 0u : base + plane;
+            const Trig2 p0 = trig2(two(oth + above + h0)), p1 = trig2(two(oth + above + h1));
+            const float jx = s.jxy[z], jzp = s.jz[z];
+            const Trig2 ym = trig2(two(oth + base + hm)), yp = trig2(two(oth + base + hp));
+            const float2 e0 = trig1(base + (kOdd ? xr : xl)), e1 = trig1(base + hx + (kOdd ? xl : xr));
+            const uint32_t unit = (base + h0) >> 1;
+            const slsf_u32x4 b0 = slsf_stream(t.seed, sweep, SLSF_PURPOSE_METRO, colour, unit);
+            const slsf_u32x4 b1 = slsf_stream(t.seed, sweep, SLSF_PURPOSE_METRO, colour, unit + (hx >> 1));
+            auto row = [&](uint32_t h, const Trig2& c, float2 e, auto row_odd, const Trig2& dn, const Trig2& up,
+                           const Trig2& zm, const Trig2& zp, const slsf_u32x4& b) {
+                constexpr bool kRowOdd = decltype(row_odd)::value;
+                /* parity 0: +x is the other colour's same compact site, -x the previous; parity 1: -x the same, +x the next */
+                Trig2 xp, xm;
+                if (kRowOdd) {
+                    xp.c = make_float2(c.c.y, e.x);
+                    xp.s = make_float2(c.s.y, e.y);
+                    xm = c;
+                } else {
+                    xp = c;
+                    xm.c = make_float2(e.x, c.c.x);
+                    xm.s = make_float2(e.y, c.s.x);
+                }
+                float2 th = two(own + base + h);
+                const Trig2 i = trig2(th);
+                if (kMeasure) {
+                    /* the site and the other colour's site of the same index: each site once */
+                    sum[0].add(i.c);
+                    sum[1].add(i.s);
+                    sum[0].add(c.c);
+                    sum[1].add(c.s);
+                    Trig2 n; /* (-cos, -sin) of the site */
+                    n.c = neg2(i.c);
+                    n.s = neg2(i.s);
+                    add_bonds2(sum[2], sum[5], jx, jx, i, n, xp, xm);
+                    add_bonds2(sum[3], sum[6], jx, jx, i, n, up, dn);
+                    add_bonds2(sum[4], sum[7], jzp, jzm, i, n, zp, zm);
+                }
+                const float2 fx = field2(jx, jzp, jzm, __fadd2_rn(xp.c, xm.c), __fadd2_rn(up.c, dn.c), zp.c, zm.c);
+                const float2 fy = field2(jx, jzp, jzm, __fadd2_rn(xp.s, xm.s), __fadd2_rn(up.s, dn.s), zp.s, zm.s);
+                accepted += metro_pair(th, i, fx, fy, t.beta, t.width, b);
+                *reinterpret_cast<float2*>(own + base + h) = th;
+            };
+            row(h0, c0, e0, std::integral_constant<bool, kOdd>(), ym, c1, m0, p0, b0);
+            row(h1, c1, e1, std::integral_constant<bool, !kOdd>(), c0, yp, m1, p1, b1);
+            m0 = c0;
+            m1 = c1;
+            c0 = p0;
+            c1 = p1;
+            jzm = jzp;
+            base += plane;
+        };
+        uint32_t z = z_lo;
+        if ((colour + z) & 1u) step(z++, std::true_type());
+        for (; z + 1 < z_hi; z += 2) {
+            step(z, std::false_type());
+            step(z + 1, std::true_type());
         }
+        if (z < z_hi) step(z, std::false_type());
     }
+    if (kMeasure)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += sum[k].total(k < 2 ? bias : s.jmax * bias);
     return accepted;
 }
 
-/* One colour half-sweep: the z walk for L_x = 32, the general form otherwise. */
+/* One colour half-sweep: the patch walk for L_x a multiple of 4, the site-by-site form for L_x = 2 mod 4, whose
+ * pairs of compact sites straddle rows (and for couplings whose biased sums could overflow). */
 template <bool kMeasure>
 __device__ __forceinline__ uint32_t sweep_colour(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
                                                  uint32_t colour, double (&acc)[8]) {
-    if (g.lx == 32) return half_sweep_walk32<kMeasure>(t, g, s, sweep, colour, acc);
+    if (g.lx % 4 == 0 && (!kMeasure || s.jmax < kJMax)) return half_sweep_quads<kMeasure>(t, g, s, sweep, colour, acc);
     return half_sweep<kMeasure>(t, g, s, sweep, colour, acc);
 }
 
 __device__ __forceinline__ float site_theta(const Geo& g, const Smem& s, uint32_t idx, const Coords& c) {
     return s.th[slot(g, idx, (c.x + c.y + c.z) & 1u)];
-}
-
-__device__ __forceinline__ float proj_of(float theta, float cphi, float sphi) {
-    float sn, cn;
-    __sincosf(theta, &sn, &cn);
-    return wolff_projection(cn, sn, cphi, sphi);
 }
 
 /* One growth pass: every row takes the cluster bits that reach it through
@@ -469,6 +579,82 @@ __device__ __forceinline__ int grow_pass(const Geo& g, Smem& s) {
     return changed;
 }
 
+/* Bond activation: the +x, +y, +z bond words of every row.  A warp holds
+ * G = 32 / L_x rows side by side (lane = x + L_x sub; the lanes past them keep
+ * no bits), sub-group sub in the planes z = 2 (G zb + sub) and z + 1, and
+ * walks columns of rows along y -- (zb, y segment) units, round robin.  The
+ * +y row's projections are the next row's own and plane z's +z partner is
+ * plane z + 1's site, so a step takes three sincos for its two sites; the two
+ * sites' arithmetic is packed (two FP32 operations per instruction) and their
+ * two Philox blocks share one key schedule.  Sub-groups past the last plane
+ * compute on the last planes and keep nothing.  Bound by instruction issue:
+ * one Philox block and three bond tests per site. */
+__device__ __forceinline__ void wolff_bonds(const TaskView& t, const Geo& g, const Smem& s, uint64_t counter,
+                                            float cphi, float sphi) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const uint32_t groups = 32u / g.lx, sub = min(lane / g.lx, groups - 1), x = lane - sub * g.lx;
+    const bool keep = x < g.lx;
+    const uint32_t xl = keep ? x : 0u, hx = g.lx >> 1, ph = g.plane >> 1;
+    const uint32_t nzb = ((g.lz >> 1) + groups - 1) / groups;
+    /* runs of at most 32 rows: lane j keeps the ballots of the run's row j until its end */
+    const uint32_t nseg = max(min(g.ly, (nwarps + nzb - 1) / nzb), (g.ly + 31u) >> 5);
+    const uint32_t seg = (g.ly + nseg - 1) / nseg;
+    const uint32_t xsrc = sub * g.lx + (xl + 1 == g.lx ? 0u : xl + 1);
+    const float2 cphi2 = make_float2(cphi, cphi), sphi2 = make_float2(sphi, sphi);
+    const float m2b = __fmul_rn(-2.0f, t.beta);
+    const float2 m2b2 = make_float2(m2b, m2b);
+    auto proj2 = [&](float ta, float tb) {
+        float2 sn, cn;
+        __sincosf(ta, &sn.x, &cn.x);
+        __sincosf(tb, &sn.y, &cn.y);
+        return __ffma2_rn(sn, sphi2, __fmul2_rn(cn, cphi2));
+    };
+    for (uint32_t u = warp; u < nzb * nseg; u += nwarps) {
+        const uint32_t zb = u / nseg, y_lo = (u - zb * nseg) * seg, y_hi = min(g.ly, y_lo + seg);
+        if (y_lo >= y_hi) continue;
+        const uint32_t z = min(2 * (zb * groups + sub), g.lz - 2), z2 = z + 2 == g.lz ? 0u : z + 2;
+        const float2 jx = make_float2(s.jxy[z], s.jxy[z + 1]), jzz = make_float2(s.jz[z], s.jz[z + 1]);
+        /* z is even: the site (x, y) has colour (x + y) & 1 on planes z and z + 2, the other on z + 1 */
+        uint32_t col = ((xl + y_lo) & 1u) ? g.stride1 : 0u;
+        uint32_t o = y_lo * hx + (xl >> 1);
+        const float *p0 = s.th + z * ph, *p1 = p0 + ph, *p2 = s.th + z2 * ph;
+        float2 r = proj2(p0[col + o], p1[g.stride1 - col + o]);
+        uint32_t idx = z * g.plane + y_lo * g.lx + xl;
+        uint32_t k[6] = {0, 0, 0, 0, 0, 0};
+        for (uint32_t y = y_lo; y < y_hi; ++y) {
+            const uint32_t on = y + 1 == g.ly ? (xl >> 1) : o + hx, coln = g.stride1 - col;
+            const float2 ry = proj2(p0[coln + on], p1[col + on]);
+            float sn, cn;
+            __sincosf(p2[col + o], &sn, &cn);
+            const float2 rz = make_float2(r.y, wolff_projection(cn, sn, cphi, sphi));
+            const float2 rx = make_float2(__shfl_sync(0xffffffffu, r.x, xsrc), __shfl_sync(0xffffffffu, r.y, xsrc));
+            const slsf_u32x4 b0 = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, idx);
+            const slsf_u32x4 b1 = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, idx + g.plane);
+            const float2 jr = __fmul2_rn(jx, r);
+            uint32_t w[6];
+            wolff_bond_words(__fmul2_rn(jr, rx), m2b2, b0.x, b1.x, w[0], w[3]);
+            wolff_bond_words(__fmul2_rn(jr, ry), m2b2, b0.y, b1.y, w[1], w[4]);
+            wolff_bond_words(__fmul2_rn(__fmul2_rn(jzz, r), rz), m2b2, b0.z, b1.z, w[2], w[5]);
+#pragma unroll
+            for (int j = 0; j < 6; ++j) k[j] = lane == y - y_lo ? w[j] : k[j];
+            r = ry;
+            col = coln;
+            o = on;
+            idx += g.lx;
+        }
+        if (lane < y_hi - y_lo)
+            for (uint32_t q = 0; q < groups && zb * groups + q < (g.lz >> 1); ++q) {
+                const uint32_t row = y_lo + lane + g.ly * 2 * (zb * groups + q), sh = q * g.lx;
+                s.bx[row] = (k[0] >> sh) & g.xmask;
+                s.by[row] = (k[1] >> sh) & g.xmask;
+                s.bz[row] = (k[2] >> sh) & g.xmask;
+                s.bx[row + g.ly] = (k[3] >> sh) & g.xmask;
+                s.by[row + g.ly] = (k[4] >> sh) & g.xmask;
+                s.bz[row + g.ly] = (k[5] >> sh) & g.xmask;
+            }
+    }
+}
+
 /* One Wolff update (src/updates.rs:551-620); adds the cluster size to *count. */
 __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Smem& s, uint64_t counter,
                                              uint32_t* s_count) {
@@ -478,196 +664,7 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
     const uint32_t x0 = slsf_range(pick.y, g.lx), y0 = slsf_range(pick.z, g.ly), z0 = slsf_range(pick.w, g.lz);
     float sphi, cphi;
     __sincosf(phi, &sphi, &cphi);
-    const float m2b = __fmul_rn(-2.0f, t.beta);
-
-    if (!g.lx_tiles_warp && g.lx < 24) { /* the general path below ORs into the rows */
-        for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) {
-            s.bx[r] = 0;
-            s.by[r] = 0;
-            s.bz[r] = 0;
-        }
-        __syncthreads();
-    }
-    if (g.lx == 32) {
-        /* A row is a warp (lane = x).  Each warp walks columns of rows along
-         * y -- (z, y segment) units, round robin -- so the projection of the
-         * +y row is the next row's own: two sincos per site instead of three,
-         * and no per-site index division. */
-        const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-        const uint32_t nseg = (nwarps + g.lz - 1) / g.lz;
-        const uint32_t seg = (g.ly + nseg - 1) / nseg;
-        for (uint32_t u = warp; u < g.lz * nseg; u += nwarps) {
-            const uint32_t z = u / nseg, y_lo = (u % nseg) * seg, y_hi = min(g.ly, y_lo + seg);
-            if (y_lo >= y_hi) continue;
-            const uint32_t zp_off = (z + 1 == g.lz) ? 0u : (z + 1) * g.plane; /* base of the +z plane */
-            const float jx = s.jxy[z], jzz = s.jz[z];
-            const uint32_t zbase = z * g.plane;
-            float ri = proj_of(s.th[slot(g, zbase + y_lo * 32u + lane, (lane + y_lo + z) & 1u)], cphi, sphi);
-            for (uint32_t y = y_lo; y < y_hi; ++y) {
-                const uint32_t idx = zbase + y * 32u + lane;
-                const uint32_t y1 = (y + 1 == g.ly) ? 0u : y + 1;
-                const float ryp = proj_of(s.th[slot(g, zbase + y1 * 32u + lane, (lane + y1 + z) & 1u)], cphi, sphi);
-                const float rzp = proj_of(s.th[slot(g, zp_off + y * 32u + lane, (lane + y + z + 1) & 1u)], cphi, sphi);
-                const float rxp = __shfl_sync(0xffffffffu, ri, (lane + 1) & 31u);
-                const slsf_u32x4 b = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, idx);
-                const uint32_t bal_x = __ballot_sync(0xffffffffu, wolff_bond_active(jx, ri, rxp, m2b, b.x));
-                const uint32_t bal_y = __ballot_sync(0xffffffffu, wolff_bond_active(jx, ri, ryp, m2b, b.y));
-                const uint32_t bal_z = __ballot_sync(0xffffffffu, wolff_bond_active(jzz, ri, rzp, m2b, b.z));
-                if (lane == 0) {
-                    const uint32_t row = y + g.ly * z;
-                    s.bx[row] = bal_x;
-                    s.by[row] = bal_y;
-                    s.bz[row] = bal_z;
-                }
-                ri = ryp;
-            }
-        }
-    } else if (g.lx >= 24) {
-        /* 24 <= L_x < 32: a row is a warp (lane = x; lanes past the row read
-         * the row's first site and keep no bits).  Each warp walks an equal run
-         * of the replica's rows in order (y fastest), so the projection of the
-         * +y row is the next row's own -- two sincos per site instead of
-         * three, and no per-site index division -- except at the first row of
-         * its run and of each plane.  (Narrower rows would leave too many
-         * lanes idle: they take the general path below.) */
-        const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-        const uint32_t nrows = g.rows;
-        const uint32_t r_lo = (uint32_t)((uint64_t)warp * nrows / nwarps);
-        const uint32_t r_hi = (uint32_t)((uint64_t)(warp + 1) * nrows / nwarps);
-        const uint32_t xl = lane < g.lx ? lane : 0u;
-        const uint32_t xsrc = lane + 1u < g.lx ? lane + 1u : 0u;
-        uint32_t z = slsf_fastdiv_div(r_lo, g.div_ly), y = r_lo - z * g.ly;
-        uint32_t zbase = 0, zp_off = 0;
-        float ri = 0.0f, jx = 0.0f, jzz = 0.0f;
-        for (uint32_t row = r_lo; row < r_hi; ++row) {
-            if (row == r_lo || y == 0) { /* a new plane: its couplings, offsets and first row */
-                zbase = z * g.plane;
-                zp_off = (z + 1 == g.lz) ? 0u : (z + 1) * g.plane; /* base of the +z plane */
-                jx = s.jxy[z];
-                jzz = s.jz[z];
-                ri = proj_of(s.th[slot(g, zbase + y * g.lx + xl, (xl + y + z) & 1u)], cphi, sphi);
-            }
-            const uint32_t idx = zbase + y * g.lx + xl;
-            const uint32_t y1 = (y + 1 == g.ly) ? 0u : y + 1;
-            const float ryp = proj_of(s.th[slot(g, zbase + y1 * g.lx + xl, (xl + y1 + z) & 1u)], cphi, sphi);
-            const float rzp = proj_of(s.th[slot(g, zp_off + y * g.lx + xl, (xl + y + z + 1) & 1u)], cphi, sphi);
-            const float rxp = __shfl_sync(0xffffffffu, ri, xsrc);
-            const slsf_u32x4 b = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, idx);
-            const uint32_t bal_x = __ballot_sync(0xffffffffu, wolff_bond_active(jx, ri, rxp, m2b, b.x));
-            const uint32_t bal_y = __ballot_sync(0xffffffffu, wolff_bond_active(jx, ri, ryp, m2b, b.y));
-            const uint32_t bal_z = __ballot_sync(0xffffffffu, wolff_bond_active(jzz, ri, rzp, m2b, b.z));
-            if (lane == 0) {
-                s.bx[row] = bal_x & g.xmask;
-                s.by[row] = bal_y & g.xmask;
-                s.bz[row] = bal_z & g.xmask;
-            }
-            ri = ryp;
-            if (++y == g.ly) {
-                y = 0;
-                ++z;
-            }
-        }
-    } else if (g.lx_tiles_warp) {
-        /* L_x = 4, 8, 16: a warp holds G = 32 / L_x rows (lane = x + L_x sub), sub-group sub
-         * in plane z = G zb + sub; each warp walks columns of rows along y --
-         * (zb, y segment) units, round robin -- so the projection of the +y
-         * row is the next row's own: two sincos per site instead of three,
-         * and no per-site index division.  Sub-groups past the last plane
-         * (L_z not a multiple of G) compute on the last plane and keep
-         * nothing. */
-        const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-        const uint32_t gsz = 32u / g.lx, sub = lane / g.lx, x = lane - sub * g.lx;
-        const uint32_t nzb = (g.lz + gsz - 1) / gsz;
-        const uint32_t nseg = (nwarps + nzb - 1) / nzb;
-        const uint32_t seg = (g.ly + nseg - 1) / nseg;
-        const uint32_t xsrc = sub * g.lx + (x + 1 == g.lx ? 0u : x + 1);
-        for (uint32_t u = warp; u < nzb * nseg; u += nwarps) {
-            const uint32_t zb = u / nseg, y_lo = (u % nseg) * seg, y_hi = min(g.ly, y_lo + seg);
-            if (y_lo >= y_hi) continue;
-            const uint32_t zq = zb * gsz + sub;
-            const bool zvalid = zq < g.lz;
-            const uint32_t z = zvalid ? zq : g.lz - 1;
-            const uint32_t zp_off = (z + 1 == g.lz) ? 0u : (z + 1) * g.plane; /* base of the +z plane */
-            const float jx = s.jxy[z], jzz = s.jz[z];
-            const uint32_t zbase = z * g.plane;
-            float ri = proj_of(s.th[slot(g, zbase + y_lo * g.lx + x, (x + y_lo + z) & 1u)], cphi, sphi);
-            for (uint32_t y = y_lo; y < y_hi; ++y) {
-                const uint32_t idx = zbase + y * g.lx + x;
-                const uint32_t y1 = (y + 1 == g.ly) ? 0u : y + 1;
-                const float ryp = proj_of(s.th[slot(g, zbase + y1 * g.lx + x, (x + y1 + z) & 1u)], cphi, sphi);
-                const float rzp = proj_of(s.th[slot(g, zp_off + y * g.lx + x, (x + y + z + 1) & 1u)], cphi, sphi);
-                const float rxp = __shfl_sync(0xffffffffu, ri, xsrc);
-                const slsf_u32x4 b = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, idx);
-                const uint32_t bal_x = __ballot_sync(0xffffffffu, wolff_bond_active(jx, ri, rxp, m2b, b.x));
-                const uint32_t bal_y = __ballot_sync(0xffffffffu, wolff_bond_active(jx, ri, ryp, m2b, b.y));
-                const uint32_t bal_z = __ballot_sync(0xffffffffu, wolff_bond_active(jzz, ri, rzp, m2b, b.z));
-                if (x == 0 && zvalid) {
-                    const uint32_t row = y + g.ly * z;
-                    s.bx[row] = (bal_x >> lane) & g.xmask;
-                    s.by[row] = (bal_y >> lane) & g.xmask;
-                    s.bz[row] = (bal_z >> lane) & g.xmask;
-                }
-                ri = ryp;
-            }
-        }
-    } else
-    /* Bond activation, one thread per site, warp-aligned site ranges. */
-    for (uint32_t i0 = (threadIdx.x & ~31u); i0 < g.volume; i0 += blockDim.x) {
-        const uint32_t idx = i0 + lane;
-        const bool valid = idx < g.volume;
-        const uint32_t ii = valid ? idx : 0;
-        const Coords c = coords_of(g, ii);
-        uint32_t xp, yp, zp;
-        forward_neighbours(g, ii, c, xp, yp, zp);
-        const float ri = proj_of(site_theta(g, s, ii, c), cphi, sphi);
-        float rxp;
-        if (g.lx_tiles_warp) {
-            rxp = __shfl_sync(0xffffffffu, ri, xp_lane(lane, g.lx));
-        } else {
-            /* the +x neighbour is the next lane unless the row or the warp ends */
-            rxp = __shfl_down_sync(0xffffffffu, ri, 1);
-            if (lane == 31 || c.x + 1 == g.lx) {
-                const Coords cx = {c.x + 1 == g.lx ? 0 : c.x + 1, c.y, c.z, c.row};
-                rxp = proj_of(site_theta(g, s, xp, cx), cphi, sphi);
-            }
-        }
-        const Coords cy = {c.x, c.y + 1 == g.ly ? 0 : c.y + 1, c.z, 0};
-        const Coords cz = {c.x, c.y, c.z + 1 == g.lz ? 0 : c.z + 1, 0};
-        const float ryp = proj_of(site_theta(g, s, yp, cy), cphi, sphi);
-        const float rzp = proj_of(site_theta(g, s, zp, cz), cphi, sphi);
-        const slsf_u32x4 b = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, ii);
-        const float jx = s.jxy[c.z], jzz = s.jz[c.z];
-        const bool ax = valid && wolff_bond_active(jx, ri, rxp, m2b, b.x);
-        const bool ay = valid && wolff_bond_active(jx, ri, ryp, m2b, b.y);
-        const bool az = valid && wolff_bond_active(jzz, ri, rzp, m2b, b.z);
-        if (g.lx_tiles_warp) {
-            const uint32_t bal_x = __ballot_sync(0xffffffffu, ax);
-            const uint32_t bal_y = __ballot_sync(0xffffffffu, ay);
-            const uint32_t bal_z = __ballot_sync(0xffffffffu, az);
-            if (valid && c.x == 0) {
-                s.bx[c.row] = (bal_x >> lane) & g.xmask;
-                s.by[c.row] = (bal_y >> lane) & g.xmask;
-                s.bz[c.row] = (bal_z >> lane) & g.xmask;
-            }
-        } else {
-            /* The warp's 32 consecutive sites cover pieces of a few rows; the
-             * first lane of each piece ORs the piece's ballot bits into its
-             * row (rows shared with another warp need the atomic). */
-            const uint32_t bal_x = __ballot_sync(0xffffffffu, ax);
-            const uint32_t bal_y = __ballot_sync(0xffffffffu, ay);
-            const uint32_t bal_z = __ballot_sync(0xffffffffu, az);
-            if (valid && (lane == 0 || c.x == 0)) {
-                const uint32_t len = min(g.lx - c.x, 32u - lane);
-                const uint32_t m = len >= 32 ? 0xffffffffu : ((1u << len) - 1u);
-                const uint32_t px = ((bal_x >> lane) & m) << c.x;
-                const uint32_t py = ((bal_y >> lane) & m) << c.x;
-                const uint32_t pz = ((bal_z >> lane) & m) << c.x;
-                if (px) atomicOr(&s.bx[c.row], px);
-                if (py) atomicOr(&s.by[c.row], py);
-                if (pz) atomicOr(&s.bz[c.row], pz);
-            }
-        }
-    }
+    wolff_bonds(t, g, s, counter, cphi, sphi);
     const uint32_t seed_row = y0 + g.ly * z0;
     for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) s.cl[r] = (r == seed_row) ? (1u << x0) : 0u;
     __syncthreads();
@@ -680,7 +677,7 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
     const uint32_t bound = t.loop_limit ? min(t.loop_limit, g.volume) : g.volume;
     uint32_t pass = 0;
     bool converged = false;
-    if (s.blk && g.lx == 32 && g.ly == 32 && g.lz == 32 && blockDim.x == 1024) {
+    if (s.blk && g.lx == 32 && g.ly == 32 && g.lz == 32 && (32u % (blockDim.x >> 5)) == 0) {
         /* a 32^3 replica is one block of the shared bit-parallel closure: warp
          * scans along y and z, a few passes instead of one row step per pass */
         typedef uint32_t Row[kGrowEdge + 1];
@@ -688,16 +685,18 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
         Row* BY = C + kGrowEdge;
         Row* BZ = BY + kGrowEdge;
         Row* BX = BZ + kGrowEdge;
-        const uint32_t z = threadIdx.x >> 5, y = threadIdx.x & 31u, r = y + 32u * z;
-        C[z][y] = s.cl[r];
-        BY[z][y] = s.by[r];
-        BZ[z][y] = s.bz[r];
-        BX[z][y] = s.bx[r];
+        for (uint32_t r = threadIdx.x; r < kGrowEdge * kGrowEdge; r += blockDim.x) {
+            const uint32_t z = r >> 5, y = r & 31u;
+            C[z][y] = s.cl[r];
+            BY[z][y] = s.by[r];
+            BZ[z][y] = s.bz[r];
+            BX[z][y] = s.bx[r];
+        }
         __syncthreads();
         const uint32_t used = close_block(C, BY, BZ, BX, true, true, true, bound + 1);
         converged = used != 0;
         pass = used ? used - 1 : bound;
-        s.cl[r] = C[z][y];
+        for (uint32_t r = threadIdx.x; r < kGrowEdge * kGrowEdge; r += blockDim.x) s.cl[r] = C[r >> 5][r & 31u];
         __syncthreads();
     } else if (g.rows <= blockDim.x) {
         /* one row per thread: its neighbour rows and bond masks stay fixed
@@ -749,11 +748,35 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
     /* Reflect the cluster (src/updates.rs:602-617) and count it. */
     uint32_t members = 0;
     for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) members += __popc(s.cl[r]);
-    for (uint32_t idx = threadIdx.x; idx < g.volume; idx += blockDim.x) {
-        const Coords c = coords_of(g, idx);
-        if ((s.cl[c.row] >> c.x) & 1u) {
-            const uint32_t sl = slot(g, idx, (c.x + c.y + c.z) & 1u);
-            s.th[sl] = slsf_reflect(s.th[sl], phi);
+    if (g.lx % 4 == 0) {
+        /* four consecutive sites of a row (a pair of each colour) per thread
+         * and step; a row's pairs are swapped between the colours by its parity */
+        const uint32_t nq = g.lx >> 2;
+        for (uint32_t i = threadIdx.x; i < (g.volume >> 2); i += blockDim.x) {
+            const uint32_t r = slsf_fastdiv_div(i, g.div_nq), q = i - r * nq;
+            const uint32_t m = s.cl[r] >> (4 * q) & 15u;
+            if (!m) continue;
+            const uint32_t z = slsf_fastdiv_div(r, g.div_ly);
+            const uint32_t p = (r - z * g.ly + z) & 1u; /* colour of the even-x sites */
+            float2* even = reinterpret_cast<float2*>(s.th + p * g.stride1 + 2 * i);
+            float2* odd = reinterpret_cast<float2*>(s.th + (p ^ 1u) * g.stride1 + 2 * i);
+            float2 e = *even, o = *odd;
+            const float ex = slsf_reflect(e.x, phi), ox = slsf_reflect(o.x, phi);
+            const float ey = slsf_reflect(e.y, phi), oy = slsf_reflect(o.y, phi);
+            e.x = (m & 1u) ? ex : e.x;
+            o.x = (m & 2u) ? ox : o.x;
+            e.y = (m & 4u) ? ey : e.y;
+            o.y = (m & 8u) ? oy : o.y;
+            *even = e;
+            *odd = o;
+        }
+    } else {
+        for (uint32_t idx = threadIdx.x; idx < g.volume; idx += blockDim.x) {
+            const Coords c = coords_of(g, idx);
+            if ((s.cl[c.row] >> c.x) & 1u) {
+                const uint32_t sl = slot(g, idx, (c.x + c.y + c.z) & 1u);
+                s.th[sl] = slsf_reflect(s.th[sl], phi);
+            }
         }
     }
 #pragma unroll
@@ -934,8 +957,8 @@ __device__ __forceinline__ void measure(const Geo& g, const Smem& s, double (&ac
 }
 
 
-template <bool kCorr>
-__global__ void __launch_bounds__(kBThreads, 1)
+template <bool kCorr, int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads, 1)
     k_resident(const TaskView* __restrict__ views, uint32_t n, uint32_t n_sweeps, unsigned int* __restrict__ queue,
                uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, unsigned long long* __restrict__ counters,
                const ResidentCorr* __restrict__ corr, uint32_t cube32) {
@@ -964,6 +987,7 @@ __global__ void __launch_bounds__(kBThreads, 1)
         }
         load_state(t, g, s);
         __syncthreads();
+        s.jmax = largest_coupling(g, s);
 #ifdef SLSF_PHASE_TIMING
         if (threadIdx.x == 0) s_phase_mark = clock64();
 #endif
@@ -1039,22 +1063,22 @@ size_t smem_bytes(uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, uint3
            8ull * corr_doubles;
 }
 
-template <bool kCorr>
+template <bool kCorr, int kMaxThreads>
 cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_sweeps, unsigned int* queue,
                               int device, cudaStream_t s, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
                               uint32_t threads, unsigned long long* counters, const ResidentCorr* corr,
                               uint32_t corr_doubles, bool cube32) {
     const size_t smem = smem_bytes(max_volume, max_rows, max_lz, corr_doubles, cube32);
-    cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr, kMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int sms = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<kCorr>, (int)threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<kCorr, kMaxThreads>, (int)threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(sms * per_sm));
-    k_resident<kCorr><<<grid, threads, smem, s>>>(views_dev, n, n_sweeps, queue, max_volume, max_rows, max_lz,
+    k_resident<kCorr, kMaxThreads><<<grid, threads, smem, s>>>(views_dev, n, n_sweeps, queue, max_volume, max_rows, max_lz,
                                                   counters, corr, cube32 ? 1u : 0u);
     return cudaGetLastError();
 }
@@ -1088,13 +1112,22 @@ cudaError_t launch_resident(const TaskView* views_dev, uint32_t n, uint32_t n_sw
     /* the padded growth blocks of 32^3 replicas, when they fit beside the largest replica */
     if (cube32 && smem_bytes(max_volume, max_rows, max_lz, corr_doubles, true) > (size_t)max_dynamic_smem(device))
         cube32 = false;
-    /* the fused correlation measurement is compiled into its own instance, so
-     * groups without it run the kernel unchanged */
+    /* the fused correlation measurement is compiled into its own instances, so
+     * groups without it run the kernel unchanged; CTAs of up to 512 threads
+     * have 128 registers a thread (the patch walk and its compensated sums
+     * need about 120), larger ones 64 and spill: 6.67e10 against 5.8e10
+     * site-updates/s at L = 32 */
     if (corr_dev && corr_doubles)
-        return launch_resident_t<true>(views_dev, n, n_sweeps, queue, device, s, max_volume, max_rows, max_lz,
-                                       threads, counters, corr_dev, corr_doubles, cube32);
-    return launch_resident_t<false>(views_dev, n, n_sweeps, queue, device, s, max_volume, max_rows, max_lz,
-                                    threads, counters, nullptr, 0, cube32);
+        return threads > 512 ? launch_resident_t<true, kBThreads>(views_dev, n, n_sweeps, queue, device, s, max_volume,
+                                                                  max_rows, max_lz, threads, counters, corr_dev,
+                                                                  corr_doubles, cube32)
+                             : launch_resident_t<true, 512>(views_dev, n, n_sweeps, queue, device, s, max_volume,
+                                                            max_rows, max_lz, threads, counters, corr_dev,
+                                                            corr_doubles, cube32);
+    return threads > 512 ? launch_resident_t<false, kBThreads>(views_dev, n, n_sweeps, queue, device, s, max_volume,
+                                                               max_rows, max_lz, threads, counters, nullptr, 0, cube32)
+                         : launch_resident_t<false, 512>(views_dev, n, n_sweeps, queue, device, s, max_volume,
+                                                         max_rows, max_lz, threads, counters, nullptr, 0, cube32);
 }
 
 }  // namespace slsf

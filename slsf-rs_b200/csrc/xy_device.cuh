@@ -78,12 +78,13 @@ __device__ __forceinline__ float wolff_projection(float c, float s, float cphi, 
     return __fmaf_rn(s, sphi, __fmul_rn(c, cphi));
 }
 
-/* e^x = 2^(x log2 e) with the hardware's 2^y, results below 2^-126 flushed to
- * zero (the instruction alone, without the range test and the two scalings
- * that keep subnormal results). */
-__device__ __forceinline__ float exp_flush(float x) {
+/* 2^y by the hardware instruction, results below 2^-126 flushed to zero (the
+ * instruction alone, without the range test and the two scalings that keep
+ * subnormal results); e^x = 2^(x log2 e). */
+constexpr float kLog2E = 1.44269504088896341f;
+__device__ __forceinline__ float exp2_flush(float y) {
     float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(x, 1.44269504088896341f)));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
     return r;
 }
 
@@ -95,12 +96,25 @@ __device__ __forceinline__ float exp_flush(float x) {
  * the spacing of [1/2, 1)), 2^32 p = 2^32 - 2^32 e in one fused step is that
  * same rounding scaled exactly, and word >> 8 < 2^24 p holds iff the word
  * itself, rounded towards zero to 24 bits, is below 2^32 p.  A flushed exp
- * gives p = 1, as a subnormal one does. */
+ * gives p = 1, as a subnormal one does, and where J r_i r_j is not positive
+ * exp is at least 1, so p <= 0 (or NaN) and no word is below it. */
 __device__ __forceinline__ bool wolff_bond_active(float coupling, float ri, float rj,
                                                   float minus_two_beta, uint32_t word) {
     const float prod = __fmul_rn(__fmul_rn(coupling, ri), rj);
-    const float e = exp_flush(__fmul_rn(minus_two_beta, prod));
-    return (prod > 0.0f) & (__uint2float_rz(word) < __fmaf_rn(e, -4294967296.0f, 4294967296.0f));
+    const float e = exp2_flush(__fmul_rn(__fmul_rn(minus_two_beta, prod), kLog2E));
+    return __uint2float_rz(word) < __fmaf_rn(e, -4294967296.0f, 4294967296.0f);
+}
+
+/* The ballots of wolff_bond_active for the bonds of two sites per lane, from
+ * their packed products J r_i r_j. */
+__device__ __forceinline__ void wolff_bond_words(float2 prod, float2 minus_two_beta, uint32_t word_a, uint32_t word_b,
+                                                 uint32_t& a, uint32_t& b) {
+    const float2 y = __fmul2_rn(__fmul2_rn(minus_two_beta, prod), make_float2(kLog2E, kLog2E));
+    const float2 e = make_float2(exp2_flush(y.x), exp2_flush(y.y));
+    const float2 p = __ffma2_rn(e, make_float2(-4294967296.0f, -4294967296.0f),
+                                make_float2(4294967296.0f, 4294967296.0f));
+    a = __ballot_sync(0xffffffffu, __uint2float_rz(word_a) < p.x);
+    b = __ballot_sync(0xffffffffu, __uint2float_rz(word_b) < p.y);
 }
 
 /* Terms of one bond a -> b = a + mu of the observables
