@@ -129,35 +129,12 @@ __device__ __forceinline__ void forward_neighbours(const Geo& g, uint32_t idx, c
     zp = (c.z + 1 == g.lz) ? idx + g.plane - g.volume : idx + g.plane;
 }
 
+/* Row word of row y of plane z (the bond and cluster words). */
+__device__ __forceinline__ uint32_t row_word(const Geo& g, uint32_t y, uint32_t z) { return y + g.ly * z; }
+
 /* Lane holding the +x neighbour when rows of lx sites tile the warp. */
 __device__ __forceinline__ uint32_t xp_lane(uint32_t lane, uint32_t lx) {
     return (lane & ~(lx - 1u)) | ((lane + 1u) & (lx - 1u));
-}
-
-__device__ __forceinline__ uint32_t rotl_row(uint32_t w, uint32_t s, uint32_t lx, uint32_t mask) {
-    return lx == 32 ? __funnelshift_l(w, w, s) : (((w << s) | (w >> (lx - s))) & mask);
-}
-
-__device__ __forceinline__ uint32_t rotr_row(uint32_t w, uint32_t s, uint32_t lx, uint32_t mask) {
-    return lx == 32 ? __funnelshift_r(w, w, s) : (((w >> s) | (w << (lx - s))) & mask);
-}
-
-/* Closure of a periodic row's cluster bits c along x through the bond bits b
- * (bit x: bond x -- x+1).  Kogge-Stone doubling in both directions: after the
- * step with shift s, every site within 2s - 1 bond steps of a seed is set;
- * shifts 1..16 cover any row of L_x <= 32 sites. */
-__device__ __forceinline__ uint32_t close_row(uint32_t c, uint32_t b, uint32_t lx, uint32_t mask) {
-    uint32_t gr = c, pr = b;                        /* rightward: bond p -> p+1 */
-    uint32_t gl = c, pl = rotl_row(b, 1, lx, mask); /* leftward: bond p-1 -> p */
-#pragma unroll
-    for (uint32_t s = 1; s < 32; s <<= 1) {
-        if (s >= lx) break;
-        gr |= rotl_row(gr & pr, s, lx, mask);
-        pr &= rotr_row(pr, s, lx, mask);
-        gl |= rotr_row(gl & pl, s, lx, mask);
-        pl &= rotl_row(pl, s, lx, mask);
-    }
-    return gr | gl;
 }
 
 struct Smem {
@@ -168,18 +145,13 @@ struct Smem {
     uint32_t* cl;
     float* jxy;
     float* jz;
-    uint32_t* blk; /* 32^3 replicas: cluster and bond words as [z][y] blocks of pitch 33 (cube32), else NULL */
     double* corr;  /* fused correlation scratch (resident_corr_doubles) */
     float jmax;    /* largest coupling of the replica (NaN and infinity become infinity) */
 };
 
 constexpr float kJMax = 1e30f;
 
-/* Words of the padded blocks of a 32^3 replica's Wolff growth (C, BY, BZ, BX). */
-constexpr uint32_t kBlockWords = 4 * kGrowEdge * (kGrowEdge + 1);
-
-__device__ __forceinline__ Smem carve(unsigned char* base, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
-                                      uint32_t cube32) {
+__device__ __forceinline__ Smem carve(unsigned char* base, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz) {
     Smem s;
     s.th = reinterpret_cast<float*>(base);
     uint32_t* w = reinterpret_cast<uint32_t*>(base + 4ull * (max_volume + 2 * kPad));
@@ -189,11 +161,8 @@ __device__ __forceinline__ Smem carve(unsigned char* base, uint32_t max_volume, 
     s.cl = w + 3 * max_rows;
     s.jxy = reinterpret_cast<float*>(w + 4 * max_rows);
     s.jz = s.jxy + max_lz;
-    uint32_t* after = reinterpret_cast<uint32_t*>(s.jz + max_lz);
-    s.blk = cube32 ? after : nullptr;
-    if (cube32) after += kBlockWords;
     /* 8-byte aligned: the volume is even, the other arrays are whole words */
-    s.corr = reinterpret_cast<double*>(after);
+    s.corr = reinterpret_cast<double*>(s.jz + max_lz);
     return s;
 }
 
@@ -553,30 +522,85 @@ __device__ __forceinline__ float site_theta(const Geo& g, const Smem& s, uint32_
     return s.th[slot(g, idx, (c.x + c.y + c.z) & 1u)];
 }
 
-/* One growth pass: every row takes the cluster bits that reach it through
- * its y and z bonds; a row that gained bits is closed along x (stored rows
- * are always closed).  Returns nonzero if any row changed.  Rows updated
- * earlier in the same pass are seen by later ones, so bits can travel more
- * than one row per pass. */
-__device__ __forceinline__ int grow_pass(const Geo& g, Smem& s) {
-    int changed = 0;
-    for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) {
-        const uint32_t old = s.cl[r];
-        const uint32_t z = slsf_fastdiv_div(r, g.div_ly);
-        const uint32_t y = r - z * g.ly;
-        const uint32_t r_yp = (y + 1 == g.ly) ? r + 1 - g.ly : r + 1;
-        const uint32_t r_ym = (y == 0) ? r + g.ly - 1 : r - 1;
-        const uint32_t r_zp = (z + 1 == g.lz) ? r + g.ly - g.rows : r + g.ly;
-        const uint32_t r_zm = (z == 0) ? r + g.rows - g.ly : r - g.ly;
-        const uint32_t in = (s.cl[r_ym] & s.by[r_ym]) | (s.cl[r_yp] & s.by[r]) | (s.cl[r_zm] & s.bz[r_zm]) |
-                            (s.cl[r_zp] & s.bz[r]);
-        const uint32_t c = old | in;
-        if (c != old) {
-            s.cl[r] = close_row(c, s.bx[r], g.lx, g.xmask);
-            changed = 1;
-        }
+/* Growth passes over row words: every row takes the cluster bits that reach
+ * it through its y and z bonds; a row that gained bits is closed along x
+ * (stored rows are always closed).  Rows updated earlier in the same pass are
+ * seen by later ones, so bits can travel more than one row per pass. */
+constexpr int kGrowSteps = 3; /* steps of every row between two block barriers */
+
+/* One step of a row from the words around it; returns whether it changed. */
+__device__ __forceinline__ bool grow_row(volatile uint32_t* cl, uint32_t w, uint32_t in, uint32_t bx, uint32_t lx) {
+    const uint32_t old = cl[w], c = old | in;
+    if (c == old) return false;
+    cl[w] = close_word(c, bx, lx, true);
+    return true;
+}
+
+/* R rows per thread, everything but the cluster words looked up once and
+ * kept in registers.  A pass takes kGrowSteps steps of every row and one block
+ * barrier with the vote: bits only ever get set, so a pass in which no row
+ * changed saw the same words throughout and the cluster is closed. */
+template <int R>
+__device__ __forceinline__ uint32_t grow_rows(const Geo& g, Smem& s, uint32_t bound) {
+    uint32_t w[R], yp[R], ym[R], zp[R], zm[R], b_yp[R], b_ym[R], b_zp[R], b_zm[R], b_x[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const uint32_t r = threadIdx.x + k * blockDim.x;
+        const bool has = r < g.rows;
+        const uint32_t z = has ? slsf_fastdiv_div(r, g.div_ly) : 0u, y = has ? r - z * g.ly : 0u;
+        w[k] = row_word(g, y, z);
+        yp[k] = row_word(g, y + 1 == g.ly ? 0 : y + 1, z);
+        ym[k] = row_word(g, y == 0 ? g.ly - 1 : y - 1, z);
+        zp[k] = row_word(g, y, z + 1 == g.lz ? 0 : z + 1);
+        zm[k] = row_word(g, y, z == 0 ? g.lz - 1 : z - 1);
+        b_yp[k] = has ? s.by[w[k]] : 0u;
+        b_ym[k] = has ? s.by[ym[k]] : 0u;
+        b_zp[k] = has ? s.bz[w[k]] : 0u;
+        b_zm[k] = has ? s.bz[zm[k]] : 0u;
+        b_x[k] = s.bx[w[k]];
     }
-    return changed;
+    volatile uint32_t* cl = s.cl;
+    for (uint32_t pass = 0; pass < bound; ++pass) {
+        int changed = 0;
+#pragma unroll 1
+        for (int step = 0; step < kGrowSteps; ++step) {
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const uint32_t in = (cl[ym[k]] & b_ym[k]) | (cl[yp[k]] & b_yp[k]) | (cl[zm[k]] & b_zm[k]) |
+                                    (cl[zp[k]] & b_zp[k]);
+                if (grow_row(cl, w[k], in, b_x[k], g.lx)) changed = 1;
+            }
+        }
+        if (!__syncthreads_or(changed)) return pass + 1;
+    }
+    return 0;
+}
+
+/* Grows the cluster (the closed seed row in cl) over the bond words; returns
+ * the passes taken, 0 if they exceeded `bound`.  A barrier every three steps
+ * against one every step takes a seventh off at L = 32 (18.4k -> 15.8k cycles
+ * per update, 2: 16.2k, 4: 15.7k); up to four rows per thread stay in
+ * registers (measured before, with words and divisions looked up in every
+ * step: L = 16 24.0k -> 12.0k, L = 24 43.5k -> 25.0k).  Scans of whole lines by
+ * shuffles need fewer passes (10 at L = 32) but longer ones: 17-19k cycles at
+ * L = 32, 39k at L = 24, 35k at L = 16. */
+__device__ __forceinline__ uint32_t grow(const Geo& g, Smem& s, uint32_t bound) {
+    if (g.rows <= blockDim.x) return grow_rows<1>(g, s, bound);
+    if (g.rows <= 2 * blockDim.x) return grow_rows<2>(g, s, bound);
+    if (g.rows <= 4 * blockDim.x) return grow_rows<4>(g, s, bound);
+    volatile uint32_t* cl = s.cl;
+    for (uint32_t pass = 0; pass < bound; ++pass) {
+        int changed = 0;
+        for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) {
+            const uint32_t z = slsf_fastdiv_div(r, g.div_ly), y = r - z * g.ly;
+            const uint32_t ym = row_word(g, y == 0 ? g.ly - 1 : y - 1, z), zm = row_word(g, y, z == 0 ? g.lz - 1 : z - 1);
+            const uint32_t in = (cl[ym] & s.by[ym]) | (cl[row_word(g, y + 1 == g.ly ? 0 : y + 1, z)] & s.by[r]) |
+                                (cl[zm] & s.bz[zm]) | (cl[row_word(g, y, z + 1 == g.lz ? 0 : z + 1)] & s.bz[r]);
+            if (grow_row(cl, r, in, s.bx[r], g.lx)) changed = 1;
+        }
+        if (!__syncthreads_or(changed)) return pass + 1;
+    }
+    return 0;
 }
 
 /* Bond activation: the +x, +y, +z bond words of every row.  A warp holds
@@ -644,7 +668,7 @@ __device__ __forceinline__ void wolff_bonds(const TaskView& t, const Geo& g, con
         }
         if (lane < y_hi - y_lo)
             for (uint32_t q = 0; q < groups && zb * groups + q < (g.lz >> 1); ++q) {
-                const uint32_t row = y_lo + lane + g.ly * 2 * (zb * groups + q), sh = q * g.lx;
+                const uint32_t row = row_word(g, y_lo + lane, 2 * (zb * groups + q)), sh = q * g.lx;
                 s.bx[row] = (k[0] >> sh) & g.xmask;
                 s.by[row] = (k[1] >> sh) & g.xmask;
                 s.bz[row] = (k[2] >> sh) & g.xmask;
@@ -665,84 +689,19 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
     float sphi, cphi;
     __sincosf(phi, &sphi, &cphi);
     wolff_bonds(t, g, s, counter, cphi, sphi);
-    const uint32_t seed_row = y0 + g.ly * z0;
-    for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) s.cl[r] = (r == seed_row) ? (1u << x0) : 0u;
+    const uint32_t seed_row = row_word(g, y0, z0);
+    for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) s.cl[r] = 0u;
     __syncthreads();
-    if (threadIdx.x == 0) s.cl[seed_row] = close_row(s.cl[seed_row], s.bx[seed_row], g.lx, g.xmask);
+    if (threadIdx.x == 0) s.cl[seed_row] = close_word(1u << x0, s.bx[seed_row], g.lx, true);
     __syncthreads();
     SLSF_PHASE(2);
 
     /* Grow the seed's component; every pass that goes on adds at least one
      * site, so the count is bounded by V (or the context's loop limit). */
-    const uint32_t bound = t.loop_limit ? min(t.loop_limit, g.volume) : g.volume;
-    uint32_t pass = 0;
-    bool converged = false;
-    if (s.blk && g.lx == 32 && g.ly == 32 && g.lz == 32 && (32u % (blockDim.x >> 5)) == 0) {
-        /* a 32^3 replica is one block of the shared bit-parallel closure: warp
-         * scans along y and z, a few passes instead of one row step per pass */
-        typedef uint32_t Row[kGrowEdge + 1];
-        Row* C = reinterpret_cast<Row*>(s.blk);
-        Row* BY = C + kGrowEdge;
-        Row* BZ = BY + kGrowEdge;
-        Row* BX = BZ + kGrowEdge;
-        for (uint32_t r = threadIdx.x; r < kGrowEdge * kGrowEdge; r += blockDim.x) {
-            const uint32_t z = r >> 5, y = r & 31u;
-            C[z][y] = s.cl[r];
-            BY[z][y] = s.by[r];
-            BZ[z][y] = s.bz[r];
-            BX[z][y] = s.bx[r];
-        }
-        __syncthreads();
-        const uint32_t used = close_block(C, BY, BZ, BX, true, true, true, bound + 1);
-        converged = used != 0;
-        pass = used ? used - 1 : bound;
-        for (uint32_t r = threadIdx.x; r < kGrowEdge * kGrowEdge; r += blockDim.x) s.cl[r] = C[r >> 5][r & 31u];
-        __syncthreads();
-    } else if (g.rows <= blockDim.x) {
-        /* one row per thread: its neighbour rows and bond masks stay fixed
-         * during the growth, so they are read once */
-        const uint32_t r = threadIdx.x;
-        const bool has = r < g.rows;
-        uint32_t r_yp = 0, r_ym = 0, r_zp = 0, r_zm = 0, b_ym = 0, b_yp = 0, b_zm = 0, b_zp = 0, b_x = 0;
-        if (has) {
-            const uint32_t z = slsf_fastdiv_div(r, g.div_ly);
-            const uint32_t y = r - z * g.ly;
-            r_yp = (y + 1 == g.ly) ? r + 1 - g.ly : r + 1;
-            r_ym = (y == 0) ? r + g.ly - 1 : r - 1;
-            r_zp = (z + 1 == g.lz) ? r + g.ly - g.rows : r + g.ly;
-            r_zm = (z == 0) ? r + g.rows - g.ly : r - g.ly;
-            b_ym = s.by[r_ym];
-            b_yp = s.by[r];
-            b_zm = s.bz[r_zm];
-            b_zp = s.bz[r];
-            b_x = s.bx[r];
-        }
-        for (; pass <= bound; ++pass) {
-            int changed = 0;
-            if (has) {
-                const uint32_t old = s.cl[r];
-                const uint32_t c = old | (s.cl[r_ym] & b_ym) | (s.cl[r_yp] & b_yp) | (s.cl[r_zm] & b_zm) |
-                                   (s.cl[r_zp] & b_zp);
-                if (c != old) {
-                    s.cl[r] = close_row(c, b_x, g.lx, g.xmask);
-                    changed = 1;
-                }
-            }
-            if (!__syncthreads_or(changed)) {
-                converged = true;
-                break;
-            }
-        }
-    } else {
-        for (; pass <= bound; ++pass)
-            if (!__syncthreads_or(grow_pass(g, s))) {
-                converged = true;
-                break;
-            }
-    }
-    if (!converged && threadIdx.x == 0) atomicOr(&t.stats[kStatError], kErrGrowthLimit);
+    const uint32_t passes = grow(g, s, (t.loop_limit ? min(t.loop_limit, g.volume) : g.volume) + 1);
+    if (passes == 0 && threadIdx.x == 0) atomicOr(&t.stats[kStatError], kErrGrowthLimit);
     SLSF_PHASE(3);
-    SLSF_PHASE_COUNT(6, pass + 1);
+    SLSF_PHASE_COUNT(6, passes);
     SLSF_PHASE_COUNT(7, 1);
 
     /* Reflect the cluster (src/updates.rs:602-617) and count it. */
@@ -754,10 +713,10 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
         const uint32_t nq = g.lx >> 2;
         for (uint32_t i = threadIdx.x; i < (g.volume >> 2); i += blockDim.x) {
             const uint32_t r = slsf_fastdiv_div(i, g.div_nq), q = i - r * nq;
-            const uint32_t m = s.cl[r] >> (4 * q) & 15u;
+            const uint32_t z = slsf_fastdiv_div(r, g.div_ly), y = r - z * g.ly;
+            const uint32_t m = s.cl[row_word(g, y, z)] >> (4 * q) & 15u;
             if (!m) continue;
-            const uint32_t z = slsf_fastdiv_div(r, g.div_ly);
-            const uint32_t p = (r - z * g.ly + z) & 1u; /* colour of the even-x sites */
+            const uint32_t p = (y + z) & 1u; /* colour of the even-x sites */
             float2* even = reinterpret_cast<float2*>(s.th + p * g.stride1 + 2 * i);
             float2* odd = reinterpret_cast<float2*>(s.th + (p ^ 1u) * g.stride1 + 2 * i);
             float2 e = *even, o = *odd;
@@ -773,7 +732,7 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
     } else {
         for (uint32_t idx = threadIdx.x; idx < g.volume; idx += blockDim.x) {
             const Coords c = coords_of(g, idx);
-            if ((s.cl[c.row] >> c.x) & 1u) {
+            if ((s.cl[row_word(g, c.y, c.z)] >> c.x) & 1u) {
                 const uint32_t sl = slot(g, idx, (c.x + c.y + c.z) & 1u);
                 s.th[sl] = slsf_reflect(s.th[sl], phi);
             }
@@ -961,7 +920,7 @@ template <bool kCorr, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_resident(const TaskView* __restrict__ views, uint32_t n, uint32_t n_sweeps, unsigned int* __restrict__ queue,
                uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, unsigned long long* __restrict__ counters,
-               const ResidentCorr* __restrict__ corr, uint32_t cube32) {
+               const ResidentCorr* __restrict__ corr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[8 * 32];
     __shared__ double bin_acc[kBinCols];
@@ -980,7 +939,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
             t.wolff_done = counters[2 * item + 1];
         }
         const Geo g = make_geo(t);
-        Smem s = carve(smem_raw, max_volume, max_rows, max_lz, cube32);
+        Smem s = carve(smem_raw, max_volume, max_rows, max_lz);
         if (threadIdx.x == 0) {
             s_cluster = 0;
             s_accepted = 0;
@@ -1057,18 +1016,16 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     }
 }
 
-size_t smem_bytes(uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, uint32_t corr_doubles = 0,
-                  bool cube32 = false) {
-    return 4ull * (max_volume + 2 * kPad) + 16ull * max_rows + 8ull * max_lz + (cube32 ? 4ull * kBlockWords : 0ull) +
-           8ull * corr_doubles;
+size_t smem_bytes(uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, uint32_t corr_doubles = 0) {
+    return 4ull * (max_volume + 2 * kPad) + 16ull * max_rows + 8ull * max_lz + 8ull * corr_doubles;
 }
 
 template <bool kCorr, int kMaxThreads>
 cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_sweeps, unsigned int* queue,
                               int device, cudaStream_t s, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
                               uint32_t threads, unsigned long long* counters, const ResidentCorr* corr,
-                              uint32_t corr_doubles, bool cube32) {
-    const size_t smem = smem_bytes(max_volume, max_rows, max_lz, corr_doubles, cube32);
+                              uint32_t corr_doubles) {
+    const size_t smem = smem_bytes(max_volume, max_rows, max_lz, corr_doubles);
     cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr, kMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int sms = 0, per_sm = 0;
@@ -1079,7 +1036,7 @@ cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(sms * per_sm));
     k_resident<kCorr, kMaxThreads><<<grid, threads, smem, s>>>(views_dev, n, n_sweeps, queue, max_volume, max_rows, max_lz,
-                                                  counters, corr, cube32 ? 1u : 0u);
+                                                  counters, corr);
     return cudaGetLastError();
 }
 
@@ -1107,11 +1064,8 @@ uint32_t resident_corr_doubles(uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t 
 cudaError_t launch_resident(const TaskView* views_dev, uint32_t n, uint32_t n_sweeps, unsigned int* queue,
                             int device, cudaStream_t s, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
                             uint32_t threads, unsigned long long* counters, const ResidentCorr* corr_dev,
-                            uint32_t corr_doubles, bool cube32) {
+                            uint32_t corr_doubles) {
     if (threads < 32 || threads > (uint32_t)kBThreads || threads % 32) return cudaErrorInvalidConfiguration;
-    /* the padded growth blocks of 32^3 replicas, when they fit beside the largest replica */
-    if (cube32 && smem_bytes(max_volume, max_rows, max_lz, corr_doubles, true) > (size_t)max_dynamic_smem(device))
-        cube32 = false;
     /* the fused correlation measurement is compiled into its own instances, so
      * groups without it run the kernel unchanged; CTAs of up to 512 threads
      * have 128 registers a thread (the patch walk and its compensated sums
@@ -1120,14 +1074,14 @@ cudaError_t launch_resident(const TaskView* views_dev, uint32_t n, uint32_t n_sw
     if (corr_dev && corr_doubles)
         return threads > 512 ? launch_resident_t<true, kBThreads>(views_dev, n, n_sweeps, queue, device, s, max_volume,
                                                                   max_rows, max_lz, threads, counters, corr_dev,
-                                                                  corr_doubles, cube32)
+                                                                  corr_doubles)
                              : launch_resident_t<true, 512>(views_dev, n, n_sweeps, queue, device, s, max_volume,
                                                             max_rows, max_lz, threads, counters, corr_dev,
-                                                            corr_doubles, cube32);
+                                                            corr_doubles);
     return threads > 512 ? launch_resident_t<false, kBThreads>(views_dev, n, n_sweeps, queue, device, s, max_volume,
-                                                               max_rows, max_lz, threads, counters, nullptr, 0, cube32)
+                                                               max_rows, max_lz, threads, counters, nullptr, 0)
                          : launch_resident_t<false, 512>(views_dev, n, n_sweeps, queue, device, s, max_volume,
-                                                         max_rows, max_lz, threads, counters, nullptr, 0, cube32);
+                                                         max_rows, max_lz, threads, counters, nullptr, 0);
 }
 
 }  // namespace slsf

@@ -262,7 +262,7 @@ __device__ bool grow_region(const WolffBits& wb, const GrowGeo& g, uint32_t r, u
         }
     }
     if (w == seed_site >> 5) c |= 1u << (seed_site & 31u);
-    c = close_word(c, bxw, g.px);
+    c = close_word(c, bxw, 32u, g.px);
     /* the stored region is closed already: without new bits nothing changes */
     const int any_new = __syncthreads_or(c != c0);
     SLSF_WB_CLOCK(5, tclk);
@@ -275,7 +275,8 @@ __device__ bool grow_region(const WolffBits& wb, const GrowGeo& g, uint32_t r, u
     BY[warp][lane] = byw;
     BZ[warp][lane] = bzw;
     __syncthreads();
-    const uint32_t passes = close_block(C, BY, BZ, BX, g.px, g.py, g.pz);
+    const GrowBlock q = {&C[0][0], &BX[0][0], &BY[0][0], &BZ[0][0], g.px, g.py, g.pz};
+    const uint32_t passes = close_block(q, kRegion * kRegion * kRegion + 1);
     SLSF_WB_COUNT(1, passes);
     SLSF_WB_CLOCK(6, tclk);
     const bool ok = passes != 0;
