@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <unordered_map>
 #include <unordered_set>
@@ -191,6 +192,7 @@ struct slsf_task {
     unsigned int* done = nullptr;
     unsigned long long* stats = nullptr;
     double* bins = nullptr;
+    float jmax = 0.0f; /* TaskView::jmax */
     slsf_batch* session = nullptr; /* open batch session holding the task's device view */
     /* correlation bins (slsf_task_corr_setup): one pool block holding the
      * launch scratch, the bin sums and the device measurement count */
@@ -224,6 +226,10 @@ struct slsf_task {
         v.n_bins = n_bins;
         v.sweeps = 0;
         v.loop_limit = ctx->loop_limit;
+        v.jmax = jmax;
+        v.partials = partials;
+        v.result = result;
+        v.done = done;
         v.stats = stats;
         return v;
     }
@@ -510,6 +516,9 @@ int slsf_task_create(slsf_ctx* ctx, const slsf_task_desc* d, slsf_task** out) {
     for (uint32_t i = 0; i < d->lz; ++i) {
         jv[i] = (float)d->j_xy[i];
         jv[d->lz + i] = (float)d->j_z[i];
+        const float j = std::max(jv[i], jv[d->lz + i]);
+        t->jmax = jv[i] < slsf::kJMax && jv[d->lz + i] < slsf::kJMax ? std::max(t->jmax, j)
+                                                                    : std::numeric_limits<float>::infinity();
     }
     /* theta, jxy and jz are separate 256-byte aligned arrays; zero the whole
      * block, then copy J.  The copy is synchronous: jv is pageable. */
@@ -714,7 +723,7 @@ int slsf_task_sweep(slsf_task* t, uint32_t n_sweeps, slsf_sweep_stats* stats) {
 int slsf_task_measure(slsf_task* t, slsf_observables* out) {
     if (!t || !out) return set_error(SLSF_ERR_INVALID, "NULL argument");
     if (int rc = bind_device(t->ctx)) return rc;
-    slsf::launch_measure(t->view(), t->partials, t->done, t->result, t->ctx->stream);
+    slsf::launch_measure(t->view(), nullptr, t->ctx->stream);
     t->ctx->launches += 1;
     SLSF_CUDA(cudaGetLastError());
     double r[8];
@@ -1094,7 +1103,7 @@ static void run_grid_task(slsf_ctx* ctx, const slsf_task* t, const TaskView& v, 
     for (uint32_t sw = 0; sw < v.sweeps; ++sw) {
         const uint64_t sweep = t->metro_sweeps + sw;
         if (pending)
-            slsf::launch_metro_colour0_measure(v, sweep, t->partials, t->done, t->result, pending, st);
+            slsf::launch_metro_colour0_measure(v, sweep, pending, st);
         else
             slsf::launch_metro_colour(v, sweep, 0, nullptr, st);
         pending = nullptr;
@@ -1128,7 +1137,7 @@ static void run_grid_task(slsf_ctx* ctx, const slsf_task* t, const TaskView& v, 
         }
     }
     if (pending) {
-        slsf::launch_measure_into_bin(v, t->partials, t->done, t->result, pending, st);
+        slsf::launch_measure(v, pending, st);
         ctx->launches += 1;
     }
 }

@@ -44,8 +44,15 @@ struct TaskView {
     uint32_t thermalization, binsize, n_bins;
     uint32_t sweeps;       /* sweeps of this task in a batched launch; 0: the launch's count */
     uint32_t loop_limit;   /* 0, or a lower bound on device loops (slsf_ctx_set_loop_limit) */
+    float jmax;            /* largest coupling; infinite if any is not below kJMax */
     unsigned long long* stats;
+    double* partials;      /* measurement scratch: block sums, totals, block counter */
+    double* result;
+    unsigned int* done;
 };
+
+/* Couplings below this keep the walks' biased FP32 sums (walk.cuh) finite. */
+constexpr float kJMax = 1e30f;
 
 /* Correlations measured inside the sweeps of the one-CTA kernel
  * (slsf_task_corr_fuse), one entry per task view of a launch; bins NULL for
@@ -77,8 +84,16 @@ void launch_metro_colour(const TaskView& t, uint64_t sweep, uint32_t colour, uin
                          cudaStream_t s);
 /* Colour 0 of a sweep fused with the measurement of the state it starts from
  * (the observables' sums into `result`, added into `bin_row` if given). */
-void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* partials, unsigned int* done,
-                                  double* result, double* bin_row, cudaStream_t s);
+void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* bin_row, cudaStream_t s);
+/* ---- walks over lattices in global memory (kernel_walk.cu) ---- */
+/* L_x a multiple of 4, L_y even, finite couplings, angles 16-byte aligned. */
+bool walk_supports(const TaskView& t);
+/* Planes per thread for n replicas of the shape in one launch. */
+uint32_t walk_seglen(const TaskView& t, uint32_t n);
+/* One colour of sweep `sweep`; with `measure` (colour 0) also the measurement
+ * of the state it starts from, into t.result and bin_row (or NULL). */
+void launch_walk_colour(const TaskView& t, uint64_t sweep, uint32_t colour, bool measure, double* bin_row, cudaStream_t s);
+void launch_walk_measure(const TaskView& t, double* bin_row, cudaStream_t s);
 /* One Wolff update; returns the number of kernels launched.  bonds [V] and
  * parent [V] are the task's scratch; with record_bonds the per-site bond
  * bits (+x, +y, +z in bits 0-2) are left in `bonds`. */
@@ -93,13 +108,10 @@ uint64_t wolff_bits_scratch_bytes(uint32_t lx, uint32_t ly, uint32_t lz);
  * the per-site bond bits, cluster_out (or NULL) the cluster mask. */
 int launch_wolff_bits(const TaskView& t, uint64_t counter, void* scratch, uint8_t* bond_bytes, uint8_t* cluster_out,
                       cudaStream_t s, float* phi_out, uint32_t seed_site[3]);
-/* Fused observables: writes 8 FP64 sums (mx, my, cos xyz, sin xyz) to result. */
-void launch_measure(const TaskView& t, double* partials, unsigned int* done, double* result,
-                    cudaStream_t s);
-/* launch_measure that also adds the measurement's kBinCols stream values to
- * bin_row (a task's bin sums row). */
-void launch_measure_into_bin(const TaskView& t, double* partials, unsigned int* done, double* result,
-                             double* bin_row, cudaStream_t s);
+/* Fused observables: writes 8 FP64 sums (mx, my, cos xyz, sin xyz) to
+ * t.result and adds the measurement's kBinCols stream values to bin_row (a
+ * task's bin sums row, or NULL). */
+void launch_measure(const TaskView& t, double* bin_row, cudaStream_t s);
 /* Blocks of a measurement launch: one per 256 sites, at most kMeasureMaxBlocks
  * (148 SMs x 8), so its per-block partial sums fit kMeasureMaxBlocks rows. */
 constexpr int kMeasureMaxBlocks = 148 * 8;

@@ -37,6 +37,7 @@
 #include "bitgrow.cuh"
 #include "engine.h"
 #include "fastdiv.h"
+#include "walk.cuh"
 #include "xy_device.cuh"
 
 namespace slsf {
@@ -146,10 +147,7 @@ struct Smem {
     float* jxy;
     float* jz;
     double* corr;  /* fused correlation scratch (resident_corr_doubles) */
-    float jmax;    /* largest coupling of the replica (NaN and infinity become infinity) */
 };
-
-constexpr float kJMax = 1e30f;
 
 __device__ __forceinline__ Smem carve(unsigned char* base, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz) {
     Smem s;
@@ -192,19 +190,6 @@ __device__ __forceinline__ void load_state(const TaskView& t, const Geo& g, Smem
         s.jxy[z] = t.jxy[z];
         s.jz[z] = t.jz[z];
     }
-}
-
-/* The same in every thread. */
-__device__ __forceinline__ float largest_coupling(const Geo& g, const Smem& s) {
-    float m = 0.0f;
-    bool fine = true;
-    for (uint32_t z = threadIdx.x & 31u; z < g.lz; z += 32) {
-        fine &= s.jxy[z] < kJMax && s.jz[z] < kJMax;
-        m = fmaxf(m, fmaxf(s.jxy[z], s.jz[z]));
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    return __all_sync(0xffffffffu, fine) ? m : __int_as_float(0x7f800000);
 }
 
 __device__ __forceinline__ void store_state(const TaskView& t, const Geo& g, const Smem& s) {
@@ -329,81 +314,6 @@ __device__ __forceinline__ uint32_t half_sweep(const TaskView& t, const Geo& g, 
  * lane, x neighbours by shuffle, L_x = 32 only) took 186 instructions per
  * update.  Operands, rounding order and randoms are those of half_sweep, so
  * decisions and new angles are bit-identical. */
-struct Trig2 {
-    float2 c, s; /* cos and sin of two sites */
-};
-
-__device__ __forceinline__ Trig2 trig2(float2 th) {
-    Trig2 t;
-    __sincosf(th.x, &t.s.x, &t.c.x);
-    __sincosf(th.y, &t.s.y, &t.c.y);
-    return t;
-}
-
-__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-
-/* Two running sums of FP32 terms carried as a value and a remainder.  The
- * value starts at a bias of at least twice what its terms can add up to, so
- * it never falls below a term's magnitude and each addition's rounding error
- * is exactly x - (t - v) (Dekker's fast two-sum); the errors add up in the
- * remainder.  total() recovers the sum to about 2^-40 of its terms'
- * magnitudes -- it agrees with FP64 sums of the same terms to 1e-12.  Four
- * packed FP32 instructions per two terms; converting each term to FP64 takes
- * eight cycles of the special-function pipe, which bound the measuring
- * half-sweep (41k of 136k cycles per sweep at L = 32 against 18k for the
- * other colour; 32k with these sums). */
-struct Sum2 {
-    float2 v, r;
-    __device__ __forceinline__ void start(float bias) {
-        v = make_float2(bias, bias);
-        r = make_float2(0.0f, 0.0f);
-    }
-    __device__ __forceinline__ void add(float2 x) {
-        const float2 minus = make_float2(-1.0f, -1.0f);
-        const float2 t = __fadd2_rn(v, x);
-        r = __fadd2_rn(r, __ffma2_rn(__ffma2_rn(v, minus, t), minus, x));
-        v = t;
-    }
-    __device__ __forceinline__ double total(float bias) const {
-        return ((double)__fsub_rn(v.x, bias) + (double)r.x) + ((double)__fsub_rn(v.y, bias) + (double)r.y);
-    }
-};
-
-/* Adds J cos and J sin of the forward bonds i -> p and the backward bonds
- * m -> i of two sites i (bond_cos, bond_sin). */
-__device__ __forceinline__ void add_bonds2(Sum2& ac, Sum2& as, float jp, float jm, const Trig2& i, const Trig2& n,
-                                           const Trig2& p, const Trig2& m) {
-    ac.add(__fmul2_rn(dup2(jp), __ffma2_rn(i.c, p.c, __fmul2_rn(i.s, p.s))));
-    as.add(__fmul2_rn(dup2(jp), __ffma2_rn(i.s, p.c, __fmul2_rn(n.c, p.s))));
-    ac.add(__fmul2_rn(dup2(jm), __ffma2_rn(m.c, i.c, __fmul2_rn(m.s, i.s))));
-    as.add(__fmul2_rn(dup2(jm), __ffma2_rn(m.s, i.c, __fmul2_rn(m.c, n.s))));
-}
-
-/* field_from_pairs of two sites. */
-__device__ __forceinline__ float2 field2(float jxy, float jzp, float jzm, float2 a01, float2 a23, float2 a4, float2 a5) {
-    return __ffma2_rn(dup2(jzm), a5, __ffma2_rn(dup2(jzp), a4, __fmul2_rn(dup2(jxy), __fadd2_rn(a01, a23))));
-}
-
-/* metro_decide for the two sites of a Philox block; returns the number accepted. */
-__device__ __forceinline__ uint32_t metro_pair(float2& th, const Trig2& own, float2 hx, float2 hy, float beta,
-                                               float width, const slsf_u32x4& b) {
-    const float2 up = make_float2((float)(b.x >> 8), (float)(b.z >> 8));
-    /* 2 u - 1 with u = word >> 8 over 2^24 */
-    const float2 d = __ffma2_rn(up, dup2(1.0f / 8388608.0f), dup2(-1.0f));
-    const float2 t = __ffma2_rn(dup2(width), d, th);
-    const float2 tn = make_float2(slsf_wrap_once(t.x), slsf_wrap_once(t.y));
-    const Trig2 n = trig2(tn);
-    const float2 dc = __fadd2_rn(own.c, neg2(n.c)), ds = __fadd2_rn(own.s, neg2(n.s));
-    const float2 de = __ffma2_rn(dc, hx, __fmul2_rn(ds, hy));
-    const float2 arg = __fmul2_rn(dup2(-beta), de);
-    const bool a0 = (de.x <= 0.0f) | (slsf_u24f(b.y) < __expf(arg.x));
-    const bool a1 = (de.y <= 0.0f) | (slsf_u24f(b.w) < __expf(arg.y));
-    th.x = a0 ? tn.x : th.x;
-    th.y = a1 ? tn.y : th.y;
-    return (a0 ? 1u : 0u) + (a1 ? 1u : 0u);
-}
-
 template <bool kMeasure>
 __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
                                                      uint32_t colour, double (&acc)[8]) {
@@ -419,7 +329,7 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
     Sum2 sum[kMeasure ? 8 : 1];
     if (kMeasure)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) sum[k].start(k < 2 ? bias : s.jmax * bias);
+        for (int k = 0; k < 8; ++k) sum[k].start(k < 2 ? bias : t.jmax * bias);
     for (uint32_t u = threadIdx.x; u < ncol * nseg; u += blockDim.x) {
         const uint32_t sg = u / ncol, col = u - sg * ncol, m = col / nq, q = col - m * nq;
         const uint32_t z_lo = sg * seglen, z_hi = min(g.lz, z_lo + seglen);
@@ -454,36 +364,9 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
             const slsf_u32x4 b1 = slsf_stream(t.seed, sweep, SLSF_PURPOSE_METRO, colour, unit + (hx >> 1));
             auto row = [&](uint32_t h, const Trig2& c, float2 e, auto row_odd, const Trig2& dn, const Trig2& up,
                            const Trig2& zm, const Trig2& zp, const slsf_u32x4& b) {
-                constexpr bool kRowOdd = decltype(row_odd)::value;
-                /* parity 0: +x is the other colour's same compact site, -x the previous; parity 1: -x the same, +x the next */
-                Trig2 xp, xm;
-                if (kRowOdd) {
-                    xp.c = make_float2(c.c.y, e.x);
-                    xp.s = make_float2(c.s.y, e.y);
-                    xm = c;
-                } else {
-                    xp = c;
-                    xm.c = make_float2(e.x, c.c.x);
-                    xm.s = make_float2(e.y, c.s.x);
-                }
                 float2 th = two(own + base + h);
-                const Trig2 i = trig2(th);
-                if (kMeasure) {
-                    /* the site and the other colour's site of the same index: each site once */
-                    sum[0].add(i.c);
-                    sum[1].add(i.s);
-                    sum[0].add(c.c);
-                    sum[1].add(c.s);
-                    Trig2 n; /* (-cos, -sin) of the site */
-                    n.c = neg2(i.c);
-                    n.s = neg2(i.s);
-                    add_bonds2(sum[2], sum[5], jx, jx, i, n, xp, xm);
-                    add_bonds2(sum[3], sum[6], jx, jx, i, n, up, dn);
-                    add_bonds2(sum[4], sum[7], jzp, jzm, i, n, zp, zm);
-                }
-                const float2 fx = field2(jx, jzp, jzm, __fadd2_rn(xp.c, xm.c), __fadd2_rn(up.c, dn.c), zp.c, zm.c);
-                const float2 fy = field2(jx, jzp, jzm, __fadd2_rn(xp.s, xm.s), __fadd2_rn(up.s, dn.s), zp.s, zm.s);
-                accepted += metro_pair(th, i, fx, fy, t.beta, t.width, b);
+                accepted += update_pair<kMeasure, decltype(row_odd)::value>(th, c, e, dn, up, zm, zp, jx, jzp, jzm,
+                                                                            t.beta, t.width, b, sum);
                 *reinterpret_cast<float2*>(own + base + h) = th;
             };
             row(h0, c0, e0, std::integral_constant<bool, kOdd>(), ym, c1, m0, p0, b0);
@@ -505,7 +388,7 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
     }
     if (kMeasure)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += sum[k].total(k < 2 ? bias : s.jmax * bias);
+        for (int k = 0; k < 8; ++k) acc[k] += sum[k].total(k < 2 ? bias : t.jmax * bias);
     return accepted;
 }
 
@@ -514,7 +397,7 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
 template <bool kMeasure>
 __device__ __forceinline__ uint32_t sweep_colour(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
                                                  uint32_t colour, double (&acc)[8]) {
-    if (g.lx % 4 == 0 && (!kMeasure || s.jmax < kJMax)) return half_sweep_quads<kMeasure>(t, g, s, sweep, colour, acc);
+    if (g.lx % 4 == 0 && (!kMeasure || t.jmax < kJMax)) return half_sweep_quads<kMeasure>(t, g, s, sweep, colour, acc);
     return half_sweep<kMeasure>(t, g, s, sweep, colour, acc);
 }
 
@@ -946,7 +829,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         }
         load_state(t, g, s);
         __syncthreads();
-        s.jmax = largest_coupling(g, s);
 #ifdef SLSF_PHASE_TIMING
         if (threadIdx.x == 0) s_phase_mark = clock64();
 #endif

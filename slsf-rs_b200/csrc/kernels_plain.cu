@@ -684,6 +684,10 @@ void launch_init_random(float* theta, uint32_t volume, uint64_t seed, cudaStream
 
 void launch_metro_colour(const TaskView& t, uint64_t sweep, uint32_t colour, uint8_t* record,
                          cudaStream_t s) {
+    if (!record && walk_supports(t)) {
+        launch_walk_colour(t, sweep, colour, false, nullptr, s);
+        return;
+    }
     const uint32_t volume = t.lx * t.ly * t.lz;
     const uint32_t npairs = ((volume >> 1) + 1) >> 1;
     const uint32_t grid = blocks_for(npairs, kThreads);
@@ -696,8 +700,11 @@ void launch_metro_colour(const TaskView& t, uint64_t sweep, uint32_t colour, uin
                                                         t.seed, sweep, colour, dhx, dly, t.stats, nullptr);
 }
 
-void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* partials, unsigned int* done,
-                                  double* result, double* bin_row, cudaStream_t s) {
+void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* bin_row, cudaStream_t s) {
+    if (walk_supports(t)) {
+        launch_walk_colour(t, sweep, 0, true, bin_row, s);
+        return;
+    }
     const uint32_t volume = t.lx * t.ly * t.lz;
     const uint32_t npairs = ((volume >> 1) + 1) >> 1;
     /* grid-stride blocks, as many as stay resident (at most kMeasureMaxBlocks,
@@ -713,7 +720,7 @@ void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* par
     const uint32_t cap = (uint32_t)std::max(1, std::min(per_sm * sms, kMeasureMaxBlocks));
     const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(blocks_for(npairs, kThreads), cap));
     const slsf_fastdiv dhx = slsf_fastdiv_make(t.lx / 2), dly = slsf_fastdiv_make(t.ly);
-    const MeasureSink sink = {partials, done, result, bin_row};
+    const MeasureSink sink = {t.partials, t.done, t.result, bin_row};
     k_metro_colour0_measure<<<grid, kThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, t.beta, t.width,
                                                       t.seed, sweep, 0, dhx, dly, t.stats, sink);
 }
@@ -756,30 +763,20 @@ int measure_partial_blocks(uint32_t volume) {
     return (int)std::max<uint32_t>(1, std::min<uint32_t>(blocks_for(volume, kMeasureThreads), kMeasureMaxBlocks));
 }
 
-void launch_measure(const TaskView& t, double* partials, unsigned int* done, double* result,
-                    cudaStream_t s) {
+void launch_measure(const TaskView& t, double* bin_row, cudaStream_t s) {
+    if (walk_supports(t)) {
+        launch_walk_measure(t, bin_row, s);
+        return;
+    }
     const uint32_t volume = t.lx * t.ly * t.lz;
     if (measure_rows_supported(t.lx, t.ly)) {
-        k_measure_rows<<<measure_partial_blocks(volume), kMeasureThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly,
-                                                                                  t.lz, partials, done, result, nullptr);
+        k_measure_rows<<<measure_partial_blocks(volume), kMeasureThreads, 0, s>>>(
+            t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, t.partials, t.done, t.result, bin_row);
         return;
     }
     k_measure<<<measure_partial_blocks(volume), kMeasureThreads, 0, s>>>(
-        t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, slsf_fastdiv_make(t.lx), slsf_fastdiv_make(t.ly), partials, done,
-        result, nullptr);
-}
-
-void launch_measure_into_bin(const TaskView& t, double* partials, unsigned int* done, double* result,
-                             double* bin_row, cudaStream_t s) {
-    const uint32_t volume = t.lx * t.ly * t.lz;
-    if (measure_rows_supported(t.lx, t.ly)) {
-        k_measure_rows<<<measure_partial_blocks(volume), kMeasureThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly,
-                                                                                  t.lz, partials, done, result, bin_row);
-        return;
-    }
-    k_measure<<<measure_partial_blocks(volume), kMeasureThreads, 0, s>>>(
-        t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, slsf_fastdiv_make(t.lx), slsf_fastdiv_make(t.ly), partials, done,
-        result, bin_row);
+        t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, slsf_fastdiv_make(t.lx), slsf_fastdiv_make(t.ly), t.partials, t.done,
+        t.result, bin_row);
 }
 
 }  // namespace slsf

@@ -25,6 +25,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <limits>
 #include <mutex>
 #include <string>
 
@@ -104,7 +105,11 @@ extern "C" int slsf_measure_noalloc(const float* theta, const float* j_xy, const
     v.lx = lx;
     v.ly = ly;
     v.lz = lz;
-    slsf::launch_measure(v, scratch->partials, &scratch->done, scratch->result, s);
+    v.jmax = std::numeric_limits<float>::infinity(); /* unknown here: the couplings are on the device */
+    v.partials = scratch->partials;
+    v.result = scratch->result;
+    v.done = &scratch->done;
+    slsf::launch_measure(v, nullptr, s);
     e = cudaGetLastError();
     double r[8];
     if (e == cudaSuccess) e = cudaMemcpyAsync(r, scratch->result, sizeof(r), cudaMemcpyDeviceToHost, s);
