@@ -57,6 +57,7 @@ constexpr uint32_t kGrowPitch = kGrowEdge + 1;
 struct GrowBlock {
     uint32_t* c;
     const uint32_t *bx, *by, *bz;
+    uint32_t lx; /* sites of a word */
     bool px, py, pz;
 };
 
@@ -110,7 +111,7 @@ struct GrowAxis {
         v = a | b;
         still = !__any_sync(0xffffffffu, v != old);
         if (!still) {
-            v = close_word(v, q.bx[at], 32, q.px);
+            v = close_word(v, q.bx[at], q.lx, q.px);
             if (v != old) q.c[at] = v;
         }
         last = v;

@@ -101,8 +101,6 @@ int launch_wolff(const TaskView& t, uint64_t wolff_counter, uint8_t* bonds, uint
                  uint8_t* cluster_out, cudaStream_t s, float* phi_out, uint32_t seed_site[3],
                  bool record_bonds = false);
 /* ---- Wolff on bit-packed bonds, the seed's cluster only (kernel_wolff_bits.cu) ---- */
-/* Sides that are multiples of 32 (regions of 32^3 sites). */
-bool wolff_bits_supports(uint32_t lx, uint32_t ly, uint32_t lz);
 uint64_t wolff_bits_scratch_bytes(uint32_t lx, uint32_t ly, uint32_t lz);
 /* `scratch` holds wolff_bits_scratch_bytes(); bond_bytes (or NULL) receives
  * the per-site bond bits, cluster_out (or NULL) the cluster mask. */
@@ -170,6 +168,9 @@ cudaError_t launch_resident(const TaskView* views_dev, uint32_t n, uint32_t n_sw
                             int device, cudaStream_t s, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
                             uint32_t threads, unsigned long long* counters, const ResidentCorr* corr_dev = nullptr,
                             uint32_t corr_doubles = 0);
+/* n_sweeps sweeps of one task (without measurements) in one launch of up to
+ * 512 threads; its counters are written, not added, to t.stats. */
+cudaError_t launch_resident_one(const TaskView& t, uint32_t n_sweeps, uint32_t threads, cudaStream_t s);
 /* Shared doubles the fused correlation measurement of one task needs (0 without). */
 uint32_t resident_corr_doubles(uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t rz);
 

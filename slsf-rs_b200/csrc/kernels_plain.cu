@@ -225,12 +225,20 @@ __global__ void __launch_bounds__(kThreads, 3)
     finish_measure(acc, scratch, sink, volume);
 }
 
-/* Smallest lattice whose Wolff update grows the seed's cluster on bit-packed
- * bonds instead of labelling 32x8x4 tiles (measured crossover on B200). */
-#ifndef SLSF_WOLFF_BITS_MIN_SITES
-#define SLSF_WOLFF_BITS_MIN_SITES (1u << 22)
-#endif
-constexpr uint64_t kWolffBitsMinSites = SLSF_WOLFF_BITS_MIN_SITES;
+/* Lattices whose Wolff update grows the seed's cluster on bit-packed bonds
+ * (kernel_wolff_bits.cu) instead of labelling 32x8x4 tiles: from 2^19 sites,
+ * and those of one growth region.  Measured on B200, us per sweep, bits against
+ * tiles: 32^3 36.7 / 53.8, 24^3 47.4 / 51.5, 48^3 69.8 / 59.4, 64^3 71.7 /
+ * 70.2, 80^3 91.2 / 86.1, 96^3 93.9 / 111, 100x90x70 88 / 97, 128^3 116 / 164,
+ * 192^3 191 / 437: between, the chain of region closures is longer than the
+ * tiles' union-find. */
+constexpr uint64_t kWolffBitsMinSites = 1u << 19;
+
+inline bool wolff_by_bits(const TaskView& t) {
+    const bool one_region = t.lx <= 32 && t.ly <= 32 && t.lz <= 32;
+    return ((uint64_t)t.lx * t.ly * t.lz >= kWolffBitsMinSites || one_region) &&
+           wolff_bits_scratch_bytes(t.lx, t.ly, t.lz) <= 4ull * t.lx * t.ly * t.lz;
+}
 
 /* ---- Wolff: union-find with links from larger to smaller roots ---- */
 
@@ -727,11 +735,8 @@ void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* bin
 
 int launch_wolff(const TaskView& t, uint64_t counter, uint8_t* bonds, uint32_t* parent,
                  uint8_t* cluster_out, cudaStream_t s, float* phi_out, uint32_t seed_site[3], bool record_bonds) {
-    /* Large lattices with sides that are multiples of 32 grow the seed's
-     * cluster on bit-packed bonds (kernel_wolff_bits.cu), in the union-find
-     * array; below kWolffBitsMinSites the tile labelling is faster. */
-    if ((uint64_t)t.lx * t.ly * t.lz >= kWolffBitsMinSites && wolff_bits_supports(t.lx, t.ly, t.lz) &&
-        wolff_bits_scratch_bytes(t.lx, t.ly, t.lz) <= 4ull * t.lx * t.ly * t.lz)
+    /* the bit planes live in the union-find array */
+    if (wolff_by_bits(t))
         return launch_wolff_bits(t, counter, parent, record_bonds ? bonds : nullptr, cluster_out, s, phi_out,
                                  seed_site);
     /* The reflection axis and seed site (src/updates.rs:564-568) come from
