@@ -116,6 +116,28 @@ TaskLayout layout_of(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t n_bins) {
 }  // namespace
 
 constexpr size_t kSmallReadBack = 256; /* bytes */
+/* Lattices up to this size sweep in one CTA even alone (slsf_task_sweep). */
+constexpr uint32_t kOneCtaSweepSites = 16384;
+
+namespace {
+
+/* Threads of the one-CTA kernel for V sites when `n` replicas share the GPU.
+ * With at least three per SM, the fewest that keep its arithmetic pipes busy
+ * (1e10 site-updates/s on B200: L = 8 2.07 / 1.56 / 1.07 on 64 / 128 / 256
+ * threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 512, L = 20 5.13 / 4.72 on 128
+ * / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93 on 512, L = 32 6.67 on 512
+ * and 5.8 on 1024); with fewer, more threads shorten each replica's sweep (us
+ * per sweep of one replica, 64 / 128 / 256 / 512 threads: L = 8 9.8 / 9.0 / 9.3
+ * / 10.4, L = 12 21 / 13.6 / 12.1 / 12.7, L = 16 30 / 17.7 / 14.4 / 14.8, L = 20
+ * 73 / 40 / 29 / 25, L = 24 128 / 67 / 43 / 37; of 296, L = 16 33 / 24 / 22 / 31,
+ * L = 24 131 / 91 / 69 / 75). */
+uint32_t resident_threads(uint64_t v, uint64_t n, uint64_t sms) {
+    if (n <= sms) return v <= 1024 ? 128 : (v <= 4096 ? 256 : 512);
+    if (n <= 2 * sms) return v <= 1024 ? 128 : (v <= 16384 ? 256 : 512);
+    return v <= 1024 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512));
+}
+
+}  // namespace
 
 struct slsf_ctx {
     int device = 0;
@@ -695,6 +717,28 @@ int slsf_task_sweep(slsf_task* t, uint32_t n_sweeps, slsf_sweep_stats* stats) {
     if (!t) return set_error(SLSF_ERR_INVALID, "task is NULL");
     if (int rc = check_sweepable(t)) return rc;
     if (int rc = bind_device(t->ctx)) return rc;
+    /* A small lattice sweeps in one launch of the one-CTA kernel, which
+     * writes the counters to the host's landing area: one sweep at L = 8 takes
+     * 9 us on the GPU against 38 us in six launches, at L = 24 37 against 47; at
+     * L = 32 59 against 37, the whole GPU being faster than one SM. */
+    if (n_sweeps && t->volume <= kOneCtaSweepSites && slsf::resident_supports(t->lx, t->ly, t->lz, t->ctx->device)) {
+        unsigned long long* st = reinterpret_cast<unsigned long long*>(t->ctx->h_small);
+        std::memset(st, 0, sizeof(unsigned long long) * slsf::kStatSlots);
+        TaskView v = t->view();
+        v.n_bins = 0; /* slsf_task_sweep does not measure */
+        v.stats = st;
+        SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->volume, 1, 1), t->ctx->stream));
+        t->ctx->launches += 1;
+        t->metro_sweeps += n_sweeps;
+        t->wolff_done += (uint64_t)n_sweeps * t->wolff_steps;
+        SLSF_CUDA(cudaStreamSynchronize(t->ctx->stream));
+        if (st[slsf::kStatError])
+            return set_error(SLSF_ERR_TIMEOUT, "a bounded device loop hit its iteration limit");
+        if (stats)
+            *stats = slsf_sweep_stats{n_sweeps, st[slsf::kStatAccepted], st[slsf::kStatClusters],
+                                      st[slsf::kStatClusterSites]};
+        return SLSF_OK;
+    }
     if (int rc = zero_stats(t)) return rc;
     for (uint32_t s = 0; s < n_sweeps; ++s) {
         TaskView v = t->view();
@@ -1163,18 +1207,12 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
     }
 }
 
-/* Without a tuned entry: the one-CTA kernel when the replica fits, with 64
- * threads up to 1024 sites, 128 up to 8192, 256 up to 16384, else 512
- * (measured on B200, 1e10 site-updates/s: L = 8 2.07 / 1.56 / 1.07 on 64 / 128
- * / 256 threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 512, L = 20 5.13 / 4.72
- * on 128 / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93 on 512, L = 32
- * 6.67 on 512 and 5.8 on 1024); else the smallest cluster that holds it, 1024
+/* Without a tuned entry: the one-CTA kernel when the replica fits (threads for
+ * a batch that fills the GPU), else the smallest cluster that holds it, 1024
  * threads; else the grid-wide kernels. */
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
-    if (slsf::resident_supports(lx, ly, lz, device)) {
-        const uint64_t v = (uint64_t)lx * ly * lz;
-        return {slsf::kKernelResident, 1, v <= 1024 ? 64u : (v <= 8192 ? 128u : (v <= 16384 ? 256u : 512u))};
-    }
+    if (slsf::resident_supports(lx, ly, lz, device))
+        return {slsf::kKernelResident, 1, resident_threads((uint64_t)lx * ly * lz, ~0ull, 1)};
     if (const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device)) return {slsf::kKernelCluster, c, 1024};
     return {slsf::kKernelGrid, 1, 256};
 }
@@ -1183,6 +1221,15 @@ slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uin
     const auto it = ctx->tune.find(shape_key(lx, ly, lz));
     if (it != ctx->tune.end()) return it->second;
     return default_choice(lx, ly, lz, ctx->device);
+}
+
+/* The default choices of one-CTA tasks fitted to how many of them run together. */
+void fit_to_batch(const slsf_ctx* ctx, slsf_task* const* tasks, std::vector<slsf::KernelChoice>& ch) {
+    uint64_t n = 0;
+    for (const slsf::KernelChoice& c : ch) n += c.kind == slsf::kKernelResident;
+    for (size_t i = 0; i < ch.size(); ++i)
+        if (ch[i].kind == slsf::kKernelResident && !ctx->tune.count(shape_key(tasks[i]->lx, tasks[i]->ly, tasks[i]->lz)))
+            ch[i].threads = resident_threads(tasks[i]->volume, n, (uint64_t)ctx->sm_count);
 }
 
 int ensure_queue_capacity(slsf_ctx* ctx, uint32_t n) {
@@ -1264,6 +1311,7 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
             return set_error(SLSF_ERR_INVALID, "the kernel choice does not hold this lattice");
         if (t->corr_interval && ch[i].kind == slsf::kKernelCluster) return set_error(SLSF_ERR_INVALID, kErrFuse);
     }
+    if (!force) fit_to_batch(ctx, tasks, ch);
     if (int rc = ensure_batch_capacity(ctx, n)) return rc;
     /* Grouped by kernel choice (one persistent launch each; cluster groups
      * first, grid-wide tasks last), largest replicas first within a group so
@@ -1419,6 +1467,7 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
                              "batch sessions hold lattices that fit one thread-block cluster's shared memory");
         if (t->corr_interval && ch[i].kind == slsf::kKernelCluster) return set_error(SLSF_ERR_INVALID, kErrFuse);
     }
+    fit_to_batch(ctx, tasks, ch);
     auto rank = [&](size_t i) {
         const slsf::KernelChoice& c = ch[i];
         const uint64_t fused = tasks[i]->corr_interval ? 1u : 0u;

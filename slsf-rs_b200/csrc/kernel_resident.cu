@@ -803,20 +803,20 @@ template <bool kCorr, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_resident(const TaskView* __restrict__ views, uint32_t n, uint32_t n_sweeps, unsigned int* __restrict__ queue,
                uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, unsigned long long* __restrict__ counters,
-               const ResidentCorr* __restrict__ corr) {
+               const ResidentCorr* __restrict__ corr, TaskView one) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[8 * 32];
     __shared__ double bin_acc[kBinCols];
     __shared__ uint32_t s_item;
     __shared__ uint32_t s_cluster;
     __shared__ uint32_t s_accepted;
-    for (;;) {
+    for (bool first = true;; first = false) {
         __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(queue, 1u);
+        if (threadIdx.x == 0) s_item = queue ? atomicAdd(queue, 1u) : (first ? 0u : n);
         __syncthreads();
         const uint32_t item = s_item;
         if (item >= n) return;
-        TaskView t = views[item];
+        TaskView t = views ? views[item] : one; /* one task by value: no view in device memory, no queue */
         if (counters) { /* a replayed launch: the counters live in their own array */
             t.metro_sweeps = counters[2 * item];
             t.wolff_done = counters[2 * item + 1];
@@ -890,10 +890,14 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         if ((threadIdx.x & 31u) == 0 && accepted) atomicAdd(&s_accepted, accepted);
         __syncthreads();
         store_state(t, g, s);
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && views) {
             atomicAdd(&t.stats[kStatAccepted], (unsigned long long)s_accepted);
             atomicAdd(&t.stats[kStatClusterSites], (unsigned long long)s_cluster);
             atomicAdd(&t.stats[kStatClusters], (unsigned long long)sweeps * t.wolff_steps);
+        } else if (threadIdx.x == 0) { /* the call's counters, to the host (t.stats is pinned memory) */
+            t.stats[kStatAccepted] = s_accepted;
+            t.stats[kStatClusterSites] = s_cluster;
+            t.stats[kStatClusters] = (unsigned long long)sweeps * t.wolff_steps;
         }
     }
 }
@@ -908,6 +912,7 @@ cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_
                               uint32_t threads, unsigned long long* counters, const ResidentCorr* corr,
                               uint32_t corr_doubles) {
     const size_t smem = smem_bytes(max_volume, max_rows, max_lz, corr_doubles);
+    const TaskView none = {};
     cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr, kMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int sms = 0, per_sm = 0;
@@ -918,7 +923,7 @@ cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(sms * per_sm));
     k_resident<kCorr, kMaxThreads><<<grid, threads, smem, s>>>(views_dev, n, n_sweeps, queue, max_volume, max_rows, max_lz,
-                                                  counters, corr);
+                                                  counters, corr, none);
     return cudaGetLastError();
 }
 
@@ -937,6 +942,18 @@ bool resident_supports(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
     if (lx > kMaxRowBits || lx < 4 || lx % 2 || ly < 2 || ly % 2 || lz < 2 || lz % 2) return false;
     const uint64_t v = (uint64_t)lx * ly * lz;
     return smem_bytes((uint32_t)v, ly * lz, lz) <= (size_t)max_dynamic_smem(device);
+}
+
+cudaError_t launch_resident_one(const TaskView& t, uint32_t n_sweeps, uint32_t threads, cudaStream_t s) {
+    const uint32_t volume = t.lx * t.ly * t.lz;
+    const size_t smem = smem_bytes(volume, t.ly * t.lz, t.lz);
+    cudaError_t e = cudaFuncSetAttribute(k_resident<false, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    TaskView v = t;
+    v.sweeps = n_sweeps;
+    k_resident<false, 512><<<1, threads, smem, s>>>(nullptr, 1, n_sweeps, nullptr, volume, t.ly * t.lz, t.lz, nullptr,
+                                                    nullptr, v);
+    return cudaGetLastError();
 }
 
 uint32_t resident_corr_doubles(uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t rz) {
