@@ -58,7 +58,7 @@ class SweepStats(C.Structure):
         return {n: getattr(self, n) for n, _ in self._fields_}
 
 
-KERNEL_KINDS = ("resident", "cluster", "grid")
+KERNEL_KINDS = ("resident", "cluster", "grid", "stream")
 
 
 class KernelChoice(C.Structure):

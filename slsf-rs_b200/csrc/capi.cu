@@ -163,6 +163,8 @@ struct slsf_ctx {
     uint32_t views_cap = 0;
     unsigned int* d_queue = nullptr; /* one counter per kernel group */
     uint32_t queue_cap = 0;
+    void* d_stream = nullptr; /* queue and per-replica state of the stream kernel, for stream_cap replicas */
+    uint32_t stream_cap = 0;
     /* side streams for the kernel groups of a batch, forked from and joined
      * back into `stream` with events, so that groups that do not fill the
      * GPU alone overlap */
@@ -249,6 +251,7 @@ struct slsf_task {
         v.sweeps = 0;
         v.loop_limit = ctx->loop_limit;
         v.jmax = jmax;
+        v.bits = parent;
         v.partials = partials;
         v.result = result;
         v.done = done;
@@ -446,6 +449,7 @@ int slsf_ctx_destroy(slsf_ctx* ctx) {
     for (void* p : dev)
         if (p) cudaFree(p);
     if (ctx->d_corr) cudaFree(ctx->d_corr);
+    if (ctx->d_stream) cudaFree(ctx->d_stream);
     void* host[] = {ctx->h_views, ctx->h_batch_stats, (void*)ctx->h_bin_src, ctx->h_bin_out, ctx->h_corr,
                     ctx->h_rcorr, ctx->h_small};
     for (void* p : host)
@@ -1202,6 +1206,8 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
                    slsf::cluster_feasible(lx, ly, lz, c.cluster, device);
         case slsf::kKernelGrid:
             return true;
+        case slsf::kKernelStream:
+            return c.cluster == 1 && c.threads == 256 && slsf::stream_fits(lx, ly, lz);
         default:
             return false;
     }
@@ -1213,8 +1219,18 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
     if (slsf::resident_supports(lx, ly, lz, device))
         return {slsf::kKernelResident, 1, resident_threads((uint64_t)lx * ly * lz, ~0ull, 1)};
-    if (const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device)) return {slsf::kKernelCluster, c, 1024};
+    const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device);
+    if (c && slsf::stream_fits(lx, ly, lz)) return {slsf::kKernelStream, 1, 256};
+    if (c) return {slsf::kKernelCluster, c, 1024};
     return {slsf::kKernelGrid, 1, 256};
+}
+
+/* A task's choice: the shape's, but tasks that the stream kernel does not take
+ * (couplings too large for the walks' sums, very many Wolff steps) go to a cluster, or the grid-wide kernels where none holds the lattice. */
+slsf::KernelChoice choice_of(const slsf_task* t, slsf::KernelChoice c) {
+    if (c.kind != slsf::kKernelStream || slsf::stream_takes(t->view())) return c;
+    const uint32_t cl = slsf::batched_cluster_size(t->lx, t->ly, t->lz, t->ctx->device);
+    return cl ? slsf::KernelChoice{slsf::kKernelCluster, cl, 1024} : slsf::KernelChoice{slsf::kKernelGrid, 1, 256};
 }
 
 slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uint32_t lz) {
@@ -1230,6 +1246,36 @@ void fit_to_batch(const slsf_ctx* ctx, slsf_task* const* tasks, std::vector<slsf
     for (size_t i = 0; i < ch.size(); ++i)
         if (ch[i].kind == slsf::kKernelResident && !ctx->tune.count(shape_key(tasks[i]->lx, tasks[i]->ly, tasks[i]->lz)))
             ch[i].threads = resident_threads(tasks[i]->volume, n, (uint64_t)ctx->sm_count);
+}
+
+/* Tasks of one group share their launches: those of one kernel choice, with
+ * or without fused correlations.  Groups run in descending rank (cluster first, grid-wide last). */
+uint64_t group_rank(const slsf_task* t, const slsf::KernelChoice& c) {
+    const uint64_t order[4] = {1, 3, 0, 2}; /* resident, cluster, grid, stream */
+    const uint64_t fused = t->corr_interval ? 1u : 0u;
+    return (order[c.kind] << 48) | (fused << 40) | ((uint64_t)c.cluster << 16) | c.threads;
+}
+
+/* Grows the context's scratch of the stream kernel to n replicas. */
+int ensure_stream_scratch(slsf_ctx* ctx, uint32_t n) {
+    if (n == 0 || n <= ctx->stream_cap) return SLSF_OK;
+    if (ctx->d_stream) {
+        SLSF_CUDA(cudaStreamSynchronize(ctx->stream));
+        for (int k = 0; k < kSideStreams; ++k) SLSF_CUDA(cudaStreamSynchronize(ctx->side[k]));
+        cudaFree(ctx->d_stream);
+        ctx->d_stream = nullptr;
+        ctx->stream_cap = 0;
+    }
+    const uint32_t cap = std::max<uint32_t>(64, n);
+    SLSF_CUDA(cudaMalloc(&ctx->d_stream, slsf::stream_scratch_bytes(cap)));
+    ctx->stream_cap = cap;
+    return SLSF_OK;
+}
+
+uint32_t stream_tasks(const std::vector<slsf::KernelChoice>& ch) {
+    uint32_t n = 0;
+    for (const slsf::KernelChoice& c : ch) n += c.kind == slsf::kKernelStream;
+    return n;
 }
 
 int ensure_queue_capacity(slsf_ctx* ctx, uint32_t n) {
@@ -1306,10 +1352,11 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
         slsf_task* t = tasks[i];
         if (!t || t->ctx != ctx) return set_error(SLSF_ERR_INVALID, "task does not belong to this context");
         if (int rc = check_sweepable(t)) return rc;
-        ch[i] = force ? *force : choice_for(ctx, t->lx, t->ly, t->lz);
+        ch[i] = choice_of(t, force ? *force : choice_for(ctx, t->lx, t->ly, t->lz));
         if (!choice_feasible(ch[i], t->lx, t->ly, t->lz, ctx->device))
             return set_error(SLSF_ERR_INVALID, "the kernel choice does not hold this lattice");
-        if (t->corr_interval && ch[i].kind == slsf::kKernelCluster) return set_error(SLSF_ERR_INVALID, kErrFuse);
+        if (t->corr_interval && (ch[i].kind == slsf::kKernelCluster || ch[i].kind == slsf::kKernelStream))
+            return set_error(SLSF_ERR_INVALID, kErrFuse);
     }
     if (!force) fit_to_batch(ctx, tasks, ch);
     if (int rc = ensure_batch_capacity(ctx, n)) return rc;
@@ -1319,9 +1366,7 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
      * slot of the batch stats array. */
     auto rank = [&](size_t i) {
         const slsf::KernelChoice& c = ch[i];
-        const uint32_t k = c.kind == slsf::kKernelCluster ? 2u : (c.kind == slsf::kKernelResident ? 1u : 0u);
-        const uint64_t fused = tasks[i]->corr_interval ? 1u : 0u;
-        return ((uint64_t)k << 48) | (fused << 40) | ((uint64_t)c.cluster << 16) | c.threads;
+        return group_rank(tasks[i], c);
     };
     std::vector<size_t> order(n);
     for (size_t i = 0; i < n; ++i) order[i] = i;
@@ -1334,6 +1379,7 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
     for (size_t k = 0; k < n; ++k)
         if (k == 0 || rank(order[k]) != rank(order[k - 1])) ++n_groups;
     if (int rc = ensure_queue_capacity(ctx, n_groups)) return rc;
+    if (int rc = ensure_stream_scratch(ctx, stream_tasks(ch))) return rc;
     bool any_fused = false;
     for (size_t k = 0; k < n; ++k) {
         TaskView v = tasks[order[k]]->view();
@@ -1376,6 +1422,9 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
         }
         if (c.kind == slsf::kKernelGrid) {
             for (size_t k = lo; k < hi; ++k) run_grid_task(ctx, tasks[order[k]], ctx->h_views[k], st);
+        } else if (c.kind == slsf::kKernelStream) {
+            SLSF_CUDA(slsf::launch_stream(ctx->d_views + lo, ctx->h_views + lo, nullptr, (uint32_t)(hi - lo), ctx->sm_count,
+                                          ctx->d_stream, st, &ctx->launches));
         } else if (c.kind == slsf::kKernelResident) {
             SLSF_CUDA(slsf::launch_resident(ctx->d_views + lo, (uint32_t)(hi - lo), n_sweeps, ctx->d_queue + q,
                                             ctx->device, st, max_vs, max_rows, max_lz, c.threads, nullptr,
@@ -1429,6 +1478,7 @@ struct slsf_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     slsf::ResidentCorr* d_rcorr = nullptr; /* fused correlations, parallel to d_views */
+    void* d_stream = nullptr; /* scratch of the stream kernel */
     unsigned long long* d_acc = nullptr; /* stats summed over the cycles of slsf_batch_step_correlations */
     unsigned long long* h_acc = nullptr; /* pinned */
 };
@@ -1436,6 +1486,7 @@ struct slsf_batch {
 static void batch_free(slsf_batch* b) {
     if (b->d_acc) cudaFree(b->d_acc);
     if (b->d_rcorr) cudaFree(b->d_rcorr);
+    if (b->d_stream) cudaFree(b->d_stream);
     if (b->h_acc) cudaFreeHost(b->h_acc);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -1461,18 +1512,17 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
         if (int rc = check_sweepable(t)) return rc;
         for (size_t j = 0; j < i; ++j)
             if (tasks[j] == t) return set_error(SLSF_ERR_INVALID, "a task appears twice in the session");
-        ch[i] = choice_for(ctx, t->lx, t->ly, t->lz);
+        ch[i] = choice_of(t, choice_for(ctx, t->lx, t->ly, t->lz));
         if (ch[i].kind == slsf::kKernelGrid || !choice_feasible(ch[i], t->lx, t->ly, t->lz, ctx->device))
             return set_error(SLSF_ERR_INVALID,
                              "batch sessions hold lattices that fit one thread-block cluster's shared memory");
-        if (t->corr_interval && ch[i].kind == slsf::kKernelCluster) return set_error(SLSF_ERR_INVALID, kErrFuse);
+        if (t->corr_interval && (ch[i].kind == slsf::kKernelCluster || ch[i].kind == slsf::kKernelStream))
+            return set_error(SLSF_ERR_INVALID, kErrFuse);
     }
     fit_to_batch(ctx, tasks, ch);
     auto rank = [&](size_t i) {
         const slsf::KernelChoice& c = ch[i];
-        const uint64_t fused = tasks[i]->corr_interval ? 1u : 0u;
-        return ((uint64_t)(c.kind == slsf::kKernelCluster ? 2u : 1u) << 48) | (fused << 40) |
-               ((uint64_t)c.cluster << 16) | c.threads;
+        return group_rank(tasks[i], c);
     };
     std::vector<size_t> order(n);
     for (size_t i = 0; i < n; ++i) order[i] = i;
@@ -1493,6 +1543,8 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
     if (e == cudaSuccess) e = cudaMalloc(&b->d_queue, sizeof(unsigned int) * n_groups);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_stats, 8 * slsf::kStatSlots * n);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counters, 16 * n);
+    if (const uint32_t ns = stream_tasks(ch))
+        if (e == cudaSuccess) e = cudaMalloc(&b->d_stream, slsf::stream_scratch_bytes(ns));
     std::vector<unsigned long long> counters(2 * n);
     for (size_t k = 0; k < n; ++k) {
         counters[2 * k] = tasks[order[k]]->metro_sweeps;
@@ -1552,7 +1604,10 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
             ++hi;
         }
         if (e == cudaSuccess) {
-            if (c.kind == slsf::kKernelResident)
+            if (c.kind == slsf::kKernelStream)
+                e = slsf::launch_stream(b->d_views + lo, views.data() + lo, b->d_counters + 2 * lo, (uint32_t)(hi - lo),
+                                        ctx->sm_count, b->d_stream, st, &launches);
+            else if (c.kind == slsf::kKernelResident)
                 e = slsf::launch_resident(b->d_views + lo, (uint32_t)(hi - lo), n_sweeps, b->d_queue + q, ctx->device,
                                           st, max_vs, max_rows, max_lz, c.threads, b->d_counters + 2 * lo,
                                           max_cd ? b->d_rcorr + lo : nullptr, max_cd);
@@ -1703,6 +1758,7 @@ int slsf_autotune(slsf_ctx* ctx, uint32_t lx, uint32_t ly, uint32_t lz, uint32_t
             const slsf::KernelChoice c = {slsf::kKernelCluster, cl, t};
             if (choice_feasible(c, lx, ly, lz, ctx->device)) cand.push_back(c);
         }
+    if (slsf::stream_fits(lx, ly, lz)) cand.push_back({slsf::kKernelStream, 1, 256});
     if (cand.empty()) cand.push_back({slsf::kKernelGrid, 1, 256});
     /* scratch replicas: about 2^25 sites, at most 4096, within the budget */
     const uint64_t v = (uint64_t)lx * ly * lz;

@@ -46,6 +46,7 @@ struct TaskView {
     uint32_t loop_limit;   /* 0, or a lower bound on device loops (slsf_ctx_set_loop_limit) */
     float jmax;            /* largest coupling; infinite if any is not below kJMax */
     unsigned long long* stats;
+    uint32_t* bits;        /* 4 V bytes of scratch: the Wolff bit planes of the stream kernels */
     double* partials;      /* measurement scratch: block sums, totals, block counter */
     double* result;
     unsigned int* done;
@@ -68,11 +69,11 @@ struct ResidentCorr {
  * choice changes neither a task's trajectory nor its bins beyond FP32
  * partial-sum rounding. */
 struct KernelChoice {
-    uint32_t kind;    /* kKernelResident, kKernelCluster or kKernelGrid */
+    uint32_t kind;    /* kKernelResident, kKernelCluster, kKernelGrid or kKernelStream */
     uint32_t cluster; /* CTAs per replica (cluster kernel), else 1 */
     uint32_t threads; /* threads per CTA (batched kernels) */
 };
-constexpr uint32_t kKernelResident = 0, kKernelCluster = 1, kKernelGrid = 2;
+constexpr uint32_t kKernelResident = 0, kKernelCluster = 1, kKernelGrid = 2, kKernelStream = 3;
 
 /* Records `message` as the calling thread's slsf_last_error text and returns
  * `code` (capi.cu). */
@@ -88,8 +89,6 @@ void launch_metro_colour0_measure(const TaskView& t, uint64_t sweep, double* bin
 /* ---- walks over lattices in global memory (kernel_walk.cu) ---- */
 /* L_x a multiple of 4, L_y even, finite couplings, angles 16-byte aligned. */
 bool walk_supports(const TaskView& t);
-/* Planes per thread for n replicas of the shape in one launch. */
-uint32_t walk_seglen(const TaskView& t, uint32_t n);
 /* One colour of sweep `sweep`; with `measure` (colour 0) also the measurement
  * of the state it starts from, into t.result and bin_row (or NULL). */
 void launch_walk_colour(const TaskView& t, uint64_t sweep, uint32_t colour, bool measure, double* bin_row, cudaStream_t s);
@@ -106,6 +105,17 @@ uint64_t wolff_bits_scratch_bytes(uint32_t lx, uint32_t ly, uint32_t lz);
  * the per-site bond bits, cluster_out (or NULL) the cluster mask. */
 int launch_wolff_bits(const TaskView& t, uint64_t counter, void* scratch, uint8_t* bond_bytes, uint8_t* cluster_out,
                       cudaStream_t s, float* phi_out, uint32_t seed_site[3]);
+/* ---- many replicas, state in global memory, persistent (kernel_stream.cu) ---- */
+/* Shapes: rows of up to 64 sites (L_x a multiple of 4), L_y and L_z even, at most 4096 rows. */
+bool stream_fits(uint32_t lx, uint32_t ly, uint32_t lz);
+/* Tasks: finite couplings, at most 1024 Wolff steps per sweep. */
+bool stream_takes(const TaskView& t);
+size_t stream_scratch_bytes(uint32_t n);
+/* Every view's sweeps, measurements included; with `counters` they come from
+ * there and are advanced, as in launch_resident.  `scratch` holds
+ * stream_scratch_bytes(n) of device memory until the launches are done. */
+cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, unsigned long long* counters, uint32_t n, int sms,
+                          void* scratch, cudaStream_t s, uint64_t* launches);
 /* Fused observables: writes 8 FP64 sums (mx, my, cos xyz, sin xyz) to
  * t.result and adds the measurement's kBinCols stream values to bin_row (a
  * task's bin sums row, or NULL). */

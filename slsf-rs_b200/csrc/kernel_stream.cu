@@ -1,0 +1,410 @@
+/*
+ * Many replicas too large for one CTA's shared memory, their state in global
+ * memory (L2 holds about a hundred 64^3 lattices): the sweeps, Wolff updates
+ * and measurements of all of them in one persistent launch.  Same role as
+ * kernel_resident.cu -- the carlo-mc Runner's task-by-task loop over
+ * ThetaModel::sweep + ThetaModel::measure (src/model.rs:379-442,
+ * src/results.rs:200-202) -- for rows of up to 64 sites, L_x a multiple of 4.
+ *
+ * A replica's sweep is a sequence of phases -- colour 0 (with the measurement
+ * of the state it starts from), colour 1, and per Wolff step bond activation,
+ * growth and reflection -- each cut into chunks of one CTA's work (growth is
+ * one chunk).  CTAs take chunks from a queue in order; the CTA that finishes a
+ * phase's last chunk queues the next phase of that replica.  So replicas
+ * advance independently of each other: the growth of one (a latency-bound
+ * chain, 65 to 200 us at 64^3 depending on the cluster) runs beside the sweeps
+ * of the others, which a launch per phase for all replicas cannot do (every
+ * phase would wait for its slowest growth: 300 us per sweep of 32 replicas
+ * against 83 us of other work).  CTAs wait only for chunks that running CTAs
+ * will queue, so no co-residency is needed; every wait is bounded.
+ *
+ * Visibility: a chunk's writes are fenced before its replica's counter is
+ * decremented, the next phase's entries are written after the counter reached
+ * zero, and a CTA fences after it has read its entry, before it reads the
+ * replica.
+ */
+#include <algorithm>
+#include <type_traits>
+
+#include "engine.h"
+#include "walk_global.cuh"
+#include "wolff_global.cuh"
+
+namespace slsf {
+
+namespace {
+
+constexpr uint32_t kStreamThreads = 512; /* one CTA per SM: 128 registers a thread */
+constexpr uint32_t kStreamRows = 8;      /* rows per thread in the growth */
+constexpr uint32_t kFlipQuads = 16;      /* quads per thread of a reflection chunk */
+constexpr uint32_t kRingEntries = 1u << 20;
+constexpr uint32_t kChunkBits = 12;
+constexpr uint32_t kMaxWolffSteps = 1024;
+
+enum Phase : uint32_t { kColour0, kColour1, kBonds, kGrow, kFlip, kMeasureLast, kDone };
+
+/* One replica's place in the launch. */
+struct StreamCtl {
+    uint32_t left; /* chunks of the phase not yet finished */
+    uint32_t phase, sweep, step;
+};
+
+/* Sizes of the chunks of a launch. */
+struct StreamShape {
+    uint32_t seglen; /* planes per thread of the walks */
+    uint32_t run;    /* rows per warp of the bond activation */
+};
+
+__host__ __device__ inline uint32_t chunks_of(const TaskView& t, const StreamShape& sh, uint32_t phase) {
+    switch (phase) {
+        case kColour0:
+        case kColour1:
+        case kMeasureLast: return (walk_units(t, sh.seglen) + kStreamThreads - 1) / kStreamThreads;
+        case kBonds: {
+            const uint32_t warps = ((t.lx + 31) / 32) * (t.lz / 2) * ((t.ly + sh.run - 1) / sh.run);
+            return (warps + kStreamThreads / 32 - 1) / (kStreamThreads / 32);
+        }
+        case kGrow: return 1;
+        case kFlip: return ((t.lx >> 2) * t.ly * t.lz + kStreamThreads * kFlipQuads - 1) / (kStreamThreads * kFlipQuads);
+        default: return 0;
+    }
+}
+
+/* The phase after `c` for sweeps below sw_hi of the launch. */
+__device__ __forceinline__ StreamCtl next_phase(const TaskView& t, const StreamShape& sh, StreamCtl c, uint32_t sw_hi) {
+    bool sweep_done = false;
+    switch (c.phase) {
+        case kColour0: c.phase = kColour1; break;
+        case kColour1:
+            c.step = 0;
+            if (t.wolff_steps) c.phase = kBonds;
+            else sweep_done = true;
+            break;
+        case kBonds: c.phase = kGrow; break;
+        case kGrow: c.phase = kFlip; break;
+        case kFlip:
+            if (++c.step < t.wolff_steps) c.phase = kBonds;
+            else sweep_done = true;
+            break;
+        default: c.phase = kDone; break;
+    }
+    if (sweep_done) {
+        ++c.sweep;
+        if (c.sweep < min(t.sweeps, sw_hi)) c.phase = kColour0;
+        else c.phase = c.sweep == t.sweeps && t.n_bins ? kMeasureLast : kDone;
+    }
+    c.left = chunks_of(t, sh, c.phase);
+    return c;
+}
+
+struct StreamQueue {
+    unsigned long long* ring; /* entry of ticket q: (q + 1) << 32 | replica << kChunkBits | chunk */
+    uint32_t* head;           /* tickets taken */
+    uint32_t* tail;           /* entries queued */
+    uint32_t* abort;          /* a wait ran out */
+};
+
+__device__ __forceinline__ void put_entry(const StreamQueue& q, uint32_t at, uint32_t replica, uint32_t chunk) {
+    *(volatile unsigned long long*)&q.ring[at] = (unsigned long long)(at + 1) << 32 | replica << kChunkBits | chunk;
+}
+
+__device__ __forceinline__ BitPlanes stream_planes(const TaskView& t) {
+    const uint32_t n = ((t.lx + 31u) >> 5) * t.ly * t.lz;
+    return {t.bits, t.bits + n, t.bits + 2 * n, t.bits + 3 * n};
+}
+
+/* Growth of a replica's cluster by the CTA, row words W of up to 32 or 64
+ * sites: row passes as in the one-CTA kernel (kernel_resident.cu), R rows per
+ * thread with their bonds in registers, the cluster words in shared memory,
+ * three steps per block barrier.  At 64^3 about 49 steps of 2,500 cycles, bound
+ * by instruction issue (visits of marked rows only, closures of whole lines by
+ * segments and scans by shuffles were no faster: 129k, 140k and more cycles
+ * against 122k). */
+template <typename W, int R>
+__device__ __forceinline__ bool grow_replica(const TaskView& t, const slsf_u32x4& pick, volatile W* cl) {
+    const uint32_t lx = t.lx, ly = t.ly, lz = t.lz, rows = ly * lz;
+    const BitPlanes planes = stream_planes(t);
+    const W *bx = reinterpret_cast<const W*>(planes.bx), *by = reinterpret_cast<const W*>(planes.by),
+            *bz = reinterpret_cast<const W*>(planes.bz);
+    const uint32_t seed_row = slsf_range(pick.z, ly) + ly * slsf_range(pick.w, lz);
+    W b_yp[R], b_ym[R], b_zp[R], b_zm[R], b_x[R];
+    uint32_t y_nb[R], z_nb[R]; /* the neighbouring rows: below in the low half, above in the high half */
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        const uint32_t r = threadIdx.x + j * kStreamThreads;
+        b_yp[j] = b_ym[j] = b_zp[j] = b_zm[j] = b_x[j] = 0;
+        y_nb[j] = z_nb[j] = 0;
+        if (r < rows) {
+            const uint32_t z = r / ly, y = r - z * ly;
+            const uint32_t ym = y == 0 ? r + ly - 1 : r - 1, yp = y + 1 == ly ? r + 1 - ly : r + 1;
+            const uint32_t zm = z == 0 ? r + rows - ly : r - ly, zp = z + 1 == lz ? r + ly - rows : r + ly;
+            b_yp[j] = by[r];
+            b_ym[j] = by[ym];
+            b_zp[j] = bz[r];
+            b_zm[j] = bz[zm];
+            b_x[j] = bx[r];
+            y_nb[j] = ym | yp << 16;
+            z_nb[j] = zm | zp << 16;
+            cl[r] = r == seed_row ? close_row((W)1 << slsf_range(pick.y, lx), b_x[j], lx) : (W)0;
+        }
+    }
+    __syncthreads();
+    constexpr int kSteps = 3;
+    const uint32_t bound = (t.loop_limit ? min(t.loop_limit, lx * rows) : lx * rows) + 1;
+    bool closed = false;
+    for (uint32_t pass = 0; pass < bound && !closed; ++pass) {
+        int changed = 0;
+#pragma unroll 1
+        for (int step = 0; step < kSteps; ++step) {
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                const uint32_t r = threadIdx.x + j * kStreamThreads;
+                if (r < rows) {
+                    const W in = (cl[y_nb[j] & 0xffffu] & b_ym[j]) | (cl[y_nb[j] >> 16] & b_yp[j]) |
+                                 (cl[z_nb[j] & 0xffffu] & b_zm[j]) | (cl[z_nb[j] >> 16] & b_zp[j]);
+                    const W old = cl[r], c = old | in;
+                    if (c != old) {
+                        cl[r] = close_row(c, b_x[j], lx);
+                        changed = 1;
+                    }
+                }
+            }
+        }
+        closed = !__syncthreads_or(changed);
+    }
+    W* out = reinterpret_cast<W*>(planes.cl);
+    for (uint32_t r = threadIdx.x; r < rows; r += kStreamThreads) out[r] = cl[r];
+    return closed;
+}
+
+/* Adds a per-thread count to stats[slot]. */
+__device__ __forceinline__ void count_into(uint32_t v, unsigned long long* stats, int slot) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(&stats[slot], (unsigned long long)v);
+}
+
+__global__ void k_stream_init(const TaskView* __restrict__ views, StreamCtl* __restrict__ ctl, StreamQueue q, uint32_t n,
+                              StreamShape sh, uint32_t sw_lo, uint32_t sw_hi) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const TaskView t = views[i];
+    if (sw_lo >= min(t.sweeps, sw_hi)) return;
+    const StreamCtl c = {chunks_of(t, sh, kColour0), kColour0, sw_lo, 0};
+    ctl[i] = c;
+    const uint32_t at = atomicAdd(q.tail, c.left);
+    for (uint32_t k = 0; k < c.left; ++k) put_entry(q, at + k, i, k);
+}
+
+__global__ void __launch_bounds__(kStreamThreads, 1)
+    k_stream(const TaskView* __restrict__ views, const unsigned long long* __restrict__ counters, StreamCtl* ctl,
+             StreamQueue q, uint32_t tickets, StreamShape sh, uint32_t sw_hi) {
+    extern __shared__ __align__(8) unsigned char grow_smem[]; /* the growth's cluster words */
+    __shared__ double scratch[8 * 32];
+    __shared__ uint32_t s_entry, s_at;
+    __shared__ StreamCtl s_ctl;
+    __shared__ bool s_last;
+    constexpr uint32_t kNone = 0xffffffffu, kSpin = 1u << 26;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t got = kNone;
+            const uint32_t ticket = atomicAdd(q.head, 1u);
+            if (ticket < tickets) {
+                volatile unsigned long long* e = q.ring + ticket;
+                for (uint32_t spin = 0;; ++spin) {
+                    const unsigned long long v = *e;
+                    if ((uint32_t)(v >> 32) == ticket + 1) {
+                        got = (uint32_t)v;
+                        break;
+                    }
+                    if (*(volatile uint32_t*)q.abort) break;
+                    if (spin == kSpin) {
+                        atomicOr(&views[0].stats[kStatError], kErrQueueLimit);
+                        atomicExch(q.abort, 1u);
+                        break;
+                    }
+                    __nanosleep(64);
+                }
+                __threadfence();
+                if (got != kNone) {
+                    const uint4 c = __ldcg(reinterpret_cast<const uint4*>(&ctl[got >> kChunkBits]));
+                    s_ctl = {c.x, c.y, c.z, c.w};
+                }
+            }
+            s_entry = got;
+        }
+        __syncthreads();
+        if (s_entry == kNone) return;
+        const uint32_t replica = s_entry >> kChunkBits, chunk = s_entry & ((1u << kChunkBits) - 1);
+        const StreamCtl c = s_ctl;
+        const TaskView t = views[replica];
+        const uint64_t sweep = (counters ? counters[2 * replica] : t.metro_sweeps) + c.sweep;
+        const uint64_t counter = (counters ? counters[2 * replica + 1] : t.wolff_done) + (uint64_t)c.sweep * t.wolff_steps + c.step;
+        /* bin row of the state that colour 0 starts from, or of the last state */
+        double* bin_row = nullptr;
+        if ((c.phase == kColour0 && c.sweep > 0) || c.phase == kMeasureLast) bin_row = bin_row_of(t, sweep);
+        if (c.phase == kColour1 || (c.phase == kColour0 && !bin_row)) {
+            count_into(walk_colour<false>(t, sweep, c.phase == kColour1, sh.seglen, chunk * kStreamThreads + threadIdx.x, nullptr),
+                       t.stats, kStatAccepted);
+        } else if (c.phase == kColour0 || c.phase == kMeasureLast) {
+            if (bin_row) {
+                Sum2 sum[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, sh.seglen, k));
+                const uint32_t unit = chunk * kStreamThreads + threadIdx.x;
+                if (c.phase == kColour0)
+                    count_into(walk_colour<true>(t, sweep, 0, sh.seglen, unit, sum), t.stats, kStatAccepted);
+                else
+                    walk_measure(t, sh.seglen, unit, sum);
+                double acc[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, sh.seglen, k));
+                block_sum<8>(acc, scratch);
+                if (threadIdx.x == 0)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) t.partials[chunk * 8 + k] = acc[k];
+            }
+        } else {
+            const slsf_u32x4 pick = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_PICK, 0, 0);
+            const float phi = slsf_angle_from_word(pick.x);
+            if (c.phase == kBonds) {
+                bond_run(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, __fmul_rn(-2.0f, t.beta), phi, t.seed, counter, stream_planes(t),
+                         sh.run, (chunk * kStreamThreads + threadIdx.x) >> 5, nullptr);
+            } else if (c.phase == kGrow) {
+                const bool closed = t.lx <= 32 ? grow_replica<uint32_t, kStreamRows>(t, pick, reinterpret_cast<uint32_t*>(grow_smem))
+                                               : grow_replica<uint64_t, kStreamRows>(t, pick, reinterpret_cast<uint64_t*>(grow_smem));
+                if (threadIdx.x == 0) {
+                    if (!closed) atomicOr(&t.stats[kStatError], kErrGrowthLimit);
+                    atomicAdd(&t.stats[kStatClusters], 1ull);
+                }
+            } else {
+                const slsf_fastdiv quads = slsf_fastdiv_make(t.lx >> 2);
+                const uint32_t* cl = stream_planes(t).cl;
+                uint32_t members = 0;
+                for (uint32_t j = 0; j < kFlipQuads; ++j)
+                    members += flip_quad(t.theta, t.lx, t.ly * t.lz, (chunk * kFlipQuads + j) * kStreamThreads + threadIdx.x,
+                                         quads, cl, phi, nullptr, true);
+                count_into(members, t.stats, kStatClusterSites);
+            }
+        }
+        /* the chunk's writes, then its count; the last chunk of the phase queues the next phase */
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicSub(&ctl[replica].left, 1u) == 1u;
+        __syncthreads();
+        if (!s_last) continue;
+        __threadfence();
+        if (bin_row) { /* the chunks' sums in chunk order */
+            if (threadIdx.x < 8) {
+                double a = 0.0;
+                for (uint32_t k = 0; k < chunks_of(t, sh, c.phase); ++k) a += __ldcg(&t.partials[k * 8 + threadIdx.x]);
+                scratch[threadIdx.x] = a;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const double tot[8] = {scratch[0], scratch[1], scratch[2], scratch[3],
+                                       scratch[4], scratch[5], scratch[6], scratch[7]};
+                add_to_bin(t, tot, bin_row);
+            }
+        }
+        const StreamCtl nx = next_phase(t, sh, c, sw_hi);
+        if (nx.phase == kDone) continue;
+        if (threadIdx.x == 0) {
+            __stcg(reinterpret_cast<uint4*>(&ctl[replica]), make_uint4(nx.left, nx.phase, nx.sweep, nx.step));
+            __threadfence();
+            s_at = atomicAdd(q.tail, nx.left);
+        }
+        __syncthreads();
+        __threadfence();
+        for (uint32_t k = threadIdx.x; k < nx.left; k += kStreamThreads) put_entry(q, s_at + k, replica, k);
+    }
+}
+
+/* Advances the counters of a replayed launch. */
+__global__ void k_stream_advance(const TaskView* __restrict__ views, unsigned long long* __restrict__ counters, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    counters[2 * i] += views[i].sweeps;
+    counters[2 * i + 1] += (uint64_t)views[i].sweeps * views[i].wolff_steps;
+}
+
+uint64_t items_per_sweep(const TaskView& t, const StreamShape& sh) {
+    return 2ull * chunks_of(t, sh, kColour0) +
+           (uint64_t)t.wolff_steps * (chunks_of(t, sh, kBonds) + 1 + chunks_of(t, sh, kFlip));
+}
+
+}  // namespace
+
+bool stream_fits(uint32_t lx, uint32_t ly, uint32_t lz) {
+    /* patches of four sites by two rows, plane pairs, one or two words per row, the growth's rows and 16-bit row numbers;
+     * the chunk numbers; the bit planes in 4 V bytes */
+    return lx >= 4 && lx <= 64 && lx % 4 == 0 && ly >= 2 && ly % 2 == 0 && lz >= 2 && lz % 2 == 0 &&
+           (uint64_t)ly * lz <= (uint64_t)kStreamThreads * kStreamRows;
+}
+
+bool stream_takes(const TaskView& t) { return walk_supports(t) && t.wolff_steps <= kMaxWolffSteps; }
+
+size_t stream_scratch_bytes(uint32_t n) { return 256 + sizeof(StreamCtl) * (size_t)n + 8ull * kRingEntries; }
+
+cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, unsigned long long* counters, uint32_t n, int sms,
+                          void* scratch, cudaStream_t s, uint64_t* launches) {
+    unsigned char* p = static_cast<unsigned char*>(scratch);
+    StreamQueue q;
+    q.head = reinterpret_cast<uint32_t*>(p);
+    q.tail = q.head + 1;
+    q.abort = q.head + 2;
+    q.ring = reinterpret_cast<unsigned long long*>(p + 256);
+    StreamCtl* ctl = reinterpret_cast<StreamCtl*>(p + 256 + 8ull * kRingEntries);
+    /* chunk sizes: the longest walks and runs that still give every SM one and a half chunks */
+    StreamShape sh = {32, 32};
+    auto total = [&](uint32_t phase) {
+        uint64_t c = 0;
+        for (uint32_t i = 0; i < n && c < 2ull * sms; ++i) c += chunks_of(host_views[i], sh, phase);
+        return c;
+    };
+    while (sh.seglen > 4 && 2 * total(kColour0) < 3ull * sms) sh.seglen >>= 1;
+    while (sh.run > 8 && 2 * total(kBonds) < 3ull * sms) sh.run >>= 1;
+    uint64_t most = 1;
+    uint32_t rows = 0, sweeps = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        most = std::max(most, items_per_sweep(host_views[i], sh) + chunks_of(host_views[i], sh, kMeasureLast));
+        rows = std::max(rows, host_views[i].ly * host_views[i].lz * (host_views[i].lx > 32 ? 2u : 1u));
+        sweeps = std::max(sweeps, host_views[i].sweeps);
+    }
+    cudaError_t e = cudaFuncSetAttribute(k_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * rows));
+    /* every launch's entries fit the ring: pieces of replicas, and of sweeps */
+    const uint32_t piece = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(n, 1u << (32 - kChunkBits)), kRingEntries / most);
+    for (uint32_t lo = 0; lo < n && e == cudaSuccess; lo += piece) {
+        const uint32_t m = std::min(piece, n - lo);
+        const TaskView* h = host_views + lo;
+        unsigned long long* c = counters ? counters + 2 * lo : nullptr;
+        const uint32_t span = (uint32_t)std::max<uint64_t>(1, kRingEntries / (most * m) > 1 ? kRingEntries / (most * m) - 1 : 1);
+        for (uint32_t sw = 0; sw < sweeps && e == cudaSuccess; sw += span) {
+            const uint32_t hi = std::min(sweeps, sw + span);
+            uint64_t tickets = 0, wide = 0;
+            for (uint32_t i = 0; i < m; ++i) {
+                if (sw >= h[i].sweeps) continue;
+                const uint32_t end = std::min(hi, h[i].sweeps);
+                tickets += (end - sw) * items_per_sweep(h[i], sh);
+                if (end == h[i].sweeps && h[i].n_bins) tickets += chunks_of(h[i], sh, kMeasureLast);
+                wide += std::max(chunks_of(h[i], sh, kColour0), chunks_of(h[i], sh, kBonds));
+            }
+            if (tickets == 0) continue;
+            if (e == cudaSuccess) e = cudaMemsetAsync(scratch, 0, 256 + 8 * tickets, s);
+            if (e != cudaSuccess) break;
+            k_stream_init<<<(m + 127) / 128, 128, 0, s>>>(views + lo, ctl + lo, q, m, sh, sw, hi);
+            k_stream<<<(uint32_t)std::min<uint64_t>(wide, (uint64_t)sms), kStreamThreads, 4 * rows, s>>>(
+                views + lo, c, ctl + lo, q, (uint32_t)tickets, sh, hi);
+            *launches += 2;
+            e = cudaGetLastError();
+        }
+        if (c && e == cudaSuccess) {
+            k_stream_advance<<<(m + 127) / 128, 128, 0, s>>>(views + lo, c, m);
+            *launches += 1;
+            e = cudaGetLastError();
+        }
+    }
+    return e;
+}
+
+}  // namespace slsf

@@ -41,6 +41,7 @@
 #include "bitgrow.cuh"
 #include "engine.h"
 #include "fastdiv.h"
+#include "wolff_global.cuh"
 #include "xy_device.cuh"
 
 namespace slsf {
@@ -96,116 +97,76 @@ struct WolffBits {
 
 __host__ __device__ inline uint64_t round256(uint64_t b) { return (b + 255) & ~255ull; }
 
-/* Bond activation.  A warp owns word w (lane = bit = x - 32 w; lanes past the
- * row keep no bits) of the plane pair z, z + 1 for a run of up to 32 rows and
- * walks it along y, so the projections of the +y row are the next row's own
- * and plane z's +z partner is plane z + 1's site: three sincos for its two
- * sites, whose arithmetic is packed and whose Philox blocks share a key
- * schedule.  (The earlier walk of one plane took 186 instructions per site and
- * 133 us at L = 256.)  Lane j keeps the words of the run's row j and writes
- * them at its end.  With an odd L_z the last pair's second plane is plane 0,
- * computed and not kept.  The seed's region is queued. */
+__host__ __device__ inline uint64_t bit_words(uint32_t lx, uint32_t ly, uint32_t lz) {
+    return (uint64_t)((lx + 31) / 32) * ly * lz;
+}
+
+__host__ __device__ inline uint64_t bit_regions(uint32_t lx, uint32_t ly, uint32_t lz) {
+    return (uint64_t)((lx + 31) / 32) * ((ly + kRegion - 1) / kRegion) * ((lz + kRegion - 1) / kRegion);
+}
+
+__host__ __device__ inline uint64_t pow2_at_least(uint64_t n) {
+    uint64_t p = 1;
+    while (p < n) p <<= 1;
+    return p;
+}
+
+__host__ __device__ inline uint64_t control_bytes(uint64_t regions) {
+    return round256(4 * regions) + round256(4 * pow2_at_least(2 * regions + 2)) + 256;
+}
+
+/* The scratch of one update: bit planes, then the control words (queued, ring, ctl; zero at its start). */
+__host__ __device__ inline WolffBits carve_bits(void* scratch, uint32_t lx, uint32_t ly, uint32_t lz) {
+    const uint64_t plane = round256(4 * bit_words(lx, ly, lz)) / 4;
+    uint32_t* p = static_cast<uint32_t*>(scratch);
+    WolffBits wb;
+    wb.bx = p;
+    wb.by = p + plane;
+    wb.bz = p + 2 * plane;
+    wb.cl = p + 3 * plane;
+    wb.regions = (uint32_t)bit_regions(lx, ly, lz);
+    wb.cap = (uint32_t)pow2_at_least(2ull * wb.regions + 2);
+    wb.queued = p + 4 * plane;
+    wb.ring = wb.queued + round256(4ull * wb.regions) / 4;
+    wb.ctl = wb.ring + round256(4ull * wb.cap) / 4;
+    return wb;
+}
+
+
+/* Makes the seed's region the first queue entry (the control words are zero). */
+__device__ __forceinline__ void queue_seed(const WolffBits& wb, uint32_t lx, uint32_t ly, uint32_t lz, uint32_t x, uint32_t y,
+                                           uint32_t z) {
+    const uint32_t words = (lx + 31u) >> 5;
+    const uint32_t r = (x >> 5) + words * ((y / kRegion) + ((ly + kRegion - 1) / kRegion) * (z / kRegion));
+    wb.queued[r] = 1;
+    wb.ring[0] = r + 1;
+    wb.ctl[1] = 1; /* tail */
+    wb.ctl[2] = 1; /* pending */
+    wb.ctl[4] = x + lx * (y + ly * z) + 1; /* the seed's bit enters its region like a face bit */
+}
+
 __global__ void __launch_bounds__(kBondThreads)
     k_wb_bonds(const float* __restrict__ theta, const float* __restrict__ jxy, const float* __restrict__ jz,
                uint32_t lx, uint32_t ly, uint32_t lz, float minus_two_beta, float phi, uint64_t seed,
                uint64_t counter, WolffBits wb, uint32_t seed_idx, uint32_t run, uint8_t* __restrict__ bond_bytes) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t words = (lx + 31u) >> 5, nrun = (ly + run - 1) / run;
-    const uint32_t w = wid % words, rest = wid / words;
-    const uint32_t z = 2u * (rest / nrun), y_lo = (rest % nrun) * run;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        /* the seed's region is the first queue entry (the scratch was zeroed) */
-        const uint32_t sx = seed_idx % lx, srow = seed_idx / lx, sy = srow % ly, sz = srow / ly;
-        const uint32_t r = (sx >> 5) + words * ((sy / kRegion) + ((ly + kRegion - 1) / kRegion) * (sz / kRegion));
-        wb.queued[r] = 1;
-        wb.ring[0] = r + 1;
-        wb.ctl[1] = 1; /* tail */
-        wb.ctl[2] = 1; /* pending */
-        wb.ctl[4] = seed_idx + 1; /* the seed's bit enters its region like a face bit */
+        const uint32_t row = seed_idx / lx;
+        queue_seed(wb, lx, ly, lz, seed_idx - row * lx, row % ly, row / ly);
     }
-    if (z >= lz) return; /* whole warps */
-    float sphi, cphi;
-    __sincosf(phi, &sphi, &cphi);
-    const float2 cphi2 = make_float2(cphi, cphi), sphi2 = make_float2(sphi, sphi);
-    auto proj2 = [&](float a, float b) {
-        float2 sn, cn;
-        __sincosf(a, &sn.x, &cn.x);
-        __sincosf(b, &sn.y, &cn.y);
-        return __ffma2_rn(sn, sphi2, __fmul2_rn(cn, cphi2));
-    };
-    const uint32_t nv = min(32u, lx - 32u * w), rows = min(run, ly - y_lo);
-    const uint32_t x = 32u * w + min(lane, nv - 1), xn = 32u * w + nv == lx ? 0u : 32u * w + 32u;
-    const bool pair = z + 1 < lz;
-    const uint32_t plane = lx * ly, z1 = pair ? z + 1 : 0u, z2 = z1 + 1 == lz ? 0u : z1 + 1;
-    const float *p0 = theta + (size_t)z * plane, *p1 = theta + (size_t)z1 * plane, *p2 = theta + (size_t)z2 * plane;
-    const float2 jx = make_float2(jxy[z], jxy[z1]), jzz = make_float2(jz[z], jz[z1]);
-    const float2 m2b2 = make_float2(minus_two_beta, minus_two_beta);
-    auto yrow = [&](uint32_t y) { return y + 1 == ly ? 0u : y + 1; };
-    uint32_t o = y_lo * lx + x;
-    float2 r = proj2(p0[o], p1[o]);
-    /* lane j: the projections of the site after the word in row y_lo + j, the +x partner of the word's last site there */
-    const uint32_t on = (y_lo + min(lane, rows - 1)) * lx + xn;
-    const float2 r_next = proj2(p0[on], p1[on]);
-    /* the angles of the next row's loads, one row ahead */
-    uint32_t oy = yrow(y_lo) * lx + x;
-    float t0 = p0[oy], t1 = p1[oy], t2 = p2[o];
-    uint32_t k[6] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t j = 0; j < rows; ++j) {
-        const float a0 = t0, a1 = t1, a2 = t2;
-        if (j + 1 < rows) {
-            const uint32_t on2 = yrow(y_lo + j + 1) * lx + x;
-            t0 = p0[on2];
-            t1 = p1[on2];
-            t2 = p2[oy];
-            oy = on2;
-        }
-        const float2 ry = proj2(a0, a1);
-        float sn, cn;
-        __sincosf(a2, &sn, &cn);
-        const float2 rz = make_float2(r.y, wolff_projection(cn, sn, cphi, sphi));
-        float2 rx = make_float2(__shfl_down_sync(0xffffffffu, r.x, 1), __shfl_down_sync(0xffffffffu, r.y, 1));
-        const float ex = __shfl_sync(0xffffffffu, r_next.x, j), ey = __shfl_sync(0xffffffffu, r_next.y, j);
-        if (lane + 1 == nv) rx = make_float2(ex, ey);
-        const slsf_u32x4 b0 = slsf_stream(seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, z * plane + o);
-        const slsf_u32x4 b1 = slsf_stream(seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, z1 * plane + o);
-        const float2 jr = __fmul2_rn(jx, r);
-        uint32_t v[6];
-        wolff_bond_words(__fmul2_rn(jr, rx), m2b2, b0.x, b1.x, v[0], v[3]);
-        wolff_bond_words(__fmul2_rn(jr, ry), m2b2, b0.y, b1.y, v[1], v[4]);
-        wolff_bond_words(__fmul2_rn(__fmul2_rn(jzz, r), rz), m2b2, b0.z, b1.z, v[2], v[5]);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) k[q] = lane == j ? v[q] : k[q];
-        if (bond_bytes && lane < nv) {
-            auto bits = [&](int q) {
-                return (uint8_t)((v[q] >> lane & 1u) | (v[q + 1] >> lane & 1u) << 1 | (v[q + 2] >> lane & 1u) << 2);
-            };
-            bond_bytes[(size_t)z * plane + o] = bits(0);
-            if (pair) bond_bytes[(size_t)z1 * plane + o] = bits(3);
-        }
-        r = ry;
-        o += lx;
-    }
-    if (lane < rows) {
-        const uint32_t m = 0xffffffffu >> (32u - nv);
-        const uint32_t i = w + words * (y_lo + lane + ly * z), i1 = i + words * ly;
-        wb.bx[i] = k[0] & m;
-        wb.by[i] = k[1] & m;
-        wb.bz[i] = k[2] & m;
-        wb.cl[i] = 0u;
-        if (pair) {
-            wb.bx[i1] = k[3] & m;
-            wb.by[i1] = k[4] & m;
-            wb.bz[i1] = k[5] & m;
-            wb.cl[i1] = 0u;
-        }
-    }
+    const BitPlanes planes = {wb.bx, wb.by, wb.bz, wb.cl};
+    bond_run(theta, jxy, jz, lx, ly, lz, minus_two_beta, phi, seed, counter, planes, run,
+             (blockIdx.x * blockDim.x + threadIdx.x) >> 5, bond_bytes);
 }
 
 struct GrowGeo {
     uint32_t lx, ly, lz, words, ry_n, rz_n;
     bool px, py, pz; /* the region spans the whole period along x (one-word rows), y (32 rows), z (32 planes) */
 };
+
+__host__ __device__ inline GrowGeo grow_geo(uint32_t lx, uint32_t ly, uint32_t lz) {
+    return {lx, ly, lz, (lx + 31) / 32, (ly + kRegion - 1) / kRegion, (lz + kRegion - 1) / kRegion,
+            lx <= 32, ly == kRegion, lz == kRegion};
+}
 
 /* Claims region r for processing unless it is claimed already (queued or
  * kept): the first neighbour a CTA claims it keeps in *keep and processes
@@ -359,8 +320,9 @@ __device__ bool grow_region(const WolffBits& wb, const GrowGeo& g, uint32_t r, u
     return ok;
 }
 
-__global__ void __launch_bounds__(kGrowThreads, 1)
-    k_wb_grow(WolffBits wb, GrowGeo g, uint32_t max_items, unsigned long long* __restrict__ stats) {
+/* Takes regions until nothing is queued or in flight. */
+__device__ __forceinline__ void grow_regions(const WolffBits& wb, const GrowGeo& g, uint32_t max_items,
+                                             unsigned long long* __restrict__ stats) {
     __shared__ uint32_t C[kRegion][kRegion + 1];
     __shared__ uint32_t BY[kRegion][kRegion + 1];
     __shared__ uint32_t BZ[kRegion][kRegion + 1];
@@ -437,65 +399,33 @@ __global__ void __launch_bounds__(kGrowThreads, 1)
     }
 }
 
-/* Reflect the cluster's sites, count them; optional byte mask.  A thread
- * takes up to four consecutive sites of a row (one 16-byte access when L_x is
- * a multiple of 4 and the angles are aligned). */
-__global__ void __launch_bounds__(kFlipThreads)
-    k_wb_flip(float* __restrict__ theta, uint32_t lx, uint32_t rows, slsf_fastdiv quads, const uint32_t* __restrict__ cl,
-              float phi, unsigned long long* __restrict__ stats, uint8_t* __restrict__ cluster_out, bool wide) {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t n = 0;
-    if (q < quads.d * rows) {
-        const uint32_t row = slsf_fastdiv_div(q, quads), x = 4u * (q - row * quads.d), sites = min(4u, lx - x);
-        const uint32_t m = (__ldcg(&cl[row * ((lx + 31u) >> 5) + (x >> 5)]) >> (x & 31u)) & 0xfu;
-        const size_t i = (size_t)row * lx + x;
-        if (m && wide) {
-            float4 v = *reinterpret_cast<float4*>(theta + i);
-            if (m & 1u) v.x = slsf_reflect(v.x, phi);
-            if (m & 2u) v.y = slsf_reflect(v.y, phi);
-            if (m & 4u) v.z = slsf_reflect(v.z, phi);
-            if (m & 8u) v.w = slsf_reflect(v.w, phi);
-            *reinterpret_cast<float4*>(theta + i) = v;
-        } else if (m) {
-            for (uint32_t k = 0; k < sites; ++k)
-                if (m >> k & 1u) theta[i + k] = slsf_reflect(theta[i + k], phi);
-        }
-        n = __popc(m);
-        if (cluster_out)
-            for (uint32_t k = 0; k < sites; ++k) cluster_out[i + k] = (uint8_t)(m >> k & 1u);
-    }
+__global__ void __launch_bounds__(kGrowThreads, 1)
+    k_wb_grow(WolffBits wb, GrowGeo g, uint32_t max_items, unsigned long long* __restrict__ stats) {
+    grow_regions(wb, g, max_items, stats);
+}
+
+/* Adds a per-thread count to stats[slot] with one global atomic per block. */
+__device__ __forceinline__ void block_count(uint32_t n, unsigned long long* stats, int slot) {
     __shared__ unsigned int s_sum;
     if (threadIdx.x == 0) s_sum = 0;
     __syncthreads();
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) n += __shfl_down_sync(0xffffffffu, n, off);
+    n = __reduce_add_sync(0xffffffffu, n);
     if ((threadIdx.x & 31) == 0 && n) atomicAdd(&s_sum, n);
     __syncthreads();
-    if (threadIdx.x == 0 && s_sum) atomicAdd(&stats[kStatClusterSites], (unsigned long long)s_sum);
+    if (threadIdx.x == 0 && s_sum) atomicAdd(&stats[slot], (unsigned long long)s_sum);
 }
 
-uint32_t pow2_at_least(uint32_t n) {
-    uint32_t p = 1;
-    while (p < n) p <<= 1;
-    return p;
-}
-
-}  // namespace
-
-namespace {
-
-uint64_t bit_words(uint32_t lx, uint32_t ly, uint32_t lz) { return (uint64_t)((lx + 31) / 32) * ly * lz; }
-
-uint64_t bit_regions(uint32_t lx, uint32_t ly, uint32_t lz) {
-    return (uint64_t)((lx + 31) / 32) * ((ly + kRegion - 1) / kRegion) * ((lz + kRegion - 1) / kRegion);
+__global__ void __launch_bounds__(kFlipThreads)
+    k_wb_flip(float* __restrict__ theta, uint32_t lx, uint32_t rows, slsf_fastdiv quads, const uint32_t* __restrict__ cl,
+              float phi, unsigned long long* __restrict__ stats, uint8_t* __restrict__ cluster_out, bool wide) {
+    block_count(flip_quad(theta, lx, rows, blockIdx.x * blockDim.x + threadIdx.x, quads, cl, phi, cluster_out, wide),
+                stats, kStatClusterSites);
 }
 
 }  // namespace
 
 uint64_t wolff_bits_scratch_bytes(uint32_t lx, uint32_t ly, uint32_t lz) {
-    const uint64_t regions = bit_regions(lx, ly, lz);
-    const uint64_t cap = pow2_at_least((uint32_t)std::min<uint64_t>(2 * regions + 2, 1u << 31));
-    return 4 * round256(4 * bit_words(lx, ly, lz)) + round256(4 * regions) + round256(4 * cap) + 256;
+    return 4 * round256(4 * bit_words(lx, ly, lz)) + control_bytes(bit_regions(lx, ly, lz));
 }
 
 int launch_wolff_bits(const TaskView& t, uint64_t counter, void* scratch, uint8_t* bond_bytes, uint8_t* cluster_out,
@@ -507,27 +437,8 @@ int launch_wolff_bits(const TaskView& t, uint64_t counter, void* scratch, uint8_
     const uint32_t x0 = slsf_range(pick.y, t.lx), y0 = slsf_range(pick.z, t.ly), z0 = slsf_range(pick.w, t.lz);
     const uint32_t volume = t.lx * t.ly * t.lz;
     const uint32_t seed_idx = x0 + t.lx * (y0 + t.ly * z0);
-    const uint64_t words = bit_words(t.lx, t.ly, t.lz);
-    WolffBits wb;
-    unsigned char* p = static_cast<unsigned char*>(scratch);
-    wb.bx = reinterpret_cast<uint32_t*>(p);
-    p += round256(4 * words);
-    wb.by = reinterpret_cast<uint32_t*>(p);
-    p += round256(4 * words);
-    wb.bz = reinterpret_cast<uint32_t*>(p);
-    p += round256(4 * words);
-    wb.cl = reinterpret_cast<uint32_t*>(p);
-    p += round256(4 * words);
-    wb.regions = (uint32_t)bit_regions(t.lx, t.ly, t.lz);
-    wb.cap = pow2_at_least(2 * wb.regions + 2);
-    unsigned char* control = p;
-    wb.queued = reinterpret_cast<uint32_t*>(p);
-    p += round256(4ull * wb.regions);
-    wb.ring = reinterpret_cast<uint32_t*>(p);
-    p += round256(4ull * wb.cap);
-    wb.ctl = reinterpret_cast<uint32_t*>(p);
-    p += 256;
-    cudaMemsetAsync(control, 0, (size_t)(p - control), s);
+    const WolffBits wb = carve_bits(scratch, t.lx, t.ly, t.lz);
+    cudaMemsetAsync(wb.queued, 0, control_bytes(wb.regions), s);
     int device = 0, sms = 148;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -539,16 +450,7 @@ int launch_wolff_bits(const TaskView& t, uint64_t counter, void* scratch, uint8_
     const uint32_t bond_blocks = (uint32_t)((warps * 32 + kBondThreads - 1) / kBondThreads);
     k_wb_bonds<<<bond_blocks, kBondThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, -2.0f * t.beta, phi,
                                                     t.seed, counter, wb, seed_idx, run, bond_bytes);
-    GrowGeo g;
-    g.lx = t.lx;
-    g.ly = t.ly;
-    g.lz = t.lz;
-    g.words = (t.lx + 31) / 32;
-    g.ry_n = (t.ly + kRegion - 1) / kRegion;
-    g.rz_n = (t.lz + kRegion - 1) / kRegion;
-    g.px = g.words == 1;
-    g.py = t.ly == kRegion;
-    g.pz = t.lz == kRegion;
+    const GrowGeo g = grow_geo(t.lx, t.ly, t.lz);
     const uint32_t grid = std::min<uint32_t>(wb.regions, (uint32_t)sms);
     /* every region is processed at most once per bit it gains */
     const uint32_t max_items = t.loop_limit ? t.loop_limit : std::max<uint32_t>(64, volume / 32);

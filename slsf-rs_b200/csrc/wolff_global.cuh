@@ -1,0 +1,162 @@
+/*
+ * Wolff update of a lattice in global memory on bit-packed bonds: the bond
+ * activation of a warp's run of rows, the reflection of four sites and the
+ * closure of rows of up to 64 sites, for kernel_wolff_bits.cu (one lattice)
+ * and kernel_stream.cu (many replicas, persistent).  Bit x mod 32 of word
+ * x / 32 of a row is site x; a row takes ceil(L_x / 32) words.
+ */
+#ifndef SLSF_WOLFF_GLOBAL_CUH
+#define SLSF_WOLFF_GLOBAL_CUH
+
+#include "bitgrow.cuh"
+#include "fastdiv.h"
+#include "xy_device.cuh"
+
+namespace slsf {
+
+/* Bond activation.  A warp owns word w (lane = bit = x - 32 w; lanes past the
+ * row keep no bits) of the plane pair z, z + 1 for a run of up to 32 rows and
+ * walks it along y, so the projections of the +y row are the next row's own
+ * and plane z's +z partner is plane z + 1's site: three sincos for its two
+ * sites, whose arithmetic is packed and whose Philox blocks share a key
+ * schedule.  (The earlier walk of one plane took 186 instructions per site and
+ * 133 us at L = 256.)  Lane j keeps the words of the run's row j and writes
+ * them at its end.  With an odd L_z the last pair's second plane is plane 0,
+ * computed and not kept. */
+struct BitPlanes {
+    uint32_t *bx, *by, *bz, *cl; /* [rows][words] */
+};
+
+/* (theta is not __restrict__: the persistent kernel changes the angles between its phases.) */
+__device__ __forceinline__ void bond_run(const float* theta, const float* __restrict__ jxy,
+                                         const float* __restrict__ jz, uint32_t lx, uint32_t ly, uint32_t lz,
+                                         float minus_two_beta, float phi, uint64_t seed, uint64_t counter,
+                                         const BitPlanes& wb, uint32_t run, uint32_t wid,
+                                         uint8_t* __restrict__ bond_bytes) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t words = (lx + 31u) >> 5, nrun = (ly + run - 1) / run;
+    const uint32_t w = wid % words, rest = wid / words;
+    const uint32_t z = 2u * (rest / nrun), y_lo = (rest % nrun) * run;
+    if (z >= lz) return; /* whole warps */
+    float sphi, cphi;
+    __sincosf(phi, &sphi, &cphi);
+    const float2 cphi2 = make_float2(cphi, cphi), sphi2 = make_float2(sphi, sphi);
+    auto proj2 = [&](float a, float b) {
+        float2 sn, cn;
+        __sincosf(a, &sn.x, &cn.x);
+        __sincosf(b, &sn.y, &cn.y);
+        return __ffma2_rn(sn, sphi2, __fmul2_rn(cn, cphi2));
+    };
+    const uint32_t nv = min(32u, lx - 32u * w), rows = min(run, ly - y_lo);
+    const uint32_t x = 32u * w + min(lane, nv - 1), xn = 32u * w + nv == lx ? 0u : 32u * w + 32u;
+    const bool pair = z + 1 < lz;
+    const uint32_t plane = lx * ly, z1 = pair ? z + 1 : 0u, z2 = z1 + 1 == lz ? 0u : z1 + 1;
+    const float *p0 = theta + (size_t)z * plane, *p1 = theta + (size_t)z1 * plane, *p2 = theta + (size_t)z2 * plane;
+    const float2 jx = make_float2(jxy[z], jxy[z1]), jzz = make_float2(jz[z], jz[z1]);
+    const float2 m2b2 = make_float2(minus_two_beta, minus_two_beta);
+    auto yrow = [&](uint32_t y) { return y + 1 == ly ? 0u : y + 1; };
+    uint32_t o = y_lo * lx + x;
+    float2 r = proj2(p0[o], p1[o]);
+    /* lane j: the projections of the site after the word in row y_lo + j, the +x partner of the word's last site there */
+    const uint32_t on = (y_lo + min(lane, rows - 1)) * lx + xn;
+    const float2 r_next = proj2(p0[on], p1[on]);
+    /* the angles of the next row's loads, one row ahead */
+    uint32_t oy = yrow(y_lo) * lx + x;
+    float t0 = p0[oy], t1 = p1[oy], t2 = p2[o];
+    uint32_t k[6] = {0, 0, 0, 0, 0, 0};
+    for (uint32_t j = 0; j < rows; ++j) {
+        const float a0 = t0, a1 = t1, a2 = t2;
+        if (j + 1 < rows) {
+            const uint32_t on2 = yrow(y_lo + j + 1) * lx + x;
+            t0 = p0[on2];
+            t1 = p1[on2];
+            t2 = p2[oy];
+            oy = on2;
+        }
+        const float2 ry = proj2(a0, a1);
+        float sn, cn;
+        __sincosf(a2, &sn, &cn);
+        const float2 rz = make_float2(r.y, wolff_projection(cn, sn, cphi, sphi));
+        float2 rx = make_float2(__shfl_down_sync(0xffffffffu, r.x, 1), __shfl_down_sync(0xffffffffu, r.y, 1));
+        const float ex = __shfl_sync(0xffffffffu, r_next.x, j), ey = __shfl_sync(0xffffffffu, r_next.y, j);
+        if (lane + 1 == nv) rx = make_float2(ex, ey);
+        const slsf_u32x4 b0 = slsf_stream(seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, z * plane + o);
+        const slsf_u32x4 b1 = slsf_stream(seed, counter, SLSF_PURPOSE_WOLFF_BOND, 0, z1 * plane + o);
+        const float2 jr = __fmul2_rn(jx, r);
+        uint32_t v[6];
+        wolff_bond_words(__fmul2_rn(jr, rx), m2b2, b0.x, b1.x, v[0], v[3]);
+        wolff_bond_words(__fmul2_rn(jr, ry), m2b2, b0.y, b1.y, v[1], v[4]);
+        wolff_bond_words(__fmul2_rn(__fmul2_rn(jzz, r), rz), m2b2, b0.z, b1.z, v[2], v[5]);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) k[q] = lane == j ? v[q] : k[q];
+        if (bond_bytes && lane < nv) {
+            auto bits = [&](int q) {
+                return (uint8_t)((v[q] >> lane & 1u) | (v[q + 1] >> lane & 1u) << 1 | (v[q + 2] >> lane & 1u) << 2);
+            };
+            bond_bytes[(size_t)z * plane + o] = bits(0);
+            if (pair) bond_bytes[(size_t)z1 * plane + o] = bits(3);
+        }
+        r = ry;
+        o += lx;
+    }
+    if (lane < rows) {
+        const uint32_t m = 0xffffffffu >> (32u - nv);
+        const uint32_t i = w + words * (y_lo + lane + ly * z), i1 = i + words * ly;
+        wb.bx[i] = k[0] & m;
+        wb.by[i] = k[1] & m;
+        wb.bz[i] = k[2] & m;
+        wb.cl[i] = 0u;
+        if (pair) {
+            wb.bx[i1] = k[3] & m;
+            wb.by[i1] = k[4] & m;
+            wb.bz[i1] = k[5] & m;
+            wb.cl[i1] = 0u;
+        }
+    }
+}
+
+/* Reflects the cluster's sites among four consecutive ones of a row (quad q of
+ * the lattice; one 16-byte access when L_x is a multiple of 4 and the angles
+ * are aligned: `wide`), with an optional byte mask; returns their number. */
+__device__ __forceinline__ uint32_t flip_quad(float* theta, uint32_t lx, uint32_t rows, uint32_t q,
+                                              const slsf_fastdiv& quads, const uint32_t* cl, float phi,
+                                              uint8_t* __restrict__ cluster_out, bool wide) {
+    if (q >= quads.d * rows) return 0;
+    const uint32_t row = slsf_fastdiv_div(q, quads), x = 4u * (q - row * quads.d), sites = min(4u, lx - x);
+    const uint32_t m = (__ldcg(&cl[row * ((lx + 31u) >> 5) + (x >> 5)]) >> (x & 31u)) & 0xfu;
+    const size_t i = (size_t)row * lx + x;
+    if (m && wide) {
+        float4 v = *reinterpret_cast<float4*>(theta + i);
+        if (m & 1u) v.x = slsf_reflect(v.x, phi);
+        if (m & 2u) v.y = slsf_reflect(v.y, phi);
+        if (m & 4u) v.z = slsf_reflect(v.z, phi);
+        if (m & 8u) v.w = slsf_reflect(v.w, phi);
+        *reinterpret_cast<float4*>(theta + i) = v;
+    } else if (m) {
+        for (uint32_t k = 0; k < sites; ++k)
+            if (m >> k & 1u) theta[i + k] = slsf_reflect(theta[i + k], phi);
+    }
+    if (cluster_out)
+        for (uint32_t k = 0; k < sites; ++k) cluster_out[i + k] = (uint8_t)(m >> k & 1u);
+    return __popc(m);
+}
+
+/* Closure of a periodic row of up to 64 sites along x (close_word). */
+__device__ __forceinline__ uint64_t carry_up64(uint64_t c, uint64_t b, uint32_t lx) {
+    uint64_t s = b + (c & b);
+    c |= lx == 64 ? (uint64_t)(s < b) : s >> lx;
+    s = b + (c & b);
+    return (s ^ b) | c;
+}
+
+__device__ __forceinline__ uint64_t close_row(uint64_t c, uint64_t b, uint32_t lx) {
+    const uint64_t mask = ~0ull >> (64 - lx), bl = ((b << 1) | (b >> (lx - 1))) & mask;
+    const uint32_t sh = 64 - lx;
+    return (carry_up64(c, b, lx) | (__brevll(carry_up64(__brevll(c) >> sh, __brevll(bl) >> sh, lx)) >> sh)) & mask;
+}
+
+__device__ __forceinline__ uint32_t close_row(uint32_t c, uint32_t b, uint32_t lx) { return close_word(c, b, lx, true); }
+
+}  // namespace slsf
+
+#endif /* SLSF_WOLFF_GLOBAL_CUH */

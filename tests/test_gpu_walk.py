@@ -45,3 +45,37 @@ def test_batched_walk_equals_one_task(slsf, ctx, dims, j, threads):
     v = float(np.prod(dims))
     scale = np.array([3 * j, 1, v * j, v * j, v * j, v * j, v * j, v * j]) * 1.3 + 1e-30
     assert np.all(np.abs(got - np.array(rows)) <= 2.0 ** -36 * scale), (got, rows)
+
+
+@pytest.mark.parametrize("dims", [(12, 6, 20), (12, 34, 6), (32, 32, 34), (36, 40, 44), (40, 6, 10), (48, 48, 48), (64, 64, 64),
+                                  (64, 2, 8), (60, 128, 32)])
+def test_stream_kernels_equal_one_task(slsf, ctx, dims):
+    """The stream kernels (one launch per phase for many replicas, in one and in two parts) give every replica the
+    one-task trajectory and measurements, also through a session whose replays continue the counters."""
+    jz = np.linspace(0.5, 1.5, dims[2])
+    make = lambda i: slsf.Task(ctx, dims, np.full(dims[2], 1.2), jz, 1.1 + 0.1 * i, wolff_steps=1 + i % 2, seed=21 + i,
+                               thermalization=1, binsize=1, n_bins=6)
+    batch, alone = [make(i) for i in range(3)], [make(i) for i in range(3)]
+    for t in batch + alone:
+        t.init_random()
+    ctx.tune_set(dims, "stream", 1, 256)
+    stats = [ctx.batch_run(batch[:1], 2)[0]] + ctx.batch_run(batch[1:], 2)
+    with ctx.session(batch, 2) as s:
+        for _ in range(2):
+            for total, more in zip(stats, s.step()):
+                for k in total:
+                    total[k] += more[k]
+    for t, st, u in zip(batch, stats, alone):
+        rows, want = [], {k: 0 for k in st}
+        for n in range(6):
+            for k, v in u.sweep(1).items():
+                want[k] += v
+            o = u.measure()
+            if n > 0:
+                rows.append([o[k] for k in ("energy", "magnetization_squared", "cos_x", "cos_y", "cos_z", "sin_x", "sin_y",
+                                            "sin_z")])
+        assert np.array_equal(t.theta.view(np.uint32), u.theta.view(np.uint32))
+        assert st == want
+        got = t.bins()[0][:5, [0, 2, 3, 4, 5, 6, 7, 8]]
+        v = float(np.prod(dims))
+        assert np.all(np.abs(got - np.array(rows)) <= 2.0 ** -36 * np.array([3, 1, v, v, v, v, v, v]) * 1.6)
