@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
             const slsf_u32x4 pick = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_PICK, 0, 0);
             const float phi = slsf_angle_from_word(pick.x);
             if (c.phase == kBonds) {
-                bond_run(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, __fmul_rn(-2.0f, t.beta), phi, t.seed, counter, stream_planes(t),
+                bond_run<2>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, __fmul_rn(-2.0f, t.beta), phi, t.seed, counter, stream_planes(t),
                          sh.run, (chunk * kStreamThreads + threadIdx.x) >> 5, nullptr);
             } else if (c.phase == kGrow) {
                 const bool closed = t.lx <= 32 ? grow_replica<uint32_t, kStreamRows>(t, pick, reinterpret_cast<uint32_t*>(grow_smem))
@@ -281,19 +281,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
                 const slsf_fastdiv quads = slsf_fastdiv_make(t.lx >> 2);
                 const uint32_t* cl = stream_planes(t).cl;
                 uint32_t members = 0;
-                for (uint32_t j = 0; j < kFlipQuads; ++j)
-                    members += flip_quad(t.theta, t.lx, t.ly * t.lz, (chunk * kFlipQuads + j) * kStreamThreads + threadIdx.x,
-                                         quads, cl, phi, nullptr, true);
+                for (uint32_t j = 0; j < kFlipQuads; j += 4)
+                    members += flip_quads<4>(t.theta, t.lx, t.ly * t.lz, (chunk * kFlipQuads + j) * kStreamThreads + threadIdx.x,
+                                             kStreamThreads, quads, cl, phi, nullptr, true);
                 count_into(members, t.stats, kStatClusterSites);
             }
         }
         /* the chunk's writes, then its count; the last chunk of the phase queues the next phase */
-        __threadfence();
         __syncthreads();
-        if (threadIdx.x == 0) s_last = atomicSub(&ctl[replica].left, 1u) == 1u;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            s_last = atomicSub(&ctl[replica].left, 1u) == 1u;
+            if (s_last) __threadfence();
+        }
         __syncthreads();
         if (!s_last) continue;
-        __threadfence();
         if (bin_row) { /* the chunks' sums in chunk order */
             if (threadIdx.x < 8) {
                 double a = 0.0;
@@ -315,8 +317,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
             s_at = atomicAdd(q.tail, nx.left);
         }
         __syncthreads();
-        __threadfence();
-        for (uint32_t k = threadIdx.x; k < nx.left; k += kStreamThreads) put_entry(q, s_at + k, replica, k);
+        for (uint32_t k = threadIdx.x; k < nx.left; k += kStreamThreads) {
+            __threadfence();
+            put_entry(q, s_at + k, replica, k);
+        }
     }
 }
 

@@ -52,6 +52,7 @@ constexpr uint32_t kRegion = kGrowEdge; /* region edge in sites along y and z; o
 constexpr uint32_t kGrowThreads = kRegion * kRegion;
 constexpr int kBondThreads = 256;
 constexpr int kFlipThreads = 256;
+constexpr int kFlipQuads = 4; /* quads of sites per thread */
 constexpr uint32_t kEmpty = 0;
 constexpr uint32_t kNoRegion = 0xffffffffu;
 
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kBondThreads)
         queue_seed(wb, lx, ly, lz, seed_idx - row * lx, row % ly, row / ly);
     }
     const BitPlanes planes = {wb.bx, wb.by, wb.bz, wb.cl};
-    bond_run(theta, jxy, jz, lx, ly, lz, minus_two_beta, phi, seed, counter, planes, run,
+    bond_run<1>(theta, jxy, jz, lx, ly, lz, minus_two_beta, phi, seed, counter, planes, run,
              (blockIdx.x * blockDim.x + threadIdx.x) >> 5, bond_bytes);
 }
 
@@ -418,7 +419,8 @@ __device__ __forceinline__ void block_count(uint32_t n, unsigned long long* stat
 __global__ void __launch_bounds__(kFlipThreads)
     k_wb_flip(float* __restrict__ theta, uint32_t lx, uint32_t rows, slsf_fastdiv quads, const uint32_t* __restrict__ cl,
               float phi, unsigned long long* __restrict__ stats, uint8_t* __restrict__ cluster_out, bool wide) {
-    block_count(flip_quad(theta, lx, rows, blockIdx.x * blockDim.x + threadIdx.x, quads, cl, phi, cluster_out, wide),
+    block_count(flip_quads<kFlipQuads>(theta, lx, rows, blockIdx.x * kFlipQuads * blockDim.x + threadIdx.x, blockDim.x, quads, cl,
+                                       phi, cluster_out, wide),
                 stats, kStatClusterSites);
 }
 
@@ -458,7 +460,7 @@ int launch_wolff_bits(const TaskView& t, uint64_t counter, void* scratch, uint8_
     const slsf_fastdiv quads = slsf_fastdiv_make((t.lx + 3) / 4);
     const uint32_t rows = t.ly * t.lz;
     const bool wide = t.lx % 4 == 0 && (reinterpret_cast<uintptr_t>(t.theta) & 15u) == 0;
-    k_wb_flip<<<(quads.d * rows + kFlipThreads - 1) / kFlipThreads, kFlipThreads, 0, s>>>(
+    k_wb_flip<<<(quads.d * rows + kFlipThreads * kFlipQuads - 1) / (kFlipThreads * kFlipQuads), kFlipThreads, 0, s>>>(
         t.theta, t.lx, rows, quads, wb.cl, phi, t.stats, cluster_out, wide);
     if (phi_out) *phi_out = phi;
     if (seed_site) {

@@ -27,7 +27,8 @@ struct BitPlanes {
     uint32_t *bx, *by, *bz, *cl; /* [rows][words] */
 };
 
-/* (theta is not __restrict__: the persistent kernel changes the angles between its phases.) */
+/* (theta is not __restrict__: the persistent kernel changes the angles between its phases.  kRows: rows in flight.) */
+template <int kRows>
 __device__ __forceinline__ void bond_run(const float* theta, const float* __restrict__ jxy,
                                          const float* __restrict__ jz, uint32_t lx, uint32_t ly, uint32_t lz,
                                          float minus_two_beta, float phi, uint64_t seed, uint64_t counter,
@@ -64,6 +65,7 @@ __device__ __forceinline__ void bond_run(const float* theta, const float* __rest
     uint32_t oy = yrow(y_lo) * lx + x;
     float t0 = p0[oy], t1 = p1[oy], t2 = p2[o];
     uint32_t k[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll kRows
     for (uint32_t j = 0; j < rows; ++j) {
         const float a0 = t0, a1 = t1, a2 = t2;
         if (j + 1 < rows) {
@@ -115,30 +117,46 @@ __device__ __forceinline__ void bond_run(const float* theta, const float* __rest
     }
 }
 
-/* Reflects the cluster's sites among four consecutive ones of a row (quad q of
- * the lattice; one 16-byte access when L_x is a multiple of 4 and the angles
+/* Reflects the cluster's sites among four consecutive ones of a row, kN quads
+ * of the lattice per thread a distance `step` apart with their loads in flight
+ * together (one 16-byte access each when L_x is a multiple of 4 and the angles
  * are aligned: `wide`), with an optional byte mask; returns their number. */
-__device__ __forceinline__ uint32_t flip_quad(float* theta, uint32_t lx, uint32_t rows, uint32_t q,
-                                              const slsf_fastdiv& quads, const uint32_t* cl, float phi,
-                                              uint8_t* __restrict__ cluster_out, bool wide) {
-    if (q >= quads.d * rows) return 0;
-    const uint32_t row = slsf_fastdiv_div(q, quads), x = 4u * (q - row * quads.d), sites = min(4u, lx - x);
-    const uint32_t m = (__ldcg(&cl[row * ((lx + 31u) >> 5) + (x >> 5)]) >> (x & 31u)) & 0xfu;
-    const size_t i = (size_t)row * lx + x;
-    if (m && wide) {
-        float4 v = *reinterpret_cast<float4*>(theta + i);
-        if (m & 1u) v.x = slsf_reflect(v.x, phi);
-        if (m & 2u) v.y = slsf_reflect(v.y, phi);
-        if (m & 4u) v.z = slsf_reflect(v.z, phi);
-        if (m & 8u) v.w = slsf_reflect(v.w, phi);
-        *reinterpret_cast<float4*>(theta + i) = v;
-    } else if (m) {
-        for (uint32_t k = 0; k < sites; ++k)
-            if (m >> k & 1u) theta[i + k] = slsf_reflect(theta[i + k], phi);
+template <int kN>
+__device__ __forceinline__ uint32_t flip_quads(float* theta, uint32_t lx, uint32_t rows, uint32_t q0, uint32_t step,
+                                               const slsf_fastdiv& quads, const uint32_t* cl, float phi,
+                                               uint8_t* __restrict__ cluster_out, bool wide) {
+    uint32_t m[kN], n = 0;
+    size_t at[kN];
+    float4 v[kN];
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+        const uint32_t q = q0 + j * step, row = slsf_fastdiv_div(q, quads), x = 4u * (q - row * quads.d);
+        at[j] = (size_t)row * lx + x;
+        m[j] = q < quads.d * rows ? (__ldcg(&cl[row * ((lx + 31u) >> 5) + (x >> 5)]) >> (x & 31u)) & 0xfu : 0u;
+        if (cluster_out && q < quads.d * rows)
+            for (uint32_t k = 0; k < min(4u, lx - x); ++k) cluster_out[at[j] + k] = (uint8_t)(m[j] >> k & 1u);
     }
-    if (cluster_out)
-        for (uint32_t k = 0; k < sites; ++k) cluster_out[i + k] = (uint8_t)(m >> k & 1u);
-    return __popc(m);
+    if (wide) {
+#pragma unroll
+        for (int j = 0; j < kN; ++j)
+            if (m[j]) v[j] = *reinterpret_cast<const float4*>(theta + at[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+        n += __popc(m[j]);
+        if (!m[j]) continue;
+        if (wide) {
+            v[j].x = m[j] & 1u ? slsf_reflect(v[j].x, phi) : v[j].x;
+            v[j].y = m[j] & 2u ? slsf_reflect(v[j].y, phi) : v[j].y;
+            v[j].z = m[j] & 4u ? slsf_reflect(v[j].z, phi) : v[j].z;
+            v[j].w = m[j] & 8u ? slsf_reflect(v[j].w, phi) : v[j].w;
+            *reinterpret_cast<float4*>(theta + at[j]) = v[j];
+        } else {
+            for (uint32_t k = 0; k < 4; ++k)
+                if (m[j] >> k & 1u) theta[at[j] + k] = slsf_reflect(theta[at[j] + k], phi);
+        }
+    }
+    return n;
 }
 
 /* Closure of a periodic row of up to 64 sites along x (close_word). */
