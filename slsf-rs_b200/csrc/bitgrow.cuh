@@ -61,7 +61,7 @@ struct GrowBlock {
     bool px, py, pz;
 };
 
-/* One axis of a thread's word: position `lane` of line `warp`.  up[k] / dn[k]
+/* One axis of one word of a thread: position `lane` of line `line`.  up[k] / dn[k]
  * are the products of the bonds over the 2^k positions below / above, so a
  * scan along the line takes one shuffle and one operation per doubling step
  * and direction. */
@@ -73,10 +73,10 @@ struct GrowAxis {
     bool still;                /* that scan changed nothing in the line */
 
     /* si, sl: strides along the line and between lines; b bonds along it, bo across */
-    __device__ __forceinline__ void start(uint32_t si, uint32_t sl, const uint32_t* b, const uint32_t* bo, bool along,
-                                          bool across) {
+    __device__ __forceinline__ void start(uint32_t line, uint32_t si, uint32_t sl, const uint32_t* b, const uint32_t* bo,
+                                          bool along, bool across) {
         constexpr uint32_t E = kGrowEdge;
-        const uint32_t lane = threadIdx.x & 31u, line = threadIdx.x >> 5;
+        const uint32_t lane = threadIdx.x & 31u;
         at = lane * si + line * sl;
         below = line > 0 ? at - sl : at + (E - 1) * sl;
         above = line + 1 < E ? at + sl : at - (E - 1) * sl;
@@ -119,20 +119,29 @@ struct GrowAxis {
     }
 };
 
-/* Closes the block (1024 threads); c must already be closed along x.  Passes
- * alternate a scan of every line along y with a scan of every line along z,
- * each with one step along the other axis and the closure along x; a pass
- * that changes nothing ends it.  The bond products stay in registers for all
- * passes.  Returns the number of passes, or 0 if max_pass passes were not
- * enough (every pass that changes something sets a bit, so 32^3 + 1 always
- * are).  Bound by shuffles and shared loads (one warp instruction per clock
- * and SM): ten shuffles per line and pass. */
+/* Closes the block (1024 / kT threads, kT lines of each axis per warp); c must
+ * already be closed along x.  Passes alternate a scan of every line along y
+ * with a scan of every line along z, each with one step along the other axis
+ * and the closure along x; a pass that changes nothing ends it.  The bond
+ * products stay in registers for all passes.  Returns the number of passes, or
+ * 0 if max_pass passes were not enough (every pass that changes something sets
+ * a bit, so 32^3 + 1 always are).  Bound by shuffles and shared loads (one warp
+ * instruction per clock and SM): ten shuffles per line and pass. */
+template <int kT>
 __device__ __forceinline__ uint32_t close_block(const GrowBlock& q, uint32_t max_pass) {
-    GrowAxis y, z;
-    y.start(1u, kGrowPitch, q.by, q.bz, q.py, q.pz);
-    z.start(kGrowPitch, 1u, q.bz, q.by, q.pz, q.py);
-    for (uint32_t pass = 0; pass < max_pass; ++pass)
-        if (!__syncthreads_or((pass & 1u) ? z.pass(q) : y.pass(q))) return pass + 1;
+    GrowAxis y[kT], z[kT];
+#pragma unroll
+    for (int p = 0; p < kT; ++p) {
+        const uint32_t line = (threadIdx.x >> 5) + p * (kGrowEdge / kT);
+        y[p].start(line, 1u, kGrowPitch, q.by, q.bz, q.py, q.pz);
+        z[p].start(line, kGrowPitch, 1u, q.bz, q.by, q.pz, q.py);
+    }
+    for (uint32_t pass = 0; pass < max_pass; ++pass) {
+        int changed = 0;
+#pragma unroll
+        for (int p = 0; p < kT; ++p) changed |= (pass & 1u) ? z[p].pass(q) : y[p].pass(q);
+        if (!__syncthreads_or(changed)) return pass + 1;
+    }
     return 0;
 }
 

@@ -121,19 +121,17 @@ constexpr uint32_t kOneCtaSweepSites = 16384;
 
 namespace {
 
-/* Threads of the one-CTA kernel for V sites when `n` replicas share the GPU.
- * With at least three per SM, the fewest that keep its arithmetic pipes busy
- * (1e10 site-updates/s on B200: L = 8 2.07 / 1.56 / 1.07 on 64 / 128 / 256
- * threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 512, L = 20 5.13 / 4.72 on 128
- * / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93 on 512, L = 32 6.67 on 512
- * and 5.8 on 1024); with fewer, more threads shorten each replica's sweep (us
- * per sweep of one replica, 64 / 128 / 256 / 512 threads: L = 8 9.8 / 9.0 / 9.3
- * / 10.4, L = 12 21 / 13.6 / 12.1 / 12.7, L = 16 30 / 17.7 / 14.4 / 14.8, L = 20
- * 73 / 40 / 29 / 25, L = 24 128 / 67 / 43 / 37; of 296, L = 16 33 / 24 / 22 / 31,
- * L = 24 131 / 91 / 69 / 75). */
-uint32_t resident_threads(uint64_t v, uint64_t n, uint64_t sms) {
-    if (n <= sms) return v <= 1024 ? 128 : (v <= 4096 ? 256 : 512);
-    if (n <= 2 * sms) return v <= 1024 ? 128 : (v <= 16384 ? 256 : 512);
+/* Threads of the one-CTA kernel for V sites.  In a batch the fewest that keep
+ * the arithmetic pipes of a full GPU busy, whatever the batch, so that a task's
+ * sums do not depend on it (1e10 site-updates/s on B200: L = 8 2.07 / 1.56 /
+ * 1.07 on 64 / 128 / 256 threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 512, L =
+ * 20 5.13 / 4.72 on 128 / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93 on
+ * 512, L = 32 6.67 on 512 and 5.8 on 1024).  Alone and without measurements
+ * (slsf_task_sweep) more threads shorten the sweep (us, 64 / 128 / 256 / 512
+ * threads: L = 8 9.8 / 9.0 / 9.3 / 10.4, L = 12 21 / 13.6 / 12.1 / 12.7, L = 16
+ * 30 / 17.7 / 14.4 / 14.8, L = 20 73 / 40 / 29 / 25, L = 24 128 / 67 / 43 / 37). */
+uint32_t resident_threads(uint64_t v, bool alone) {
+    if (alone) return v <= 1024 ? 128 : (v <= 4096 ? 256 : 512);
     return v <= 1024 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512));
 }
 
@@ -731,7 +729,7 @@ int slsf_task_sweep(slsf_task* t, uint32_t n_sweeps, slsf_sweep_stats* stats) {
         TaskView v = t->view();
         v.n_bins = 0; /* slsf_task_sweep does not measure */
         v.stats = st;
-        SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->volume, 1, 1), t->ctx->stream));
+        SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->volume, true), t->ctx->stream));
         t->ctx->launches += 1;
         t->metro_sweeps += n_sweeps;
         t->wolff_done += (uint64_t)n_sweeps * t->wolff_steps;
@@ -771,11 +769,13 @@ int slsf_task_sweep(slsf_task* t, uint32_t n_sweeps, slsf_sweep_stats* stats) {
 int slsf_task_measure(slsf_task* t, slsf_observables* out) {
     if (!t || !out) return set_error(SLSF_ERR_INVALID, "NULL argument");
     if (int rc = bind_device(t->ctx)) return rc;
-    slsf::launch_measure(t->view(), nullptr, t->ctx->stream);
+    /* the last block writes the totals to the host's landing area itself */
+    TaskView view = t->view();
+    view.result = t->ctx->h_small;
+    slsf::launch_measure(view, nullptr, t->ctx->stream);
     t->ctx->launches += 1;
     SLSF_CUDA(cudaGetLastError());
     double r[8];
-    SLSF_CUDA(cudaMemcpyAsync(t->ctx->h_small, t->result, sizeof(r), cudaMemcpyDeviceToHost, t->ctx->stream));
     SLSF_CUDA(cudaStreamSynchronize(t->ctx->stream));
     std::memcpy(r, t->ctx->h_small, sizeof(r));
     const double v = (double)t->volume;
@@ -1218,7 +1218,7 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
  * threads; else the grid-wide kernels. */
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
     if (slsf::resident_supports(lx, ly, lz, device))
-        return {slsf::kKernelResident, 1, resident_threads((uint64_t)lx * ly * lz, ~0ull, 1)};
+        return {slsf::kKernelResident, 1, resident_threads((uint64_t)lx * ly * lz, false)};
     const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device);
     if (c && slsf::stream_fits(lx, ly, lz)) return {slsf::kKernelStream, 1, 256};
     if (c) return {slsf::kKernelCluster, c, 1024};
@@ -1237,15 +1237,6 @@ slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uin
     const auto it = ctx->tune.find(shape_key(lx, ly, lz));
     if (it != ctx->tune.end()) return it->second;
     return default_choice(lx, ly, lz, ctx->device);
-}
-
-/* The default choices of one-CTA tasks fitted to how many of them run together. */
-void fit_to_batch(const slsf_ctx* ctx, slsf_task* const* tasks, std::vector<slsf::KernelChoice>& ch) {
-    uint64_t n = 0;
-    for (const slsf::KernelChoice& c : ch) n += c.kind == slsf::kKernelResident;
-    for (size_t i = 0; i < ch.size(); ++i)
-        if (ch[i].kind == slsf::kKernelResident && !ctx->tune.count(shape_key(tasks[i]->lx, tasks[i]->ly, tasks[i]->lz)))
-            ch[i].threads = resident_threads(tasks[i]->volume, n, (uint64_t)ctx->sm_count);
 }
 
 /* Tasks of one group share their launches: those of one kernel choice, with
@@ -1358,7 +1349,6 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
         if (t->corr_interval && (ch[i].kind == slsf::kKernelCluster || ch[i].kind == slsf::kKernelStream))
             return set_error(SLSF_ERR_INVALID, kErrFuse);
     }
-    if (!force) fit_to_batch(ctx, tasks, ch);
     if (int rc = ensure_batch_capacity(ctx, n)) return rc;
     /* Grouped by kernel choice (one persistent launch each; cluster groups
      * first, grid-wide tasks last), largest replicas first within a group so
@@ -1519,7 +1509,6 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
         if (t->corr_interval && (ch[i].kind == slsf::kKernelCluster || ch[i].kind == slsf::kKernelStream))
             return set_error(SLSF_ERR_INVALID, kErrFuse);
     }
-    fit_to_batch(ctx, tasks, ch);
     auto rank = [&](size_t i) {
         const slsf::KernelChoice& c = ch[i];
         return group_rank(tasks[i], c);

@@ -458,7 +458,9 @@ __global__ void __launch_bounds__(kFinThreads) k_corr_finalize(const CorrTask* _
     for (uint32_t j = threadIdx.x; j < lz * R; j += blockDim.x) {
         const uint32_t z = j / R, r = j % R;
         double a = 0.0, b = 0.0;
+#pragma unroll 4
         for (uint32_t c = 0; c < sh.cx; ++c) a += part[(size_t)(z * sh.cx + c) * sh.rp + r];
+#pragma unroll 4
         for (uint32_t c = 0; c < sh.cy; ++c) b += part[(size_t)(sh.nx + z * sh.cy + c) * sh.rp + r];
         lsx[j] = a;
         lsy[j] = b;
@@ -466,10 +468,21 @@ __global__ void __launch_bounds__(kFinThreads) k_corr_finalize(const CorrTask* _
     }
     __syncthreads(); /* the layer sums are visible to the whole block */
     for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) {
+        /* in layer order; 16 layers' loads in flight before their adds */
         double sx = 0.0, sy = 0.0;
-        for (uint32_t z = 0; z < lz; ++z) {
-            sx += lsx[(size_t)z * R + r];
-            sy += lsy[(size_t)z * R + r];
+        for (uint32_t z0 = 0; z0 < lz; z0 += 16) {
+            double vx[16], vy[16];
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                const bool in = z0 + j < lz;
+                vx[j] = in ? lsx[(size_t)(z0 + j) * R + r] : 0.0;
+                vy[j] = in ? lsy[(size_t)(z0 + j) * R + r] : 0.0;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) {
+                sx += vx[j];
+                sy += vy[j];
+            }
         }
         const double cx = sx / volume, cy = sy / volume;
         emit(r, cx);
@@ -517,9 +530,13 @@ __global__ void __launch_bounds__(kFinThreads) k_corr_finalize(const CorrTask* _
         if (sh.spectral) {
             /* lag r + 1 from the summed folded spectrum, in frequency order */
             const uint32_t n = lz, lag = r + 1;
-            sz = 0.0;
-            for (uint32_t q = 0; q <= n / 2; ++q) sz += zcol[q] * ctab[(q * lag) % n];
-            sz /= (double)n;
+            /* four interleaved sums (n is a power of two) */
+            double part4[4] = {0.0, 0.0, 0.0, 0.0};
+            for (uint32_t q = 0; q + 3 <= n / 2; q += 4)
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) part4[j] += zcol[q + j] * ctab[((q + j) * lag) & (n - 1)];
+            for (uint32_t q = (n / 2 + 1) & ~3u; q <= n / 2; ++q) part4[0] += zcol[q] * ctab[(q * lag) & (n - 1)];
+            sz = ((part4[0] + part4[1]) + (part4[2] + part4[3])) / (double)n;
         }
         emit(3 * R + lz * R + r, sz / volume);
     }
@@ -581,11 +598,13 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
     if (n_items > 0) {
         const size_t smem = (size_t)max_len * kCorrPitch * sizeof(float2);
         cudaError_t e = cudaSuccess;
-        if (smem > 48 * 1024)
+        /* a task whose only lines are spectral z lines has no item for k_corr_lines */
+        const bool lines = !(one && one->rxy == 0 && n_zunits > 0);
+        if (lines && smem > 48 * 1024)
             e = cudaFuncSetAttribute(k_corr_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         const uint32_t grid = std::min<uint32_t>(n_items, 1u << 30);
-        k_corr_lines<<<grid, line_threads, smem, s>>>(one ? nullptr : tasks_dev, by_value, n_tasks, n_items);
+        if (lines) k_corr_lines<<<grid, line_threads, smem, s>>>(one ? nullptr : tasks_dev, by_value, n_tasks, n_items);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (n_zunits > 0) {

@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "engine.h"
+#include "region_grow.cuh"
 #include "walk_global.cuh"
 #include "wolff_global.cuh"
 
@@ -36,7 +37,9 @@ namespace {
 
 constexpr uint32_t kStreamThreads = 512; /* one CTA per SM: 128 registers a thread */
 constexpr uint32_t kStreamRows = 8;      /* rows per thread in the growth */
-constexpr uint32_t kFlipQuads = 16;      /* quads per thread of a reflection chunk */
+constexpr uint32_t kSegPlanes = 8;       /* planes per thread of a walk */
+constexpr uint32_t kBondRun = 16;        /* rows per warp of the bond activation */
+constexpr uint32_t kFlipQuads = 8;       /* quads per thread of a reflection */
 constexpr uint32_t kRingEntries = 1u << 20;
 constexpr uint32_t kChunkBits = 12;
 constexpr uint32_t kMaxWolffSteps = 1024;
@@ -49,25 +52,34 @@ struct StreamCtl {
     uint32_t phase, sweep, step;
 };
 
-/* Sizes of the chunks of a launch. */
+/* Sizes of the chunks of a launch.  A phase is a row of blocks of one CTA's
+ * threads (walks of kSegPlanes planes per thread, a run of rows per warp,
+ * kFlipQuads quads per thread); a chunk takes `per` of them one after the other.  The
+ * blocks, and so the order of the measured sums, are the same in every launch. */
 struct StreamShape {
-    uint32_t seglen; /* planes per thread of the walks */
-    uint32_t run;    /* rows per warp of the bond activation */
+    uint32_t per;     /* blocks per chunk */
+    uint32_t growers; /* CTAs that grow a replica's cluster together by regions; 1: one CTA by rows */
 };
 
-__host__ __device__ inline uint32_t chunks_of(const TaskView& t, const StreamShape& sh, uint32_t phase) {
+__host__ __device__ inline uint32_t smaller(uint32_t a, uint32_t b) { return a < b ? a : b; }
+
+__host__ __device__ inline uint32_t blocks_of(const TaskView& t, uint32_t phase) {
     switch (phase) {
         case kColour0:
         case kColour1:
-        case kMeasureLast: return (walk_units(t, sh.seglen) + kStreamThreads - 1) / kStreamThreads;
+        case kMeasureLast: return (walk_units(t, kSegPlanes) + kStreamThreads - 1) / kStreamThreads;
         case kBonds: {
-            const uint32_t warps = ((t.lx + 31) / 32) * (t.lz / 2) * ((t.ly + sh.run - 1) / sh.run);
+            const uint32_t warps = ((t.lx + 31) / 32) * (t.lz / 2) * ((t.ly + kBondRun - 1) / kBondRun);
             return (warps + kStreamThreads / 32 - 1) / (kStreamThreads / 32);
         }
-        case kGrow: return 1;
         case kFlip: return ((t.lx >> 2) * t.ly * t.lz + kStreamThreads * kFlipQuads - 1) / (kStreamThreads * kFlipQuads);
         default: return 0;
     }
+}
+
+__host__ __device__ inline uint32_t chunks_of(const TaskView& t, const StreamShape& sh, uint32_t phase) {
+    if (phase == kGrow) return smaller(sh.growers, (uint32_t)bit_regions(t.lx, t.ly, t.lz));
+    return (blocks_of(t, phase) + sh.per - 1) / sh.per;
 }
 
 /* The phase after `c` for sweeps below sw_hi of the launch. */
@@ -109,8 +121,8 @@ __device__ __forceinline__ void put_entry(const StreamQueue& q, uint32_t at, uin
 }
 
 __device__ __forceinline__ BitPlanes stream_planes(const TaskView& t) {
-    const uint32_t n = ((t.lx + 31u) >> 5) * t.ly * t.lz;
-    return {t.bits, t.bits + n, t.bits + 2 * n, t.bits + 3 * n};
+    const WolffBits wb = carve_bits(t.bits, t.lx, t.ly, t.lz);
+    return {wb.bx, wb.by, wb.bz, wb.cl};
 }
 
 /* Growth of a replica's cluster by the CTA, row words W of up to 32 or 64
@@ -243,33 +255,53 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         /* bin row of the state that colour 0 starts from, or of the last state */
         double* bin_row = nullptr;
         if ((c.phase == kColour0 && c.sweep > 0) || c.phase == kMeasureLast) bin_row = bin_row_of(t, sweep);
+        const uint32_t b_lo = chunk * sh.per, b_hi = smaller(b_lo + sh.per, blocks_of(t, c.phase));
         if (c.phase == kColour1 || (c.phase == kColour0 && !bin_row)) {
-            count_into(walk_colour<false>(t, sweep, c.phase == kColour1, sh.seglen, chunk * kStreamThreads + threadIdx.x, nullptr),
-                       t.stats, kStatAccepted);
+            uint32_t accepted = 0;
+            for (uint32_t b = b_lo; b < b_hi; ++b)
+                accepted += walk_colour<false>(t, sweep, c.phase == kColour1, kSegPlanes, b * kStreamThreads + threadIdx.x, nullptr);
+            count_into(accepted, t.stats, kStatAccepted);
         } else if (c.phase == kColour0 || c.phase == kMeasureLast) {
-            if (bin_row) {
+            uint32_t accepted = 0;
+            for (uint32_t b = b_lo; b < b_hi && bin_row; ++b) {
                 Sum2 sum[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, sh.seglen, k));
-                const uint32_t unit = chunk * kStreamThreads + threadIdx.x;
+                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, kSegPlanes, k));
+                const uint32_t unit = b * kStreamThreads + threadIdx.x;
                 if (c.phase == kColour0)
-                    count_into(walk_colour<true>(t, sweep, 0, sh.seglen, unit, sum), t.stats, kStatAccepted);
+                    accepted += walk_colour<true>(t, sweep, 0, kSegPlanes, unit, sum);
                 else
-                    walk_measure(t, sh.seglen, unit, sum);
+                    walk_measure(t, kSegPlanes, unit, sum);
                 double acc[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, sh.seglen, k));
+                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, kSegPlanes, k));
                 block_sum<8>(acc, scratch);
                 if (threadIdx.x == 0)
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) t.partials[chunk * 8 + k] = acc[k];
+                    for (int k = 0; k < 8; ++k) t.partials[b * 8 + k] = acc[k];
             }
+            if (c.phase == kColour0) count_into(accepted, t.stats, kStatAccepted);
         } else {
             const slsf_u32x4 pick = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_PICK, 0, 0);
             const float phi = slsf_angle_from_word(pick.x);
             if (c.phase == kBonds) {
-                bond_run<2>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, __fmul_rn(-2.0f, t.beta), phi, t.seed, counter, stream_planes(t),
-                         sh.run, (chunk * kStreamThreads + threadIdx.x) >> 5, nullptr);
+                if (chunk == 0 && sh.growers > 1) { /* the region queue, with the seed's region its first entry */
+                    const WolffBits wb = carve_bits(t.bits, t.lx, t.ly, t.lz);
+                    const uint32_t n = (uint32_t)(control_bytes(wb.regions) / 4);
+                    for (uint32_t i = threadIdx.x; i < n; i += kStreamThreads) wb.queued[i] = 0;
+                    __syncthreads();
+                    if (threadIdx.x == 0)
+                        queue_seed(wb, t.lx, t.ly, t.lz, slsf_range(pick.y, t.lx), slsf_range(pick.z, t.ly),
+                                   slsf_range(pick.w, t.lz));
+                }
+                const BitPlanes planes = stream_planes(t);
+                for (uint32_t b = b_lo; b < b_hi; ++b)
+                    bond_run<2>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, __fmul_rn(-2.0f, t.beta), phi, t.seed, counter, planes,
+                                kBondRun, (b * kStreamThreads + threadIdx.x) >> 5, nullptr);
+            } else if (c.phase == kGrow && sh.growers > 1) {
+                grow_regions<2>(carve_bits(t.bits, t.lx, t.ly, t.lz), grow_geo(t.lx, t.ly, t.lz),
+                                t.loop_limit ? t.loop_limit : max(64u, t.lx * t.ly * t.lz / 32), t.stats);
+                if (chunk == 0 && threadIdx.x == 0) atomicAdd(&t.stats[kStatClusters], 1ull);
             } else if (c.phase == kGrow) {
                 const bool closed = t.lx <= 32 ? grow_replica<uint32_t, kStreamRows>(t, pick, reinterpret_cast<uint32_t*>(grow_smem))
                                                : grow_replica<uint64_t, kStreamRows>(t, pick, reinterpret_cast<uint64_t*>(grow_smem));
@@ -281,9 +313,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
                 const slsf_fastdiv quads = slsf_fastdiv_make(t.lx >> 2);
                 const uint32_t* cl = stream_planes(t).cl;
                 uint32_t members = 0;
-                for (uint32_t j = 0; j < kFlipQuads; j += 4)
-                    members += flip_quads<4>(t.theta, t.lx, t.ly * t.lz, (chunk * kFlipQuads + j) * kStreamThreads + threadIdx.x,
-                                             kStreamThreads, quads, cl, phi, nullptr, true);
+                for (uint32_t j = b_lo * kFlipQuads; j < b_hi * kFlipQuads; j += 4)
+                    members += flip_quads<4>(t.theta, t.lx, t.ly * t.lz, j * kStreamThreads + threadIdx.x, kStreamThreads, quads,
+                                             cl, phi, nullptr, true);
                 count_into(members, t.stats, kStatClusterSites);
             }
         }
@@ -296,10 +328,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         }
         __syncthreads();
         if (!s_last) continue;
-        if (bin_row) { /* the chunks' sums in chunk order */
+        if (bin_row) { /* the blocks' sums in order */
             if (threadIdx.x < 8) {
                 double a = 0.0;
-                for (uint32_t k = 0; k < chunks_of(t, sh, c.phase); ++k) a += __ldcg(&t.partials[k * 8 + threadIdx.x]);
+                for (uint32_t k = 0; k < blocks_of(t, c.phase); ++k) a += __ldcg(&t.partials[k * 8 + threadIdx.x]);
                 scratch[threadIdx.x] = a;
             }
             __syncthreads();
@@ -334,7 +366,7 @@ __global__ void k_stream_advance(const TaskView* __restrict__ views, unsigned lo
 
 uint64_t items_per_sweep(const TaskView& t, const StreamShape& sh) {
     return 2ull * chunks_of(t, sh, kColour0) +
-           (uint64_t)t.wolff_steps * (chunks_of(t, sh, kBonds) + 1 + chunks_of(t, sh, kFlip));
+           (uint64_t)t.wolff_steps * (chunks_of(t, sh, kBonds) + chunks_of(t, sh, kGrow) + chunks_of(t, sh, kFlip));
 }
 
 }  // namespace
@@ -343,7 +375,8 @@ bool stream_fits(uint32_t lx, uint32_t ly, uint32_t lz) {
     /* patches of four sites by two rows, plane pairs, one or two words per row, the growth's rows and 16-bit row numbers;
      * the chunk numbers; the bit planes in 4 V bytes */
     return lx >= 4 && lx <= 64 && lx % 4 == 0 && ly >= 2 && ly % 2 == 0 && lz >= 2 && lz % 2 == 0 &&
-           (uint64_t)ly * lz <= (uint64_t)kStreamThreads * kStreamRows;
+           (uint64_t)ly * lz <= (uint64_t)kStreamThreads * kStreamRows &&
+           wolff_bits_scratch_bytes(lx, ly, lz) <= 4ull * lx * ly * lz;
 }
 
 bool stream_takes(const TaskView& t) { return walk_supports(t) && t.wolff_steps <= kMaxWolffSteps; }
@@ -359,15 +392,25 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
     q.abort = q.head + 2;
     q.ring = reinterpret_cast<unsigned long long*>(p + 256);
     StreamCtl* ctl = reinterpret_cast<StreamCtl*>(p + 256 + 8ull * kRingEntries);
-    /* chunk sizes: the longest walks and runs that still give every SM one and a half chunks */
-    StreamShape sh = {32, 32};
-    auto total = [&](uint32_t phase) {
+    /* as many blocks per chunk as leave three chunks of the walks per SM (each
+     * chunk costs about 2 us in the queue and its fences: 1.42 against 1.28 ms per
+     * sweep of 300 replicas of 64^3) */
+    StreamShape sh = {8, 1};
+    uint64_t sites = 0;
+    for (uint32_t i = 0; i < n; ++i) sites = std::max(sites, (uint64_t)host_views[i].lx * host_views[i].ly * host_views[i].lz);
+    auto chunks = [&]() {
         uint64_t c = 0;
-        for (uint32_t i = 0; i < n && c < 2ull * sms; ++i) c += chunks_of(host_views[i], sh, phase);
+        for (uint32_t i = 0; i < n && c < 3ull * sms; ++i) c += chunks_of(host_views[i], sh, kColour0);
         return c;
     };
-    while (sh.seglen > 4 && 2 * total(kColour0) < 3ull * sms) sh.seglen >>= 1;
-    while (sh.run > 8 && 2 * total(kBonds) < 3ull * sms) sh.run >>= 1;
+    while (sh.per > 1 && chunks() < 3ull * sms) sh.per >>= 1;
+    /* several CTAs grow a large replica together while there are SMs for them
+     * (us per sweep, together / by rows: one 64^3 150 / 178, sixteen 180 / 226,
+     * thirty-two 236 / 248, sixty-four 373 / 336; at 48^3 and 36^3 the cut regions
+     * make it slower: sixteen 136 / 121 and 126 / 100) */
+    if (sites >= 200000)
+        while (sh.growers < 8 && 2ull * sh.growers * n <= (uint64_t)sms) sh.growers <<= 1;
+    if (sh.growers < 4) sh.growers = 1;
     uint64_t most = 1;
     uint32_t rows = 0, sweeps = 0;
     for (uint32_t i = 0; i < n; ++i) {
