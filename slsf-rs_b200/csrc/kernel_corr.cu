@@ -103,8 +103,8 @@ __host__ __device__ inline uint32_t corr_zunits_of(const CorrShape& sh) {
 }
 
 /* Twiddles of the spectral route (FP32), laid out so that a warp reads 32
- * consecutive entries: stage[k][t] = w_(2h)^(t mod h) for the lane stage of
- * half-size h = 16 >> k, slot[j][t] = w_n^(t bitrev(j)) for register slot j,
+ * consecutive entries: stage[k][t] = w_(2h)^(t mod h) in the upper lanes (t & h)
+ * of the lane stage of half-size h = 16 >> k and 1 in the lower ones, slot[j][t] = w_n^(t bitrev(j)) for register slot j,
  * reg[q] = w_n^q for q < n (the register stages), with w_N = exp(-2 pi i / N)
  * evaluated in FP64 and rounded. */
 struct FftTables {
@@ -131,7 +131,7 @@ __device__ void fft_tables(FftTables& T, uint32_t n) {
     for (uint32_t q = threadIdx.x; q < n; q += blockDim.x) T.reg[q] = w(q);
     for (uint32_t e = threadIdx.x; e < 5 * 32; e += blockDim.x) {
         const uint32_t k = e / 32, t = e % 32, h = 16u >> k;
-        T.stage[k][t] = w((t & (h - 1)) * (n / (2 * h)));
+        T.stage[k][t] = (t & h) ? w((t & (h - 1)) * (n / (2 * h))) : make_float2(1.0f, 0.0f);
     }
     for (uint32_t e = threadIdx.x; e < n1 * 32; e += blockDim.x) {
         const uint32_t j = e / 32, t = e % 32;
@@ -238,16 +238,17 @@ __device__ void corr_z_unit(const CorrTask& Tk, const CorrShape& sh, uint32_t g,
              * ends with frequency index bitrev5(t) */
 #pragma unroll
             for (uint32_t k = 0; k < 5; ++k) {
+                /* the lower lane keeps X + Y, the upper one (Y - X) w, Y being
+                 * its partner's: one fused multiply-add by the lane's sign per
+                 * component, then the twiddle, which is 1 in the lower lanes */
                 const uint32_t h = 16u >> k;
-                const bool upper = lane & h;
+                const float sign = (lane & h) ? -1.0f : 1.0f;
                 const float2 w = T.stage[k][lane];
 #pragma unroll
                 for (uint32_t j = 0; j < N1; ++j) {
                     const float yx = __shfl_xor_sync(0xffffffffu, X[j].x, h);
                     const float yy = __shfl_xor_sync(0xffffffffu, X[j].y, h);
-                    const float2 sum = make_float2(X[j].x + yx, X[j].y + yy);
-                    const float2 dif = cmulf(make_float2(yx - X[j].x, yy - X[j].y), w);
-                    X[j] = upper ? dif : sum;
+                    X[j] = cmulf(make_float2(__fmaf_rn(sign, X[j].x, yx), __fmaf_rn(sign, X[j].y, yy)), w);
                 }
             }
 #pragma unroll

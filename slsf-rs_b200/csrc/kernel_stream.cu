@@ -132,7 +132,7 @@ __device__ __forceinline__ BitPlanes stream_planes(const TaskView& t) {
  * by instruction issue (visits of marked rows only, closures of whole lines by
  * segments and scans by shuffles were no faster: 129k, 140k and more cycles
  * against 122k). */
-template <typename W, int R>
+template <typename W, int R, bool kWhole>
 __device__ __forceinline__ bool grow_replica(const TaskView& t, const slsf_u32x4& pick, volatile W* cl) {
     const uint32_t lx = t.lx, ly = t.ly, lz = t.lz, rows = ly * lz;
     const BitPlanes planes = stream_planes(t);
@@ -157,7 +157,7 @@ __device__ __forceinline__ bool grow_replica(const TaskView& t, const slsf_u32x4
             b_x[j] = bx[r];
             y_nb[j] = ym | yp << 16;
             z_nb[j] = zm | zp << 16;
-            cl[r] = r == seed_row ? close_row((W)1 << slsf_range(pick.y, lx), b_x[j], lx) : (W)0;
+            cl[r] = r == seed_row ? close_row<kWhole>((W)1 << slsf_range(pick.y, lx), b_x[j], lx) : (W)0;
         }
     }
     __syncthreads();
@@ -176,7 +176,7 @@ __device__ __forceinline__ bool grow_replica(const TaskView& t, const slsf_u32x4
                                  (cl[z_nb[j] & 0xffffu] & b_zm[j]) | (cl[z_nb[j] >> 16] & b_zp[j]);
                     const W old = cl[r], c = old | in;
                     if (c != old) {
-                        cl[r] = close_row(c, b_x[j], lx);
+                        cl[r] = close_row<kWhole>(c, b_x[j], lx);
                         changed = 1;
                     }
                 }
@@ -303,8 +303,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
                                 t.loop_limit ? t.loop_limit : max(64u, t.lx * t.ly * t.lz / 32), t.stats);
                 if (chunk == 0 && threadIdx.x == 0) atomicAdd(&t.stats[kStatClusters], 1ull);
             } else if (c.phase == kGrow) {
-                const bool closed = t.lx <= 32 ? grow_replica<uint32_t, kStreamRows>(t, pick, reinterpret_cast<uint32_t*>(grow_smem))
-                                               : grow_replica<uint64_t, kStreamRows>(t, pick, reinterpret_cast<uint64_t*>(grow_smem));
+                uint32_t* cl = reinterpret_cast<uint32_t*>(grow_smem);
+                uint64_t* cl2 = reinterpret_cast<uint64_t*>(grow_smem);
+                const bool closed = t.lx <= 32 ? grow_replica<uint32_t, kStreamRows, false>(t, pick, cl)
+                                    : t.lx == 64 ? grow_replica<uint64_t, kStreamRows, true>(t, pick, cl2)
+                                                 : grow_replica<uint64_t, kStreamRows, false>(t, pick, cl2);
                 if (threadIdx.x == 0) {
                     if (!closed) atomicOr(&t.stats[kStatError], kErrGrowthLimit);
                     atomicAdd(&t.stats[kStatClusters], 1ull);

@@ -159,21 +159,31 @@ __device__ __forceinline__ uint32_t flip_quads(float* theta, uint32_t lx, uint32
     return n;
 }
 
-/* Closure of a periodic row of up to 64 sites along x (close_word). */
+/* Closure of a periodic row of up to 64 sites along x (close_word); kWhole: a
+ * row of exactly one or two words, whose reversal and carry need no shifts. */
+template <bool kWhole>
 __device__ __forceinline__ uint64_t carry_up64(uint64_t c, uint64_t b, uint32_t lx) {
     uint64_t s = b + (c & b);
-    c |= lx == 64 ? (uint64_t)(s < b) : s >> lx;
+    c |= kWhole ? (uint64_t)(s < b) : s >> lx;
     s = b + (c & b);
     return (s ^ b) | c;
 }
 
+template <bool kWhole>
 __device__ __forceinline__ uint64_t close_row(uint64_t c, uint64_t b, uint32_t lx) {
+    if (kWhole) {
+        const uint64_t bl = (b << 1) | (b >> 63);
+        return carry_up64<true>(c, b, 64) | __brevll(carry_up64<true>(__brevll(c), __brevll(bl), 64));
+    }
     const uint64_t mask = ~0ull >> (64 - lx), bl = ((b << 1) | (b >> (lx - 1))) & mask;
     const uint32_t sh = 64 - lx;
-    return (carry_up64(c, b, lx) | (__brevll(carry_up64(__brevll(c) >> sh, __brevll(bl) >> sh, lx)) >> sh)) & mask;
+    return (carry_up64<false>(c, b, lx) | (__brevll(carry_up64<false>(__brevll(c) >> sh, __brevll(bl) >> sh, lx)) >> sh)) & mask;
 }
 
-__device__ __forceinline__ uint32_t close_row(uint32_t c, uint32_t b, uint32_t lx) { return close_word(c, b, lx, true); }
+template <bool kWhole>
+__device__ __forceinline__ uint32_t close_row(uint32_t c, uint32_t b, uint32_t lx) {
+    return close_word(c, b, kWhole ? 32u : lx, true);
+}
 
 }  // namespace slsf
 
