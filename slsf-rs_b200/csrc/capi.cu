@@ -72,8 +72,11 @@ bool width_ok(double w) { return w >= 0.0 && std::isfinite(w); }
 uint64_t align256(uint64_t b) { return (b + 255) & ~255ull; }
 
 /* Kernels of one correlation measurement (launch_corr): the line items, the
- * spectral z items when there are z items, and the finalize. */
-uint32_t corr_launch_count(uint32_t items, uint32_t z_items) { return items ? (z_items ? 3u : 2u) : 1u; }
+ * spectral z items when there are z items, the layers' sums when they are
+ * many, and the finalize. */
+uint32_t corr_launch_count(uint32_t items, uint32_t z_items, uint32_t layers) {
+    return (items ? (z_items ? 3u : 2u) : 1u) + (slsf::corr_layers_launch(layers) ? 1u : 0u);
+}
 
 /* Side streams for the kernel groups of a batch after the first (group g
  * runs on side[(g - 1) % kSideStreams]); each group has its own work-queue
@@ -188,7 +191,7 @@ struct slsf_ctx {
      * repeated batch reuses it without an upload */
     std::vector<const slsf_task*> corr_last;
     std::vector<uint64_t> corr_last_gen;
-    uint32_t corr_last_items = 0, corr_last_zunits = 0, corr_last_len = 0, corr_last_r = 0, corr_last_nz = 0;
+    uint32_t corr_last_items = 0, corr_last_zunits = 0, corr_last_len = 0, corr_last_r = 0, corr_last_nz = 0, corr_last_layers = 0;
     uint64_t corr_gen = 0; /* slsf_task_corr_setup calls so far */
 };
 
@@ -815,8 +818,10 @@ int slsf_task_correlations(slsf_task* t, uint32_t rmax_xy, uint32_t rmax_z, doub
     const uint32_t items = slsf::corr_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z);
     e = slsf::launch_corr(nullptr, &ct, 1, items, slsf::corr_z_units(t->lx, t->ly, t->lz, rmax_xy, rmax_z),
                           slsf::corr_len(t->lx, t->ly, t->lz, rmax_xy, rmax_z), std::max(rmax_xy, rmax_z),
-                          slsf::corr_z_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z), ctx->sm_count, ctx->stream);
-    ctx->launches += corr_launch_count(items, slsf::corr_z_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z));
+                          slsf::corr_z_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z), t->lz * rmax_xy, ctx->sm_count,
+                          ctx->stream);
+    ctx->launches += corr_launch_count(items, slsf::corr_z_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z),
+                                       t->lz * rmax_xy);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), ct.values, 8ull * nv, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     ctx->pool.free(dv, bytes);
@@ -957,7 +962,7 @@ int slsf_batch_correlations(slsf_ctx* ctx, slsf_task* const* tasks, size_t n) {
             SLSF_CUDA(cudaHostAlloc(&ctx->h_corr, sizeof(slsf::CorrTask) * n, cudaHostAllocDefault));
             ctx->corr_cap = n;
         }
-        uint32_t items = 0, zunits = 0, max_len = 0, max_r = 0, max_nz = 0;
+        uint32_t items = 0, zunits = 0, max_len = 0, max_r = 0, max_nz = 0, max_layers = 0;
         for (size_t i = 0; i < n; ++i) {
             slsf_task* t = tasks[i];
             ctx->h_corr[i] = slsf::CorrTask{t->theta, t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz, items,
@@ -968,6 +973,7 @@ int slsf_batch_correlations(slsf_ctx* ctx, slsf_task* const* tasks, size_t n) {
             max_len = std::max(max_len, slsf::corr_len(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz));
             max_r = std::max(max_r, std::max(t->corr_rxy, t->corr_rz));
             max_nz = std::max(max_nz, slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz));
+            max_layers = std::max(max_layers, t->lz * t->corr_rxy);
         }
         SLSF_CUDA(cudaMemcpyAsync(ctx->d_corr, ctx->h_corr, sizeof(slsf::CorrTask) * n, cudaMemcpyHostToDevice,
                                   ctx->stream));
@@ -979,11 +985,12 @@ int slsf_batch_correlations(slsf_ctx* ctx, slsf_task* const* tasks, size_t n) {
         ctx->corr_last_len = max_len;
         ctx->corr_last_r = max_r;
         ctx->corr_last_nz = max_nz;
+        ctx->corr_last_layers = max_layers;
     }
     SLSF_CUDA(slsf::launch_corr(ctx->d_corr, nullptr, (uint32_t)n, ctx->corr_last_items, ctx->corr_last_zunits,
                                 ctx->corr_last_len,
-                                ctx->corr_last_r, ctx->corr_last_nz, ctx->sm_count, ctx->stream));
-    ctx->launches += corr_launch_count(ctx->corr_last_items, ctx->corr_last_nz);
+                                ctx->corr_last_r, ctx->corr_last_nz, ctx->corr_last_layers, ctx->sm_count, ctx->stream));
+    ctx->launches += corr_launch_count(ctx->corr_last_items, ctx->corr_last_nz, ctx->corr_last_layers);
     for (size_t i = 0; i < n; ++i) tasks[i]->corr_count += 1;
     return SLSF_OK;
 }
@@ -1179,9 +1186,11 @@ static void run_grid_task(slsf_ctx* ctx, const slsf_task* t, const TaskView& v, 
             slsf::launch_corr(nullptr, &ct, 1, items, slsf::corr_z_units(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz),
                               slsf::corr_len(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz),
                               std::max(t->corr_rxy, t->corr_rz),
-                              slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz), ctx->sm_count, st);
+                              slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz), t->lz * t->corr_rxy,
+                              ctx->sm_count, st);
             ctx->launches +=
-                corr_launch_count(items, slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz));
+                corr_launch_count(items, slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz),
+                                  t->lz * t->corr_rxy);
         }
     }
     if (pending) {

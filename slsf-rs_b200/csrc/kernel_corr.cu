@@ -432,95 +432,133 @@ __global__ void __launch_bounds__(kCorrThreads)
     }
 }
 
+/* Where a measurement's value goes: the task's values and / or its bin row
+ * *count / binsize (the finalize advances the count after both kernels). */
+struct CorrSink {
+    double *values, *bin;
+    __device__ __forceinline__ void put(uint32_t j, double v) const {
+        if (values) values[j] = v;
+        if (bin) bin[j] += v;
+    }
+};
+
+/* The block's task, by value: a reference that is either the list's entry or
+ * the by-value parameter would have the parameter's copy on the thread's stack
+ * read by the loads that __restrict__ makes read-only global ones. */
+__device__ __forceinline__ CorrTask corr_task(const CorrTask* tasks, const CorrTask& one, uint32_t i) {
+    if (tasks) return tasks[i];
+    return one;
+}
+
+__device__ __forceinline__ CorrSink corr_sink(const CorrTask& T) {
+    const unsigned long long row = T.count ? *T.count / (T.binsize ? T.binsize : 1) : 0;
+    const uint32_t nv = 3 * T.rxy + T.lz * T.rxy + T.rz;
+    return {T.values, (T.bins && row < T.n_bins) ? T.bins + row * nv : nullptr};
+}
+
+/* Entry j = z R + r of the layers' sums over their items along x and y
+ * ([L_z][R] each, after the partials), and its value C_xy(z, r). */
+__device__ __forceinline__ void layer_sum(const CorrTask& T, const CorrShape& sh, const CorrSink& sink, uint32_t j) {
+    const uint32_t R = T.rxy, z = j / R, r = j - z * R;
+    const double* __restrict__ part = T.partial;
+    double* lsx = T.partial + (size_t)(sh.nx + sh.ny + sh.nz) * sh.rp;
+    double* lsy = lsx + (size_t)T.lz * R;
+    double a = 0.0, b = 0.0;
+#pragma unroll 4
+    for (uint32_t c = 0; c < sh.cx; ++c) a += part[(size_t)(z * sh.cx + c) * sh.rp + r];
+#pragma unroll 4
+    for (uint32_t c = 0; c < sh.cy; ++c) b += part[(size_t)(sh.nx + z * sh.cy + c) * sh.rp + r];
+    lsx[j] = a;
+    lsy[j] = b;
+    sink.put(3 * R + j, (a + b) / (2.0 * (double)T.lx * T.ly));
+}
+
+/* The layers' sums of every task, one thread each, blockIdx.y's task: a
+ * launch of its own from kLayerSums sums on (launch_corr).  Latency bounds
+ * both places: in the finalize's one block per task the 4,608 sums of 96^3
+ * with R = 48 and the columns after them took 28 us, here 6 and 11 after
+ * them; the 128 sums of 16^3 with R = 8 cost less inside the finalize (54 us
+ * for 300 tasks' measurements, 58 with the launch; 12.5 and 15.6 for one 8^3). */
+constexpr int kLayerThreads = 128;
+constexpr uint32_t kLayerSums = 256;
+
+__global__ void __launch_bounds__(kLayerThreads) k_corr_layers(const CorrTask* tasks, CorrTask one) {
+    const CorrTask T = corr_task(tasks, one, blockIdx.y);
+    const uint32_t j = blockIdx.x * kLayerThreads + threadIdx.x;
+    if (j < T.lz * T.rxy) layer_sum(T, corr_shape(T.lx, T.ly, T.lz, T.rxy, T.rz), corr_sink(T), j);
+}
+
 constexpr int kFinThreads = 1024;
 constexpr uint32_t kZParts = 8;     /* interleaved partial sums per C_z lag */
 constexpr uint32_t kMaxZLags = 400; /* R_z <= corr_ext - L_z < 775 / 2 */
 
-__global__ void __launch_bounds__(kFinThreads) k_corr_finalize(const CorrTask* __restrict__ tasks, CorrTask one) {
-    const CorrTask& T = tasks ? tasks[blockIdx.x] : one;
+__global__ void __launch_bounds__(kFinThreads) k_corr_finalize(const CorrTask* tasks, CorrTask one, bool layers_done) {
+    const CorrTask T = corr_task(tasks, one, blockIdx.x);
     const uint32_t R = T.rxy, Rz = T.rz, lz = T.lz;
     if (R == 0 && Rz == 0) return;
     const CorrShape sh = corr_shape(T.lx, T.ly, lz, R, Rz);
     const uint32_t items = sh.nx + sh.ny + sh.nz;
-    const uint32_t nv = 3 * R + lz * R + Rz;
-    const double volume = (double)T.lx * T.ly * lz, area = (double)T.lx * T.ly;
+    const double volume = (double)T.lx * T.ly * lz;
     const double* __restrict__ part = T.partial;
-    double* lsx = T.partial + (size_t)items * sh.rp; /* [lz][R] layer sums */
-    double* lsy = lsx + (size_t)lz * R;
-    __shared__ unsigned long long row_s;
-    if (threadIdx.x == 0) row_s = T.count ? *T.count / (T.binsize ? T.binsize : 1) : 0;
+    const double* lsx = T.partial + (size_t)items * sh.rp; /* [lz][R] layer sums */
+    const double* lsy = lsx + (size_t)lz * R;
+    __shared__ CorrSink sink_s;
+    if (threadIdx.x == 0) sink_s = corr_sink(T);
     __syncthreads();
-    const unsigned long long row = row_s;
-    double* bin = (T.bins && row < T.n_bins) ? T.bins + row * nv : nullptr;
-    auto emit = [&](uint32_t j, double v) {
-        if (T.values) T.values[j] = v;
-        if (bin) bin[j] += v;
-    };
-    for (uint32_t j = threadIdx.x; j < lz * R; j += blockDim.x) {
-        const uint32_t z = j / R, r = j % R;
-        double a = 0.0, b = 0.0;
-#pragma unroll 4
-        for (uint32_t c = 0; c < sh.cx; ++c) a += part[(size_t)(z * sh.cx + c) * sh.rp + r];
-#pragma unroll 4
-        for (uint32_t c = 0; c < sh.cy; ++c) b += part[(size_t)(sh.nx + z * sh.cy + c) * sh.rp + r];
-        lsx[j] = a;
-        lsy[j] = b;
-        emit(3 * R + j, (a + b) / (2.0 * area));
-    }
-    __syncthreads(); /* the layer sums are visible to the whole block */
-    for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) {
-        /* in layer order; 16 layers' loads in flight before their adds */
-        double sx = 0.0, sy = 0.0;
-        for (uint32_t z0 = 0; z0 < lz; z0 += 16) {
-            double vx[16], vy[16];
+    const CorrSink sink = sink_s;
+    auto emit = [&](uint32_t j, double v) { sink.put(j, v); };
+    /* sums over columns in kZParts interleaved partial sums (rows p = q mod
+     * kZParts, in order; 16 loads in flight), then the partial sums in order --
+     * the same order whatever the block size, so every launch of a task gives
+     * the same bits */
+    __shared__ double zpart[kZParts * kMaxZLags];
+    __shared__ double zcol[kMaxZLags];
+    auto column_sums = [&](const double* base, size_t pitch, uint32_t cols, uint32_t rows) {
+        for (uint32_t idx = threadIdx.x; idx < cols * kZParts; idx += blockDim.x) {
+            const uint32_t r = idx % cols, q = idx / cols;
+            const double* col = base + r;
+            double a = 0.0;
+            uint32_t p = q;
+            for (; p + 15 * kZParts < rows; p += 16 * kZParts) {
+                double v[16];
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) {
-                const bool in = z0 + j < lz;
-                vx[j] = in ? lsx[(size_t)(z0 + j) * R + r] : 0.0;
-                vy[j] = in ? lsy[(size_t)(z0 + j) * R + r] : 0.0;
-            }
+                for (uint32_t j = 0; j < 16; ++j) v[j] = col[(size_t)(p + j * kZParts) * pitch];
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) {
-                sx += vx[j];
-                sy += vy[j];
+                for (uint32_t j = 0; j < 16; ++j) a += v[j];
             }
+#pragma unroll 4
+            for (; p < rows; p += kZParts) a += col[(size_t)p * pitch];
+            zpart[idx] = a;
         }
-        const double cx = sx / volume, cy = sy / volume;
-        emit(r, cx);
-        emit(R + r, cy);
-        emit(2 * R + r, (cx + cy) / 2.0);
+        __syncthreads();
+        for (uint32_t r = threadIdx.x; r < cols; r += blockDim.x) {
+            double v = 0.0;
+            for (uint32_t q = 0; q < kZParts; ++q) v += zpart[q * cols + r];
+            zcol[r] = v;
+        }
+        __syncthreads();
+    };
+    if (!layers_done) {
+        for (uint32_t j = threadIdx.x; j < lz * R; j += blockDim.x) layer_sum(T, sh, sink, j);
+        __syncthreads(); /* visible to the whole block */
+    }
+    if (R) {
+        column_sums(lsx, R, R, lz);
+        for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) emit(r, zcol[r] / volume);
+        const double cx = threadIdx.x < R ? zcol[threadIdx.x] / volume : 0.0; /* R < 128 threads or kFinThreads */
+        __syncthreads();
+        column_sums(lsy, R, R, lz);
+        for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) {
+            const double cy = zcol[r] / volume;
+            emit(R + r, cy);
+            emit(2 * R + r, (cx + cy) / 2.0);
+        }
+        __syncthreads();
     }
     /* C_z: each column of the z items' rows (a lag, or on the spectral route
-     * a frequency of the folded spectrum) summed over the items in kZParts
-     * interleaved partial sums (items p = q mod kZParts, in order), then the
-     * partial sums in order -- the same order whatever the block size, so
-     * every launch of a task gives the same bits */
-    __shared__ double zpart[kZParts * kMaxZLags];
-    const uint32_t zc = sh.spectral ? lz / 2 + 1 : Rz; /* columns */
-    const uint32_t zrows = sh.spectral ? corr_zunits_of(sh) : sh.nz; /* rows: units, or items */
-    for (uint32_t idx = threadIdx.x; idx < zc * kZParts; idx += blockDim.x) {
-        const uint32_t r = idx % zc, q = idx / zc;
-        const double* col = part + (size_t)(sh.nx + sh.ny) * sh.rp + r;
-        /* in item order; 16 loads in flight before their adds */
-        double a = 0.0;
-        uint32_t p = q;
-        for (; p + 15 * kZParts < zrows; p += 16 * kZParts) {
-            double v[16];
-#pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) v[j] = col[(size_t)(p + j * kZParts) * sh.rp];
-#pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) a += v[j];
-        }
-        for (; p < zrows; p += kZParts) a += col[(size_t)p * sh.rp];
-        zpart[idx] = a;
-    }
-    __syncthreads();
-    __shared__ double zcol[kMaxZLags];
-    for (uint32_t r = threadIdx.x; r < zc; r += blockDim.x) {
-        double sz = 0.0;
-        for (uint32_t q = 0; q < kZParts; ++q) sz += zpart[q * zc + r];
-        zcol[r] = sz;
-    }
+     * a frequency of the folded spectrum) over the items, or the units */
+    const uint32_t zc = sh.spectral ? lz / 2 + 1 : Rz;
+    if (Rz) column_sums(part + (size_t)(sh.nx + sh.ny) * sh.rp, sh.rp, zc, sh.spectral ? corr_zunits_of(sh) : sh.nz);
     /* cos(2 pi m / n) for the n residues m of q * lag, evaluated once each */
     __shared__ double ctab[kFftMax];
     if (sh.spectral)
@@ -585,15 +623,18 @@ bool corr_supports(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t
     return (size_t)corr_ext(lx, ly, lz, rxy, rz) * kCorrPitch * sizeof(float2) <= kCorrMaxTile;
 }
 
+bool corr_layers_launch(uint32_t max_layers) { return max_layers >= kLayerSums; }
+
 cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t n_tasks, uint32_t n_items,
-                        uint32_t n_zunits, uint32_t max_len, uint32_t max_r, uint32_t max_nz, int sm_count,
-                        cudaStream_t s) {
+                        uint32_t n_zunits, uint32_t max_len, uint32_t max_r, uint32_t max_nz, uint32_t max_layers,
+                        int sm_count, cudaStream_t s) {
     /* a warp takes 8 lags per pass: blocks of one or two warps for small
      * radii, so that short lines do not hold idle warps */
     const int line_threads = max_r <= 16 ? 64 : (max_r <= 32 ? 128 : kCorrThreads);
+    const bool layers = corr_layers_launch(max_layers);
     /* the finalize splits each C_z sum over its z items only when there are
      * many; each lag needs a thread of its own (R_z <= 258 < kFinThreads) */
-    const int fin_threads = (max_nz > 64 || max_r > 128) ? kFinThreads : 128;
+    const int fin_threads = (max_nz > 64 || max_r > 128 || layers) ? kFinThreads : 128;
     if (n_tasks == 0 || (!tasks_dev && (!one || n_tasks != 1))) return cudaErrorInvalidValue;
     const CorrTask by_value = one ? *one : CorrTask{};
     if (n_items > 0) {
@@ -622,7 +663,14 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
             if (e != cudaSuccess) return e;
         }
     }
-    k_corr_finalize<<<n_tasks, fin_threads, 0, s>>>(one ? nullptr : tasks_dev, by_value);
+    if (layers) {
+        for (uint32_t lo = 0; lo < n_tasks; lo += 65535) /* tasks of one launch (grid.y) */
+            k_corr_layers<<<dim3((max_layers + kLayerThreads - 1) / kLayerThreads, std::min(65535u, n_tasks - lo)), kLayerThreads, 0, s>>>(
+                one ? nullptr : tasks_dev + lo, by_value);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    k_corr_finalize<<<n_tasks, fin_threads, 0, s>>>(one ? nullptr : tasks_dev, by_value, layers);
     return cudaGetLastError();
 }
 
