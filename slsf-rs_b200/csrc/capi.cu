@@ -216,6 +216,7 @@ struct slsf_task {
     double* result = nullptr;
     unsigned int* done = nullptr;
     unsigned long long* stats = nullptr;
+    bool stats_open = false; /* a call is between begin_stats and read_stats */
     double* bins = nullptr;
     float jmax = 0.0f; /* TaskView::jmax */
     slsf_batch* session = nullptr; /* open batch session holding the task's device view */
@@ -252,6 +253,7 @@ struct slsf_task {
         v.sweeps = 0;
         v.loop_limit = ctx->loop_limit;
         v.jmax = jmax;
+        v.wolff_only = 0;
         v.bits = parent;
         v.partials = partials;
         v.result = result;
@@ -282,19 +284,49 @@ int check_free(const slsf_task* t) {
     return SLSF_OK;
 }
 
+/* The task's counters are clear between calls: read_stats' kernel writes them
+ * to the host's landing area and clears them for the next call (one launch in
+ * place of a memset before the call's kernels and a copy after them).  A call
+ * that failed before its read_stats leaves them to the next one. */
+int begin_stats(slsf_task* t) {
+    if (t->stats_open)
+        SLSF_CUDA(cudaMemsetAsync(t->stats, 0, sizeof(unsigned long long) * slsf::kStatSlots, t->ctx->stream));
+    t->stats_open = true;
+    return SLSF_OK;
+}
+
 int read_stats(slsf_task* t, unsigned long long out[slsf::kStatSlots]) {
     static_assert(sizeof(unsigned long long) * slsf::kStatSlots <= kSmallReadBack, "stats fit the landing area");
-    SLSF_CUDA(cudaMemcpyAsync(t->ctx->h_small, t->stats, sizeof(unsigned long long) * slsf::kStatSlots,
-                              cudaMemcpyDeviceToHost, t->ctx->stream));
+    slsf::launch_publish_stats(t->stats, reinterpret_cast<unsigned long long*>(t->ctx->h_small), t->ctx->stream);
+    t->ctx->launches += 1;
+    SLSF_CUDA(cudaGetLastError());
     SLSF_CUDA(cudaStreamSynchronize(t->ctx->stream));
+    t->stats_open = false;
     std::memcpy(out, t->ctx->h_small, sizeof(unsigned long long) * slsf::kStatSlots);
     if (out[slsf::kStatError])
         return set_error(SLSF_ERR_TIMEOUT, "a bounded device loop hit its iteration limit");
     return SLSF_OK;
 }
 
-int zero_stats(slsf_task* t) {
-    SLSF_CUDA(cudaMemsetAsync(t->stats, 0, sizeof(unsigned long long) * slsf::kStatSlots, t->ctx->stream));
+/* A small lattice's updates in one launch of the one-CTA kernel, which writes
+ * the counters to the host's landing area: one sweep at L = 8 takes 9 us on
+ * the GPU against 38 us in six launches, at L = 24 37 against 47; at L = 32 59
+ * against 37, the whole GPU being faster than one SM. */
+bool one_cta_updates(const slsf_task* t) {
+    return t->volume <= kOneCtaSweepSites && slsf::resident_supports(t->lx, t->ly, t->lz, t->ctx->device);
+}
+
+int run_one_cta(slsf_task* t, TaskView v, uint32_t n_sweeps, unsigned long long out[slsf::kStatSlots]) {
+    unsigned long long* st = reinterpret_cast<unsigned long long*>(t->ctx->h_small);
+    std::memset(st, 0, sizeof(unsigned long long) * slsf::kStatSlots);
+    v.n_bins = 0; /* single-task updates do not measure */
+    v.stats = st;
+    SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->volume, true), t->ctx->stream));
+    t->ctx->launches += 1;
+    SLSF_CUDA(cudaStreamSynchronize(t->ctx->stream));
+    std::memcpy(out, st, sizeof(unsigned long long) * slsf::kStatSlots);
+    if (out[slsf::kStatError])
+        return set_error(SLSF_ERR_TIMEOUT, "a bounded device loop hit its iteration limit");
     return SLSF_OK;
 }
 
@@ -647,7 +679,7 @@ int slsf_task_metropolis_color(slsf_task* t, uint32_t colour, uint8_t* accept_ma
         d_mask = t->bonds;
         SLSF_CUDA(cudaMemsetAsync(d_mask, 0, t->volume, t->ctx->stream));
     }
-    if (int rc = zero_stats(t)) return rc;
+    if (int rc = begin_stats(t)) return rc;
     slsf::launch_metro_colour(t->view(), t->metro_sweeps, colour, d_mask, t->ctx->stream);
     t->ctx->launches += 1;
     SLSF_CUDA(cudaGetLastError());
@@ -663,14 +695,19 @@ int slsf_task_metropolis_sweep(slsf_task* t, double* acceptance) {
     if (!t) return set_error(SLSF_ERR_INVALID, "task is NULL");
     if (int rc = check_sweepable(t)) return rc;
     if (int rc = bind_device(t->ctx)) return rc;
-    if (int rc = zero_stats(t)) return rc;
-    const TaskView v = t->view();
-    slsf::launch_metro_colour(v, t->metro_sweeps, 0, nullptr, t->ctx->stream);
-    slsf::launch_metro_colour(v, t->metro_sweeps, 1, nullptr, t->ctx->stream);
-    t->ctx->launches += 2;
-    SLSF_CUDA(cudaGetLastError());
     unsigned long long st[slsf::kStatSlots];
-    if (int rc = read_stats(t, st)) return rc;
+    TaskView v = t->view();
+    if (one_cta_updates(t)) {
+        v.wolff_steps = 0;
+        if (int rc = run_one_cta(t, v, 1, st)) return rc;
+    } else {
+        if (int rc = begin_stats(t)) return rc;
+        slsf::launch_metro_colour(v, t->metro_sweeps, 0, nullptr, t->ctx->stream);
+        slsf::launch_metro_colour(v, t->metro_sweeps, 1, nullptr, t->ctx->stream);
+        t->ctx->launches += 2;
+        SLSF_CUDA(cudaGetLastError());
+        if (int rc = read_stats(t, st)) return rc;
+    }
     t->metro_sweeps += 1;
     if (acceptance) *acceptance = (double)st[slsf::kStatAccepted] / (double)t->volume;
     return SLSF_OK;
@@ -683,7 +720,7 @@ int slsf_task_wolff_step_debug(slsf_task* t, uint8_t* bonds, uint8_t* cluster, f
     /* wolff_cluster_step_with_theta_scratch validates T (src/updates.rs:558). */
     if (!temperature_ok(t->temperature)) return set_error(SLSF_ERR_INVALID, kErrTemperature);
     if (int rc = bind_device(t->ctx)) return rc;
-    if (int rc = zero_stats(t)) return rc;
+    if (int rc = begin_stats(t)) return rc;
     /* The exported cluster mask needs a byte per site of its own; it comes
      * from the pool and goes back after the copy. */
     void* d_cluster = nullptr;
@@ -700,13 +737,14 @@ int slsf_task_wolff_step_debug(slsf_task* t, uint8_t* bonds, uint8_t* cluster, f
         e = cudaMemcpyAsync(bonds, t->bonds, t->volume, cudaMemcpyDeviceToHost, t->ctx->stream);
     if (e == cudaSuccess && cluster)
         e = cudaMemcpyAsync(cluster, d_cluster, t->volume, cudaMemcpyDeviceToHost, t->ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(t->ctx->stream);
+    if (e != cudaSuccess) cudaStreamSynchronize(t->ctx->stream);
+    unsigned long long st[slsf::kStatSlots];
+    const int rc = e == cudaSuccess ? read_stats(t, st) : SLSF_OK;
     if (d_cluster) t->ctx->pool.free(d_cluster, align256(t->volume));
     if (e != cudaSuccess) return cuda_error(e, "wolff step");
     if (bonds) /* the bond bits only (the kernels mark tile roots in bit 3) */
         for (uint32_t i = 0; i < t->volume; ++i) bonds[i] &= 7u;
-    unsigned long long st[slsf::kStatSlots];
-    if (int rc = read_stats(t, st)) return rc;
+    if (rc) return rc;
     t->wolff_done += 1;
     if (phi) *phi = phi_h;
     if (seed_site) std::memcpy(seed_site, site, sizeof(site));
@@ -715,6 +753,17 @@ int slsf_task_wolff_step_debug(slsf_task* t, uint8_t* bonds, uint8_t* cluster, f
 }
 
 int slsf_task_wolff_step(slsf_task* t, uint64_t* cluster_size) {
+    if (t && !t->session && temperature_ok(t->temperature) && one_cta_updates(t)) {
+        if (int rc = bind_device(t->ctx)) return rc;
+        unsigned long long st[slsf::kStatSlots];
+        TaskView v = t->view();
+        v.wolff_steps = 1;
+        v.wolff_only = 1;
+        if (int rc = run_one_cta(t, v, 1, st)) return rc;
+        t->wolff_done += 1;
+        if (cluster_size) *cluster_size = st[slsf::kStatClusterSites];
+        return SLSF_OK;
+    }
     return slsf_task_wolff_step_debug(t, nullptr, nullptr, nullptr, nullptr, cluster_size);
 }
 
@@ -722,29 +771,19 @@ int slsf_task_sweep(slsf_task* t, uint32_t n_sweeps, slsf_sweep_stats* stats) {
     if (!t) return set_error(SLSF_ERR_INVALID, "task is NULL");
     if (int rc = check_sweepable(t)) return rc;
     if (int rc = bind_device(t->ctx)) return rc;
-    /* A small lattice sweeps in one launch of the one-CTA kernel, which
-     * writes the counters to the host's landing area: one sweep at L = 8 takes
-     * 9 us on the GPU against 38 us in six launches, at L = 24 37 against 47; at
-     * L = 32 59 against 37, the whole GPU being faster than one SM. */
-    if (n_sweeps && t->volume <= kOneCtaSweepSites && slsf::resident_supports(t->lx, t->ly, t->lz, t->ctx->device)) {
-        unsigned long long* st = reinterpret_cast<unsigned long long*>(t->ctx->h_small);
-        std::memset(st, 0, sizeof(unsigned long long) * slsf::kStatSlots);
-        TaskView v = t->view();
-        v.n_bins = 0; /* slsf_task_sweep does not measure */
-        v.stats = st;
-        SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->volume, true), t->ctx->stream));
-        t->ctx->launches += 1;
+    if (n_sweeps && one_cta_updates(t)) {
+        unsigned long long st[slsf::kStatSlots];
+        const int rc = run_one_cta(t, t->view(), n_sweeps, st);
+        if (rc && rc != SLSF_ERR_TIMEOUT) return rc;
         t->metro_sweeps += n_sweeps;
         t->wolff_done += (uint64_t)n_sweeps * t->wolff_steps;
-        SLSF_CUDA(cudaStreamSynchronize(t->ctx->stream));
-        if (st[slsf::kStatError])
-            return set_error(SLSF_ERR_TIMEOUT, "a bounded device loop hit its iteration limit");
+        if (rc) return rc;
         if (stats)
             *stats = slsf_sweep_stats{n_sweeps, st[slsf::kStatAccepted], st[slsf::kStatClusters],
                                       st[slsf::kStatClusterSites]};
         return SLSF_OK;
     }
-    if (int rc = zero_stats(t)) return rc;
+    if (int rc = begin_stats(t)) return rc;
     for (uint32_t s = 0; s < n_sweeps; ++s) {
         TaskView v = t->view();
         slsf::launch_metro_colour(v, t->metro_sweeps, 0, nullptr, t->ctx->stream);

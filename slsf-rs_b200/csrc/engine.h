@@ -45,6 +45,7 @@ struct TaskView {
     uint32_t sweeps;       /* sweeps of this task in a batched launch; 0: the launch's count */
     uint32_t loop_limit;   /* 0, or a lower bound on device loops (slsf_ctx_set_loop_limit) */
     float jmax;            /* largest coupling; infinite if any is not below kJMax */
+    uint32_t wolff_only;   /* the one-CTA kernel leaves the Metropolis half-sweeps out (slsf_task_wolff_step) */
     unsigned long long* stats;
     uint32_t* bits;        /* 4 V bytes of scratch: the Wolff bit planes of the stream kernels */
     double* partials;      /* measurement scratch: block sums, totals, block counter */
@@ -80,6 +81,8 @@ constexpr uint32_t kKernelResident = 0, kKernelCluster = 1, kKernelGrid = 2, kKe
 int report_error(int code, const std::string& message);
 
 /* ---- single-task kernels (kernels_plain.cu) ---- */
+/* Copies a task's counters to pinned host memory and clears them. */
+void launch_publish_stats(unsigned long long* stats, unsigned long long* host, cudaStream_t s);
 void launch_init_random(float* theta, uint32_t volume, uint64_t seed, cudaStream_t s);
 void launch_metro_colour(const TaskView& t, uint64_t sweep, uint32_t colour, uint8_t* record,
                          cudaStream_t s);

@@ -841,22 +841,24 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         const bool measuring = t.n_bins > 0;
         for (uint32_t sw = 0; sw < sweeps; ++sw) {
             const uint64_t sweep = t.metro_sweeps + sw;
-            double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (measuring && sw > 0 && sweep > t.thermalization) {
-                accepted += sweep_colour<true>(t, g, s, sweep, 0, acc);
-                double tot[8];
+            if (!t.wolff_only) {
+                double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                if (measuring && sw > 0 && sweep > t.thermalization) {
+                    accepted += sweep_colour<true>(t, g, s, sweep, 0, acc);
+                    double tot[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) tot[k] = acc[k];
-                block_sum<8>(tot, red);
-                if (threadIdx.x == 0) bin_measurement(t, g.volume, sweep, tot, bin_acc, bin_cur);
-            } else {
-                accepted += sweep_colour<false>(t, g, s, sweep, 0, acc);
+                    for (int k = 0; k < 8; ++k) tot[k] = acc[k];
+                    block_sum<8>(tot, red);
+                    if (threadIdx.x == 0) bin_measurement(t, g.volume, sweep, tot, bin_acc, bin_cur);
+                } else {
+                    accepted += sweep_colour<false>(t, g, s, sweep, 0, acc);
+                }
+                __syncthreads();
+                SLSF_PHASE(0);
+                accepted += sweep_colour<false>(t, g, s, sweep, 1, acc);
+                __syncthreads();
+                SLSF_PHASE(1);
             }
-            __syncthreads();
-            SLSF_PHASE(0);
-            accepted += sweep_colour<false>(t, g, s, sweep, 1, acc);
-            __syncthreads();
-            SLSF_PHASE(1);
             for (uint32_t k = 0; k < t.wolff_steps; ++k)
                 wolff_update(t, g, s, t.wolff_done + (uint64_t)sw * t.wolff_steps + k, &s_cluster);
             /* ThetaModel::measure's correlations of the state after this sweep:

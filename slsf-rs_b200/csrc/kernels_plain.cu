@@ -679,7 +679,17 @@ __global__ void k_gather(const double* const* __restrict__ src, uint32_t per, do
     for (uint32_t k = threadIdx.x; k < per; k += blockDim.x) d[k] = s[k];
 }
 
+__global__ void k_publish_stats(unsigned long long* __restrict__ stats, unsigned long long* __restrict__ host) {
+    const unsigned long long v = stats[threadIdx.x];
+    host[threadIdx.x] = v;
+    stats[threadIdx.x] = 0;
+}
+
 }  // namespace
+
+void launch_publish_stats(unsigned long long* stats, unsigned long long* host, cudaStream_t s) {
+    k_publish_stats<<<1, kStatSlots, 0, s>>>(stats, host);
+}
 
 void launch_gather(const double* const* src, uint32_t n, uint32_t per, double* dst, cudaStream_t s) {
     k_gather<<<n, 128, 0, s>>>(src, per, dst);
