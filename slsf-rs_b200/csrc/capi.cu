@@ -126,16 +126,22 @@ namespace {
 
 /* Threads of the one-CTA kernel for V sites.  In a batch the fewest that keep
  * the arithmetic pipes of a full GPU busy, whatever the batch, so that a task's
- * sums do not depend on it (1e10 site-updates/s on B200: L = 8 2.07 / 1.56 /
- * 1.07 on 64 / 128 / 256 threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 512, L =
- * 20 5.13 / 4.72 on 128 / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93 on
- * 512, L = 32 6.67 on 512 and 5.8 on 1024).  Alone and without measurements
- * (slsf_task_sweep) more threads shorten the sweep (us, 64 / 128 / 256 / 512
- * threads: L = 8 9.8 / 9.0 / 9.3 / 10.4, L = 12 21 / 13.6 / 12.1 / 12.7, L = 16
- * 30 / 17.7 / 14.4 / 14.8, L = 20 73 / 40 / 29 / 25, L = 24 128 / 67 / 43 / 37). */
-uint32_t resident_threads(uint64_t v, bool alone) {
-    if (alone) return v <= 1024 ? 128 : (v <= 4096 ? 256 : 512);
-    return v <= 1024 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512));
+ * sums do not depend on it (1e10 site-updates/s on B200: L = 8 2.37 / 2.05 on
+ * 64 / 128 threads, L = 16 5.24 / 5.73 / 5.18 and 3.53 on 64 / 128 / 256 and 512,
+ * L = 20 5.13 / 4.72 on 128 / 256, L = 24 5.00 / 4.18 on 256 / 512, L = 28 4.93
+ * on 512, L = 32 6.67 on 512 and 5.8 on 1024).  Lattices that sweep a site per
+ * lane lose little with twice the threads and a few replicas gain much (us per
+ * sweep of 1184 or more replicas per 148, and of 8: 6x8x16 4.5 / 13.6 on 64 and
+ * 4.9 / 9.6 on 128, L = 10 5.0 / 15.7 and 5.1 / 9.9; L = 18 22.0 / 45 on 128 and
+ * 23.9 / 32 on 256, L = 22 37.1 / 46 on 256 and 38.2 / 37 on 512).  Alone and
+ * without measurements (slsf_task_sweep) more threads shorten the sweep (us, 64
+ * / 128 / 256 / 512 threads: L = 8 9.8 / 9.0 / 9.3 / 10.4, L = 12 21 / 13.6 / 12.1
+ * / 12.7, L = 16 30 / 17.7 / 14.4 / 14.8, L = 20 73 / 40 / 29 / 25, L = 24 128 /
+ * 67 / 43 / 37). */
+uint32_t resident_threads(uint32_t lx, uint64_t v, bool alone) {
+    if (alone) return v <= 512 ? 128 : (v <= 4096 ? 256 : 512);
+    if (lx % 4) return v <= 512 ? 64 : (v <= 4096 ? 128 : (v <= 8192 ? 256 : 512));
+    return v <= 512 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512));
 }
 
 }  // namespace
@@ -321,7 +327,7 @@ int run_one_cta(slsf_task* t, TaskView v, uint32_t n_sweeps, unsigned long long 
     std::memset(st, 0, sizeof(unsigned long long) * slsf::kStatSlots);
     v.n_bins = 0; /* single-task updates do not measure */
     v.stats = st;
-    SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->volume, true), t->ctx->stream));
+    SLSF_CUDA(slsf::launch_resident_one(v, n_sweeps, resident_threads(t->lx, t->volume, true), t->ctx->stream));
     t->ctx->launches += 1;
     SLSF_CUDA(cudaStreamSynchronize(t->ctx->stream));
     std::memcpy(out, st, sizeof(unsigned long long) * slsf::kStatSlots);
@@ -1266,7 +1272,7 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
  * threads; else the grid-wide kernels. */
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
     if (slsf::resident_supports(lx, ly, lz, device))
-        return {slsf::kKernelResident, 1, resident_threads((uint64_t)lx * ly * lz, false)};
+        return {slsf::kKernelResident, 1, resident_threads(lx, (uint64_t)lx * ly * lz, false)};
     const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device);
     if (c && slsf::stream_fits(lx, ly, lz)) return {slsf::kKernelStream, 1, 256};
     if (c) return {slsf::kKernelCluster, c, 1024};

@@ -394,10 +394,19 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
 
 /* One colour half-sweep: the patch walk for L_x a multiple of 4, the site-by-site form for L_x = 2 mod 4, whose
  * pairs of compact sites straddle rows (and for couplings whose biased sums could overflow). */
+/* The patch walk from 1,024 sites on, where its units fill the block: a thread
+ * has at least one plane's four updates to do one after the other, and in a
+ * smaller lattice that chain is longer than half_sweep's, with a site per lane
+ * (us per sweep of 8 replicas alone, and of 2048 per 148 of them, walk and
+ * half_sweep: 4^3 8.2 / 3.2 and 5.6 / 2.4, 8^3 9.3 / 3.8 and 8.5 / 3.2; 12^3
+ * 13.3 / 7.4 and 27.7 / 9.5). */
+constexpr uint32_t kQuadSites = 1024;
+
 template <bool kMeasure>
 __device__ __forceinline__ uint32_t sweep_colour(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
                                                  uint32_t colour, double (&acc)[8]) {
-    if (g.lx % 4 == 0 && (!kMeasure || t.jmax < kJMax)) return half_sweep_quads<kMeasure>(t, g, s, sweep, colour, acc);
+    if (g.lx % 4 == 0 && g.volume >= kQuadSites && (!kMeasure || t.jmax < kJMax))
+        return half_sweep_quads<kMeasure>(t, g, s, sweep, colour, acc);
     return half_sweep<kMeasure>(t, g, s, sweep, colour, acc);
 }
 
