@@ -585,12 +585,12 @@ int slsf_task_create(slsf_ctx* ctx, const slsf_task_desc* d, slsf_task** out) {
         t->jmax = jv[i] < slsf::kJMax && jv[d->lz + i] < slsf::kJMax ? std::max(t->jmax, j)
                                                                     : std::numeric_limits<float>::infinity();
     }
-    /* theta, jxy and jz are separate 256-byte aligned arrays; zero the whole
-     * block, then copy J.  The copy is synchronous: jv is pageable. */
+    /* zero the whole block, then write the couplings, which travel in the
+     * launch; one wait for all of it */
     e = cudaMemsetAsync(block, 0, L.total, ctx->stream);
+    if (e == cudaSuccess) e = slsf::launch_set_couplings(t->jxy, t->jz, jv.data(), d->lz, ctx->stream);
+    ctx->launches += (d->lz + slsf::kCouplingsPerLaunch - 1) / slsf::kCouplingsPerLaunch;
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(t->jxy, jv.data(), 4ull * d->lz, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(t->jz, jv.data() + d->lz, 4ull * d->lz, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         ctx->pool.free(block, L.total);
         delete t;
@@ -1294,9 +1294,14 @@ slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uin
 }
 
 /* Tasks of one group share their launches: those of one kernel choice, with
- * or without fused correlations.  Groups run in descending rank (cluster first, grid-wide last). */
+ * or without fused correlations.  Groups start in descending rank: clusters,
+ * which need several free SMs at once, then the one-CTA kernel, then the
+ * stream kernel, whose CTAs fill an SM each and take up work as they find
+ * room, and grid-wide tasks last.  (With the stream kernel's 148 CTAs ahead the
+ * one-CTA groups waited for its end: 192 requests of 8^3 to 64^3 took 43.6 ms,
+ * 27.7 and 16.2 of them alone; behind them 38.2.) */
 uint64_t group_rank(const slsf_task* t, const slsf::KernelChoice& c) {
-    const uint64_t order[4] = {1, 3, 0, 2}; /* resident, cluster, grid, stream */
+    const uint64_t order[4] = {2, 3, 0, 1}; /* resident, cluster, grid, stream */
     const uint64_t fused = t->corr_interval ? 1u : 0u;
     return (order[c.kind] << 48) | (fused << 40) | ((uint64_t)c.cluster << 16) | c.threads;
 }

@@ -679,6 +679,16 @@ __global__ void k_gather(const double* const* __restrict__ src, uint32_t per, do
     for (uint32_t k = threadIdx.x; k < per; k += blockDim.x) d[k] = s[k];
 }
 
+struct Couplings {
+    float xy[kCouplingsPerLaunch], z[kCouplingsPerLaunch];
+};
+
+__global__ void k_set_couplings(float* __restrict__ jxy, float* __restrict__ jz, uint32_t n, const __grid_constant__ Couplings c) {
+    if (threadIdx.x >= n) return;
+    jxy[threadIdx.x] = c.xy[threadIdx.x];
+    jz[threadIdx.x] = c.z[threadIdx.x];
+}
+
 __global__ void k_publish_stats(unsigned long long* __restrict__ stats, unsigned long long* __restrict__ host) {
     const unsigned long long v = stats[threadIdx.x];
     host[threadIdx.x] = v;
@@ -686,6 +696,17 @@ __global__ void k_publish_stats(unsigned long long* __restrict__ stats, unsigned
 }
 
 }  // namespace
+
+cudaError_t launch_set_couplings(float* jxy, float* jz, const float* j, uint32_t lz, cudaStream_t s) {
+    for (uint32_t lo = 0; lo < lz; lo += kCouplingsPerLaunch) {
+        const uint32_t n = std::min(kCouplingsPerLaunch, lz - lo);
+        Couplings c = {};
+        std::copy(j + lo, j + lo + n, c.xy);
+        std::copy(j + lz + lo, j + lz + lo + n, c.z);
+        k_set_couplings<<<1, kCouplingsPerLaunch, 0, s>>>(jxy + lo, jz + lo, n, c);
+    }
+    return cudaGetLastError();
+}
 
 void launch_publish_stats(unsigned long long* stats, unsigned long long* host, cudaStream_t s) {
     k_publish_stats<<<1, kStatSlots, 0, s>>>(stats, host);
