@@ -748,8 +748,6 @@ int slsf_task_wolff_step_debug(slsf_task* t, uint8_t* bonds, uint8_t* cluster, f
     const int rc = e == cudaSuccess ? read_stats(t, st) : SLSF_OK;
     if (d_cluster) t->ctx->pool.free(d_cluster, align256(t->volume));
     if (e != cudaSuccess) return cuda_error(e, "wolff step");
-    if (bonds) /* the bond bits only (the kernels mark tile roots in bit 3) */
-        for (uint32_t i = 0; i < t->volume; ++i) bonds[i] &= 7u;
     if (rc) return rc;
     t->wolff_done += 1;
     if (phi) *phi = phi_h;

@@ -294,9 +294,6 @@ __device__ __forceinline__ bool uf_union(uint32_t* parent, uint32_t a, uint32_t 
 constexpr uint32_t kTileX = 32, kTileY = 8, kTileZ = 4;
 constexpr uint32_t kTileSites = kTileX * kTileY * kTileZ;
 static_assert(kTileX == 32, "a tile row is one warp");
-/* Bit 3 of a site's bond byte: the site is the root of its component inside
- * its tile (bits 0-2 are the +x/+y/+z bonds). */
-constexpr uint8_t kTileRoot = 8;
 
 /* Local union-find in shared memory: hook the larger root under the smaller
  * with a CAS; bounded like the global one. */
@@ -412,7 +409,6 @@ __global__ void __launch_bounds__(kThreads)
         const uint32_t rx = r % kTileX, ry = (r / kTileX) % kTileY, rz = r / (kTileX * kTileY);
         const uint32_t i = (x0 + ax) + lx * ((y0 + ay) + ly * (z0 + az));
         parent[i] = (x0 + rx) + lx * ((y0 + ry) + ly * (z0 + rz));
-        if (r == l) bonds[i] = (uint8_t)(lbits[l] | kTileRoot); /* marks the tile's roots for k_wolff_compress */
     }
     if (!ok) atomicOr(&stats[kStatError], kErrUnionFindLimit);
 }
@@ -466,43 +462,30 @@ __global__ void __launch_bounds__(kThreads)
     if (!ok) atomicOr(&stats[kStatError], kErrUnionFindLimit);
 }
 
-/* After the joins between tiles, every tile root points at its component's
- * root (path compression from the roots only: the other sites point at a
- * tile root, and nobody points at them). */
-__global__ void __launch_bounds__(kThreads)
-    k_wolff_compress(const uint8_t* __restrict__ bonds, uint32_t volume, uint32_t* parent,
-                     unsigned long long* stats, uint32_t limit) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= volume || !(bonds[i] & kTileRoot)) return;
-    /* A find without path splitting: the only writes in this kernel set a
-     * tile root's parent to its component's root, so every parent a thread
-     * reads leads to the same root (a split could write back a stale
-     * ancestor over a root already written). */
-    const volatile uint32_t* par = parent;
-    const uint32_t bound = uf_bounds(volume, limit).find;
-    uint32_t x = i;
-    for (uint32_t it = 0;; ++it) {
-        const uint32_t p = par[x];
-        if (p == x) break;
-        if (it >= bound) {
-            atomicOr(&stats[kStatError], kErrUnionFindLimit);
-            return;
-        }
-        x = p;
-    }
-    parent[i] = x;
-}
-
 /* Reflect the seed's component (src/updates.rs:602-617).  A site's parent is
- * a tile root whose parent is the component's root, so two loads find it. */
+ * its tile's root, which reaches the component's root in the few steps that
+ * the joins left; the array no longer changes, so every chain ends there.
+ * Finding the roots here, where the tiles' few roots come from the cache,
+ * saves a kernel that shortened the chains first (4.8 us of 58 at 64^3). */
 __global__ void __launch_bounds__(kThreads)
     k_wolff_flip(float* __restrict__ theta, uint32_t volume, const uint32_t* __restrict__ parent, uint32_t seed_idx,
-                 float phi, unsigned long long* stats, uint8_t* __restrict__ cluster_out) {
+                 float phi, unsigned long long* stats, uint8_t* __restrict__ cluster_out, uint32_t limit) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t bound = uf_bounds(volume, limit).find;
+    bool ok = true;
+    auto root_of = [&](uint32_t x) {
+        for (uint32_t it = 0; it <= bound; ++it) {
+            const uint32_t p = parent[x];
+            if (p == x) return x;
+            x = p;
+        }
+        ok = false;
+        return x;
+    };
     uint32_t in = 0;
     if (i < volume) {
-        const uint32_t root = parent[parent[seed_idx]];
-        in = (parent[parent[i]] == root) ? 1u : 0u;
+        in = root_of(i) == root_of(seed_idx) ? 1u : 0u;
+        if (!ok) atomicOr(&stats[kStatError], kErrUnionFindLimit);
         if (in) theta[i] = slsf_reflect(theta[i], phi);
         if (cluster_out) cluster_out[i] = (uint8_t)in;
     }
@@ -784,15 +767,14 @@ int launch_wolff(const TaskView& t, uint64_t counter, uint8_t* bonds, uint32_t* 
                                              t.seed, counter, bonds, parent, t.stats, t.loop_limit);
     k_wolff_boundary<<<blocks_for((uint64_t)tiles * kFaceRows * 32, kThreads), kThreads, 0, s>>>(
         bonds, t.lx, t.ly, t.lz, tiles, parent, t.stats, t.loop_limit);
-    k_wolff_compress<<<grid, kThreads, 0, s>>>(bonds, volume, parent, t.stats, t.loop_limit);
-    k_wolff_flip<<<grid, kThreads, 0, s>>>(t.theta, volume, parent, seed_idx, phi, t.stats, cluster_out);
+    k_wolff_flip<<<grid, kThreads, 0, s>>>(t.theta, volume, parent, seed_idx, phi, t.stats, cluster_out, t.loop_limit);
     if (phi_out) *phi_out = phi;
     if (seed_site) {
         seed_site[0] = x0;
         seed_site[1] = y0;
         seed_site[2] = z0;
     }
-    return 4;
+    return 3;
 }
 
 int measure_partial_blocks(uint32_t volume) {
