@@ -226,66 +226,60 @@ __global__ void __launch_bounds__(kThreads, 3)
 }
 
 /* Lattices whose Wolff update grows the seed's cluster on bit-packed bonds
- * (kernel_wolff_bits.cu) instead of labelling 32x8x4 tiles: from 2^19 sites,
- * and those of one growth region.  Measured on B200, us per sweep, bits against
- * tiles: 32^3 36.7 / 53.8, 24^3 47.4 / 51.5, 48^3 69.8 / 59.4, 64^3 71.7 /
- * 70.2, 80^3 91.2 / 86.1, 96^3 93.9 / 111, 100x90x70 88 / 97, 128^3 116 / 164,
- * 192^3 191 / 437: between, the chain of region closures is longer than the
- * tiles' union-find. */
-constexpr uint64_t kWolffBitsMinSites = 1u << 19;
+ * (kernel_wolff_bits.cu) instead of labelling 32x8x4 tiles: from 2^21 sites.
+ * Measured on B200, us per Metropolis and Wolff call, bits against tiles: 32^3
+ * 66 / 60, 30x32x24 74 / 58, 96^3 117 / 104, 150x148x30 135 / 100, 112^3 136 /
+ * 126, 128^3 141 / 141, 160^3 172 / 212: below, the chain of region closures is
+ * longer than the tiles' union-find, which labels every component. */
+constexpr uint64_t kWolffBitsMinSites = 1u << 21;
 
 inline bool wolff_by_bits(const TaskView& t) {
-    const bool one_region = t.lx <= 32 && t.ly <= 32 && t.lz <= 32;
-    return ((uint64_t)t.lx * t.ly * t.lz >= kWolffBitsMinSites || one_region) &&
+    return (uint64_t)t.lx * t.ly * t.lz >= kWolffBitsMinSites &&
            wolff_bits_scratch_bytes(t.lx, t.ly, t.lz) <= 4ull * t.lx * t.ly * t.lz;
 }
 
-/* ---- Wolff: union-find with links from larger to smaller roots ---- */
+/* ---- Wolff: union-find with links from larger to smaller indices ---- */
 
-/* Loop bounds of the union-find: a path is strictly decreasing, so at most
- * `volume` long; a union retries at most 2^22 times.  A nonzero `limit`
+/* Loop bounds of the union-find: parents are at most their children, so a path
+ * has at most `volume` steps and a union, which takes one down one of two
+ * paths each time round, at most twice as many.  A nonzero `limit`
  * (slsf_ctx_set_loop_limit) lowers both, to exercise the error path. */
 struct UfBounds {
-    uint32_t find, uni;
+    uint32_t find;
+    uint64_t uni;
 };
 
 __device__ __forceinline__ UfBounds uf_bounds(uint32_t volume, uint32_t limit) {
-    const uint32_t u = 1u << 22;
-    return {limit ? min(limit, volume) : volume, limit ? min(limit, u) : u};
+    const uint64_t u = 2ull * volume + 2;
+    return {limit ? min(limit, volume) : volume, limit && limit < u ? limit : u};
 }
 
-/* Root of x with path splitting.  parent[i] <= i always holds, so every path
- * is strictly decreasing; the loop is bounded by b.find. */
-__device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x, UfBounds b, bool* ok) {
+/* Lock-free union after Rem (Dijkstra, A Discipline of Programming, 1976; with
+ * splicing, Patwary, Blair and Manne 2010): climb both paths together, always
+ * from the node with the larger parent; a root is hooked under the other's
+ * parent by a CAS, any other node is pointed there as it is left (both belong
+ * to one component once this union is done, and parents stay below their
+ * children, so a store that another overtakes loses nothing but a shortcut).
+ * One dependent read a step, where finding both roots first took four: those
+ * reads of the global array, 300 ns each, are the time of k_wolff_boundary. */
+__device__ __forceinline__ bool uf_union(uint32_t* parent, uint32_t a, uint32_t b, uint64_t bound) {
     volatile uint32_t* par = parent;
-    for (uint32_t it = 0; it <= b.find; ++it) {
-        const uint32_t p = par[x];
-        if (p == x) return x;
-        const uint32_t gp = par[p];
-        if (gp != p) par[x] = gp;
-        x = p;
-    }
-    *ok = false;
-    return x;
-}
-
-/* Lock-free union: hook the larger root under the smaller with a CAS.  A
- * failed CAS means another thread linked that root; every retry follows some
- * other thread's progress, and the retry count is bounded. */
-__device__ __forceinline__ bool uf_union(uint32_t* parent, uint32_t a, uint32_t b, UfBounds bd) {
-    bool ok = true;
-    for (uint32_t it = 0; it < bd.uni; ++it) {
-        a = uf_find(parent, a, bd, &ok);
-        b = uf_find(parent, b, bd, &ok);
-        if (!ok) return false;
-        if (a == b) return true;
-        if (a > b) {
-            const uint32_t t = a;
-            a = b;
-            b = t;
+    uint32_t pa = par[a], pb = par[b];
+    for (uint64_t it = 0; it < bound; ++it) {
+        if (pa == pb) return true;
+        if (pa < pb) {
+            const uint32_t t = a, pt = pa;
+            a = b, pa = pb;
+            b = t, pb = pt;
         }
-        const uint32_t old = atomicCAS(&parent[b], b, a);
-        if (old == b) return true;
+        if (pa == a) { /* a root, as last read */
+            pa = atomicCAS(&parent[a], a, pb);
+            if (pa == a) return true;
+        } else {
+            par[a] = pb;
+            a = pa;
+            pa = par[a];
+        }
     }
     return false;
 }
@@ -294,37 +288,25 @@ __device__ __forceinline__ bool uf_union(uint32_t* parent, uint32_t a, uint32_t 
 constexpr uint32_t kTileX = 32, kTileY = 8, kTileZ = 4;
 constexpr uint32_t kTileSites = kTileX * kTileY * kTileZ;
 static_assert(kTileX == 32, "a tile row is one warp");
+/* Two rows a warp and phase: the unions' chains run side by side (us per call of
+ * Metropolis and Wolff on 256 / 512 / 1024 threads: 48^3 83 / 76 / 74, 100x12x138
+ * 87 / 81 / 79, 128^3 - / 141 / 152). */
+constexpr int kTileThreads = 512;
 
-/* Local union-find in shared memory: hook the larger root under the smaller
- * with a CAS; bounded like the global one. */
-__device__ __forceinline__ uint32_t tile_find(uint32_t* lpar, uint32_t x, UfBounds bd, bool* ok) {
+/* Root of x in a tile's shared array, splitting the path. */
+__device__ __forceinline__ uint32_t tile_find(uint32_t* lpar, uint32_t x, uint32_t bound, bool* ok) {
     volatile uint32_t* par = lpar;
-    for (uint32_t it = 0; it <= bd.find; ++it) {
-        const uint32_t p = par[x];
+    uint32_t p = par[x];
+    for (uint32_t it = 0; it <= bound; ++it) {
         if (p == x) return x;
         const uint32_t gp = par[p];
-        if (gp != p) par[x] = gp;
+        if (gp == p) return p;
+        par[x] = gp;
         x = p;
+        p = gp;
     }
     *ok = false;
     return x;
-}
-
-__device__ __forceinline__ bool tile_union(uint32_t* lpar, uint32_t a, uint32_t b, UfBounds bd) {
-    bool ok = true;
-    for (uint32_t it = 0; it < bd.uni; ++it) {
-        a = tile_find(lpar, a, bd, &ok);
-        b = tile_find(lpar, b, bd, &ok);
-        if (!ok) return false;
-        if (a == b) return true;
-        if (a > b) {
-            const uint32_t t = a;
-            a = b;
-            b = t;
-        }
-        if (atomicCAS(&lpar[b], b, a) == b) return true;
-    }
-    return false;
 }
 
 /* Bond activation (try_add_wolff_neighbor, src/updates.rs:537-548) for every
@@ -332,7 +314,7 @@ __device__ __forceinline__ bool tile_union(uint32_t* lpar, uint32_t a, uint32_t 
  * gets parent = the smallest site of its component inside the tile (local
  * order is global order inside a tile, so parent[i] <= i holds).  Bonds that
  * leave the tile are joined by k_wolff_boundary. */
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kTileThreads)
     k_wolff_tiles(const float* __restrict__ theta, const float* __restrict__ jxy,
                   const float* __restrict__ jz, uint32_t lx, uint32_t ly, uint32_t lz,
                   float minus_two_beta, float phi, uint64_t seed, uint64_t counter,
@@ -340,7 +322,6 @@ __global__ void __launch_bounds__(kThreads)
                   unsigned long long* __restrict__ stats, uint32_t limit) {
     __shared__ uint32_t lpar[kTileSites];
     const UfBounds bd = uf_bounds(kTileSites, limit);
-    const UfBounds bu = {bd.find, limit ? min(limit, 4 * kTileSites) : 4 * kTileSites};
     __shared__ uint8_t lbits[kTileSites];
     const uint32_t ntx = (lx + kTileX - 1) / kTileX, nty = (ly + kTileY - 1) / kTileY;
     const uint32_t tx = blockIdx.x % ntx, rest = blockIdx.x / ntx;
@@ -398,14 +379,14 @@ __global__ void __launch_bounds__(kThreads)
         const unsigned yrow = yin ? __ballot_sync(0xffffffffu, (lbits[l + kTileX] & 1u) && xin) : 0u;
         const unsigned zrow = zin ? __ballot_sync(0xffffffffu, (lbits[l + kTileX * kTileY] & 1u) && xin) : 0u;
         const unsigned ylead = yb & ~((yb & own & yrow) << 1), zlead = zb & ~((zb & own & zrow) << 1);
-        if ((ylead >> lane) & 1u) ok &= tile_union(lpar, l, l + kTileX, bu);
-        if ((zlead >> lane) & 1u) ok &= tile_union(lpar, l, l + kTileX * kTileY, bu);
+        if ((ylead >> lane) & 1u) ok &= uf_union(lpar, l, l + kTileX, bd.uni);
+        if ((zlead >> lane) & 1u) ok &= uf_union(lpar, l, l + kTileX * kTileY, bd.uni);
     }
     __syncthreads();
     for (uint32_t l = threadIdx.x; l < kTileSites; l += blockDim.x) {
         const uint32_t ax = l % kTileX, ay = (l / kTileX) % kTileY, az = l / (kTileX * kTileY);
         if (ax >= ex || ay >= ey || az >= ez) continue;
-        const uint32_t r = tile_find(lpar, l, bd, &ok);
+        const uint32_t r = tile_find(lpar, l, bd.find, &ok);
         const uint32_t rx = r % kTileX, ry = (r / kTileX) % kTileY, rz = r / (kTileX * kTileY);
         const uint32_t i = (x0 + ax) + lx * ((y0 + ay) + ly * (z0 + az));
         parent[i] = (x0 + rx) + lx * ((y0 + ry) + ly * (z0 + rz));
@@ -458,7 +439,7 @@ __global__ void __launch_bounds__(kThreads)
     const unsigned long long key = act ? (((unsigned long long)a << 32) | b) : ~0ull;
     const unsigned grp = __match_any_sync(0xffffffffu, key);
     bool ok = true;
-    if (act && lane == (uint32_t)(__ffs(grp) - 1) && a != b) ok = uf_union(parent, a, b, uf_bounds(volume, limit));
+    if (act && lane == (uint32_t)(__ffs(grp) - 1) && a != b) ok = uf_union(parent, a, b, uf_bounds(volume, limit).uni);
     if (!ok) atomicOr(&stats[kStatError], kErrUnionFindLimit);
 }
 
@@ -763,7 +744,7 @@ int launch_wolff(const TaskView& t, uint64_t counter, uint8_t* bonds, uint32_t* 
     const uint32_t grid = blocks_for(volume, kThreads);
     const uint32_t tiles = ((t.lx + kTileX - 1) / kTileX) * ((t.ly + kTileY - 1) / kTileY) *
                            ((t.lz + kTileZ - 1) / kTileZ);
-    k_wolff_tiles<<<tiles, kThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, -2.0f * t.beta, phi,
+    k_wolff_tiles<<<tiles, kTileThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, -2.0f * t.beta, phi,
                                              t.seed, counter, bonds, parent, t.stats, t.loop_limit);
     k_wolff_boundary<<<blocks_for((uint64_t)tiles * kFaceRows * 32, kThreads), kThreads, 0, s>>>(
         bonds, t.lx, t.ly, t.lz, tiles, parent, t.stats, t.loop_limit);
