@@ -119,8 +119,13 @@ TaskLayout layout_of(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t n_bins) {
 }  // namespace
 
 constexpr size_t kSmallReadBack = 256; /* bytes */
-/* Lattices up to this size sweep in one CTA even alone (slsf_task_sweep). */
-constexpr uint32_t kOneCtaSweepSites = 16384;
+/* Lattices up to these sizes run in one CTA even alone: whole sweeps
+ * (slsf_task_sweep), and a Metropolis sweep or Wolff step by itself, which the
+ * grid-wide kernels need fewer launches for (us per call with its round trip,
+ * one CTA / grid-wide: a sweep and a measurement at 16^3 49 / 60, 18^3 59 / 59,
+ * 20^3 58 / 61, 22^3 72 / 60, 24^3 69 / 61; the two updates at 16^3 46 / 55,
+ * 4x4x250 54 / 58, 18^3 62 / 55, 20^3 58 / 56, 24^3 71 / 56). */
+constexpr uint32_t kOneCtaSweepSites = 8192, kOneCtaUpdateSites = 5120;
 
 namespace {
 
@@ -314,12 +319,10 @@ int read_stats(slsf_task* t, unsigned long long out[slsf::kStatSlots]) {
     return SLSF_OK;
 }
 
-/* A small lattice's updates in one launch of the one-CTA kernel, which writes
- * the counters to the host's landing area: one sweep at L = 8 takes 9 us on
- * the GPU against 38 us in six launches, at L = 24 37 against 47; at L = 32 59
- * against 37, the whole GPU being faster than one SM. */
-bool one_cta_updates(const slsf_task* t) {
-    return t->volume <= kOneCtaSweepSites && slsf::resident_supports(t->lx, t->ly, t->lz, t->ctx->device);
+/* Whether an update of the task alone runs in one launch of the one-CTA
+ * kernel, which writes the counters to the host's landing area. */
+bool one_cta_updates(const slsf_task* t, uint32_t most) {
+    return t->volume <= most && slsf::resident_supports(t->lx, t->ly, t->lz, t->ctx->device);
 }
 
 int run_one_cta(slsf_task* t, TaskView v, uint32_t n_sweeps, unsigned long long out[slsf::kStatSlots]) {
@@ -703,7 +706,7 @@ int slsf_task_metropolis_sweep(slsf_task* t, double* acceptance) {
     if (int rc = bind_device(t->ctx)) return rc;
     unsigned long long st[slsf::kStatSlots];
     TaskView v = t->view();
-    if (one_cta_updates(t)) {
+    if (one_cta_updates(t, kOneCtaUpdateSites)) {
         v.wolff_steps = 0;
         if (int rc = run_one_cta(t, v, 1, st)) return rc;
     } else {
@@ -757,7 +760,7 @@ int slsf_task_wolff_step_debug(slsf_task* t, uint8_t* bonds, uint8_t* cluster, f
 }
 
 int slsf_task_wolff_step(slsf_task* t, uint64_t* cluster_size) {
-    if (t && !t->session && temperature_ok(t->temperature) && one_cta_updates(t)) {
+    if (t && !t->session && temperature_ok(t->temperature) && one_cta_updates(t, kOneCtaUpdateSites)) {
         if (int rc = bind_device(t->ctx)) return rc;
         unsigned long long st[slsf::kStatSlots];
         TaskView v = t->view();
@@ -775,7 +778,7 @@ int slsf_task_sweep(slsf_task* t, uint32_t n_sweeps, slsf_sweep_stats* stats) {
     if (!t) return set_error(SLSF_ERR_INVALID, "task is NULL");
     if (int rc = check_sweepable(t)) return rc;
     if (int rc = bind_device(t->ctx)) return rc;
-    if (n_sweeps && one_cta_updates(t)) {
+    if (n_sweeps && one_cta_updates(t, kOneCtaSweepSites)) {
         unsigned long long st[slsf::kStatSlots];
         const int rc = run_one_cta(t, t->view(), n_sweeps, st);
         if (rc && rc != SLSF_ERR_TIMEOUT) return rc;
