@@ -418,6 +418,7 @@ __device__ __forceinline__ float site_theta(const Geo& g, const Smem& s, uint32_
  * it through its y and z bonds; a row that gained bits is closed along x
  * (stored rows are always closed).  Rows updated earlier in the same pass are
  * seen by later ones, so bits can travel more than one row per pass. */
+constexpr int kLongRuns = 4; /* rows unrolled in the bond activation of 512-thread CTAs */
 constexpr int kGrowSteps = 3; /* steps of every row between two block barriers */
 
 /* One step of a row from the words around it; returns whether it changed. */
@@ -505,6 +506,7 @@ __device__ __forceinline__ uint32_t grow(const Geo& g, Smem& s, uint32_t bound) 
  * two Philox blocks share one key schedule.  Sub-groups past the last plane
  * compute on the last planes and keep nothing.  Bound by instruction issue:
  * one Philox block and three bond tests per site. */
+template <int kUnroll>
 __device__ __forceinline__ void wolff_bonds(const TaskView& t, const Geo& g, const Smem& s, uint64_t counter,
                                             float cphi, float sphi) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -537,6 +539,7 @@ __device__ __forceinline__ void wolff_bonds(const TaskView& t, const Geo& g, con
         float2 r = proj2(p0[col + o], p1[g.stride1 - col + o]);
         uint32_t idx = z * g.plane + y_lo * g.lx + xl;
         uint32_t k[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll kUnroll
         for (uint32_t y = y_lo; y < y_hi; ++y) {
             const uint32_t on = y + 1 == g.ly ? (xl >> 1) : o + hx, coln = g.stride1 - col;
             const float2 ry = proj2(p0[coln + on], p1[col + on]);
@@ -572,6 +575,7 @@ __device__ __forceinline__ void wolff_bonds(const TaskView& t, const Geo& g, con
 }
 
 /* One Wolff update (src/updates.rs:551-620); adds the cluster size to *count. */
+template <int kUnroll>
 __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Smem& s, uint64_t counter,
                                              uint32_t* s_count) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -580,7 +584,7 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
     const uint32_t x0 = slsf_range(pick.y, g.lx), y0 = slsf_range(pick.z, g.ly), z0 = slsf_range(pick.w, g.lz);
     float sphi, cphi;
     __sincosf(phi, &sphi, &cphi);
-    wolff_bonds(t, g, s, counter, cphi, sphi);
+    wolff_bonds<kUnroll>(t, g, s, counter, cphi, sphi);
     const uint32_t seed_row = row_word(g, y0, z0);
     for (uint32_t r = threadIdx.x; r < g.rows; r += blockDim.x) s.cl[r] = 0u;
     __syncthreads();
@@ -808,7 +812,7 @@ __device__ __forceinline__ void measure(const Geo& g, const Smem& s, double (&ac
 }
 
 
-template <bool kCorr, int kMaxThreads>
+template <bool kCorr, int kMaxThreads, int kUnroll>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_resident(const TaskView* __restrict__ views, uint32_t n, uint32_t n_sweeps, unsigned int* __restrict__ queue,
                uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, unsigned long long* __restrict__ counters,
@@ -869,7 +873,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
                 SLSF_PHASE(1);
             }
             for (uint32_t k = 0; k < t.wolff_steps; ++k)
-                wolff_update(t, g, s, t.wolff_done + (uint64_t)sw * t.wolff_steps + k, &s_cluster);
+                wolff_update<kUnroll>(t, g, s, t.wolff_done + (uint64_t)sw * t.wolff_steps + k, &s_cluster);
             /* ThetaModel::measure's correlations of the state after this sweep:
              * measurement m = sweep - thermalization, every corr_interval-th */
             if constexpr (kCorr) {
@@ -917,23 +921,23 @@ size_t smem_bytes(uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, uint3
     return 4ull * (max_volume + 2 * kPad) + 16ull * max_rows + 8ull * max_lz + 8ull * corr_doubles;
 }
 
-template <bool kCorr, int kMaxThreads>
+template <bool kCorr, int kMaxThreads, int kUnroll>
 cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_sweeps, unsigned int* queue,
                               int device, cudaStream_t s, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
                               uint32_t threads, unsigned long long* counters, const ResidentCorr* corr,
                               uint32_t corr_doubles) {
     const size_t smem = smem_bytes(max_volume, max_rows, max_lz, corr_doubles);
     const TaskView none = {};
-    cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr, kMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr, kMaxThreads, kUnroll>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int sms = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<kCorr, kMaxThreads>, (int)threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<kCorr, kMaxThreads, kUnroll>, (int)threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     const uint32_t grid = std::min<uint32_t>(n, (uint32_t)(sms * per_sm));
-    k_resident<kCorr, kMaxThreads><<<grid, threads, smem, s>>>(views_dev, n, n_sweeps, queue, max_volume, max_rows, max_lz,
+    k_resident<kCorr, kMaxThreads, kUnroll><<<grid, threads, smem, s>>>(views_dev, n, n_sweeps, queue, max_volume, max_rows, max_lz,
                                                   counters, corr, none);
     return cudaGetLastError();
 }
@@ -958,11 +962,11 @@ bool resident_supports(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
 cudaError_t launch_resident_one(const TaskView& t, uint32_t n_sweeps, uint32_t threads, cudaStream_t s) {
     const uint32_t volume = t.lx * t.ly * t.lz;
     const size_t smem = smem_bytes(volume, t.ly * t.lz, t.lz);
-    cudaError_t e = cudaFuncSetAttribute(k_resident<false, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_resident<false, 512, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     TaskView v = t;
     v.sweeps = n_sweeps;
-    k_resident<false, 512><<<1, threads, smem, s>>>(nullptr, 1, n_sweeps, nullptr, volume, t.ly * t.lz, t.lz, nullptr,
+    k_resident<false, 512, 1><<<1, threads, smem, s>>>(nullptr, 1, n_sweeps, nullptr, volume, t.ly * t.lz, t.lz, nullptr,
                                                     nullptr, v);
     return cudaGetLastError();
 }
@@ -976,22 +980,27 @@ cudaError_t launch_resident(const TaskView* views_dev, uint32_t n, uint32_t n_sw
                             uint32_t threads, unsigned long long* counters, const ResidentCorr* corr_dev,
                             uint32_t corr_doubles) {
     if (threads < 32 || threads > (uint32_t)kBThreads || threads % 32) return cudaErrorInvalidConfiguration;
-    /* the fused correlation measurement is compiled into its own instances, so
+    /* lattices that take 512 threads have long bond runs and an SM to
+     * themselves: four rows unrolled give 7.34e10 site-updates/s over 1184
+     * replicas of 32^3 for 7.20e10 (22^3 to 30^3 and 12x50x50 2 to 3 % more);
+     * smaller ones, whose CTAs share an SM's instruction cache, lose by it
+     *
+     * the fused correlation measurement is compiled into its own instances, so
      * groups without it run the kernel unchanged; CTAs of up to 512 threads
      * have 128 registers a thread (the patch walk and its compensated sums
      * need about 120), larger ones 64 and spill: 6.67e10 against 5.8e10
      * site-updates/s at L = 32 */
     if (corr_dev && corr_doubles)
-        return threads > 512 ? launch_resident_t<true, kBThreads>(views_dev, n, n_sweeps, queue, device, s, max_volume,
+        return threads > 512 ? launch_resident_t<true, kBThreads, 1>(views_dev, n, n_sweeps, queue, device, s, max_volume,
                                                                   max_rows, max_lz, threads, counters, corr_dev,
                                                                   corr_doubles)
-                             : launch_resident_t<true, 512>(views_dev, n, n_sweeps, queue, device, s, max_volume,
+                             : launch_resident_t<true, 512, 1>(views_dev, n, n_sweeps, queue, device, s, max_volume,
                                                             max_rows, max_lz, threads, counters, corr_dev,
                                                             corr_doubles);
-    return threads > 512 ? launch_resident_t<false, kBThreads>(views_dev, n, n_sweeps, queue, device, s, max_volume,
-                                                               max_rows, max_lz, threads, counters, nullptr, 0)
-                         : launch_resident_t<false, 512>(views_dev, n, n_sweeps, queue, device, s, max_volume,
-                                                         max_rows, max_lz, threads, counters, nullptr, 0);
+    const auto launch = threads > 512    ? launch_resident_t<false, kBThreads, 1>
+                        : threads == 512 ? launch_resident_t<false, 512, kLongRuns>
+                                         : launch_resident_t<false, 512, 1>;
+    return launch(views_dev, n, n_sweeps, queue, device, s, max_volume, max_rows, max_lz, threads, counters, nullptr, 0);
 }
 
 }  // namespace slsf
