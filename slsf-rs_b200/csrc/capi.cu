@@ -7,7 +7,7 @@
  *   theta    FP32 [V]          the state, x fastest (src/types.rs:146-149)
  *   jxy, jz  FP32 [Lz]         layer couplings
  *   bonds    u8   [V]          Wolff active-bond bits (+x, +y, +z)
- *   parent   u32  [V]          Wolff union-find forest
+ *   parent   u32  [V]          Wolff union-find forest, or bit planes and region queue
  *   partials FP64 [blocks][8]  measurement block sums
  *   result   FP64 [8]          measurement sums
  *   done     u32               last-block counter of the measurement
@@ -148,6 +148,14 @@ uint32_t resident_threads(uint32_t lx, uint64_t v, bool alone) {
     if (lx % 4) return v <= 512 ? 64 : (v <= 4096 ? 128 : (v <= 8192 ? 256 : 512));
     return v <= 512 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512));
 }
+
+/* The same for tasks that measure their correlations inside the sweeps: a lag
+ * takes a warp, so twice the threads cost a full GPU little and a few replicas
+ * gain much (us per sweep of 600 replicas, and of 16: 4x18x4 56 / 28 on 64 and
+ * 57 / 18 on 128, L = 8 49 / 23 and 51 / 15, L = 16 117 / 39 on 128 and 113 / 30
+ * on 256, L = 24 360 / 94 on 256 and 392 / 79 on 512; L = 4 30 / 13 on 64 and 35 /
+ * 10 on 128). */
+uint32_t fused_threads(uint64_t v) { return v <= 100 ? 64 : (v <= 1024 ? 128 : (v <= 16384 ? 256 : 512)); }
 
 }  // namespace
 
@@ -1271,9 +1279,11 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
 /* Without a tuned entry: the one-CTA kernel when the replica fits (threads for
  * a batch that fills the GPU), else the smallest cluster that holds it, 1024
  * threads; else the grid-wide kernels. */
-slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
-    if (slsf::resident_supports(lx, ly, lz, device))
-        return {slsf::kKernelResident, 1, resident_threads(lx, (uint64_t)lx * ly * lz, false)};
+slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device, bool fused = false) {
+    if (slsf::resident_supports(lx, ly, lz, device)) {
+        const uint64_t v = (uint64_t)lx * ly * lz;
+        return {slsf::kKernelResident, 1, fused ? fused_threads(v) : resident_threads(lx, v, false)};
+    }
     const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device);
     if (c && slsf::stream_fits(lx, ly, lz)) return {slsf::kKernelStream, 1, 256};
     if (c) return {slsf::kKernelCluster, c, 1024};
@@ -1288,10 +1298,10 @@ slsf::KernelChoice choice_of(const slsf_task* t, slsf::KernelChoice c) {
     return cl ? slsf::KernelChoice{slsf::kKernelCluster, cl, 1024} : slsf::KernelChoice{slsf::kKernelGrid, 1, 256};
 }
 
-slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uint32_t lz) {
+slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uint32_t lz, bool fused = false) {
     const auto it = ctx->tune.find(shape_key(lx, ly, lz));
     if (it != ctx->tune.end()) return it->second;
-    return default_choice(lx, ly, lz, ctx->device);
+    return default_choice(lx, ly, lz, ctx->device, fused);
 }
 
 /* Tasks of one group share their launches: those of one kernel choice, with
@@ -1394,7 +1404,7 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
     slsf_task* const* tasks = task_list.data();
     if (n == 0) return SLSF_OK;
     if (int rc = bind_device(ctx)) return rc;
-    /* Kernel of each task (kernel_resident.cu, kernel_cluster.cu, or the
+    /* Kernel of each task (kernel_resident.cu, kernel_stream.cu, kernel_cluster.cu, or the
      * grid-wide single-task kernels of kernels_plain.cu for lattices too
      * large for one cluster's shared memory, which fill the GPU on their
      * own), from the context's tuning table or the default. */
@@ -1403,7 +1413,7 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
         slsf_task* t = tasks[i];
         if (!t || t->ctx != ctx) return set_error(SLSF_ERR_INVALID, "task does not belong to this context");
         if (int rc = check_sweepable(t)) return rc;
-        ch[i] = choice_of(t, force ? *force : choice_for(ctx, t->lx, t->ly, t->lz));
+        ch[i] = choice_of(t, force ? *force : choice_for(ctx, t->lx, t->ly, t->lz, t->corr_interval != 0));
         if (!choice_feasible(ch[i], t->lx, t->ly, t->lz, ctx->device))
             return set_error(SLSF_ERR_INVALID, "the kernel choice does not hold this lattice");
         if (t->corr_interval && (ch[i].kind == slsf::kKernelCluster || ch[i].kind == slsf::kKernelStream))
@@ -1562,7 +1572,7 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
         if (int rc = check_sweepable(t)) return rc;
         for (size_t j = 0; j < i; ++j)
             if (tasks[j] == t) return set_error(SLSF_ERR_INVALID, "a task appears twice in the session");
-        ch[i] = choice_of(t, choice_for(ctx, t->lx, t->ly, t->lz));
+        ch[i] = choice_of(t, choice_for(ctx, t->lx, t->ly, t->lz, t->corr_interval != 0));
         if (ch[i].kind == slsf::kKernelGrid || !choice_feasible(ch[i], t->lx, t->ly, t->lz, ctx->device))
             return set_error(SLSF_ERR_INVALID,
                              "batch sessions hold lattices that fit one thread-block cluster's shared memory");

@@ -37,8 +37,6 @@ namespace {
 
 constexpr uint32_t kStreamThreads = 512; /* one CTA per SM: 128 registers a thread */
 constexpr uint32_t kStreamRows = 8;      /* rows per thread in the growth */
-constexpr uint32_t kSegPlanes = 8;       /* planes per thread of a walk */
-constexpr uint32_t kBondRun = 16;        /* rows per warp of the bond activation */
 constexpr uint32_t kFlipQuads = 8;       /* quads per thread of a reflection */
 constexpr uint32_t kRingEntries = 1u << 20;
 constexpr uint32_t kChunkBits = 12;
@@ -53,23 +51,31 @@ struct StreamCtl {
 };
 
 /* Sizes of the chunks of a launch.  A phase is a row of blocks of one CTA's
- * threads (walks of kSegPlanes planes per thread, a run of rows per warp,
+ * threads (walks of seg_planes planes per thread, a run of rows per warp,
  * kFlipQuads quads per thread); a chunk takes `per` of them one after the other.  The
  * blocks, and so the order of the measured sums, are the same in every launch. */
 struct StreamShape {
-    uint32_t per;     /* blocks per chunk */
+    uint32_t per;      /* blocks per chunk */
+    uint32_t bond_run; /* rows per warp of the bond activation */
     uint32_t growers; /* CTAs that grow a replica's cluster together by regions; 1: one CTA by rows */
 };
 
 __host__ __device__ inline uint32_t smaller(uint32_t a, uint32_t b) { return a < b ? a : b; }
 
-__host__ __device__ inline uint32_t blocks_of(const TaskView& t, uint32_t phase) {
+/* Planes per thread of a replica's walks, by its size alone: the order of the
+ * measured sums hangs on it.  Fewer planes shorten a lone replica's phases and
+ * start more walks (us per sweep, 4 and 8 planes: one 40^3 84 / 96, one 56^3 109
+ * / 120, thirty-two 64x64x40 137 / 144); the largest replicas fill the GPU with
+ * 8 already (thirty-two 64^3 233 / 218). */
+__host__ __device__ inline uint32_t seg_planes(const TaskView& t) { return t.lx * t.ly * t.lz >= 200000 ? 8 : 4; }
+
+__host__ __device__ inline uint32_t blocks_of(const TaskView& t, const StreamShape& sh, uint32_t phase) {
     switch (phase) {
         case kColour0:
         case kColour1:
-        case kMeasureLast: return (walk_units(t, kSegPlanes) + kStreamThreads - 1) / kStreamThreads;
+        case kMeasureLast: return (walk_units(t, seg_planes(t)) + kStreamThreads - 1) / kStreamThreads;
         case kBonds: {
-            const uint32_t warps = ((t.lx + 31) / 32) * (t.lz / 2) * ((t.ly + kBondRun - 1) / kBondRun);
+            const uint32_t warps = ((t.lx + 31) / 32) * (t.lz / 2) * ((t.ly + sh.bond_run - 1) / sh.bond_run);
             return (warps + kStreamThreads / 32 - 1) / (kStreamThreads / 32);
         }
         case kFlip: return ((t.lx >> 2) * t.ly * t.lz + kStreamThreads * kFlipQuads - 1) / (kStreamThreads * kFlipQuads);
@@ -79,7 +85,7 @@ __host__ __device__ inline uint32_t blocks_of(const TaskView& t, uint32_t phase)
 
 __host__ __device__ inline uint32_t chunks_of(const TaskView& t, const StreamShape& sh, uint32_t phase) {
     if (phase == kGrow) return smaller(sh.growers, (uint32_t)bit_regions(t.lx, t.ly, t.lz));
-    return (blocks_of(t, phase) + sh.per - 1) / sh.per;
+    return (blocks_of(t, sh, phase) + sh.per - 1) / sh.per;
 }
 
 /* The phase after `c` for sweeps below sw_hi of the launch. */
@@ -255,26 +261,26 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         /* bin row of the state that colour 0 starts from, or of the last state */
         double* bin_row = nullptr;
         if ((c.phase == kColour0 && c.sweep > 0) || c.phase == kMeasureLast) bin_row = bin_row_of(t, sweep);
-        const uint32_t b_lo = chunk * sh.per, b_hi = smaller(b_lo + sh.per, blocks_of(t, c.phase));
+        const uint32_t b_lo = chunk * sh.per, b_hi = smaller(b_lo + sh.per, blocks_of(t, sh, c.phase));
         if (c.phase == kColour1 || (c.phase == kColour0 && !bin_row)) {
             uint32_t accepted = 0;
             for (uint32_t b = b_lo; b < b_hi; ++b)
-                accepted += walk_colour<false>(t, sweep, c.phase == kColour1, kSegPlanes, b * kStreamThreads + threadIdx.x, nullptr);
+                accepted += walk_colour<false>(t, sweep, c.phase == kColour1, seg_planes(t), b * kStreamThreads + threadIdx.x, nullptr);
             count_into(accepted, t.stats, kStatAccepted);
         } else if (c.phase == kColour0 || c.phase == kMeasureLast) {
             uint32_t accepted = 0;
             for (uint32_t b = b_lo; b < b_hi && bin_row; ++b) {
                 Sum2 sum[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, kSegPlanes, k));
+                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, seg_planes(t), k));
                 const uint32_t unit = b * kStreamThreads + threadIdx.x;
                 if (c.phase == kColour0)
-                    accepted += walk_colour<true>(t, sweep, 0, kSegPlanes, unit, sum);
+                    accepted += walk_colour<true>(t, sweep, 0, seg_planes(t), unit, sum);
                 else
-                    walk_measure(t, kSegPlanes, unit, sum);
+                    walk_measure(t, seg_planes(t), unit, sum);
                 double acc[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, kSegPlanes, k));
+                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, seg_planes(t), k));
                 block_sum<8>(acc, scratch);
                 if (threadIdx.x == 0)
 #pragma unroll
@@ -297,7 +303,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
                 const BitPlanes planes = stream_planes(t);
                 for (uint32_t b = b_lo; b < b_hi; ++b)
                     bond_run<2>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, __fmul_rn(-2.0f, t.beta), phi, t.seed, counter, planes,
-                                kBondRun, (b * kStreamThreads + threadIdx.x) >> 5, nullptr);
+                                sh.bond_run, (b * kStreamThreads + threadIdx.x) >> 5, nullptr);
             } else if (c.phase == kGrow && sh.growers > 1) {
                 grow_regions<2>(carve_bits(t.bits, t.lx, t.ly, t.lz), grow_geo(t.lx, t.ly, t.lz),
                                 t.loop_limit ? t.loop_limit : max(64u, t.lx * t.ly * t.lz / 32), t.stats);
@@ -334,7 +340,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         if (bin_row) { /* the blocks' sums in order */
             if (threadIdx.x < 8) {
                 double a = 0.0;
-                for (uint32_t k = 0; k < blocks_of(t, c.phase); ++k) a += __ldcg(&t.partials[k * 8 + threadIdx.x]);
+                for (uint32_t k = 0; k < blocks_of(t, sh, c.phase); ++k) a += __ldcg(&t.partials[k * 8 + threadIdx.x]);
                 scratch[threadIdx.x] = a;
             }
             __syncthreads();
@@ -398,7 +404,7 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
     /* as many blocks per chunk as leave three chunks of the walks per SM (each
      * chunk costs about 2 us in the queue and its fences: 1.42 against 1.28 ms per
      * sweep of 300 replicas of 64^3) */
-    StreamShape sh = {8, 1};
+    StreamShape sh = {8, 16, 1};
     uint64_t sites = 0;
     for (uint32_t i = 0; i < n; ++i) sites = std::max(sites, (uint64_t)host_views[i].lx * host_views[i].ly * host_views[i].lz);
     auto chunks = [&]() {
@@ -407,12 +413,14 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
         return c;
     };
     while (sh.per > 1 && chunks() < 3ull * sms) sh.per >>= 1;
+    if (chunks() < (uint64_t)sms) sh.bond_run = 8; /* few walks: one 56^3 109 -> 104 us, eight 117 -> 112 */
     /* several CTAs grow a large replica together while there are SMs for them
      * (us per sweep, together / by rows: one 64^3 150 / 178, sixteen 180 / 226,
-     * thirty-two 236 / 248, sixty-four 373 / 336; at 48^3 and 36^3 the cut regions
+     * thirty-two 236 / 248, sixty-four 373 / 336; one 56^3 121 / 130, sixteen 133 /
+     * 139, thirty-two 171 / 145; at 48^3 and 36^3 the cut regions
      * make it slower: sixteen 136 / 121 and 126 / 100) */
-    if (sites >= 200000)
-        while (sh.growers < 8 && 2ull * sh.growers * n <= (uint64_t)sms) sh.growers <<= 1;
+    if (sites >= 150000)
+        while (sh.growers < 8 && (sites >= 200000 ? 2ull : 4ull) * sh.growers * n <= (uint64_t)sms) sh.growers <<= 1;
     if (sh.growers < 4) sh.growers = 1;
     uint64_t most = 1;
     uint32_t rows = 0, sweeps = 0;
