@@ -656,7 +656,7 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
             e = cudaFuncSetAttribute(k_corr_zfft, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem);
             if (e != cudaSuccess) return e;
             /* blocks loop over the units, so each computes its twiddle tables
-             * once: four per SM (the kernel's occupancy) */
+             * once: three per SM (the kernel's occupancy) */
             const uint32_t zgrid = sm_count > 0 ? std::min<uint32_t>(n_zunits, 3u * (uint32_t)sm_count) : n_zunits;
             k_corr_zfft<<<zgrid, kCorrThreads, zsmem, s>>>(one ? nullptr : tasks_dev, by_value, n_tasks, n_zunits);
             e = cudaGetLastError();

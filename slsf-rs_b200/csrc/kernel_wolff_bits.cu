@@ -1,9 +1,8 @@
 /*
  * Single-task Wolff update on bit-packed bonds: grows the seed's cluster
- * only, for lattices whose three sides are multiples of 32 (the large
- * single-replica lattices: L = 64 ... 256 and more).
+ * only, for large single-replica lattices of any sides (kWolffBitsMinSites).
  *
- * Replaces, for those shapes, the whole-lattice union-find labelling of
+ * Replaces, for those sizes, the whole-lattice union-find labelling of
  * kernels_plain.cu.  The reference grows one cluster from a random seed by
  * depth-first search (wolff_cluster_step_with_theta_scratch,
  * src/updates.rs:551-620); with one counter-based random per bond, that

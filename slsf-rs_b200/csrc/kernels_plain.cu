@@ -9,18 +9,19 @@
  *                        it starts from (the batched grid path)
  *   k_wolff_tiles        per-site +x/+y/+z bond activation of
  *   k_wolff_boundary     wolff_cluster_step_with_theta_scratch
- *   k_wolff_compress     (src/updates.rs:551-620): components inside
- *   k_wolff_flip         32x8x4 tiles by union-find in shared memory, the
+ *   k_wolff_flip         (src/updates.rs:551-620): components inside
+ *                        32x8x4 tiles by union-find in shared memory, the
  *                        bonds between tiles by a lock-free global
- *                        union-find over the tile roots, the tile roots
- *                        pointed at their component's root, then reflect
- *                        the seed's component
+ *                        union-find over the tile roots, then reflect the
+ *                        seed's component
  *   k_measure            measure_theta_observables_with_scratch
  *                        (src/observables.rs:80-154), FP64 block sums, fixed
  *                        summation order (last block reduces the partials);
  *   k_measure_rows       the same with warps walking rows (L_x a multiple of
  *                        32): two sincos per site instead of four
  *
+ * Metropolis and measurement here take the shapes that the patch walks of
+ * kernel_walk.cu do not; the Wolff kernels lattices below kWolffBitsMinSites.
  * (The correlation functions are in kernel_corr.cu, batched over tasks.)
  */
 #include <algorithm>
