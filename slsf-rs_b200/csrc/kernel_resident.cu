@@ -626,12 +626,21 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
             *odd = o;
         }
     } else {
-        for (uint32_t idx = threadIdx.x; idx < g.volume; idx += blockDim.x) {
-            const Coords c = coords_of(g, idx);
-            if ((s.cl[row_word(g, c.y, c.z)] >> c.x) & 1u) {
-                const uint32_t sl = slot(g, idx, (c.x + c.y + c.z) & 1u);
-                s.th[sl] = slsf_reflect(s.th[sl], phi);
-            }
+        /* rows of 2 mod 4: a pair of neighbours, one site of each colour (a site
+         * per thread took 53 us per sweep of a few 26^3 where this takes 51, and
+         * 95 of 30^3 on 256 threads for 87) */
+        const uint32_t hx = g.lx >> 1;
+        for (uint32_t i = threadIdx.x; i < g.half; i += blockDim.x) {
+            const uint32_t r = slsf_fastdiv_div(i, g.div_hx), k = i - r * hx;
+            const uint32_t z = slsf_fastdiv_div(r, g.div_ly), y = r - z * g.ly;
+            const uint32_t m = s.cl[row_word(g, y, z)] >> (2 * k) & 3u;
+            if (!m) continue;
+            const uint32_t p = (y + z) & 1u;
+            float* even = s.th + p * g.stride1 + i;
+            float* odd = s.th + (p ^ 1u) * g.stride1 + i;
+            const float e = *even, o = *odd, e_new = slsf_reflect(e, phi), o_new = slsf_reflect(o, phi);
+            *even = (m & 1u) ? e_new : e;
+            *odd = (m & 2u) ? o_new : o;
         }
     }
 #pragma unroll
