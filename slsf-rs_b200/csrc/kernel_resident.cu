@@ -574,11 +574,9 @@ __device__ __forceinline__ void wolff_bonds(const TaskView& t, const Geo& g, con
     }
 }
 
-/* One Wolff update (src/updates.rs:551-620); adds the cluster size to *count. */
+/* One Wolff update (src/updates.rs:551-620); returns the thread's share of the cluster size. */
 template <int kUnroll>
-__device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Smem& s, uint64_t counter,
-                                             uint32_t* s_count) {
-    const uint32_t lane = threadIdx.x & 31u;
+__device__ __forceinline__ uint32_t wolff_update(const TaskView& t, const Geo& g, Smem& s, uint64_t counter) {
     const slsf_u32x4 pick = slsf_stream(t.seed, counter, SLSF_PURPOSE_WOLFF_PICK, 0, 0);
     const float phi = slsf_angle_from_word(pick.x);
     const uint32_t x0 = slsf_range(pick.y, g.lx), y0 = slsf_range(pick.z, g.ly), z0 = slsf_range(pick.w, g.lz);
@@ -643,11 +641,16 @@ __device__ __forceinline__ void wolff_update(const TaskView& t, const Geo& g, Sm
             *odd = (m & 2u) ? o_new : o;
         }
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) members += __shfl_down_sync(0xffffffffu, members, off);
-    if (lane == 0 && members) atomicAdd(s_count, members);
     __syncthreads();
     SLSF_PHASE(4);
+    return members;
+}
+
+/* Adds a per-thread count of the whole item to a shared total. */
+__device__ __forceinline__ void item_total(unsigned long long v, unsigned long long* total) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31u) == 0 && v) atomicAdd(total, v);
 }
 
 /* (cos, sin) of the site (x, y, z) of the resident state. */
@@ -830,8 +833,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     __shared__ double red[8 * 32];
     __shared__ double bin_acc[kBinCols];
     __shared__ uint32_t s_item;
-    __shared__ uint32_t s_cluster;
-    __shared__ uint32_t s_accepted;
+    /* 64 bits: an item's counts run over all of its sweeps (2^32 accepted sites are 131,072 sweeps at 32^3) */
+    __shared__ unsigned long long s_cluster;
+    __shared__ unsigned long long s_accepted;
     for (bool first = true;; first = false) {
         __syncthreads();
         if (threadIdx.x == 0) s_item = queue ? atomicAdd(queue, 1u) : (first ? 0u : n);
@@ -855,7 +859,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         if (threadIdx.x == 0) s_phase_mark = clock64();
 #endif
         const uint32_t sweeps = t.sweeps ? t.sweeps : n_sweeps;
-        uint32_t accepted = 0;
+        unsigned long long accepted = 0, cluster_sites = 0;
         int64_t bin_cur = -1;
         /* ThetaModel::measure after every sweep past thermalization: the state
          * after sweep k is measured inside sweep k+1's colour-0 half-sweep,
@@ -882,7 +886,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
                 SLSF_PHASE(1);
             }
             for (uint32_t k = 0; k < t.wolff_steps; ++k)
-                wolff_update<kUnroll>(t, g, s, t.wolff_done + (uint64_t)sw * t.wolff_steps + k, &s_cluster);
+                cluster_sites += wolff_update<kUnroll>(t, g, s, t.wolff_done + (uint64_t)sw * t.wolff_steps + k);
             /* ThetaModel::measure's correlations of the state after this sweep:
              * measurement m = sweep - thermalization, every corr_interval-th */
             if constexpr (kCorr) {
@@ -909,14 +913,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
             if (threadIdx.x == 0) bin_measurement(t, g.volume, last, acc, bin_acc, bin_cur);
         }
         if (threadIdx.x == 0) flush_bin(t, bin_acc, bin_cur);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) accepted += __shfl_down_sync(0xffffffffu, accepted, off);
-        if ((threadIdx.x & 31u) == 0 && accepted) atomicAdd(&s_accepted, accepted);
+        item_total(accepted, &s_accepted);
+        item_total(cluster_sites, &s_cluster);
         __syncthreads();
         store_state(t, g, s);
         if (threadIdx.x == 0 && views) {
-            atomicAdd(&t.stats[kStatAccepted], (unsigned long long)s_accepted);
-            atomicAdd(&t.stats[kStatClusterSites], (unsigned long long)s_cluster);
+            atomicAdd(&t.stats[kStatAccepted], s_accepted);
+            atomicAdd(&t.stats[kStatClusterSites], s_cluster);
             atomicAdd(&t.stats[kStatClusters], (unsigned long long)sweeps * t.wolff_steps);
         } else if (threadIdx.x == 0) { /* the call's counters, to the host (t.stats is pinned memory) */
             t.stats[kStatAccepted] = s_accepted;
