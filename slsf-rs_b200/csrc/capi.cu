@@ -83,6 +83,24 @@ uint32_t corr_launch_count(uint32_t items, uint32_t z_items, uint32_t layers) {
  * counter. */
 constexpr int kSideStreams = 7;
 
+/* Largest of n couplings (none is negative, but a NaN passes the checks of
+ * slsf_task_create); infinite if any is not below kJMax.  The bits of
+ * nonnegative floats compare as integers, NaN above all others: a maximum that
+ * the compiler vectorises, where one over floats (100 us for 2^17 layers) is a
+ * serial chain. */
+float largest_coupling(const float* j, size_t n) {
+    int32_t most = 0;
+    for (size_t i = 0; i < n; ++i) {
+        int32_t bits;
+        std::memcpy(&bits, &j[i], 4);
+        bits &= 0x7fffffff;
+        most = bits > most ? bits : most;
+    }
+    float v;
+    std::memcpy(&v, &most, 4);
+    return v < slsf::kJMax ? v : std::numeric_limits<float>::infinity();
+}
+
 /* Offsets of the arrays inside a task's block. */
 struct TaskLayout {
     uint64_t theta, jxy, jz, bonds, parent, partials, result, done, stats, bins, total;
@@ -589,18 +607,14 @@ int slsf_task_create(slsf_ctx* ctx, const slsf_task_desc* d, slsf_task** out) {
     t->stats = reinterpret_cast<unsigned long long*>(b + L.stats);
     t->bins = reinterpret_cast<double*>(b + L.bins);
     std::vector<float> jv(2 * (size_t)d->lz);
-    for (uint32_t i = 0; i < d->lz; ++i) {
-        jv[i] = (float)d->j_xy[i];
-        jv[d->lz + i] = (float)d->j_z[i];
-        const float j = std::max(jv[i], jv[d->lz + i]);
-        t->jmax = jv[i] < slsf::kJMax && jv[d->lz + i] < slsf::kJMax ? std::max(t->jmax, j)
-                                                                    : std::numeric_limits<float>::infinity();
-    }
+    for (uint32_t i = 0; i < d->lz; ++i) jv[i] = (float)d->j_xy[i];
+    for (uint32_t i = 0; i < d->lz; ++i) jv[d->lz + i] = (float)d->j_z[i];
+    t->jmax = largest_coupling(jv.data(), jv.size());
     /* zero the whole block, then write the couplings, which travel in the
      * launch; one wait for all of it */
     e = cudaMemsetAsync(block, 0, L.total, ctx->stream);
     if (e == cudaSuccess) e = slsf::launch_set_couplings(t->jxy, t->jz, jv.data(), d->lz, ctx->stream);
-    ctx->launches += (d->lz + slsf::kCouplingsPerLaunch - 1) / slsf::kCouplingsPerLaunch;
+    ctx->launches += slsf::set_couplings_launches(d->lz);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         ctx->pool.free(block, L.total);

@@ -81,9 +81,12 @@ constexpr uint32_t kKernelResident = 0, kKernelCluster = 1, kKernelGrid = 2, kKe
 int report_error(int code, const std::string& message);
 
 /* ---- single-task kernels (kernels_plain.cu) ---- */
-/* Writes a task's couplings (j: lz of J_xy, then lz of J_z), carried by the
- * launches' parameters, kCouplingsPerLaunch layers each. */
-constexpr uint32_t kCouplingsPerLaunch = 256;
+/* Writes a task's couplings (j: lz of J_xy, then lz of J_z; kept by the caller
+ * until the stream is done): carried by the launches' parameters,
+ * kCouplingsPerLaunch layers each, or by two copies where that takes more than
+ * kCouplingsLaunches launches.  set_couplings_launches: kernels launched. */
+constexpr uint32_t kCouplingsPerLaunch = 256, kCouplingsLaunches = 4;
+uint32_t set_couplings_launches(uint32_t lz);
 cudaError_t launch_set_couplings(float* jxy, float* jz, const float* j, uint32_t lz, cudaStream_t s);
 /* Copies a task's counters to pinned host memory and clears them. */
 void launch_publish_stats(unsigned long long* stats, unsigned long long* host, cudaStream_t s);

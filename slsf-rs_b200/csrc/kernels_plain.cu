@@ -662,7 +662,16 @@ __global__ void k_publish_stats(unsigned long long* __restrict__ stats, unsigned
 
 }  // namespace
 
+uint32_t set_couplings_launches(uint32_t lz) {
+    const uint32_t n = (lz + kCouplingsPerLaunch - 1) / kCouplingsPerLaunch;
+    return n <= kCouplingsLaunches ? n : 0;
+}
+
 cudaError_t launch_set_couplings(float* jxy, float* jz, const float* j, uint32_t lz, cudaStream_t s) {
+    if (set_couplings_launches(lz) == 0) {
+        const cudaError_t e = cudaMemcpyAsync(jxy, j, 4ull * lz, cudaMemcpyHostToDevice, s);
+        return e != cudaSuccess ? e : cudaMemcpyAsync(jz, j + lz, 4ull * lz, cudaMemcpyHostToDevice, s);
+    }
     for (uint32_t lo = 0; lo < lz; lo += kCouplingsPerLaunch) {
         const uint32_t n = std::min(kCouplingsPerLaunch, lz - lo);
         Couplings c = {};
