@@ -239,10 +239,10 @@ inline bool wolff_by_bits(const TaskView& t) {
            wolff_bits_scratch_bytes(t.lx, t.ly, t.lz) <= 4ull * t.lx * t.ly * t.lz;
 }
 
-/* ---- Wolff: union-find with links from larger to smaller indices ---- */
+/* ---- Wolff: union-find with links down a total order of the nodes ---- */
 
-/* Loop bounds of the union-find: parents are at most their children, so a path
- * has at most `volume` steps and a union, which takes one down one of two
+/* Loop bounds of the union-find: parents are at most their children in the
+ * order, so a path has at most `volume` steps and a union, which takes one down one of two
  * paths each time round, at most twice as many.  A nonzero `limit`
  * (slsf_ctx_set_loop_limit) lowers both, to exercise the error path. */
 struct UfBounds {
@@ -262,13 +262,27 @@ __device__ __forceinline__ UfBounds uf_bounds(uint32_t volume, uint32_t limit) {
  * to one component once this union is done, and parents stay below their
  * children, so a store that another overtakes loses nothing but a shortcut).
  * One dependent read a step, where finding both roots first took four: those
- * reads of the global array, 300 ns each, are the time of k_wolff_boundary. */
+ * reads of the global array, 300 ns each, are the time of k_wolff_boundary.
+ *
+ * The order is that of the indices in a tile (kScatter false), where a warp's
+ * runs are short, and that of a bijective hash of them between the tiles: a
+ * row of tiles ordered by index hangs every root on its neighbour's, a chain
+ * as long as the row that the union across the period and every thread of the
+ * reflection climb, while a random order (Goel, Khanna, Larkin and Tarjan,
+ * Disjoint set union with randomized linking, 2014) keeps the expected depth
+ * logarithmic. */
+template <bool kScatter>
+__device__ __forceinline__ uint32_t uf_order(uint32_t i) {
+    return kScatter ? i * 2654435769u : i; /* odd factor, 2^32 / golden ratio */
+}
+
+template <bool kScatter>
 __device__ __forceinline__ bool uf_union(uint32_t* parent, uint32_t a, uint32_t b, uint64_t bound) {
     volatile uint32_t* par = parent;
     uint32_t pa = par[a], pb = par[b];
     for (uint64_t it = 0; it < bound; ++it) {
         if (pa == pb) return true;
-        if (pa < pb) {
+        if (uf_order<kScatter>(pa) < uf_order<kScatter>(pb)) {
             const uint32_t t = a, pt = pa;
             a = b, pa = pb;
             b = t, pb = pt;
@@ -380,8 +394,8 @@ __global__ void __launch_bounds__(kTileThreads)
         const unsigned yrow = yin ? __ballot_sync(0xffffffffu, (lbits[l + kTileX] & 1u) && xin) : 0u;
         const unsigned zrow = zin ? __ballot_sync(0xffffffffu, (lbits[l + kTileX * kTileY] & 1u) && xin) : 0u;
         const unsigned ylead = yb & ~((yb & own & yrow) << 1), zlead = zb & ~((zb & own & zrow) << 1);
-        if ((ylead >> lane) & 1u) ok &= uf_union(lpar, l, l + kTileX, bd.uni);
-        if ((zlead >> lane) & 1u) ok &= uf_union(lpar, l, l + kTileX * kTileY, bd.uni);
+        if ((ylead >> lane) & 1u) ok &= uf_union<false>(lpar, l, l + kTileX, bd.uni);
+        if ((zlead >> lane) & 1u) ok &= uf_union<false>(lpar, l, l + kTileX * kTileY, bd.uni);
     }
     __syncthreads();
     for (uint32_t l = threadIdx.x; l < kTileSites; l += blockDim.x) {
@@ -440,7 +454,7 @@ __global__ void __launch_bounds__(kThreads)
     const unsigned long long key = act ? (((unsigned long long)a << 32) | b) : ~0ull;
     const unsigned grp = __match_any_sync(0xffffffffu, key);
     bool ok = true;
-    if (act && lane == (uint32_t)(__ffs(grp) - 1) && a != b) ok = uf_union(parent, a, b, uf_bounds(volume, limit).uni);
+    if (act && lane == (uint32_t)(__ffs(grp) - 1) && a != b) ok = uf_union<true>(parent, a, b, uf_bounds(volume, limit).uni);
     if (!ok) atomicOr(&stats[kStatError], kErrUnionFindLimit);
 }
 

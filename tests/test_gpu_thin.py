@@ -1,0 +1,48 @@
+"""Wolff updates of long thin lattices (marked gpu): the joins between tiles keep their trees shallow, so that no device
+loop takes a number of steps that grows with the lattice's length, and the cluster is the seed's component."""
+import numpy as np
+import pytest
+from scipy.sparse import coo_matrix
+from scipy.sparse.csgraph import connected_components
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(slsf):
+    slsf.build()
+    c = slsf.Context()
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("temperature", [0.4, 1.3])
+@pytest.mark.parametrize("dims", [(32, 8, 4096), (4, 4, 20000), (20000, 4, 4), (4, 20000, 2)])
+def test_rows_of_tiles_join_in_few_steps(slsf, dims, temperature):
+    # 1,024 to 5,000 tiles in a row: 128 steps are far above the logarithm of either
+    with slsf.Context() as ctx:
+        t = slsf.Task(ctx, dims, np.full(dims[2], 1.2), np.full(dims[2], 1.0), temperature, wolff_steps=1, seed=7)
+        t.init_cold()
+        ctx.set_loop_limit(128)
+        for _ in range(4):
+            t.metropolis_sweep()
+            t.wolff_step()
+        t.close()
+
+
+@pytest.mark.parametrize("dims", [(32, 8, 1024), (4, 4, 3001), (5001, 4, 4), (4, 3000, 2)])
+def test_cluster_of_a_thin_lattice(slsf, ctx, dims):
+    t = slsf.Task(ctx, dims, np.full(dims[2], 1.2), np.linspace(0.5, 1.5, dims[2]), 0.8, wolff_steps=1, seed=9)
+    t.init_cold()
+    lx, ly, lz = dims
+    site = np.arange(t.volume).reshape(lz, ly, lx)
+    for _ in range(3):
+        dbg = t.wolff_step_debug()
+        bonds = dbg["bonds"].reshape(lz, ly, lx)
+        ends = [(site[bonds & (1 << bit) != 0], np.roll(site, -1, axis)[bonds & (1 << bit) != 0])
+                for bit, axis in ((0, 2), (1, 1), (2, 0))]
+        a, b = (np.concatenate([e[k] for e in ends]) for k in (0, 1))
+        label = connected_components(coo_matrix((np.ones(a.size, np.int8), (a, b)), shape=(t.volume,) * 2), directed=False)[1]
+        x, y, z = dbg["seed_site"]
+        assert np.array_equal(dbg["cluster"].astype(bool), label == label[site[z, y, x]])
+    t.close()
