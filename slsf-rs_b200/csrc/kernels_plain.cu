@@ -226,17 +226,34 @@ __global__ void __launch_bounds__(kThreads, 3)
     finish_measure(acc, scratch, sink, volume);
 }
 
+/* Wolff tiles: a CTA labels one tile of kTileX x kTileY x kTileZ sites. */
+constexpr uint32_t kTileX = 32, kTileY = 8, kTileZ = 4;
+constexpr uint32_t kTileSites = kTileX * kTileY * kTileZ;
+static_assert(kTileX == 32, "a tile row is one warp");
+
+inline uint32_t wolff_tiles(const TaskView& t) {
+    return ((t.lx + kTileX - 1) / kTileX) * ((t.ly + kTileY - 1) / kTileY) * ((t.lz + kTileZ - 1) / kTileZ);
+}
+
 /* Lattices whose Wolff update grows the seed's cluster on bit-packed bonds
- * (kernel_wolff_bits.cu) instead of labelling 32x8x4 tiles: from 2^21 sites.
- * Measured on B200, us per Metropolis and Wolff call, bits against tiles: 32^3
- * 66 / 60, 30x32x24 74 / 58, 96^3 117 / 104, 150x148x30 135 / 100, 112^3 136 /
- * 126, 128^3 141 / 141, 160^3 172 / 212: below, the chain of region closures is
- * longer than the tiles' union-find, which labels every component. */
+ * (kernel_wolff_bits.cu) instead of labelling 32x8x4 tiles: from 2^21 sites,
+ * where that is the shorter of the two.  The tiles take 30 ns each, whatever
+ * the lattice's form.  The growth is a chain of region closures, half the
+ * regions of each axis one after the other, 11 us each (5.5 us for every region
+ * of L_x / 32 + L_y / 32 + L_z / 32), and 6 us per 2^20 sites for the bonds and
+ * the reflection.  Measured on B200, us per Wolff update at T = 1.2, bits against
+ * tiles: 128^3 110 / 106, 150x150x100 116 / 125, 160^3 131 / 169, 256^3 257 / 562,
+ * 128x128x1024 309 / 613, 1024x1024x16 440 / 546; 2048x32x32 346 / 106,
+ * 1024x1024x2 256 / 117, 512x512x8 182 / 104, 32x32x4096 483 / 179, 64x64x1024
+ * 227 / 185. */
 constexpr uint64_t kWolffBitsMinSites = 1u << 21;
+constexpr uint64_t kRegionTiles = 180, kTileSitesByBits = 5400; /* tiles' worth of a region; sites by bits in a tile's time */
 
 inline bool wolff_by_bits(const TaskView& t) {
-    return (uint64_t)t.lx * t.ly * t.lz >= kWolffBitsMinSites &&
-           wolff_bits_scratch_bytes(t.lx, t.ly, t.lz) <= 4ull * t.lx * t.ly * t.lz;
+    const uint64_t v = (uint64_t)t.lx * t.ly * t.lz;
+    const uint64_t chain = (uint64_t)(t.lx + 31) / 32 + (t.ly + 31) / 32 + (t.lz + 31) / 32;
+    return v >= kWolffBitsMinSites && kRegionTiles * chain + v / kTileSitesByBits < wolff_tiles(t) &&
+           wolff_bits_scratch_bytes(t.lx, t.ly, t.lz) <= 4ull * v;
 }
 
 /* ---- Wolff: union-find with links down a total order of the nodes ---- */
@@ -299,10 +316,6 @@ __device__ __forceinline__ bool uf_union(uint32_t* parent, uint32_t a, uint32_t 
     return false;
 }
 
-/* Wolff tiles: a CTA labels one tile of kTileX x kTileY x kTileZ sites. */
-constexpr uint32_t kTileX = 32, kTileY = 8, kTileZ = 4;
-constexpr uint32_t kTileSites = kTileX * kTileY * kTileZ;
-static_assert(kTileX == 32, "a tile row is one warp");
 /* Two rows a warp and phase: the unions' chains run side by side (us per call of
  * Metropolis and Wolff on 256 / 512 / 1024 threads: 48^3 83 / 76 / 74, 100x12x138
  * 87 / 81 / 79, 128^3 - / 141 / 152). */
@@ -766,8 +779,7 @@ int launch_wolff(const TaskView& t, uint64_t counter, uint8_t* bonds, uint32_t* 
     const uint32_t volume = t.lx * t.ly * t.lz;
     const uint32_t seed_idx = x0 + t.lx * (y0 + t.ly * z0);
     const uint32_t grid = blocks_for(volume, kThreads);
-    const uint32_t tiles = ((t.lx + kTileX - 1) / kTileX) * ((t.ly + kTileY - 1) / kTileY) *
-                           ((t.lz + kTileZ - 1) / kTileZ);
+    const uint32_t tiles = wolff_tiles(t);
     k_wolff_tiles<<<tiles, kTileThreads, 0, s>>>(t.theta, t.jxy, t.jz, t.lx, t.ly, t.lz, -2.0f * t.beta, phi,
                                              t.seed, counter, bonds, parent, t.stats, t.loop_limit);
     k_wolff_boundary<<<blocks_for((uint64_t)tiles * kFaceRows * 32, kThreads), kThreads, 0, s>>>(

@@ -1,4 +1,4 @@
-"""Wolff updates of long thin lattices (marked gpu): the joins between tiles keep their trees shallow, so that no device
+"""Wolff updates of lattices of extreme form (marked gpu): the joins between tiles keep their trees shallow, so that no device
 loop takes a number of steps that grows with the lattice's length, and the cluster is the seed's component."""
 import numpy as np
 import pytest
@@ -30,13 +30,16 @@ def test_rows_of_tiles_join_in_few_steps(slsf, dims, temperature):
         t.close()
 
 
-@pytest.mark.parametrize("dims", [(32, 8, 1024), (4, 4, 3001), (5001, 4, 4), (4, 3000, 2)])
-def test_cluster_of_a_thin_lattice(slsf, ctx, dims):
+# rows of tiles; then both sides of the choice between tiles and growth on bits, from 2^21 sites on: whole and cut words,
+# rows of less than a word, an odd number of planes
+@pytest.mark.parametrize("dims", [(32, 8, 1024), (4, 4, 3001), (5001, 4, 4), (4, 3000, 2), (160, 160, 160), (100, 160, 160),
+                                  (100, 160, 161), (6, 600, 600), (6, 590, 601), (64, 64, 512), (2048, 32, 32), (31, 10, 7000)])
+def test_cluster_is_the_seeds_component(slsf, ctx, dims):
     t = slsf.Task(ctx, dims, np.full(dims[2], 1.2), np.linspace(0.5, 1.5, dims[2]), 0.8, wolff_steps=1, seed=9)
     t.init_cold()
     lx, ly, lz = dims
     site = np.arange(t.volume).reshape(lz, ly, lx)
-    for _ in range(3):
+    for _ in range(3 if t.volume < 2 ** 20 else 1):
         dbg = t.wolff_step_debug()
         bonds = dbg["bonds"].reshape(lz, ly, lx)
         ends = [(site[bonds & (1 << bit) != 0], np.roll(site, -1, axis)[bonds & (1 << bit) != 0])
