@@ -147,6 +147,18 @@ constexpr uint32_t kOneCtaSweepSites = 8192, kOneCtaUpdateSites = 5120;
 
 namespace {
 
+/* At least `t` threads, and enough that the growth keeps its rows in registers
+ * (four a thread, kernel_resident.cu): thin lattices have many short rows. Past
+ * 3,072 rows the 1,024-thread instance pays, although it spills. us per sweep of
+ * 8 replicas at T = 0.9, and of 1200, by volume alone and by rows: 4x4x1000 146 /
+ * 89 and 1152 / 701 (256, 1024 threads), 4x8x256 198 / 58 and 681 / 443 (128, 512),
+ * 8x8x128 88 / 43 and 338 / 272 (128, 256), 4x64x64 163 / 107 and 1316 / 884 (256,
+ * 1024); 8x8x300, 2,400 rows, 159 / 161 and 1205 / 1252 on 512 and 1,024. */
+uint32_t threads_for_rows(uint32_t t, uint32_t rows) {
+    while (t < 512 && rows > 4 * t) t <<= 1;
+    return rows > 3072 ? 1024 : t;
+}
+
 /* Threads of the one-CTA kernel for V sites.  In a batch the fewest that keep
  * the arithmetic pipes of a full GPU busy, whatever the batch, so that a task's
  * sums do not depend on it (1e10 site-updates/s on B200: L = 8 2.37 / 2.05 on
@@ -163,8 +175,9 @@ namespace {
  * 67 / 43 / 37). */
 uint32_t resident_threads(uint32_t lx, uint64_t v, bool alone) {
     if (alone) return v <= 512 ? 128 : (v <= 4096 ? 256 : 512);
-    if (lx % 4) return v <= 512 ? 64 : (v <= 4096 ? 128 : (v <= 8192 ? 256 : 512));
-    return v <= 512 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512));
+    const uint32_t t = lx % 4 ? (v <= 512 ? 64 : (v <= 4096 ? 128 : (v <= 8192 ? 256 : 512)))
+                              : (v <= 512 ? 64 : (v <= 8192 ? 128 : (v <= 16384 ? 256 : 512)));
+    return threads_for_rows(t, (uint32_t)(v / lx));
 }
 
 /* The same for tasks that measure their correlations inside the sweeps: a lag
@@ -173,7 +186,9 @@ uint32_t resident_threads(uint32_t lx, uint64_t v, bool alone) {
  * 57 / 18 on 128, L = 8 49 / 23 and 51 / 15, L = 16 117 / 39 on 128 and 113 / 30
  * on 256, L = 24 360 / 94 on 256 and 392 / 79 on 512; L = 4 30 / 13 on 64 and 35 /
  * 10 on 128). */
-uint32_t fused_threads(uint64_t v) { return v <= 100 ? 64 : (v <= 1024 ? 128 : (v <= 16384 ? 256 : 512)); }
+uint32_t fused_threads(uint32_t lx, uint64_t v) {
+    return threads_for_rows(v <= 100 ? 64 : (v <= 1024 ? 128 : (v <= 16384 ? 256 : 512)), (uint32_t)(v / lx));
+}
 
 }  // namespace
 
@@ -1296,7 +1311,7 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device, bool fused = false) {
     if (slsf::resident_supports(lx, ly, lz, device)) {
         const uint64_t v = (uint64_t)lx * ly * lz;
-        return {slsf::kKernelResident, 1, fused ? fused_threads(v) : resident_threads(lx, v, false)};
+        return {slsf::kKernelResident, 1, fused ? fused_threads(lx, v) : resident_threads(lx, v, false)};
     }
     const uint32_t c = slsf::batched_cluster_size(lx, ly, lz, device);
     if (c && slsf::stream_fits(lx, ly, lz)) return {slsf::kKernelStream, 1, 256};

@@ -49,3 +49,21 @@ def test_cluster_is_the_seeds_component(slsf, ctx, dims):
         x, y, z = dbg["seed_site"]
         assert np.array_equal(dbg["cluster"].astype(bool), label == label[site[z, y, x]])
     t.close()
+
+
+@pytest.mark.parametrize("dims", [(4, 4, 130), (4, 8, 256), (8, 8, 128), (8, 8, 300), (4, 64, 64), (6, 10, 60)])
+def test_batched_thin_replicas(slsf, dims):
+    """The one-CTA kernel's default block keeps the rows of thin lattices in registers (four a thread up to 512
+    threads), and their trajectories are the one-task trajectories."""
+    with slsf.Context() as ctx:
+        choice = ctx.tune_get(dims)
+        assert choice["kind"] == "resident" and 4 * choice["threads"] >= min(dims[1] * dims[2], 2048)
+        make = lambda: slsf.Task(ctx, dims, np.full(dims[2], 1.2), np.linspace(0.5, 1.5, dims[2]), 0.9, wolff_steps=1, seed=4)
+        a, b = make(), make()
+        a.init_random()
+        b.init_random()
+        stats, alone = ctx.batch_run([a], 4)[0], b.sweep(4)
+        assert stats == alone
+        assert np.array_equal(a.theta.view(np.uint32), b.theta.view(np.uint32))
+        a.close()
+        b.close()
