@@ -405,8 +405,13 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
      * chunk costs about 2 us in the queue and its fences: 1.42 against 1.28 ms per
      * sweep of 300 replicas of 64^3) */
     StreamShape sh = {8, 16, 1};
-    uint64_t sites = 0;
-    for (uint32_t i = 0; i < n; ++i) sites = std::max(sites, (uint64_t)host_views[i].lx * host_views[i].ly * host_views[i].lz);
+    uint64_t sites = 0, gain = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const TaskView& t = host_views[i];
+        const uint64_t chain = (t.lx + 31) / 32 + (t.ly + kRegion - 1) / kRegion + (t.lz + kRegion - 1) / kRegion;
+        sites = std::max(sites, (uint64_t)t.lx * t.ly * t.lz);
+        gain = std::max(gain, (uint64_t)t.ly * t.lz * (t.ly + t.lz) / (kStreamThreads * chain));
+    }
     auto chunks = [&]() {
         uint64_t c = 0;
         for (uint32_t i = 0; i < n && c < 3ull * sms; ++i) c += chunks_of(host_views[i], sh, kColour0);
@@ -414,13 +419,21 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
     };
     while (sh.per > 1 && chunks() < 3ull * sms) sh.per >>= 1;
     if (chunks() < (uint64_t)sms) sh.bond_run = 8; /* few walks: one 56^3 109 -> 104 us, eight 117 -> 112 */
-    /* several CTAs grow a large replica together while there are SMs for them
-     * (us per sweep, together / by rows: one 64^3 150 / 178, sixteen 180 / 226,
-     * thirty-two 236 / 248, sixty-four 373 / 336; one 56^3 121 / 130, sixteen 133 /
-     * 139, thirty-two 171 / 145; at 48^3 and 36^3 the cut regions
-     * make it slower: sixteen 136 / 121 and 126 / 100) */
-    if (sites >= 150000)
-        while (sh.growers < 8 && (sites >= 200000 ? 2ull : 4ull) * sh.growers * n <= (uint64_t)sms) sh.growers <<= 1;
+    /* Several CTAs grow a replica together, by regions, where one CTA's row
+     * passes would take long and while there are SMs for them.  A pass visits
+     * rows / 512 rows a thread and there are as many as the cluster is long,
+     * L_y + L_z; the regions are a chain of their number along the axes: `gain` is
+     * the one over the other.  us per sweep at T = 0.9, by rows / by 8 CTAs: one
+     * 40^3 (gain 42) 85 / 90, 48^3 (72) 98 / 96, 36x4x512 (108) 189 / 157, 56^3
+     * (114) 114 / 104, 36x256x12 (146) 215 / 121, 64^3 (170) 151 / 119, 36x8x512
+     * (219) 276 / 176; sixteen 48^3 109 / 113, 56^3 137 / 126, 64^3 175 / 143,
+     * 36x8x512 369 / 206.  Four CTAs each for up to 37 replicas pay at the larger
+     * gains alone (thirty-two 56^3 145 / 171, 36x256x12 273 / 190, 64^3 248 / 236,
+     * 36x8x512 375 / 310). */
+    if (gain > 140)
+        while (sh.growers < 8 && 2ull * sh.growers * n <= (uint64_t)sms) sh.growers <<= 1;
+    else if ((gain > 100 || sites >= 150000) && 8ull * n <= (uint64_t)sms)
+        sh.growers = 8;
     if (sh.growers < 4) sh.growers = 1;
     uint64_t most = 1;
     uint32_t rows = 0, sweeps = 0;
