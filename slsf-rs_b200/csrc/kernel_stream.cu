@@ -51,29 +51,33 @@ struct StreamCtl {
 };
 
 /* Sizes of the chunks of a launch.  A phase is a row of blocks of one CTA's
- * threads (walks of seg_planes planes per thread, a run of rows per warp,
+ * threads (walks of walk_planes planes per thread, a run of rows per warp,
  * kFlipQuads quads per thread); a chunk takes `per` of them one after the other.  The
  * blocks, and so the order of the measured sums, are the same in every launch. */
 struct StreamShape {
     uint32_t per;      /* blocks per chunk */
     uint32_t bond_run; /* rows per warp of the bond activation */
-    uint32_t growers; /* CTAs that grow a replica's cluster together by regions; 1: one CTA by rows */
+    uint32_t planes;   /* planes per thread of colour 1, at most; 0: as colour 0 */
+    uint32_t growers;  /* CTAs that grow a replica's cluster together by regions; 1: one CTA by rows */
 };
 
 __host__ __device__ inline uint32_t smaller(uint32_t a, uint32_t b) { return a < b ? a : b; }
 
-/* Planes per thread of a replica's walks, by its size alone: the order of the
- * measured sums hangs on it.  Fewer planes shorten a lone replica's phases and
- * start more walks (us per sweep, 4 and 8 planes: one 40^3 84 / 96, one 56^3 109
+/* Planes per thread of a replica's walks, for colour 0 and the measurement by its
+ * size alone: the order of the measured sums hangs on it.  Fewer planes shorten a
+ * lone replica's phases and start more walks (us per sweep, 4 and 8 planes: one 40^3 84 / 96, one 56^3 109
  * / 120, thirty-two 64x64x40 137 / 144); the largest replicas fill the GPU with
  * 8 already (thirty-two 64^3 233 / 218). */
-__host__ __device__ inline uint32_t seg_planes(const TaskView& t) { return t.lx * t.ly * t.lz >= 200000 ? 8 : 4; }
+__host__ __device__ inline uint32_t walk_planes(const TaskView& t, const StreamShape& sh, uint32_t phase) {
+    if (phase == kColour1 && sh.planes) return sh.planes;
+    return t.lx * t.ly * t.lz >= 200000 ? 8 : 4;
+}
 
 __host__ __device__ inline uint32_t blocks_of(const TaskView& t, const StreamShape& sh, uint32_t phase) {
     switch (phase) {
         case kColour0:
         case kColour1:
-        case kMeasureLast: return (walk_units(t, seg_planes(t)) + kStreamThreads - 1) / kStreamThreads;
+        case kMeasureLast: return (walk_units(t, walk_planes(t, sh, phase)) + kStreamThreads - 1) / kStreamThreads;
         case kBonds: {
             const uint32_t warps = ((t.lx + 31) / 32) * (t.lz / 2) * ((t.ly + sh.bond_run - 1) / sh.bond_run);
             return (warps + kStreamThreads / 32 - 1) / (kStreamThreads / 32);
@@ -261,26 +265,27 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         /* bin row of the state that colour 0 starts from, or of the last state */
         double* bin_row = nullptr;
         if ((c.phase == kColour0 && c.sweep > 0) || c.phase == kMeasureLast) bin_row = bin_row_of(t, sweep);
+        const uint32_t planes = walk_planes(t, sh, c.phase);
         const uint32_t b_lo = chunk * sh.per, b_hi = smaller(b_lo + sh.per, blocks_of(t, sh, c.phase));
         if (c.phase == kColour1 || (c.phase == kColour0 && !bin_row)) {
             uint32_t accepted = 0;
             for (uint32_t b = b_lo; b < b_hi; ++b)
-                accepted += walk_colour<false>(t, sweep, c.phase == kColour1, seg_planes(t), b * kStreamThreads + threadIdx.x, nullptr);
+                accepted += walk_colour<false>(t, sweep, c.phase == kColour1, planes, b * kStreamThreads + threadIdx.x, nullptr);
             count_into(accepted, t.stats, kStatAccepted);
         } else if (c.phase == kColour0 || c.phase == kMeasureLast) {
             uint32_t accepted = 0;
             for (uint32_t b = b_lo; b < b_hi && bin_row; ++b) {
                 Sum2 sum[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, seg_planes(t), k));
+                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, planes, k));
                 const uint32_t unit = b * kStreamThreads + threadIdx.x;
                 if (c.phase == kColour0)
-                    accepted += walk_colour<true>(t, sweep, 0, seg_planes(t), unit, sum);
+                    accepted += walk_colour<true>(t, sweep, 0, planes, unit, sum);
                 else
-                    walk_measure(t, seg_planes(t), unit, sum);
+                    walk_measure(t, planes, unit, sum);
                 double acc[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, seg_planes(t), k));
+                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, planes, k));
                 block_sum<8>(acc, scratch);
                 if (threadIdx.x == 0)
 #pragma unroll
@@ -374,7 +379,7 @@ __global__ void k_stream_advance(const TaskView* __restrict__ views, unsigned lo
 }
 
 uint64_t items_per_sweep(const TaskView& t, const StreamShape& sh) {
-    return 2ull * chunks_of(t, sh, kColour0) +
+    return (uint64_t)chunks_of(t, sh, kColour0) + chunks_of(t, sh, kColour1) +
            (uint64_t)t.wolff_steps * (chunks_of(t, sh, kBonds) + chunks_of(t, sh, kGrow) + chunks_of(t, sh, kFlip));
 }
 
@@ -404,7 +409,7 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
     /* as many blocks per chunk as leave three chunks of the walks per SM (each
      * chunk costs about 2 us in the queue and its fences: 1.42 against 1.28 ms per
      * sweep of 300 replicas of 64^3) */
-    StreamShape sh = {8, 16, 1};
+    StreamShape sh = {8, 16, 0, 1};
     uint64_t sites = 0, gain = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const TaskView& t = host_views[i];
@@ -418,7 +423,15 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
         return c;
     };
     while (sh.per > 1 && chunks() < 3ull * sms) sh.per >>= 1;
-    if (chunks() < (uint64_t)sms) sh.bond_run = 8; /* few walks: one 56^3 109 -> 104 us, eight 117 -> 112 */
+    /* Few walks: shorter phases, in colour 1's planes and the bonds' rows, which
+     * no sum's order hangs on.  us per sweep with 16 rows, 8, 8 and two planes, 4 and
+     * two planes: one 64x64x40 102 / 99 / 98 / 94, eight 116 / 113 / 111 / 107; one
+     * 64^3 121 / 113 / 111 / 106, twelve 138 / 135 / 131 / 135; thirty-two 36x40x44
+     * 103 / 101 / 98 / 104; sixteen 64x64x40, more walks than SMs, 121 / 119 / 120 / 125. */
+    if (const uint64_t walks = chunks(); walks < (uint64_t)sms) {
+        sh.planes = 2;
+        sh.bond_run = 8 * walks < 5ull * sms ? 4 : 8;
+    }
     /* Several CTAs grow a replica together, by regions, where one CTA's row
      * passes would take long and while there are SMs for them.  A pass visits
      * rows / 512 rows a thread and there are as many as the cluster is long,
@@ -458,7 +471,7 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
                 const uint32_t end = std::min(hi, h[i].sweeps);
                 tickets += (end - sw) * items_per_sweep(h[i], sh);
                 if (end == h[i].sweeps && h[i].n_bins) tickets += chunks_of(h[i], sh, kMeasureLast);
-                wide += std::max(chunks_of(h[i], sh, kColour0), chunks_of(h[i], sh, kBonds));
+                wide += std::max(std::max(chunks_of(h[i], sh, kColour0), chunks_of(h[i], sh, kColour1)), chunks_of(h[i], sh, kBonds));
             }
             if (tickets == 0) continue;
             if (e == cudaSuccess) e = cudaMemsetAsync(scratch, 0, 256 + 8 * tickets, s);
