@@ -270,7 +270,7 @@ struct slsf_task {
     unsigned long long* stats = nullptr;
     bool stats_open = false; /* a call is between begin_stats and read_stats */
     double* bins = nullptr;
-    float jmax = 0.0f; /* TaskView::jmax */
+    float jxy_max = 0.0f, jz_max = 0.0f; /* TaskView's */
     slsf_batch* session = nullptr; /* open batch session holding the task's device view */
     /* correlation bins (slsf_task_corr_setup): one pool block holding the
      * launch scratch, the bin sums and the device measurement count */
@@ -304,7 +304,8 @@ struct slsf_task {
         v.n_bins = n_bins;
         v.sweeps = 0;
         v.loop_limit = ctx->loop_limit;
-        v.jmax = jmax;
+        v.jxy_max = jxy_max;
+        v.jz_max = jz_max;
         v.wolff_only = 0;
         v.bits = parent;
         v.partials = partials;
@@ -624,7 +625,8 @@ int slsf_task_create(slsf_ctx* ctx, const slsf_task_desc* d, slsf_task** out) {
     std::vector<float> jv(2 * (size_t)d->lz);
     for (uint32_t i = 0; i < d->lz; ++i) jv[i] = (float)d->j_xy[i];
     for (uint32_t i = 0; i < d->lz; ++i) jv[d->lz + i] = (float)d->j_z[i];
-    t->jmax = largest_coupling(jv.data(), jv.size());
+    t->jxy_max = largest_coupling(jv.data(), d->lz);
+    t->jz_max = largest_coupling(jv.data() + d->lz, d->lz);
     /* zero the whole block, then write the couplings, which travel in the
      * launch; one wait for all of it */
     e = cudaMemsetAsync(block, 0, L.total, ctx->stream);

@@ -44,7 +44,7 @@ struct TaskView {
     uint32_t thermalization, binsize, n_bins;
     uint32_t sweeps;       /* sweeps of this task in a batched launch; 0: the launch's count */
     uint32_t loop_limit;   /* 0, or a lower bound on device loops (slsf_ctx_set_loop_limit) */
-    float jmax;            /* largest coupling; infinite if any is not below kJMax */
+    float jxy_max, jz_max; /* largest couplings in the planes and between them; infinite if one is not below kJMax */
     uint32_t wolff_only;   /* the one-CTA kernel leaves the Metropolis half-sweeps out (slsf_task_wolff_step) */
     unsigned long long* stats;
     uint32_t* bits;        /* 4 V bytes of scratch: the Wolff bit planes of the stream kernels */

@@ -329,7 +329,7 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
     Sum2 sum[kMeasure ? 8 : 1];
     if (kMeasure)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) sum[k].start(k < 2 ? bias : t.jmax * bias);
+        for (int k = 0; k < 8; ++k) sum[k].start(bias * term_bound(t.jxy_max, t.jz_max, k));
     for (uint32_t u = threadIdx.x; u < ncol * nseg; u += blockDim.x) {
         const uint32_t sg = u / ncol, col = u - sg * ncol, m = col / nq, q = col - m * nq;
         const uint32_t z_lo = sg * seglen, z_hi = min(g.lz, z_lo + seglen);
@@ -388,7 +388,7 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
     }
     if (kMeasure)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += sum[k].total(k < 2 ? bias : t.jmax * bias);
+        for (int k = 0; k < 8; ++k) acc[k] += sum[k].total(bias * term_bound(t.jxy_max, t.jz_max, k));
     return accepted;
 }
 
@@ -405,7 +405,7 @@ constexpr uint32_t kQuadSites = 1024;
 template <bool kMeasure>
 __device__ __forceinline__ uint32_t sweep_colour(const TaskView& t, const Geo& g, Smem& s, uint64_t sweep,
                                                  uint32_t colour, double (&acc)[8]) {
-    if (g.lx % 4 == 0 && g.volume >= kQuadSites && (!kMeasure || t.jmax < kJMax))
+    if (g.lx % 4 == 0 && g.volume >= kQuadSites && (!kMeasure || fmaxf(t.jxy_max, t.jz_max) < kJMax))
         return half_sweep_quads<kMeasure>(t, g, s, sweep, colour, acc);
     return half_sweep<kMeasure>(t, g, s, sweep, colour, acc);
 }

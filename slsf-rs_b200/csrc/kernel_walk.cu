@@ -112,7 +112,7 @@ int sm_count() {
 bool walk_supports(const TaskView& t) {
     /* patches of four sites by two rows; the biased sums need finite couplings; 32-bit site indices; a block sum per
      * block of the partials' rows */
-    return t.lx % 4 == 0 && t.ly % 2 == 0 && t.lz >= 2 && t.jmax < kJMax &&
+    return t.lx % 4 == 0 && t.ly % 2 == 0 && t.lz >= 2 && fmaxf(t.jxy_max, t.jz_max) < kJMax &&
            (reinterpret_cast<uintptr_t>(t.theta) & 15u) == 0 && (uint64_t)t.lx * t.ly * t.lz <= 0x7fffffffull &&
            walk_blocks(t, t.lz) <= (uint32_t)kMeasureMaxBlocks;
 }

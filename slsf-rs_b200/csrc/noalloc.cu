@@ -105,7 +105,7 @@ extern "C" int slsf_measure_noalloc(const float* theta, const float* j_xy, const
     v.lx = lx;
     v.ly = ly;
     v.lz = lz;
-    v.jmax = std::numeric_limits<float>::infinity(); /* unknown here: the couplings are on the device */
+    v.jxy_max = v.jz_max = std::numeric_limits<float>::infinity(); /* unknown here: the couplings are on the device */
     v.partials = scratch->partials;
     v.result = scratch->result;
     v.done = &scratch->done;

@@ -56,6 +56,13 @@ struct Sum2 {
     }
 };
 
+/* Bound of the terms of sum k (mx, my, cos xyz, sin xyz): each direction's own
+ * largest coupling, so that the weaker one's terms are not lost under the
+ * other's bias. */
+__device__ __forceinline__ float term_bound(float jxy_max, float jz_max, int k) {
+    return k < 2 ? 1.0f : (k == 4 || k == 7 ? jz_max : jxy_max);
+}
+
 /* Adds J cos and J sin of the forward bonds i -> p and the backward bonds
  * m -> i of two sites i (bond_cos, bond_sin). */
 __device__ __forceinline__ void add_bonds2(Sum2& ac, Sum2& as, float jp, float jm, const Trig2& i, const Trig2& n,

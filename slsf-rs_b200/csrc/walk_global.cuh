@@ -58,9 +58,10 @@ __host__ __device__ inline uint32_t walk_units(const TaskView& t, uint32_t segle
     return (t.lx >> 2) * (t.ly >> 1) * ((t.lz + seglen - 1) / seglen);
 }
 
-/* Bias of a thread's sums (walk.cuh): each takes four terms per plane, at most 1 or J in magnitude. */
+/* Bias of a thread's sums (walk.cuh): each takes four terms per plane, at most
+ * 1 or the direction's largest J in magnitude. */
 __device__ __forceinline__ float walk_bias(const TaskView& t, uint32_t seglen, int k) {
-    return 8.0f * (float)seglen * (k < 2 ? 1.0f : t.jmax);
+    return 8.0f * (float)seglen * term_bound(t.jxy_max, t.jz_max, k);
 }
 
 /* One colour of unit `unit`'s patch; returns the accepted sites and, with
