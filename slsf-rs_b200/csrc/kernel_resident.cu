@@ -324,12 +324,9 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
     float* own = s.th + colour * g.stride1;
     const float* oth = s.th + (colour ^ 1u) * g.stride1;
     uint32_t accepted = 0;
-    /* each of a thread's sums takes four terms per plane, at most 1 or J in magnitude */
-    const float bias = 8.0f * (float)(seglen * ((ncol * nseg + blockDim.x - 1) / blockDim.x));
-    Sum2 sum[kMeasure ? 8 : 1];
-    if (kMeasure)
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sum[k].start(bias * term_bound(t.jxy_max, t.jz_max, k));
+    WalkSums sums;
+    if (kMeasure) sums.start(t.jxy_max, t.jz_max);
+    Sum2* sum = kMeasure ? sums.run : nullptr;
     for (uint32_t u = threadIdx.x; u < ncol * nseg; u += blockDim.x) {
         const uint32_t sg = u / ncol, col = u - sg * ncol, m = col / nq, q = col - m * nq;
         const uint32_t z_lo = sg * seglen, z_hi = min(g.lz, z_lo + seglen);
@@ -383,12 +380,14 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
         for (; z + 1 < z_hi; z += 2) {
             step(z, std::false_type());
             step(z + 1, std::true_type());
+            if (kMeasure) sums.flush();
         }
         if (z < z_hi) step(z, std::false_type());
+        if (kMeasure) sums.flush();
     }
     if (kMeasure)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += sum[k].total(bias * term_bound(t.jxy_max, t.jz_max, k));
+        for (int k = 0; k < 8; ++k) acc[k] += sums.acc[k];
     return accepted;
 }
 

@@ -275,21 +275,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         } else if (c.phase == kColour0 || c.phase == kMeasureLast) {
             uint32_t accepted = 0;
             for (uint32_t b = b_lo; b < b_hi && bin_row; ++b) {
-                Sum2 sum[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, planes, k));
+                WalkSums sums;
+                sums.start(t.jxy_max, t.jz_max);
                 const uint32_t unit = b * kStreamThreads + threadIdx.x;
                 if (c.phase == kColour0)
-                    accepted += walk_colour<true>(t, sweep, 0, planes, unit, sum);
+                    accepted += walk_colour<true>(t, sweep, 0, planes, unit, &sums);
                 else
-                    walk_measure(t, planes, unit, sum);
-                double acc[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, planes, k));
-                block_sum<8>(acc, scratch);
+                    walk_measure(t, planes, unit, sums);
+                block_sum<8>(sums.acc, scratch);
                 if (threadIdx.x == 0)
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) t.partials[b * 8 + k] = acc[k];
+                    for (int k = 0; k < 8; ++k) t.partials[b * 8 + k] = sums.acc[k];
             }
             if (c.phase == kColour0) count_into(accepted, t.stats, kStatAccepted);
         } else {

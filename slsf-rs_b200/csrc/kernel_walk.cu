@@ -66,34 +66,23 @@ __device__ __forceinline__ void finish_sums(double (&acc)[8], const TaskView& t,
 template <bool kMeasure>
 __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm)
     k_walk_colour(TaskView t, uint64_t sweep, uint32_t colour, uint32_t seglen, double* bin_row) {
-    Sum2 sum[kMeasure ? 8 : 1];
-    if (kMeasure)
-#pragma unroll
-        for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, seglen, k));
-    const uint32_t accepted = walk_colour<kMeasure>(t, sweep, colour, seglen, blockIdx.x * kWalkThreads + threadIdx.x, sum);
+    WalkSums sums;
+    if (kMeasure) sums.start(t.jxy_max, t.jz_max);
+    const uint32_t accepted = walk_colour<kMeasure>(t, sweep, colour, seglen, blockIdx.x * kWalkThreads + threadIdx.x, &sums);
     block_count(accepted, t.stats, kStatAccepted);
-    if (kMeasure) {
-        double acc[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, seglen, k));
-        finish_sums(acc, t, bin_row);
-    }
+    if (kMeasure) finish_sums(sums.acc, t, bin_row);
 }
 
-/* The observables of the state: 14 sincos per eight sites.  The sums in FP32
- * value and remainder (Sum2) instead of FP64 conversions on the
+/* The observables of the state: 14 sincos per eight sites.  The terms gathered
+ * in FP32 value and remainder (Sum2) instead of an FP64 conversion each on the
  * special-function pipe, which bound the earlier row walk (72% of it busy, 86
  * us at L = 256). */
 __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm)
     k_walk_measure(TaskView t, uint32_t seglen, double* bin_row) {
-    Sum2 sum[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) sum[k].start(walk_bias(t, seglen, k));
-    walk_measure(t, seglen, blockIdx.x * kWalkThreads + threadIdx.x, sum);
-    double acc[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = sum[k].total(walk_bias(t, seglen, k));
-    finish_sums(acc, t, bin_row);
+    WalkSums sums;
+    sums.start(t.jxy_max, t.jz_max);
+    walk_measure(t, seglen, blockIdx.x * kWalkThreads + threadIdx.x, sums);
+    finish_sums(sums.acc, t, bin_row);
 }
 
 uint32_t walk_blocks(const TaskView& t, uint32_t seglen) {
@@ -110,7 +99,7 @@ int sm_count() {
 }  // namespace
 
 bool walk_supports(const TaskView& t) {
-    /* patches of four sites by two rows; the biased sums need finite couplings; 32-bit site indices; a block sum per
+    /* patches of four sites by two rows; the biased runs need finite couplings; 32-bit site indices; a block sum per
      * block of the partials' rows */
     return t.lx % 4 == 0 && t.ly % 2 == 0 && t.lz >= 2 && fmaxf(t.jxy_max, t.jz_max) < kJMax &&
            (reinterpret_cast<uintptr_t>(t.theta) & 15u) == 0 && (uint64_t)t.lx * t.ly * t.lz <= 0x7fffffffull &&

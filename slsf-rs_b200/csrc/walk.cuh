@@ -29,16 +29,23 @@ __device__ __forceinline__ Trig2 trig2(float2 th) {
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
-/* Two running sums of FP32 terms carried as a value and a remainder.  The
- * value starts at a bias of at least twice what its terms can add up to, so
- * it never falls below a term's magnitude and each addition's rounding error
- * is exactly x - (t - v) (Dekker's fast two-sum); the errors add up in the
- * remainder.  total() recovers the sum to about 2^-40 of its terms'
- * magnitudes -- it agrees with FP64 sums of the same terms to 1e-12.  Four
- * packed FP32 instructions per two terms; converting each term to FP64 takes
- * eight cycles of the special-function pipe, which bound the measuring
- * half-sweep (41k of 136k cycles per sweep at L = 32 against 18k for the
- * other colour; 32k with these sums). */
+/* FP64 sums of FP32 terms of two sites, a few planes of them gathered in FP32
+ * first: a value and a remainder per site.  The value starts at a bias that
+ * keeps it above every term's magnitude, so each addition's rounding error is
+ * exactly x - (t - v) (Dekker's fast two-sum); the errors add up in the
+ * remainder.  Before kWalkRun planes and one are over, the two are added to the
+ * thread's FP64 sum and start anew.  Up to then the value stays below 2^6 times
+ * the terms' bound and the remainder below 2^-14, which rounds only where small
+ * terms have bits past 2^-38 of the bound: against FP64 sums of the same terms
+ * 2^-52 of their total, 2^-47 where the layers' couplings spread over six decades
+ * (value and remainder kept for a whole walk: 2^-41 there, at 64 planes a
+ * thread).  Four packed FP32 instructions per two terms and three conversions
+ * per run, 1 to 2 % of a sweep more than one run per walk; converting each term
+ * takes eight cycles of the special-function pipe, which bound the measuring
+ * half-sweep (41k of 136k cycles per sweep at L = 32 against 18k for the other
+ * colour; 32k with one run per walk). */
+constexpr int kWalkRun = 2;
+constexpr float kWalkBias = 8.0f * (kWalkRun + 1); /* twice the terms, four a plane, of kWalkRun + 1 planes */
 struct Sum2 {
     float2 v, r;
     __device__ __forceinline__ void start(float bias) {
@@ -51,8 +58,11 @@ struct Sum2 {
         r = __fadd2_rn(r, __ffma2_rn(__ffma2_rn(v, minus, t), minus, x));
         v = t;
     }
-    __device__ __forceinline__ double total(float bias) const {
-        return ((double)__fsub_rn(v.x, bias) + (double)r.x) + ((double)__fsub_rn(v.y, bias) + (double)r.y);
+    /* The sum so far (v - bias is exact: v stays within a factor of two of the bias); starts anew. */
+    __device__ __forceinline__ double take(float bias) {
+        const double s = ((double)__fsub_rn(v.x, bias) + (double)__fsub_rn(v.y, bias)) + (double)__fadd_rn(r.x, r.y);
+        start(bias);
+        return s;
     }
 };
 
@@ -62,6 +72,28 @@ struct Sum2 {
 __device__ __forceinline__ float term_bound(float jxy_max, float jz_max, int k) {
     return k < 2 ? 1.0f : (k == 4 || k == 7 ? jz_max : jxy_max);
 }
+
+/* A walk's sums (mx, my, cos xyz, sin xyz): `flush` at the latest after kWalkRun
+ * + 1 planes, `acc` holds them after it. */
+struct WalkSums {
+    Sum2 run[8];
+    double acc[8];
+    float jxy, jz;
+    __device__ __forceinline__ float bias(int k) const { return kWalkBias * term_bound(jxy, jz, k); }
+    __device__ __forceinline__ void start(float jxy_max, float jz_max) {
+        jxy = jxy_max;
+        jz = jz_max;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            run[k].start(bias(k));
+            acc[k] = 0.0;
+        }
+    }
+    __device__ __forceinline__ void flush() {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[k] += run[k].take(bias(k));
+    }
+};
 
 /* Adds J cos and J sin of the forward bonds i -> p and the backward bonds
  * m -> i of two sites i (bond_cos, bond_sin). */

@@ -58,17 +58,11 @@ __host__ __device__ inline uint32_t walk_units(const TaskView& t, uint32_t segle
     return (t.lx >> 2) * (t.ly >> 1) * ((t.lz + seglen - 1) / seglen);
 }
 
-/* Bias of a thread's sums (walk.cuh): each takes four terms per plane, at most
- * 1 or the direction's largest J in magnitude. */
-__device__ __forceinline__ float walk_bias(const TaskView& t, uint32_t seglen, int k) {
-    return 8.0f * (float)seglen * term_bound(t.jxy_max, t.jz_max, k);
-}
-
 /* One colour of unit `unit`'s patch; returns the accepted sites and, with
- * kMeasure, adds the terms of the state before the update to sum. */
+ * kMeasure, adds the terms of the state before the update to sums. */
 template <bool kMeasure>
 __device__ __forceinline__ uint32_t walk_colour(const TaskView& t, uint64_t sweep, uint32_t colour, uint32_t seglen,
-                                                uint32_t unit_index, Sum2* sum) {
+                                                uint32_t unit_index, WalkSums* sums) {
     const uint32_t lx = t.lx, plane = lx * t.ly;
     uint32_t accepted = 0;
     Patch pt;
@@ -96,6 +90,7 @@ __device__ __forceinline__ uint32_t walk_colour(const TaskView& t, uint64_t swee
     Trig2 m0 = trig2(pick(four(below + i0), par_lo)), m1 = trig2(pick(four(below + i1), !par_lo));
     Trig2 c0 = trig2(pick(r0, !par_lo)), c1 = trig2(pick(r1, par_lo));
     float jzm = jz[pt.z_lo == 0 ? t.lz - 1 : pt.z_lo - 1];
+    Sum2* sum = kMeasure ? sums->run : nullptr;
     auto step = [&](uint32_t z, auto odd) {
         constexpr bool kOdd = decltype(odd)::value;
         const uint32_t above = z + 1 == t.lz ? 0u : base + plane;
@@ -132,8 +127,10 @@ __device__ __forceinline__ uint32_t walk_colour(const TaskView& t, uint64_t swee
     for (; z + 1 < pt.z_hi; z += 2) {
         step(z, std::false_type());
         step(z + 1, std::true_type());
+        if (kMeasure) sums->flush();
     }
     if (z < pt.z_hi) step(z, std::false_type());
+    if (kMeasure) sums->flush();
     return accepted;
 }
 
@@ -143,8 +140,8 @@ __device__ __forceinline__ void add_bond2(Sum2& ac, Sum2& as, float j, const Tri
     as.add(__fmul2_rn(dup2(j), __ffma2_rn(a.s, b.c, __fmul2_rn(neg2(a.c), b.s))));
 }
 
-/* The observables' terms of unit `unit`'s patch, added to sum. */
-__device__ __forceinline__ void walk_measure(const TaskView& t, uint32_t seglen, uint32_t unit_index, Sum2* sum) {
+/* The observables' terms of unit `unit`'s patch, added to sums. */
+__device__ __forceinline__ void walk_measure(const TaskView& t, uint32_t seglen, uint32_t unit_index, WalkSums& sums) {
     const uint32_t lx = t.lx, plane = lx * t.ly;
     Patch pt;
     if (!patch_of(t, unit_index, seglen, pt)) return;
@@ -172,6 +169,7 @@ __device__ __forceinline__ void walk_measure(const TaskView& t, uint32_t seglen,
         r.b.s = make_float2(c.b.s.y, sn);
         return r;
     };
+    Sum2* sum = sums.run;
     uint32_t base = pt.z_lo * plane;
     Quad c0 = quad(base + i0), c1 = quad(base + i1);
     for (uint32_t z = pt.z_lo; z < pt.z_hi; ++z) {
@@ -193,7 +191,9 @@ __device__ __forceinline__ void walk_measure(const TaskView& t, uint32_t seglen,
         c0 = n0;
         c1 = n1;
         base += plane;
+        if (z & 1u) sums.flush();
     }
+    sums.flush();
 }
 
 }  // namespace slsf
