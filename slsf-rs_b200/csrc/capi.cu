@@ -71,13 +71,6 @@ bool width_ok(double w) { return w >= 0.0 && std::isfinite(w); }
 
 uint64_t align256(uint64_t b) { return (b + 255) & ~255ull; }
 
-/* Kernels of one correlation measurement (launch_corr): the line items, the
- * spectral z items when there are z items, the layers' sums when they are
- * many, and the finalize. */
-uint32_t corr_launch_count(uint32_t items, uint32_t z_items, uint32_t layers) {
-    return (items ? (z_items ? 3u : 2u) : 1u) + (slsf::corr_layers_launch(layers) ? 1u : 0u);
-}
-
 /* Side streams for the kernel groups of a batch after the first (group g
  * runs on side[(g - 1) % kSideStreams]); each group has its own work-queue
  * counter. */
@@ -904,9 +897,7 @@ int slsf_task_correlations(slsf_task* t, uint32_t rmax_xy, uint32_t rmax_z, doub
     e = slsf::launch_corr(nullptr, &ct, 1, items, slsf::corr_z_units(t->lx, t->ly, t->lz, rmax_xy, rmax_z),
                           slsf::corr_len(t->lx, t->ly, t->lz, rmax_xy, rmax_z), std::max(rmax_xy, rmax_z),
                           slsf::corr_z_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z), t->lz * rmax_xy, ctx->sm_count,
-                          ctx->stream);
-    ctx->launches += corr_launch_count(items, slsf::corr_z_items(t->lx, t->ly, t->lz, rmax_xy, rmax_z),
-                                       t->lz * rmax_xy);
+                          ctx->stream, &ctx->launches);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), ct.values, 8ull * nv, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     ctx->pool.free(dv, bytes);
@@ -1074,8 +1065,8 @@ int slsf_batch_correlations(slsf_ctx* ctx, slsf_task* const* tasks, size_t n) {
     }
     SLSF_CUDA(slsf::launch_corr(ctx->d_corr, nullptr, (uint32_t)n, ctx->corr_last_items, ctx->corr_last_zunits,
                                 ctx->corr_last_len,
-                                ctx->corr_last_r, ctx->corr_last_nz, ctx->corr_last_layers, ctx->sm_count, ctx->stream));
-    ctx->launches += corr_launch_count(ctx->corr_last_items, ctx->corr_last_nz, ctx->corr_last_layers);
+                                ctx->corr_last_r, ctx->corr_last_nz, ctx->corr_last_layers, ctx->sm_count, ctx->stream,
+                                &ctx->launches));
     for (size_t i = 0; i < n; ++i) tasks[i]->corr_count += 1;
     return SLSF_OK;
 }
@@ -1272,10 +1263,7 @@ static void run_grid_task(slsf_ctx* ctx, const slsf_task* t, const TaskView& v, 
                               slsf::corr_len(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz),
                               std::max(t->corr_rxy, t->corr_rz),
                               slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz), t->lz * t->corr_rxy,
-                              ctx->sm_count, st);
-            ctx->launches +=
-                corr_launch_count(items, slsf::corr_z_items(t->lx, t->ly, t->lz, t->corr_rxy, t->corr_rz),
-                                  t->lz * t->corr_rxy);
+                              ctx->sm_count, st, &ctx->launches);
         }
     }
     if (pending) {

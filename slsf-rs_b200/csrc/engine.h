@@ -167,12 +167,11 @@ bool corr_supports(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t
  * n_items and n_zunits in all) in device memory; or, for one task, `one` on
  * the host (passed to the kernels by value, no copy).  max_len, max_r,
  * max_nz, max_layers: the largest corr_len, radius, corr_z_items and L_z times
- * in-plane radius of them (they size the launches). */
+ * in-plane radius of them (they size the launches).  Adds the kernels launched
+ * to *launches. */
 cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t n_tasks, uint32_t n_items,
                         uint32_t n_zunits, uint32_t max_len, uint32_t max_r, uint32_t max_nz, uint32_t max_layers,
-                        int sm_count, cudaStream_t s);
-/* Whether launch_corr gives the layers' sums a launch of their own. */
-bool corr_layers_launch(uint32_t max_layers);
+                        int sm_count, cudaStream_t s, uint64_t* launches);
 /* z-line work items of a task (0 without C_z). */
 uint32_t corr_z_items(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t rz);
 /* Spectral z units of a task: groups of consecutive z items whose power

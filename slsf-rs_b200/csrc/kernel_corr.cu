@@ -623,15 +623,13 @@ bool corr_supports(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t
     return (size_t)corr_ext(lx, ly, lz, rxy, rz) * kCorrPitch * sizeof(float2) <= kCorrMaxTile;
 }
 
-bool corr_layers_launch(uint32_t max_layers) { return max_layers >= kLayerSums; }
-
 cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t n_tasks, uint32_t n_items,
                         uint32_t n_zunits, uint32_t max_len, uint32_t max_r, uint32_t max_nz, uint32_t max_layers,
-                        int sm_count, cudaStream_t s) {
+                        int sm_count, cudaStream_t s, uint64_t* launches) {
     /* a warp takes 8 lags per pass: blocks of one or two warps for small
      * radii, so that short lines do not hold idle warps */
     const int line_threads = max_r <= 16 ? 64 : (max_r <= 32 ? 128 : kCorrThreads);
-    const bool layers = corr_layers_launch(max_layers);
+    const bool layers = max_layers >= kLayerSums;
     /* the finalize splits each C_z sum over its z items only when there are
      * many; each lag needs a thread of its own (R_z <= 258 < kFinThreads) */
     const int fin_threads = (max_nz > 64 || max_r > 128 || layers) ? kFinThreads : 128;
@@ -646,7 +644,10 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
             e = cudaFuncSetAttribute(k_corr_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         const uint32_t grid = std::min<uint32_t>(n_items, 1u << 30);
-        if (lines) k_corr_lines<<<grid, line_threads, smem, s>>>(one ? nullptr : tasks_dev, by_value, n_tasks, n_items);
+        if (lines) {
+            k_corr_lines<<<grid, line_threads, smem, s>>>(one ? nullptr : tasks_dev, by_value, n_tasks, n_items);
+            *launches += 1;
+        }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (n_zunits > 0) {
@@ -659,18 +660,22 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
              * once: three per SM (the kernel's occupancy) */
             const uint32_t zgrid = sm_count > 0 ? std::min<uint32_t>(n_zunits, 3u * (uint32_t)sm_count) : n_zunits;
             k_corr_zfft<<<zgrid, kCorrThreads, zsmem, s>>>(one ? nullptr : tasks_dev, by_value, n_tasks, n_zunits);
+            *launches += 1;
             e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }
     }
     if (layers) {
-        for (uint32_t lo = 0; lo < n_tasks; lo += 65535) /* tasks of one launch (grid.y) */
+        for (uint32_t lo = 0; lo < n_tasks; lo += 65535) { /* tasks of one launch (grid.y) */
             k_corr_layers<<<dim3((max_layers + kLayerThreads - 1) / kLayerThreads, std::min(65535u, n_tasks - lo)), kLayerThreads, 0, s>>>(
                 one ? nullptr : tasks_dev + lo, by_value);
+            *launches += 1;
+        }
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     k_corr_finalize<<<n_tasks, fin_threads, 0, s>>>(one ? nullptr : tasks_dev, by_value, layers);
+    *launches += 1;
     return cudaGetLastError();
 }
 
