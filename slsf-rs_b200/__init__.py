@@ -58,6 +58,8 @@ class SweepStats(C.Structure):
         return {n: getattr(self, n) for n, _ in self._fields_}
 
 
+# Bytes of one task's entry in the table that every batched call uploads (sizeof(TaskView), asserted in capi.cu).
+TASK_VIEW_BYTES = 152
 KERNEL_KINDS = ("resident", "cluster", "grid", "stream")
 
 

@@ -129,6 +129,8 @@ TaskLayout layout_of(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t n_bins) {
 
 }  // namespace
 
+/* The package's TASK_VIEW_BYTES, from which the benchmark counts a call's uploads. */
+static_assert(sizeof(TaskView) == 152, "TASK_VIEW_BYTES");
 constexpr size_t kSmallReadBack = 256; /* bytes */
 /* Lattices up to these sizes run in one CTA even alone: whole sweeps
  * (slsf_task_sweep), and a Metropolis sweep or Wolff step by itself, which the
