@@ -78,9 +78,9 @@ __device__ __forceinline__ float wolff_projection(float c, float s, float cphi, 
     return __fmaf_rn(s, sphi, __fmul_rn(c, cphi));
 }
 
-/* 2^y by the hardware instruction, results below 2^-126 flushed to zero (the
- * instruction alone, without the range test and the two scalings that keep
- * subnormal results); e^x = 2^(x log2 e). */
+/* 2^y by the PTX instruction ex2.approx.ftz.f32 (PTX ISA, ex2: a fast
+ * approximation of 2^a; with .ftz subnormal operands and results are flushed to
+ * zero).  e^x = 2^(x log2 e). */
 constexpr float kLog2E = 1.44269504088896341f;
 __device__ __forceinline__ float exp2_flush(float y) {
     float r;
@@ -97,7 +97,8 @@ __device__ __forceinline__ float exp2_flush(float y) {
  * same rounding scaled exactly, and word >> 8 < 2^24 p holds iff the word
  * itself, rounded towards zero to 24 bits, is below 2^32 p.  A flushed exp
  * gives p = 1, as a subnormal one does, and where J r_i r_j is not positive
- * exp is at least 1, so p <= 0 (or NaN) and no word is below it. */
+ * exp is at least 1, so p <= 0 (or NaN) and no word is below it.  The decisions
+ * are those of 1 - __expf for every FP32 product (tests/c/bond_exp.cu). */
 __device__ __forceinline__ bool wolff_bond_active(float coupling, float ri, float rj,
                                                   float minus_two_beta, uint32_t word) {
     const float prod = __fmul_rn(__fmul_rn(coupling, ri), rj);
