@@ -359,7 +359,7 @@ int read_stats(slsf_task* t, unsigned long long out[slsf::kStatSlots]) {
 /* Whether an update of the task alone runs in one launch of the one-CTA
  * kernel, which writes the counters to the host's landing area. */
 bool one_cta_updates(const slsf_task* t, uint32_t most) {
-    return t->volume <= most && slsf::resident_supports(t->lx, t->ly, t->lz, t->ctx->device);
+    return t->volume <= most && slsf::resident_supports(t->lx, t->ly, t->lz);
 }
 
 int run_one_cta(slsf_task* t, TaskView v, uint32_t n_sweeps, unsigned long long out[slsf::kStatSlots]) {
@@ -1284,7 +1284,7 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
     switch (c.kind) {
         case slsf::kKernelResident:
             return c.cluster == 1 && c.threads >= 64 && c.threads <= 1024 && c.threads % 32 == 0 &&
-                   slsf::resident_supports(lx, ly, lz, device);
+                   slsf::resident_supports(lx, ly, lz);
         case slsf::kKernelCluster:
             return c.threads >= 64 && c.threads <= 1024 && c.threads % 32 == 0 &&
                    slsf::cluster_feasible(lx, ly, lz, c.cluster, device);
@@ -1301,7 +1301,7 @@ bool choice_feasible(const slsf::KernelChoice& c, uint32_t lx, uint32_t ly, uint
  * a batch that fills the GPU), else the smallest cluster that holds it, 1024
  * threads; else the grid-wide kernels. */
 slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int device, bool fused = false) {
-    if (slsf::resident_supports(lx, ly, lz, device)) {
+    if (slsf::resident_supports(lx, ly, lz)) {
         const uint64_t v = (uint64_t)lx * ly * lz;
         return {slsf::kKernelResident, 1, fused ? fused_threads(lx, v) : resident_threads(lx, v, false)};
     }

@@ -179,7 +179,7 @@ uint32_t corr_z_items(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t rxy, uint3
 uint32_t corr_z_units(uint32_t lx, uint32_t ly, uint32_t lz, uint32_t rxy, uint32_t rz);
 
 /* ---- batched persistent engine, one CTA per replica (kernel_resident.cu) ---- */
-bool resident_supports(uint32_t lx, uint32_t ly, uint32_t lz, int device);
+bool resident_supports(uint32_t lx, uint32_t ly, uint32_t lz);
 /* Runs n_sweeps sweeps of every view in `views_dev` (device array of n);
  * `queue` is a zeroed device counter.  With `counters` (2 per view, may be
  * NULL) the Metropolis and Wolff counters come from there instead of the

@@ -1031,7 +1031,12 @@ cudaError_t launch_w(const TaskView* views_dev, uint32_t n, uint32_t n_sweeps, u
                      cudaStream_t s, uint32_t cluster, uint32_t threads, const Limits& lim,
                      unsigned long long* counters) {
     const size_t smem = smem_bytes(lim, sizeof(W));
-    cudaError_t e = cudaFuncSetAttribute(k_cluster<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    /* the device's limit, whatever this launch needs: another thread's launch may need more */
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_cluster<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 std::max((int)smem, max_dynamic_smem(device)));
     if (e != cudaSuccess) return e;
     if (cluster > 8) {
         e = cudaFuncSetAttribute(k_cluster<W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

@@ -641,7 +641,7 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
         /* a task whose only lines are spectral z lines has no item for k_corr_lines */
         const bool lines = !(one && one->rxy == 0 && n_zunits > 0);
         if (lines && smem > 48 * 1024)
-            e = cudaFuncSetAttribute(k_corr_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = cudaFuncSetAttribute(k_corr_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCorrMaxTile);
         if (e != cudaSuccess) return e;
         const uint32_t grid = std::min<uint32_t>(n_items, 1u << 30);
         if (lines) {

@@ -932,6 +932,17 @@ size_t smem_bytes(uint32_t max_volume, uint32_t max_rows, uint32_t max_lz, uint3
     return 4ull * (max_volume + 2 * kPad) + 16ull * max_rows + 8ull * max_lz + 8ull * corr_doubles;
 }
 
+/* Compute capability 10.0 gives a block 227 KB; the kernel's static arrays need room in it. */
+constexpr size_t kMaxDynamicSmem = 227 * 1024 - 4096;
+
+/* Lets a kernel be launched with `smem` bytes: its limit goes to the device's
+ * at once, since a limit as low as one launch needs would refuse the larger
+ * launch that another thread, with a context of its own, is about to make. */
+template <typename K>
+cudaError_t allow_smem(K kernel, size_t smem) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, kMaxDynamicSmem));
+}
+
 template <bool kCorr, int kMaxThreads, int kUnroll>
 cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_sweeps, unsigned int* queue,
                               int device, cudaStream_t s, uint32_t max_volume, uint32_t max_rows, uint32_t max_lz,
@@ -939,7 +950,7 @@ cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_
                               uint32_t corr_doubles) {
     const size_t smem = smem_bytes(max_volume, max_rows, max_lz, corr_doubles);
     const TaskView none = {};
-    cudaError_t e = cudaFuncSetAttribute(k_resident<kCorr, kMaxThreads, kUnroll>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k_resident<kCorr, kMaxThreads, kUnroll>, smem);
     if (e != cudaSuccess) return e;
     int sms = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -953,27 +964,20 @@ cudaError_t launch_resident_t(const TaskView* views_dev, uint32_t n, uint32_t n_
     return cudaGetLastError();
 }
 
-int max_dynamic_smem(int device) {
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    /* leave room for the kernel's static shared arrays */
-    return v - 4096;
-}
-
 }  // namespace
 
-bool resident_supports(uint32_t lx, uint32_t ly, uint32_t lz, int device) {
+bool resident_supports(uint32_t lx, uint32_t ly, uint32_t lz) {
     /* Row words hold L_x <= 32 bits; the colour-split layout needs even
      * dimensions (L_x = 2 mod 4 copies the state site by site). */
     if (lx > kMaxRowBits || lx < 4 || lx % 2 || ly < 2 || ly % 2 || lz < 2 || lz % 2) return false;
     const uint64_t v = (uint64_t)lx * ly * lz;
-    return smem_bytes((uint32_t)v, ly * lz, lz) <= (size_t)max_dynamic_smem(device);
+    return smem_bytes((uint32_t)v, ly * lz, lz) <= kMaxDynamicSmem;
 }
 
 cudaError_t launch_resident_one(const TaskView& t, uint32_t n_sweeps, uint32_t threads, cudaStream_t s) {
     const uint32_t volume = t.lx * t.ly * t.lz;
     const size_t smem = smem_bytes(volume, t.ly * t.lz, t.lz);
-    cudaError_t e = cudaFuncSetAttribute(k_resident<false, 512, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k_resident<false, 512, 1>, smem);
     if (e != cudaSuccess) return e;
     TaskView v = t;
     v.sweeps = n_sweeps;

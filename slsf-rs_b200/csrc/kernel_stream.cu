@@ -451,7 +451,8 @@ cudaError_t launch_stream(const TaskView* views, const TaskView* host_views, uns
         rows = std::max(rows, host_views[i].ly * host_views[i].lz * (host_views[i].lx > 32 ? 2u : 1u));
         sweeps = std::max(sweeps, host_views[i].sweeps);
     }
-    cudaError_t e = cudaFuncSetAttribute(k_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * rows));
+    /* the largest growth's words, whatever this launch needs: another thread's launch may need more */
+    cudaError_t e = cudaFuncSetAttribute(k_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kStreamThreads * kStreamRows));
     /* every launch's entries fit the ring: pieces of replicas, and of sweeps */
     const uint32_t piece = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(n, 1u << (32 - kChunkBits)), kRingEntries / most);
     for (uint32_t lo = 0; lo < n && e == cudaSuccess; lo += piece) {
