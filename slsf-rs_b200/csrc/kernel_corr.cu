@@ -474,13 +474,14 @@ __device__ __forceinline__ void layer_sum(const CorrTask& T, const CorrShape& sh
 }
 
 /* The layers' sums of every task, one thread each, blockIdx.y's task: a
- * launch of its own from kLayerSums sums on (launch_corr).  Latency bounds
- * both places: in the finalize's one block per task the 4,608 sums of 96^3
- * with R = 48 and the columns after them took 28 us, here 6 and 11 after
- * them; the 128 sums of 16^3 with R = 8 cost less inside the finalize (54 us
- * for 300 tasks' measurements, 58 with the launch; 12.5 and 15.6 for one 8^3). */
+ * launch of its own from kLayerSums sums on (launch_corr): where the finalize's
+ * one block per task takes them one after the other for longer than a launch
+ * lasts.  us per measurement, inside the finalize of 1,024 threads and by the
+ * launch: 96^3 with R = 48 (4,608 sums) 50.4 / 48.3, 128^3 R = 64 (8,192) 85.8 /
+ * 81.9; 80^3 R = 40 (3,200) 40.1 / 40.7, 64^3 R = 32 37.5 / 41.4, 32^3 R = 16 31.5 /
+ * 33.7. */
 constexpr int kLayerThreads = 128;
-constexpr uint32_t kLayerSums = 256;
+constexpr uint32_t kLayerSums = 4096;
 
 __global__ void __launch_bounds__(kLayerThreads) k_corr_layers(const CorrTask* tasks, CorrTask one) {
     const CorrTask T = corr_task(tasks, one, blockIdx.y);
@@ -545,7 +546,7 @@ __global__ void __launch_bounds__(kFinThreads) k_corr_finalize(const CorrTask* t
     if (R) {
         column_sums(lsx, R, R, lz);
         for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) emit(r, zcol[r] / volume);
-        const double cx = threadIdx.x < R ? zcol[threadIdx.x] / volume : 0.0; /* R < 128 threads or kFinThreads */
+        const double cx = threadIdx.x < R ? zcol[threadIdx.x] / volume : 0.0; /* R is at most the block */
         __syncthreads();
         column_sums(lsy, R, R, lz);
         for (uint32_t r = threadIdx.x; r < R; r += blockDim.x) {
@@ -631,8 +632,12 @@ cudaError_t launch_corr(const CorrTask* tasks_dev, const CorrTask* one, uint32_t
     const int line_threads = max_r <= 16 ? 64 : (max_r <= 32 ? 128 : kCorrThreads);
     const bool layers = max_layers >= kLayerSums;
     /* the finalize splits each C_z sum over its z items only when there are
-     * many; each lag needs a thread of its own (R_z <= 258 < kFinThreads) */
-    const int fin_threads = (max_nz > 64 || max_r > 128 || layers) ? kFinThreads : 128;
+     * many; each lag needs a thread of its own (R_z <= 258 < kFinThreads).  Blocks
+     * by the layers' sums too (us per measurement of one task, and of 300, on 128 /
+     * 256 / 1,024 threads: 16^3 R = 8, 128 sums, 16.0 / 16.0 / 16.1 and 55.1 / 55.1 /
+     * 65.5; 24^3 R = 12, 288 sums, 19.4 / 17.2 / 17.2 and 94 / 94 / 102; 48^3 R = 24,
+     * 1,152 sums, 30.9 / 22.6 / 18.6) */
+    const int fin_threads = (max_nz > 64 || max_r > 128 || max_layers > 1024) ? kFinThreads : (max_layers >= 256 ? 256 : 128);
     if (n_tasks == 0 || (!tasks_dev && (!one || n_tasks != 1))) return cudaErrorInvalidValue;
     const CorrTask by_value = one ? *one : CorrTask{};
     if (n_items > 0) {

@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
                                                 ((16, 16, 24), (8, 12), ("lines", "finalize")),
                                                 ((16, 16, 8), (8, 0), ("lines", "finalize")),
                                                 ((16, 16, 64), (2, 32), ("lines", "zfft", "finalize")),
-                                                ((16, 16, 64), (8, 0), ("lines", "layers", "finalize")),
-                                                ((16, 16, 64), (8, 32), ("lines", "zfft", "layers", "finalize"))])
+                                                ((16, 16, 512), (7, 0), ("lines", "finalize")),
+                                                ((16, 16, 512), (8, 0), ("lines", "layers", "finalize")),
+                                                ((128, 64, 128), (32, 64), ("lines", "zfft", "layers", "finalize"))])
 def test_correlation_launches(slsf, dims, radii, kernels):
     with slsf.Context() as ctx:
         t = slsf.Task(ctx, dims, np.full(dims[2], 1.2), np.full(dims[2], 1.0), 1.2, seed=3)
