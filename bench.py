@@ -679,7 +679,7 @@ def main():
                                    f"in [1.1,1.5], L={L}, J_xy=1.2, J_z~U[0.5,1.5], Metropolis (width pi) + 1 Wolff "
                                    f"+ measure per sweep, {total_sweeps} sweeps total, {S} sweeps per step",
                        "replicas_per_gpu": n, "L": L, "sweeps_per_step": S, "parallelism": f"replicas x{world}",
-                       "l2": "inputs larger than L2 (state 512 MiB per GPU)", "reductions": "fp64",
+                       "l2": "inputs larger than L2 (state 512 MiB per GPU)", "reductions": "fp64 (terms of up to three planes a thread gathered as FP32 value and remainder)",
                        "kernel_choice": choice},
             "clocks": clk, "gpu_launches": launches,
             "e2e": {"value": e2e_value, "unit": "site-updates/s", "h2d_bytes_per_step": h2d,

@@ -150,10 +150,11 @@ int slsf_batch_step_correlations(slsf_batch* b, uint32_t n_cycles, slsf_sweep_st
  * How the batched entry points run each lattice shape: the one-CTA kernel
  * with a CTA of `threads`, the cluster kernel with `cluster` CTAs per replica
  * (a power of two up to 16) of `threads` each, the grid-wide single-task
- * kernels, or the stream kernels (the replicas' state in global memory, one
- * launch per phase of a sweep for all of them; cluster 1, threads 256; L_x a
- * multiple of 4 up to 64, at most 4096 rows L_y L_z).  The choice changes neither a task's trajectory nor its bins
- * beyond FP32 partial-sum rounding, only the speed.  A context starts from a
+ * kernels, or the stream kernel (the replicas' state in global memory, the
+ * phases of all their sweeps as chunks of one persistent launch; L_x a multiple
+ * of 4 up to 64, at most 4096 rows L_y L_z; written as cluster 1, threads 256,
+ * which do not size its CTAs).  The choice changes neither a task's trajectory
+ * nor its bins beyond partial-sum rounding, only the speed.  A context starts from a
  * default per shape; slsf_autotune times every feasible choice on scratch
  * replicas and keeps the fastest; the table can be saved and loaded.  No
  * reference counterpart (the reference's tasks are single-threaded). */
@@ -266,7 +267,7 @@ int slsf_task_corr_setup(slsf_task* task, uint32_t rmax_xy, uint32_t rmax_z, uin
  * one-CTA kernel (even L_x <= 32 and a replica that fits shared memory), or
  * by the correlation kernels queued after those sweeps on the grid-wide
  * kernels (lattices too large for one cluster; not in sessions).  Tasks on
- * the cluster or stream kernels are refused.  0 turns it off.
+ * the cluster or stream kernel are refused.  0 turns it off.
  * Such a task refuses the separate measurements (slsf_batch_correlations,
  * slsf_batch_step_correlations).  Values agree with the separate kernels to
  * FP32 partial-sum rounding. */

@@ -23,9 +23,9 @@
  * Wolff labelling is bit-parallel: the active +x/+y/+z bonds of a row of
  * L_x <= 32 sites are three 32-bit words; the cluster grows from the seed by
  * OR-ing neighbour rows through the bond words and closing every row that
- * gained bits along x, until a pass changes nothing.  (In one CTA a pass is
- * a single block barrier, which for replicas of this size beats the
- * column-scan rounds of kernel_cluster.cu.)  The result is the seed's
+ * gained bits along x, until a pass changes nothing: three steps of every row
+ * and one block barrier a pass, which for replicas of this size beats scans of
+ * whole lines (grow, below).  The result is the seed's
  * connected component over the active bonds -- the set the reference's DFS
  * (src/updates.rs:577-597) collects when fed the same per-bond randoms.
  * Growth is monotone, so the pass count is bounded by V.
@@ -391,9 +391,10 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
     return accepted;
 }
 
-/* One colour half-sweep: the patch walk for L_x a multiple of 4, the site-by-site form for L_x = 2 mod 4, whose
- * pairs of compact sites straddle rows (and for couplings whose biased sums could overflow). */
-/* The patch walk from 1,024 sites on, where its units fill the block: a thread
+/* One colour half-sweep: the patch walk for L_x a multiple of 4, the
+ * site-by-site form for L_x = 2 mod 4, whose pairs of compact sites straddle rows
+ * (and for couplings whose biased sums could overflow).  The walk from 1,024
+ * sites on, where its units fill the block: a thread
  * has at least one plane's four updates to do one after the other, and in a
  * smaller lattice that chain is longer than half_sweep's, with a site per lane
  * (us per sweep of 8 replicas alone, and of 2048 per 148 of them, walk and
@@ -417,7 +418,6 @@ __device__ __forceinline__ float site_theta(const Geo& g, const Smem& s, uint32_
  * it through its y and z bonds; a row that gained bits is closed along x
  * (stored rows are always closed).  Rows updated earlier in the same pass are
  * seen by later ones, so bits can travel more than one row per pass. */
-constexpr int kLongRuns = 4; /* rows unrolled in the bond activation of 512-thread CTAs */
 constexpr int kGrowSteps = 3; /* steps of every row between two block barriers */
 
 /* One step of a row from the words around it; returns whether it changed. */
@@ -823,6 +823,9 @@ __device__ __forceinline__ void measure(const Geo& g, const Smem& s, double (&ac
 }
 
 
+constexpr int kLongRuns = 4; /* kUnroll of 512-thread CTAs (launch_resident) */
+
+/* kCorr: with fused correlations; kUnroll: rows unrolled in the bond activation. */
 template <bool kCorr, int kMaxThreads, int kUnroll>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_resident(const TaskView* __restrict__ views, uint32_t n, uint32_t n_sweeps, unsigned int* __restrict__ queue,

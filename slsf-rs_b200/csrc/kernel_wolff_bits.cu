@@ -1,6 +1,7 @@
 /*
  * Single-task Wolff update on bit-packed bonds: grows the seed's cluster
- * only, for large single-replica lattices of any sides (kWolffBitsMinSites).
+ * only, for large single-replica lattices that are not too long for their size
+ * (wolff_by_bits, kernels_plain.cu).
  *
  * Replaces, for those sizes, the whole-lattice union-find labelling of
  * kernels_plain.cu.  The reference grows one cluster from a random seed by
@@ -10,9 +11,9 @@
  * it is needed.
  *
  *   k_wb_bonds   per-site +x/+y/+z bond activation (try_add_wolff_neighbor,
- *                src/updates.rs:537-548) into three bit planes: bit i of the
- *                flat bitmap is site i (site index x + Lx (y + Ly z), so a
- *                32-bit word is 32 consecutive sites of one row); clears the
+ *                src/updates.rs:537-548) into three bit planes: bit x mod 32
+ *                of word x / 32 of a row is site x, a row of L_x sites takes
+ *                ceil(L_x / 32) words (wolff_global.cuh); clears the
  *                cluster bitmap and queues the seed's region, whose first
  *                processing adds the seed's bit.
  *   k_wb_grow    the cluster over the active bonds.  The lattice is cut into

@@ -21,7 +21,8 @@
  *                        32): two sincos per site instead of four
  *
  * Metropolis and measurement here take the shapes that the patch walks of
- * kernel_walk.cu do not; the Wolff kernels lattices below kWolffBitsMinSites.
+ * kernel_walk.cu do not; the Wolff kernels lattices whose cluster is not grown
+ * on bits (wolff_by_bits).
  * (The correlation functions are in kernel_corr.cu, batched over tasks.)
  */
 #include <algorithm>
