@@ -266,8 +266,9 @@ int slsf_task_corr_setup(slsf_task* task, uint32_t rmax_xy, uint32_t rmax_z, uin
  * correlation_interval = interval): from the replica in shared memory on the
  * one-CTA kernel (even L_x <= 32 and a replica that fits shared memory), or
  * by the correlation kernels queued after those sweeps on the grid-wide
- * kernels (lattices too large for one cluster; not in sessions).  Tasks on
- * the cluster or stream kernel are refused.  0 turns it off.
+ * kernels (lattices too large for one cluster, whatever kernel the tuner keeps
+ * for them; not in sessions).  Tasks of other shapes on the cluster or stream
+ * kernel are refused.  0 turns it off.
  * Such a task refuses the separate measurements (slsf_batch_correlations,
  * slsf_batch_step_correlations).  Values agree with the separate kernels to
  * FP32 partial-sum rounding. */

@@ -970,6 +970,10 @@ int slsf_task_corr_setup(slsf_task* t, uint32_t rmax_xy, uint32_t rmax_z, uint32
     return SLSF_OK;
 }
 
+namespace {
+slsf::KernelChoice fused_choice(const slsf_task* t); /* the task's kernel with correlations inside its sweeps */
+}
+
 int slsf_task_corr_fuse(slsf_task* t, uint32_t interval) {
     if (!t) return set_error(SLSF_ERR_INVALID, "task is NULL");
     if (int rc = check_free(t)) return rc;
@@ -978,10 +982,10 @@ int slsf_task_corr_fuse(slsf_task* t, uint32_t interval) {
     /* the context's kernel choice for this shape (default or tuned) must be the
      * one-CTA kernel (correlations from the replica in shared memory) or the
      * grid-wide kernels (the correlation launches queued after the sweep) */
-    slsf_kernel_choice kc = {};
-    if (interval && (slsf_tune_get(t->ctx, t->lx, t->ly, t->lz, &kc) != SLSF_OK ||
-                     (kc.kind != SLSF_KERNEL_RESIDENT && kc.kind != SLSF_KERNEL_GRID)))
-        return set_error(SLSF_ERR_INVALID, kErrFuse);
+    if (interval) {
+        const slsf::KernelChoice c = fused_choice(t);
+        if (c.kind != slsf::kKernelResident && c.kind != slsf::kKernelGrid) return set_error(SLSF_ERR_INVALID, kErrFuse);
+    }
     t->corr_interval = interval;
     return SLSF_OK;
 }
@@ -1312,11 +1316,14 @@ slsf::KernelChoice default_choice(uint32_t lx, uint32_t ly, uint32_t lz, int dev
 }
 
 /* A task's choice: the shape's, but tasks that the stream kernel does not take
- * (couplings too large for the walks' sums, very many Wolff steps) go to a cluster, or the grid-wide kernels where none holds the lattice. */
-slsf::KernelChoice choice_of(const slsf_task* t, slsf::KernelChoice c) {
-    if (c.kind != slsf::kKernelStream || slsf::stream_takes(t->view())) return c;
+ * (couplings too large for the walks' sums, very many Wolff steps) go to a cluster, or the grid-wide kernels where none holds the lattice.
+ * With correlations inside its sweeps a task of a shape that only the tuner
+ * gave to the stream kernel stays on the grid-wide kernels, which measure them. */
+slsf::KernelChoice choice_of(const slsf_task* t, slsf::KernelChoice c, bool fused) {
+    if (c.kind != slsf::kKernelStream || (!fused && slsf::stream_takes(t->view()))) return c;
     const uint32_t cl = slsf::batched_cluster_size(t->lx, t->ly, t->lz, t->ctx->device);
-    return cl ? slsf::KernelChoice{slsf::kKernelCluster, cl, 1024} : slsf::KernelChoice{slsf::kKernelGrid, 1, 256};
+    if (cl == 0) return {slsf::kKernelGrid, 1, 256};
+    return fused ? c : slsf::KernelChoice{slsf::kKernelCluster, cl, 1024};
 }
 
 slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uint32_t lz, bool fused = false) {
@@ -1324,6 +1331,8 @@ slsf::KernelChoice choice_for(const slsf_ctx* ctx, uint32_t lx, uint32_t ly, uin
     if (it != ctx->tune.end()) return it->second;
     return default_choice(lx, ly, lz, ctx->device, fused);
 }
+
+slsf::KernelChoice fused_choice(const slsf_task* t) { return choice_of(t, choice_for(t->ctx, t->lx, t->ly, t->lz, true), true); }
 
 /* Tasks of one group share their launches: those of one kernel choice, with
  * or without fused correlations.  Groups start in descending rank: clusters,
@@ -1434,7 +1443,7 @@ static int batch_run_impl(slsf_ctx* ctx, slsf_task* const* all_tasks, size_t n_a
         slsf_task* t = tasks[i];
         if (!t || t->ctx != ctx) return set_error(SLSF_ERR_INVALID, "task does not belong to this context");
         if (int rc = check_sweepable(t)) return rc;
-        ch[i] = choice_of(t, force ? *force : choice_for(ctx, t->lx, t->ly, t->lz, t->corr_interval != 0));
+        ch[i] = choice_of(t, force ? *force : choice_for(ctx, t->lx, t->ly, t->lz, t->corr_interval != 0), t->corr_interval != 0);
         if (!choice_feasible(ch[i], t->lx, t->ly, t->lz, ctx->device))
             return set_error(SLSF_ERR_INVALID, "the kernel choice does not hold this lattice");
         if (t->corr_interval && (ch[i].kind == slsf::kKernelCluster || ch[i].kind == slsf::kKernelStream))
@@ -1593,7 +1602,7 @@ int slsf_batch_open(slsf_ctx* ctx, slsf_task* const* tasks, size_t n, uint32_t n
         if (int rc = check_sweepable(t)) return rc;
         for (size_t j = 0; j < i; ++j)
             if (tasks[j] == t) return set_error(SLSF_ERR_INVALID, "a task appears twice in the session");
-        ch[i] = choice_of(t, choice_for(ctx, t->lx, t->ly, t->lz, t->corr_interval != 0));
+        ch[i] = choice_of(t, choice_for(ctx, t->lx, t->ly, t->lz, t->corr_interval != 0), t->corr_interval != 0);
         if (ch[i].kind == slsf::kKernelGrid || !choice_feasible(ch[i], t->lx, t->ly, t->lz, ctx->device))
             return set_error(SLSF_ERR_INVALID,
                              "batch sessions hold lattices that fit one thread-block cluster's shared memory");
