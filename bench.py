@@ -102,6 +102,14 @@ def max_over_ranks(value, dist, device):
     return float(t.item())
 
 
+def kernel_label(choice):
+    """The batched kernel that runs the replicas, for the roofline entry."""
+    return {"resident": "k_resident (one launch = S sweeps of every replica, each replica resident in one CTA's shared memory)",
+            "cluster": f"k_cluster ({choice['cluster']} CTAs per replica)",
+            "stream": "k_stream (one launch = S sweeps of every replica, their state in L2)",
+            "grid": "grid-wide kernels"}[choice["kind"]]
+
+
 def peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -640,10 +648,10 @@ def main():
     achieved = alg_bytes / avg_launch_s / 1e9
     tps = traffic_per_site()
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": (tps * n * L ** 3) if tps is not None else None,
+                # counted for kernels that keep a replica on chip for the whole launch
+                "traffic": (tps * n * L ** 3) if tps is not None and choice["kind"] != "stream" else None,
                 "peak_kind": peak_kind,
-                "kernel": "k_resident (one launch = S sweeps of every replica, each replica resident in one CTA's shared memory)"
-                if choice["kind"] == "resident" else f"k_cluster ({choice['cluster']} CTAs per replica)",
+                "kernel": kernel_label(choice),
                 "algorithmic_bytes_per_launch": alg_bytes}
 
     extra = {}
