@@ -376,14 +376,22 @@ __device__ __forceinline__ uint32_t half_sweep_quads(const TaskView& t, const Ge
             base += plane;
         };
         uint32_t z = z_lo;
-        if ((colour + z) & 1u) step(z++, std::true_type());
+        bool open = false; /* terms that are not in the FP64 sums yet */
+        if ((colour + z) & 1u) {
+            step(z++, std::true_type());
+            open = true;
+        }
         for (; z + 1 < z_hi; z += 2) {
             step(z, std::false_type());
             step(z + 1, std::true_type());
             if (kMeasure) sums.flush();
+            open = false;
         }
-        if (z < z_hi) step(z, std::false_type());
-        if (kMeasure) sums.flush();
+        if (z < z_hi) {
+            step(z, std::false_type());
+            open = true;
+        }
+        if (kMeasure && open) sums.flush();
     }
     if (kMeasure)
 #pragma unroll

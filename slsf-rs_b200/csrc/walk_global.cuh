@@ -122,15 +122,17 @@ __device__ __forceinline__ uint32_t walk_colour(const TaskView& t, uint64_t swee
         jzm = jzp;
         base += plane;
     };
-    uint32_t z = pt.z_lo;
-    if (par_lo) step(z++, std::true_type());
+    uint32_t z = pt.z_lo + par_lo;
+    if (par_lo) step(pt.z_lo, std::true_type());
     for (; z + 1 < pt.z_hi; z += 2) {
         step(z, std::false_type());
         step(z + 1, std::true_type());
         if (kMeasure) sums->flush();
     }
+    /* planes that no pair has flushed: the last, or an only one */
+    const bool open = z < pt.z_hi || pt.z_hi - pt.z_lo == 1;
     if (z < pt.z_hi) step(z, std::false_type());
-    if (kMeasure) sums->flush();
+    if (kMeasure && open) sums->flush();
     return accepted;
 }
 
@@ -193,7 +195,7 @@ __device__ __forceinline__ void walk_measure(const TaskView& t, uint32_t seglen,
         base += plane;
         if (z & 1u) sums.flush();
     }
-    sums.flush();
+    if (pt.z_hi & 1u) sums.flush(); /* the last plane's terms */
 }
 
 }  // namespace slsf
