@@ -60,9 +60,10 @@ __device__ __forceinline__ void finish_sums(double (&acc)[8], const TaskView& t,
     }
 }
 
-/* One colour.  Bound by instruction issue (two Philox blocks, 14 neighbour
- * and 8 own sincos per four updates); angles come from L2 or HBM, 12 bytes
- * per update. */
+/* One colour.  Bound by instruction issue and the special-function pipe (two
+ * Philox blocks, 14 neighbour and 8 own sincos per four updates: 53 and 52% of
+ * their cycles); angles come from L2 or HBM, 12 bytes per update.  At L = 256
+ * 41 us, 82 with the measurement (one thread per Philox block: 70 and 115). */
 template <bool kMeasure>
 __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm)
     k_walk_colour(TaskView t, uint64_t sweep, uint32_t colour, uint32_t seglen, double* bin_row) {
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm)
 /* The observables of the state: 14 sincos per eight sites.  The terms gathered
  * in FP32 value and remainder (Sum2) instead of an FP64 conversion each on the
  * special-function pipe, which bound the earlier row walk (72% of it busy, 86
- * us at L = 256). */
+ * us at L = 256; now 45% and 52 us). */
 __global__ void __launch_bounds__(kWalkThreads, kWalkBlocksPerSm)
     k_walk_measure(TaskView t, uint32_t seglen, double* bin_row) {
     WalkSums sums;

@@ -20,8 +20,8 @@ namespace slsf {
  * and plane z's +z partner is plane z + 1's site: three sincos for its two
  * sites, whose arithmetic is packed and whose Philox blocks share a key
  * schedule.  (The earlier walk of one plane took 186 instructions per site and
- * 133 us at L = 256.)  Lane j keeps the words of the run's row j and writes
- * them at its end.  With an odd L_z the last pair's second plane is plane 0,
+ * 133 us at L = 256, this one 100 and 84.)  Lane j keeps the words of the
+ * run's row j and writes them at its end.  With an odd L_z the last pair's second plane is plane 0,
  * computed and not kept. */
 struct BitPlanes {
     uint32_t *bx, *by, *bz, *cl; /* [rows][words] */
